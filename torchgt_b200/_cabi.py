@@ -1,14 +1,17 @@
-"""ctypes binding of ``libtorchgt_b200.so`` (the C ABI declared in ``include/torchgt_b200.h``).
+"""ctypes binding of ``libtorchgt_b200.so`` (the C ABI declared in ``include/torchgt_b200.h``) and the loader of
+the host module built on top of it.
 
 There is no CPU fallback: if the library is missing or a call fails this module raises.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 from ctypes import POINTER, c_char_p, c_float, c_int, c_int64, c_size_t, c_uint32, c_void_p
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libtorchgt_b200.so"
+NATIVE_PATH = LIB_PATH.with_name("_native.so")
 
 TGT_OK = 0
 TGT_ERR_INDEX_RANGE = 5
@@ -133,6 +136,25 @@ def load() -> ctypes.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The host module (``csrc/binding*.cpp``): edge layouts, autograd nodes and launches of the hot calls.
+    Raises if it is not built."""
+    global _native
+    if _native is not None:
+        return _native
+    load()
+    if not NATIVE_PATH.exists():
+        raise RuntimeError(f"{NATIVE_PATH} is missing: build it with `python -m torchgt_b200.build`")
+    spec = importlib.util.spec_from_file_location("torchgt_b200._native", NATIVE_PATH)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    _native = module
+    return module
 
 
 def last_error() -> str:

@@ -1,0 +1,322 @@
+// Python module torchgt_b200._native: edge layouts and the autograd node of the sparse attention.
+#include "binding.h"
+
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/utils/pybind.h>
+
+namespace py = pybind11;
+
+namespace tgt_host {
+
+void* stream_of(const at::Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+namespace {
+
+void check_cuda(cudaError_t e, const char* what) {
+  if (e != cudaSuccess) throw TgtFailure(TGT_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+}
+
+bool capturing(const at::Tensor& t) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  check_cuda(cudaStreamIsCapturing(static_cast<cudaStream_t>(stream_of(t)), &status), "cudaStreamIsCapturing");
+  return status != cudaStreamCaptureStatusNone;
+}
+
+// Pinned words that receive the range-check results of layout builds, each with an event: at most kMost per
+// process, allocated 64 at a time and handed out again once their copy has landed.  A layout that finds none free
+// (a thousand builds outstanding) goes without and reads the device word when it is asked.
+class CheckWords {
+ public:
+  struct Word { int32_t* host = nullptr; cudaEvent_t event = nullptr; int device = -1; };
+
+  int take(int device) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (size_t i = 0; i < returned_.size(); ++i) {
+      const int slot = returned_[i];
+      if (words_[slot].device == device && cudaEventQuery(words_[slot].event) == cudaSuccess) {
+        returned_.erase(returned_.begin() + i);
+        return slot;
+      }
+      if (i >= 3) break;        // the oldest ones are done first
+    }
+    cudaGetLastError();         // "not ready" is not an error
+    if (fresh_ == 0) {
+      if (words_.size() + kChunk > kMost) return -1;
+      int32_t* p = nullptr;
+      if (cudaHostAlloc(reinterpret_cast<void**>(&p), kChunk * sizeof(int32_t), cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+      }
+      for (int i = 0; i < kChunk; ++i) words_.push_back({p + i, nullptr, -1});
+      fresh_ = kChunk;
+    }
+    const int slot = int(words_.size()) - fresh_;
+    if (cudaEventCreateWithFlags(&words_[slot].event, cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      return -1;
+    }
+    words_[slot].device = device;
+    --fresh_;
+    return slot;
+  }
+  void give_back(int slot) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    returned_.push_back(slot);
+  }
+  Word at(int slot) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    return words_[slot];
+  }
+
+ private:
+  static constexpr int kChunk = 64, kMost = 1024;
+  std::mutex mutex_;
+  std::vector<Word> words_;
+  std::vector<int> returned_;
+  int fresh_ = 0;
+};
+
+CheckWords& check_words() {
+  static CheckWords* words = new CheckWords;   // outlives every layout, whatever the order of destruction
+  return *words;
+}
+
+}  // namespace
+
+// ---- layouts ------------------------------------------------------------------------------------------------
+Layout::Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by_) : group_by(group_by_) {
+  const int64_t n_edges = edge_index.size(1);
+  size_t ws = 0;
+  check(tgt_edge_layout_sizes(n_rows, n_edges, &ws));
+  const c10::cuda::CUDAGuard guard(edge_index.device());
+  const auto i32 = edge_index.options().dtype(at::kInt);
+  ptr = at::empty({n_rows + 1}, i32);
+  other = at::empty({n_edges}, i32);
+  perm = at::empty({n_edges}, i32);
+  seg = at::empty({n_edges}, i32);
+  bad_index = at::empty({1}, i32);
+  at::Tensor workspace = at::empty({int64_t(ws < 16 ? 16 : ws)}, edge_index.options().dtype(at::kByte));
+  auto words = [](const at::Tensor& t) { return static_cast<int32_t*>(tgt_host::ptr(t)); };
+  const void* edges = tgt_host::ptr(edge_index);
+  void* stream = stream_of(edge_index);
+  check(edge_index.scalar_type() == at::kLong
+            ? tgt_edge_layout_build(static_cast<const int64_t*>(edges), n_edges, n_rows, group_by, words(ptr),
+                                    words(other), words(perm), words(seg), workspace.data_ptr(), workspace.numel(),
+                                    words(bad_index), stream)
+            : tgt_edge_layout_build_i32(static_cast<const int32_t*>(edges), n_edges, n_rows, group_by, words(ptr),
+                                        words(other), words(perm), words(seg), workspace.data_ptr(),
+                                        workspace.numel(), words(bad_index), stream));
+  c.n_rows = n_rows;
+  c.n_edges = n_edges;
+  c.ptr = words(ptr);
+  c.other = words(other);
+  c.perm = words(perm);
+  c.seg = words(seg);
+  if (!capturing(edge_index)) {
+    slot_ = check_words().take(edge_index.device().index());
+    if (slot_ >= 0) {
+      const auto w = check_words().at(slot_);
+      check_cuda(cudaMemcpyAsync(w.host, bad_index.data_ptr(), 4, cudaMemcpyDeviceToHost,
+                                 static_cast<cudaStream_t>(stream)), "cudaMemcpyAsync");
+      check_cuda(cudaEventRecord(w.event, static_cast<cudaStream_t>(stream)), "cudaEventRecord");
+    }
+  }
+}
+
+Layout::~Layout() {
+  if (slot_ >= 0) check_words().give_back(slot_);
+}
+
+void Layout::settle(bool bad) {
+  state_ = bad ? kBad : kGood;
+  if (slot_ >= 0) {
+    check_words().give_back(slot_);
+    slot_ = -1;
+  }
+  if (bad)
+    throw TgtFailure(TGT_ERR_INDEX_RANGE, "edge_index holds a node id outside [0, " + std::to_string(c.n_rows) + ")");
+}
+
+void Layout::poll() {
+  if (state_ == kGood) return;
+  if (state_ == kBad) settle(true);
+  if (slot_ < 0 || capturing(ptr)) return;
+  const auto w = check_words().at(slot_);
+  const cudaError_t e = cudaEventQuery(w.event);
+  if (e == cudaSuccess) return settle(*static_cast<volatile int32_t*>(w.host) != 0);
+  if (e != cudaErrorNotReady) check_cuda(e, "cudaEventQuery");
+  cudaGetLastError();
+}
+
+void Layout::verify() {
+  if (state_ == kGood) return;
+  if (state_ == kBad) settle(true);
+  if (slot_ < 0) return settle(bad_index.item<int32_t>() != 0);
+  const auto w = check_words().at(slot_);
+  check_cuda(cudaEventSynchronize(w.event), "cudaEventSynchronize");
+  settle(*static_cast<volatile int32_t*>(w.host) != 0);
+}
+
+Graph::Graph(const at::Tensor& edge_index, int64_t rows)
+    : n_rows(rows), n_edges(edge_index.size(1)), edge_index_(edge_index),
+      by_dst_(std::make_shared<Layout>(edge_index, rows, 1)) {}
+
+std::shared_ptr<Layout> Graph::by_src() {
+  std::lock_guard<std::mutex> lock(mutex_);
+  if (!by_src_) {
+    by_src_ = std::make_shared<Layout>(edge_index_, n_rows, 0);
+    edge_index_.reset();
+  }
+  return by_src_;
+}
+
+void Graph::poll() {
+  by_dst_->poll();
+  if (by_src_) by_src_->poll();
+}
+
+size_t Graph::scratch_bytes(int heads, int head_dim, int dtype, int phase) {
+  {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (const Need& n : needs_)
+      if (n.heads == heads && n.head_dim == head_dim && n.dtype == dtype && n.phase == phase) return n.bytes;
+  }
+  size_t bytes = 0;
+  check(tgt_sparse_attn_scratch_bytes(&by_dst_->c, phase == 1 ? &by_src()->c : nullptr, heads, head_dim, dtype, phase,
+                                      &bytes));
+  bytes = bytes < 16 ? 16 : bytes;
+  std::lock_guard<std::mutex> lock(mutex_);
+  needs_.push_back({heads, head_dim, dtype, phase, bytes});
+  return bytes;
+}
+
+// ---- attention ----------------------------------------------------------------------------------------------
+namespace {
+
+int bias_heads(const at::Tensor& bias) {
+  return bias.defined() ? (bias.dim() == 1 ? 1 : int(bias.size(1))) : 0;
+}
+
+at::Tensor scratch(Graph& g, int heads, int head_dim, int dtype, int phase, const at::Tensor& like) {
+  return at::empty({int64_t(g.scratch_bytes(heads, head_dim, dtype, phase))}, like.options().dtype(at::kByte));
+}
+
+}  // namespace
+
+void attention_forward(Graph& g, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
+                       const at::Tensor& out, const at::Tensor& z, int heads, int head_dim, int dtype) {
+  at::Tensor tmp = scratch(g, heads, head_dim, dtype, 0, q);
+  check(tgt_sparse_attn_fwd(ptr(q), ptr(k), ptr(v), fptr(bias), bias_heads(bias), &g.by_dst()->c, ptr(out), fptr(z),
+                            heads, head_dim, dtype, tmp.data_ptr(), tmp.numel(), stream_of(q)));
+}
+
+void attention_backward(Graph& g, const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                        const at::Tensor& bias, const at::Tensor& out, const at::Tensor& z, const at::Tensor& dq,
+                        const at::Tensor& dk, const at::Tensor& dv, const at::Tensor& dbias, int heads, int head_dim,
+                        int dtype) {
+  at::Tensor tmp = scratch(g, heads, head_dim, dtype, 1, q);
+  check(tgt_sparse_attn_bwd(ptr(dout), ptr(q), ptr(k), ptr(v), fptr(bias), bias_heads(bias), ptr(out), fptr(z),
+                            &g.by_dst()->c, &g.by_src()->c, ptr(dq), ptr(dk), ptr(dv), fptr(dbias), heads, head_dim,
+                            dtype, tmp.data_ptr(), tmp.numel(), stream_of(q)));
+}
+
+namespace {
+
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+struct SparseGraphAttentionBackward : public torch::autograd::Node {
+  std::shared_ptr<Graph> graph;
+  SavedVariable q, k, v, bias, out;
+  at::Tensor z;
+  int dtype = 0;
+  bool with_dbias = false;   // the statistics of the forward's output are read only then, so only then is it kept
+
+  variable_list apply(variable_list&& grads) override {
+    if (!grads[0].defined()) return variable_list(4);
+    const at::Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack();
+    const at::Tensor out_ = with_dbias ? out.unpack(shared_from_this()) : at::Tensor();
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard guard(q_.device());
+    const at::Tensor dout = grads[0].contiguous();
+    at::Tensor dq = at::empty_like(q_), dk = at::empty_like(k_), dv = at::empty_like(v_), dbias;
+    if (with_dbias) dbias = at::empty_like(bias_);
+    attention_backward(*graph, dout, q_, k_, v_, bias_, out_, z, dq, dk, dv, dbias, int(q_.size(1)), int(q_.size(2)),
+                       dtype);
+    return {dq, dk, dv, dbias};
+  }
+  std::string name() const override { return "SparseGraphAttentionBackward"; }
+  void release_variables() override {
+    q.reset_data(); k.reset_data(); v.reset_data(); bias.reset_data(); out.reset_data();
+    z.reset();
+  }
+};
+
+at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in,
+                     const std::optional<at::Tensor>& bias_in, const std::shared_ptr<Graph>& graph) {
+  const at::Tensor bias = bias_in.has_value() ? *bias_in : at::Tensor();
+  const at::Tensor q = q_in.contiguous(), k = k_in.contiguous(), v = v_in.contiguous();
+  const int heads = int(q.size(1)), head_dim = int(q.size(2));
+  const int dtype = q.scalar_type() == at::kFloat ? TGT_F32 : TGT_BF16;
+  const c10::cuda::CUDAGuard guard(q.device());
+  at::Tensor out, z;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    out = at::empty_like(q);
+    z = at::empty({q.size(0), heads}, q.options().dtype(at::kFloat));
+    attention_forward(*graph, q, k, v, bias, out, z, heads, head_dim, dtype);
+  }
+  if (torch::autograd::compute_requires_grad(q, k, v, bias)) {
+    auto node = std::shared_ptr<SparseGraphAttentionBackward>(new SparseGraphAttentionBackward(),
+                                                             torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(q, k, v, bias));
+    node->graph = graph;
+    node->dtype = dtype;
+    node->with_dbias = bias.defined() && bias.requires_grad();
+    node->q = SavedVariable(q, false);
+    node->k = SavedVariable(k, false);
+    node->v = SavedVariable(v, false);
+    node->bias = SavedVariable(bias, false);
+    node->z = z;
+    torch::autograd::set_history(out, node);
+    if (node->with_dbias) node->out = SavedVariable(out, true);
+  }
+  return out;
+}
+
+}  // namespace
+}  // namespace tgt_host
+
+PYBIND11_MODULE(_native, m) {
+  using namespace tgt_host;
+  static py::object tgt_error = py::module_::import("torchgt_b200._cabi").attr("TgtError");
+  tgt_error.inc_ref();
+  py::register_exception_translator([](std::exception_ptr p) {
+    try {
+      if (p) std::rethrow_exception(p);
+    } catch (const TgtFailure& e) {
+      PyErr_SetObject(tgt_error.ptr(), tgt_error(e.code, e.message).ptr());
+    }
+  });
+  py::class_<Layout, std::shared_ptr<Layout>>(m, "Layout")
+      .def(py::init<const at::Tensor&, int64_t, int>())
+      .def("poll", &Layout::poll)
+      .def("verify", &Layout::verify)
+      .def_property_readonly("verified", &Layout::verified)
+      .def_readonly("ptr", &Layout::ptr)
+      .def_readonly("other", &Layout::other)
+      .def_readonly("perm", &Layout::perm)
+      .def_readonly("seg", &Layout::seg)
+      .def_readonly("bad_index", &Layout::bad_index)
+      .def_readonly("group_by", &Layout::group_by);
+  py::class_<Graph, std::shared_ptr<Graph>>(m, "Graph")
+      .def(py::init<const at::Tensor&, int64_t>())
+      .def("by_dst", &Graph::by_dst)
+      .def("by_src", &Graph::by_src)
+      .def("has_by_src", &Graph::has_by_src)
+      .def("poll", &Graph::poll);
+  m.def("attention", &attention);
+}

@@ -1,0 +1,93 @@
+// Host path between PyTorch and the C ABI (include/torchgt_b200.h): what the binding's translation units share.
+// The Python modules keep their interfaces; argument checks, allocation, autograd bookkeeping and launches of the
+// hot calls run here, because a small call is bound by exactly that: one attention forward + backward on 4,097
+// rows and 45,056 edges took 132 us per call issued from Python through ctypes and takes 77 us from here (its
+// kernels: 49 us).
+#pragma once
+
+#include <ATen/ATen.h>
+#include <cuda_runtime_api.h>
+#include <pybind11/pybind11.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+
+#include <cstdint>
+#include <memory>
+#include <mutex>
+#include <vector>
+
+#include "../../include/torchgt_b200.h"
+
+namespace tgt_host {
+
+// A C-ABI call returned a non-zero code; Python sees torchgt_b200._cabi.TgtError.
+struct TgtFailure : std::exception {
+  int code;
+  std::string message;
+  TgtFailure(int c, std::string m) : code(c), message(std::move(m)) {}
+  const char* what() const noexcept override { return message.c_str(); }
+};
+
+inline void check(int code) {
+  if (code != TGT_OK) throw TgtFailure(code, tgt_last_error());
+}
+
+void* stream_of(const at::Tensor& t);   // the current stream of t's device
+
+inline void* ptr(const at::Tensor& t) { return t.defined() && t.numel() > 0 ? t.data_ptr() : nullptr; }
+inline float* fptr(const at::Tensor& t) { return static_cast<float*>(ptr(t)); }
+
+// One orientation of a graph (see torchgt_b200.graph.EdgeLayout).  The build enqueues kernels and does not wait;
+// the result of its range check arrives in a pinned word behind an event.
+class Layout {
+ public:
+  Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by);
+  ~Layout();
+  Layout(const Layout&) = delete;
+  Layout& operator=(const Layout&) = delete;
+
+  void poll();     // throws if the build is known to have seen a bad node id; never waits
+  void verify();   // waits for the build first
+  bool verified() const { return state_ == kGood; }
+
+  tgt_layout c{};
+  at::Tensor ptr, other, perm, seg, bad_index;
+  int group_by;
+
+ private:
+  enum State { kPending, kGood, kBad };
+  void settle(bool bad);
+  State state_ = kPending;
+  int slot_ = -1;   // pinned word and event of a pending check (-1: none, the device word is read instead)
+};
+
+// Both orientations of one batch graph; by_src is built on first use.
+class Graph {
+ public:
+  Graph(const at::Tensor& edge_index, int64_t n_rows);
+  std::shared_ptr<Layout> by_dst() const { return by_dst_; }
+  std::shared_ptr<Layout> by_src();
+  bool has_by_src() const { return by_src_ != nullptr; }
+  void poll();
+  // bytes of scratch the attention kernels need (asked from the library once per shape and phase)
+  size_t scratch_bytes(int heads, int head_dim, int dtype, int phase);
+  int64_t n_rows, n_edges;
+
+ private:
+  std::mutex mutex_;
+  at::Tensor edge_index_;   // kept until by_src is built
+  std::shared_ptr<Layout> by_dst_, by_src_;
+  struct Need { int heads, head_dim, dtype, phase; size_t bytes; };
+  std::vector<Need> needs_;
+};
+
+// z is the forward's sum of weights; forward on contiguous CUDA tensors, no autograd
+void attention_forward(Graph& g, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
+                       const at::Tensor& out, const at::Tensor& z, int heads, int head_dim, int dtype);
+void attention_backward(Graph& g, const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                        const at::Tensor& bias, const at::Tensor& out, const at::Tensor& z, const at::Tensor& dq,
+                        const at::Tensor& dk, const at::Tensor& dv, const at::Tensor& dbias, int heads, int head_dim,
+                        int dtype);
+
+}  // namespace tgt_host

@@ -14,24 +14,6 @@ import torch
 
 from . import _cabi
 
-class _StatusRing:
-    """Pinned host words that receive the range-check result of layout builds (one small pinned
-    allocation per process instead of one per layout)."""
-
-    SLOTS = 256
-
-    def __init__(self):
-        self.words = torch.zeros(self.SLOTS, dtype=torch.int32).pin_memory()
-        self.next = 0
-
-    def take(self) -> torch.Tensor:
-        slot = self.words[self.next:self.next + 1]
-        self.next = (self.next + 1) % self.SLOTS
-        return slot
-
-
-_status_ring: Optional[_StatusRing] = None
-
 
 class EdgeLayout:
     """One orientation of the graph: edges sorted by destination (``group_by=1``) or source (0).
@@ -39,76 +21,39 @@ class EdgeLayout:
     ``perm`` is the stable argsort of the grouping endpoint, ``seg`` that endpoint in sorted order,
     ``other`` the opposite endpoint in sorted order, ``ptr`` the row pointers (all int32, on the GPU).
 
-    The build never synchronises: the result of its index-range check is copied to pinned host memory
-    behind an event, and :meth:`poll` / :meth:`verify` read it later."""
+    The build (``csrc/binding.cpp``) never synchronises: the result of its index-range check is copied to
+    pinned host memory behind an event, and :meth:`poll` / :meth:`verify` read it later."""
 
-    def __init__(self, edge_index: torch.Tensor, n_rows: int, group_by: int):
-        global _status_ring
-        lib = _cabi.load()
-        dev = edge_index.device
-        n_edges = int(edge_index.shape[1])
-        ws = ctypes.c_size_t()
-        _cabi.check(lib.tgt_edge_layout_sizes(n_rows, n_edges, ctypes.byref(ws)))
-        i32 = dict(dtype=torch.int32, device=dev)
-        self.ptr = torch.empty(n_rows + 1, **i32)
-        self.other = torch.empty(n_edges, **i32)
-        self.perm = torch.empty(n_edges, **i32)
-        self.seg = torch.empty(n_edges, **i32)
-        workspace = torch.empty(max(ws.value, 16), dtype=torch.uint8, device=dev)
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        nz = lambda t: t.data_ptr() if t.numel() else None
-        self.bad_index = torch.empty(1, **i32)     # written by the build: 1 if a node id was out of range
-        wide = edge_index.dtype == torch.int64
-        build = lib.tgt_edge_layout_build if wide else lib.tgt_edge_layout_build_i32
-        _cabi.check(build(nz(edge_index), n_edges, n_rows, group_by, self.ptr.data_ptr(), nz(self.other),
-                          nz(self.perm), nz(self.seg), workspace.data_ptr(), workspace.numel(),
-                          self.bad_index.data_ptr(), stream))
-        self.n_rows, self.n_edges, self.group_by = n_rows, n_edges, group_by
-        self.c = _cabi.TgtLayout(n_rows=n_rows, n_edges=n_edges, ptr=self.ptr.data_ptr(), other=nz(self.other),
-                                 perm=nz(self.perm), seg=nz(self.seg))
-        self.verified = False
-        self._host_flag: Optional[torch.Tensor] = None
-        self._flag_ready: Optional[torch.cuda.Event] = None
-        if not torch.cuda.is_current_stream_capturing():
-            if _status_ring is None:
-                _status_ring = _StatusRing()
-            self._host_flag = _status_ring.take()
-            self._host_flag.copy_(self.bad_index, non_blocking=True)
-            self._flag_ready = torch.cuda.Event()
-            self._flag_ready.record(torch.cuda.current_stream(dev))
+    def __init__(self, native, n_rows: int, n_edges: int):
+        self.native = native
+        self.ptr, self.other, self.perm, self.seg = native.ptr, native.other, native.perm, native.seg
+        self.bad_index = native.bad_index     # written by the build: 1 if a node id was out of range
+        self.n_rows, self.n_edges, self.group_by = n_rows, n_edges, native.group_by
+        self._c = None
+
+    @property
+    def c(self) -> "_cabi.TgtLayout":
+        """``struct tgt_layout`` for calls of the C ABI."""
+        if self._c is None:
+            nz = lambda t: t.data_ptr() if t.numel() else None
+            self._c = _cabi.TgtLayout(n_rows=self.n_rows, n_edges=self.n_edges, ptr=self.ptr.data_ptr(),
+                                      other=nz(self.other), perm=nz(self.perm), seg=nz(self.seg))
+        return self._c
 
     def byref(self):
         return ctypes.byref(self.c)
 
-    def _raise_if_bad(self, flag: int) -> None:
-        self.verified = True
-        self._host_flag = self._flag_ready = None
-        if flag != 0:
-            self.verified = False
-            self._failed = True
-            raise _cabi.TgtError(_cabi.TGT_ERR_INDEX_RANGE,
-                                 f"edge_index holds a node id outside [0, {self.n_rows})")
+    @property
+    def verified(self) -> bool:
+        return self.native.verified
 
     def poll(self) -> None:
         """Raise if the build is known to have seen a bad node id; never waits for the GPU."""
-        if getattr(self, "_failed", False):
-            self._raise_if_bad(1)
-        if self.verified or self._flag_ready is None or torch.cuda.is_current_stream_capturing():
-            return
-        if self._flag_ready.query():
-            self._raise_if_bad(int(self._host_flag[0]))
+        self.native.poll()
 
     def verify(self) -> None:
         """As :meth:`poll`, but waits for the build to finish."""
-        if getattr(self, "_failed", False):
-            self._raise_if_bad(1)
-        if self.verified:
-            return
-        if self._flag_ready is not None:
-            self._flag_ready.synchronize()
-            self._raise_if_bad(int(self._host_flag[0]))
-        else:
-            self._raise_if_bad(int(self.bad_index.item()))
+        self.native.verify()
 
 
 class SparseGraph:
@@ -132,32 +77,35 @@ class SparseGraph:
         self.n_rows = int(n_rows)
         self.n_edges = int(edge_index.shape[1])
         self.device = edge_index.device
-        self.by_dst = EdgeLayout(edge_index, self.n_rows, 1)
-        self._edge_index = edge_index  # kept until by_src is built
+        self.native = _cabi.native().Graph(edge_index, self.n_rows)
+        self._by_dst: Optional[EdgeLayout] = None
         self._by_src: Optional[EdgeLayout] = None
         self.scratch_bytes: dict = {}  # (heads, head_dim, dtype, phase) -> bytes the attention kernels need
         if not defer_check:
             self.check()
 
     @property
+    def by_dst(self) -> EdgeLayout:
+        if self._by_dst is None:
+            self._by_dst = EdgeLayout(self.native.by_dst(), self.n_rows, self.n_edges)
+        return self._by_dst
+
+    @property
     def by_src(self) -> EdgeLayout:
         """Built on first backward (inference never needs it)."""
         if self._by_src is None:
-            self._by_src = EdgeLayout(self._edge_index, self.n_rows, 0)
-            self._edge_index = None
+            self._by_src = EdgeLayout(self.native.by_src(), self.n_rows, self.n_edges)
         return self._by_src
 
     def poll(self) -> None:
         """Raise a pending index-range error without waiting for the GPU."""
-        self.by_dst.poll()
-        if self._by_src is not None:
-            self._by_src.poll()
+        self.native.poll()
 
     def check(self) -> None:
         """Raise if a build saw a node id outside [0, n_rows) (waits for the builds to finish)."""
-        self.by_dst.verify()
-        if self._by_src is not None:
-            self._by_src.verify()
+        self.native.by_dst().verify()
+        if self.native.has_by_src():
+            self.native.by_src().verify()
 
     def same_edges(self, edge_index: torch.Tensor) -> torch.Tensor:
         """0-d bool tensor on the device: is ``edge_index`` ([2, E], same E) exactly the list this graph was

@@ -1,4 +1,4 @@
-"""Autograd wrapper of the fused sparse graph-attention kernels.
+"""Entry point of the fused sparse graph-attention kernels (their autograd node is in csrc/binding.cpp).
 
 ``sparse_graph_attention(q, k, v, graph, bias)`` computes, for every edge e = (s -> d) and head h,
 
@@ -24,10 +24,6 @@ def _stream(t: torch.Tensor) -> int:
     return torch.cuda.current_stream(t.device).cuda_stream
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None or t.numel() == 0 else t.data_ptr()
-
-
 def _scratch(graph: SparseGraph, heads: int, head_dim: int, dtype: int, phase: int, device) -> torch.Tensor:
     """Scratch of one call; its size is asked from the library once per (graph, shape, phase)."""
     key = (heads, head_dim, dtype, phase)
@@ -40,42 +36,6 @@ def _scratch(graph: SparseGraph, heads: int, head_dim: int, dtype: int, phase: i
                                                       ctypes.byref(n)))
         nbytes = graph.scratch_bytes[key] = max(n.value, 16)
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
-
-
-class _SparseGraphAttention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, bias, graph: SparseGraph):
-        lib = _cabi.load()
-        n_rows, heads, head_dim = q.shape
-        out = torch.empty_like(q)
-        z = torch.empty((n_rows, heads), dtype=torch.float32, device=q.device)
-        bias_heads = 0 if bias is None else (1 if bias.dim() == 1 else int(bias.shape[1]))
-        scratch = _scratch(graph, heads, head_dim, _DTYPES[q.dtype], 0, q.device)
-        _cabi.check(lib.tgt_sparse_attn_fwd(
-            _ptr(q), _ptr(k), _ptr(v), _ptr(bias), bias_heads, graph.by_dst.byref(), _ptr(out), _ptr(z),
-            heads, head_dim, _DTYPES[q.dtype], scratch.data_ptr(), scratch.numel(), _stream(q)))
-        ctx.graph = graph
-        ctx.bias_heads = bias_heads
-        ctx.save_for_backward(q, k, v, bias, out, z)
-        return out
-
-    @staticmethod
-    def backward(ctx, dout):
-        lib = _cabi.load()
-        q, k, v, bias, out, z = ctx.saved_tensors
-        graph: SparseGraph = ctx.graph
-        n_rows, heads, head_dim = q.shape
-        dout = dout.contiguous()
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        dbias = None
-        if bias is not None and ctx.needs_input_grad[3]:
-            dbias = torch.empty_like(bias)
-        scratch = _scratch(graph, heads, head_dim, _DTYPES[q.dtype], 1, q.device)
-        _cabi.check(lib.tgt_sparse_attn_bwd(
-            _ptr(dout), _ptr(q), _ptr(k), _ptr(v), _ptr(bias), ctx.bias_heads, _ptr(out), _ptr(z),
-            graph.by_dst.byref(), graph.by_src.byref(), _ptr(dq), _ptr(dk), _ptr(dv), _ptr(dbias), heads,
-            head_dim, _DTYPES[q.dtype], scratch.data_ptr(), scratch.numel(), _stream(q)))
-        return dq, dk, dv, dbias, None
 
 
 def _heads_fit_one_group(heads: int, head_dim: int, dtype: torch.dtype) -> bool:
@@ -102,8 +62,7 @@ def sparse_graph_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
         raise TypeError("q, k, v must all be float32 or all bfloat16")
     n_rows, heads, head_dim = q.shape
     graph = graph_for(edge_index, n_rows)
-    graph.poll()   # a node id outside [0, N) found by the (asynchronous) layout build is raised here
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+    graph.native.poll()   # a node id outside [0, N) found by the (asynchronous) layout build is raised here
     if bias is not None:
         if bias.dim() == 2 and bias.shape[1] == 1 and heads != 1:
             bias = bias[:, 0]
@@ -118,4 +77,4 @@ def sparse_graph_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
         bias = bias.contiguous()
         if graph.n_edges == 0:
             bias = None  # nothing to add the (empty) bias to
-    return _SparseGraphAttention.apply(q, k, v, bias, graph)
+    return _cabi.native().attention(q, k, v, bias, graph.native)
