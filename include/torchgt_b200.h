@@ -154,6 +154,47 @@ TGT_API int tgt_edge_prepare(const int64_t* raw_edges, int64_t raw_total, const 
                              int64_t out_total, void* stream);
 
 /*
+ * Edges among the nodes idx[0 .. n_idx) of a graph, renumbered by position in idx (gen_sub_edge_index,
+ * gt_sp/utils.py:202-215): existing self loops dropped, kept edges in their order, then one self loop per listed
+ * node in node-id order.  In two calls, because the caller allocates the result: tgt_subgraph_count leaves
+ * {number of kept edges, 1 if an id was out of range} in the device words *result (inside the workspace), and after
+ * reading them the caller passes n_kept (+ 2 * n_idx with add_global_token) as out_total to tgt_subgraph_write with
+ * the same workspace.  add_global_token and sub_seq_len as in tgt_edge_prepare.  edge_index: device int64
+ * [2, n_edges]; idx: device int64; out: device int64 [2, out_total].  Negative ids count from the end, as PyTorch's
+ * indexing does.  Neither call synchronises.
+ */
+TGT_API int tgt_subgraph_workspace_bytes(int64_t n_edges, int64_t n_nodes, size_t* bytes);
+TGT_API int tgt_subgraph_count(const int64_t* edge_index, int64_t n_edges, int64_t n_nodes, const int64_t* idx,
+                               int64_t n_idx, void* workspace, size_t workspace_bytes, const int64_t** result,
+                               void* stream);
+TGT_API int tgt_subgraph_write(int64_t n_edges, int64_t n_nodes, int64_t n_idx, int add_global_token,
+                               int64_t sub_seq_len, const void* workspace, int64_t* out, int64_t out_total,
+                               void* stream);
+
+/* out[r] = x[idx[r]] for rows of row_bytes bytes; idx: device int64 [n_out], negative ids count from the end, rows
+ * whose id is out of range are left unwritten. */
+TGT_API int tgt_gather_rows(const void* x, int64_t n_rows, int64_t row_bytes, const int64_t* idx, int64_t n_out,
+                            void* out, void* stream);
+
+/*
+ * Cluster-sparse block generator (generate_new_edges_optimized, gt_sp/utils.py:218-305): every pair of the k
+ * partitions gets dense block x block blocks at block coordinates drawn as numpy's RandomState draws them.
+ * partition: device int64 [n_nodes], or NULL for k contiguous ranges (partition of v = v * k / n_nodes).
+ * tgt_blocks_plan leaves {blocks, grid rows, 1 if some pair is denser than p and keeps its original edges (which
+ * these calls do not produce), 1 if an id was out of range} in the device words *result; tgt_blocks_write writes
+ * blocks * block * block edges (device int64 [2, ...]) pair by pair, or with by_source = 1 in the order of a stable
+ * sort by source.  sub_seq_len as in tgt_edge_prepare.  Neither call synchronises.
+ */
+TGT_API int tgt_blocks_workspace_bytes(int k, int64_t n_nodes, int64_t block, size_t* bytes);
+TGT_API int tgt_blocks_plan(const int64_t* edge_index, int64_t n_edges, int64_t n_nodes, const int64_t* partition,
+                            int k, double p, int64_t block, void* workspace, size_t workspace_bytes,
+                            const int64_t** result, void* stream);
+TGT_API int tgt_blocks_list_bytes(int64_t blocks, size_t* bytes);
+TGT_API int tgt_blocks_write(int64_t n_nodes, int k, int64_t block, const void* workspace, void* list,
+                             size_t list_bytes, int64_t blocks, int by_source, int64_t sub_seq_len, int64_t* out,
+                             void* stream);
+
+/*
  * Bytes of scratch tgt_sparse_attn_fwd (phase 0) / tgt_sparse_attn_bwd (phase 1) need for these
  * layouts (partial sums of rows that cross a tile boundary; row statistics of the backward).
  * by_src may be NULL for phase 0.

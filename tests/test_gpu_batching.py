@@ -1,0 +1,82 @@
+"""Batch construction on the GPU (csrc/batching.cu) against the PyTorch / numpy formulation on the CPU, which the
+reference's own vectors pin (test_batching_gloo.py).  Integer work: every array bit for bit."""
+import types
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _no_group():
+    import torchgt_b200.gt_sp.initialize as init
+    init.destroy_sequence_parallel()
+    yield
+    init.destroy_sequence_parallel()
+
+
+def _graph(seed, n, m):
+    gen = torch.Generator().manual_seed(seed)
+    return torch.randint(0, n, (2, m), generator=gen), torch.randperm(n, generator=gen)
+
+
+# sizes around the marking pass's chunk of 2048 candidates and its 256 threads, self loops and duplicates among them
+@pytest.mark.parametrize("n,m,b", [(1, 0, 1), (5, 40, 5), (100, 1948, 60), (100, 1949, 99), (255, 5000, 1), (3000, 20000, 1500),
+                                   (40000, 300001, 20000)])
+def test_induced_subgraph(n, m, b):
+    from torchgt_b200.gt_sp.utils import gen_sub_edge_index
+    edges, perm = _graph(n + m, n, m)
+    idx = perm[:b]
+    want = gen_sub_edge_index(edges, idx, n)
+    assert torch.equal(gen_sub_edge_index(edges.cuda(), idx.cuda(), n).cpu(), want)
+    assert torch.equal(gen_sub_edge_index(edges.cuda(), (idx - n).cuda(), n).cpu(), want)   # counted from the end
+    if m:
+        edges[1, m // 2] = n
+        with pytest.raises(IndexError):
+            gen_sub_edge_index(edges.cuda(), idx.cuda(), n)
+
+
+# unequal partitions (different bounds for rows and columns), one block per side (no random number drawn), more than
+# 624 coordinates for a pair, partitions smaller than a block
+@pytest.mark.parametrize("n,m,k,block", [(64, 500, 1, 4), (97, 400, 3, 4), (50, 300, 8, 5), (33, 200, 4, 16), (2000, 60000, 3, 4),
+                                         (5000, 30000, 8, 16), (700, 3000, 70, 2)])
+def test_block_generator(n, m, k, block):
+    from torchgt_b200.gt_sp.batching import contiguous_partition, generate_new_edges_optimized, reformat_graph
+    edges, perm = _graph(n * k + block, n, m)
+    for part in (contiguous_partition(edges, n, k), (perm.double() / n).pow(1.5).mul(k).long()):
+        mapping = np.argsort(np.argsort(part.numpy(), kind="stable"), kind="stable")
+        for p in (1, 0.02):
+            want = generate_new_edges_optimized(edges, k, part, p, block, mapping)
+            assert torch.equal(generate_new_edges_optimized(edges.cuda(), k, part, p, block, mapping).cpu(), want)
+        for ids in (part, None):
+            want, order = reformat_graph(edges, k, block, partition_ids=ids)
+            got, got_order = reformat_graph(edges.cuda(), k, block, partition_ids=ids)
+            assert torch.equal(got.cpu(), want) and torch.equal(got_order.cpu(), order)
+
+
+@pytest.mark.parametrize("model", ["graphormer", "gt"])
+@pytest.mark.parametrize("reorder", [False, True])
+@pytest.mark.parametrize("features,dtype", [(64, torch.float32), (3, torch.float32), (5, torch.bfloat16)])
+def test_training_batch(model, reorder, features, dtype):
+    from torchgt_b200.gt_sp.batching import get_batch_reorder_blockize, set_partitioner
+    from torchgt_b200.gt_sp.initialize import get_last_batch_flag
+    n, seq_len = 3001, 1000
+    edges, perm = _graph(9, n, 25000)
+    gen = torch.Generator().manual_seed(1)
+    x, y = torch.randn(n, features, generator=gen).to(dtype), torch.randint(0, 40, (n,), generator=gen)
+    args = types.SimpleNamespace(seq_len=seq_len, model=model, reorder=reorder)
+    scatter = lambda e, nodes, k: ((torch.arange(nodes) * 13) % nodes) * k // nodes
+    for idx, rest in ((perm[:seq_len], None), (perm[:777], [777]), (perm[:777], [800])):
+        for partitioner in (None, scatter):
+            set_partitioner(partitioner)
+            try:
+                want = get_batch_reorder_blockize(args, x, y, idx, rest, "cpu", edges, n, 4, 8)
+                flag = get_last_batch_flag()
+                got = get_batch_reorder_blockize(args, x.cuda(), y.cuda(), idx.cuda(), rest, "cuda", edges.cuda(), n, 4, 8)
+            finally:
+                set_partitioner(None)
+            assert got[3] is None and get_last_batch_flag() == flag
+            for a, b in zip(got[:3], want[:3]):
+                assert a.dtype == b.dtype and torch.equal(a.cpu(), b)

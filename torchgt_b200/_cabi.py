@@ -63,6 +63,17 @@ SIGNATURES = {
                                           c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "tgt_edge_prepare": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int, c_int, c_int64, c_int64,
                                  c_void_p, c_int64, c_void_p]),
+    "tgt_subgraph_workspace_bytes": (c_int, [c_int64, c_int64, POINTER(c_size_t)]),
+    "tgt_subgraph_count": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_size_t, POINTER(c_void_p),
+                                   c_void_p]),
+    "tgt_subgraph_write": (c_int, [c_int64, c_int64, c_int64, c_int, c_int64, c_void_p, c_void_p, c_int64, c_void_p]),
+    "tgt_gather_rows": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_void_p]),
+    "tgt_blocks_workspace_bytes": (c_int, [c_int, c_int64, c_int64, POINTER(c_size_t)]),
+    "tgt_blocks_plan": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int, ctypes.c_double, c_int64, c_void_p, c_size_t,
+                                POINTER(c_void_p), c_void_p]),
+    "tgt_blocks_list_bytes": (c_int, [c_int64, POINTER(c_size_t)]),
+    "tgt_blocks_write": (c_int, [c_int64, c_int, c_int64, c_void_p, c_void_p, c_size_t, c_int64, c_int, c_int64, c_void_p,
+                                 c_void_p]),
     "tgt_sparse_attn_scratch_bytes": (c_int, [_PL, _PL, c_int, c_int, c_int, c_int, POINTER(c_size_t)]),
     "tgt_sparse_attn_fwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int, _PL, c_void_p,
                                     c_void_p, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p]),

@@ -319,4 +319,5 @@ PYBIND11_MODULE(_native, m) {
       .def("has_by_src", &Graph::has_by_src)
       .def("poll", &Graph::poll);
   m.def("attention", &attention);
+  bind_batching(m);
 }

@@ -15,6 +15,7 @@
 #include <cstdint>
 #include <memory>
 #include <mutex>
+#include <string>
 #include <vector>
 
 #include "../../include/torchgt_b200.h"
@@ -89,5 +90,7 @@ void attention_backward(Graph& g, const at::Tensor& dout, const at::Tensor& q, c
                         const at::Tensor& bias, const at::Tensor& out, const at::Tensor& z, const at::Tensor& dq,
                         const at::Tensor& dk, const at::Tensor& dv, const at::Tensor& dbias, int heads, int head_dim,
                         int dtype);
+
+void bind_batching(pybind11::module_& m);   // binding_batch.cpp
 
 }  // namespace tgt_host

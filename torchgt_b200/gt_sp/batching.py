@@ -3,7 +3,9 @@ generator and the per-rank batch slicing of the reference's gt_sp/utils.py.
 
 Function names, argument order and results follow the reference (gt_sp/utils.py:61-82, 187-215,
 218-305, 319-359, 409-520).  Everything is integer work on node ids and must be bit-exact; it runs on
-whatever device its inputs live on (the reference runs it on the host for every batch).
+whatever device its inputs live on (the reference runs it on the host for every batch).  int64 tensors on a GPU
+take the kernels of ``csrc/batching.cu``; the PyTorch / numpy formulation below is what they are checked against
+and what every other tensor takes.
 
 Two third-party pieces of the reference are not available here and are restated from their published
 behaviour: the three ``torch_geometric.utils`` calls inside ``gen_sub_edge_index``
@@ -24,6 +26,7 @@ import torch
 import torch.distributed as dist
 from torch import Tensor
 
+from .. import _cabi
 from .initialize import (get_sequence_parallel_group, get_sequence_parallel_rank, get_sequence_parallel_src_rank,
                          get_sequence_parallel_world_size, last_batch_flag, sequence_parallel_is_initialized)
 from .utils import adjust_edge_index_nomerge, fix_edge_index
@@ -60,12 +63,21 @@ def random_split_idx(data_y, frac_train: float, frac_valid: float, frac_test: fl
     return {"train": torch.tensor(all_idx[:a]), "valid": torch.tensor(all_idx[a:b]), "test": torch.tensor(all_idx[b:])}
 
 
+def _on_device(edge_index, *ids) -> bool:
+    """Can the kernels take this edge list and these id lists?"""
+    return (isinstance(edge_index, Tensor) and edge_index.is_cuda and edge_index.dtype == torch.int64 and
+            edge_index.dim() == 2 and edge_index.shape[0] == 2 and
+            all(t.device == edge_index.device and t.dtype == torch.int64 and t.dim() == 1 for t in ids))
+
+
 # ---- induced sub-graph of a batch (gt_sp/utils.py:202-215) --------------------------------------------
 def gen_sub_edge_index(edge_index: Tensor, idx_batch: Tensor, N: int) -> Tensor:
     """Edges among the nodes ``idx_batch`` of the whole graph, renumbered by position in ``idx_batch``:
     existing self loops are dropped, one self loop per node is added, and the kept columns keep their
     order (original edges first, then the self loops in node-id order)."""
     idx_batch = idx_batch.to(edge_index.device)
+    if _on_device(edge_index, idx_batch) and N > 0:
+        return _cabi.native().batch(edge_index.contiguous(), idx_batch.contiguous(), N, False, 0, [], 0, 0)[0]
     src, dst = edge_index[0], edge_index[1]
     keep = src != dst                                              # remove_self_loops
     loops = torch.arange(N, dtype=edge_index.dtype, device=edge_index.device)
@@ -105,8 +117,13 @@ def generate_new_edges_optimized(edge_index, k: int, partition_ids, p: float, bl
     counts of all later pairs), and pairs in which a partition has fewer than ``blocksize`` nodes get
     no edges at all.  Returns [2, E_new] int64 in the renumbered ids, on the device of ``edge_index``."""
     device = edge_index.device if isinstance(edge_index, Tensor) else torch.device("cpu")
+    part = torch.as_tensor(partition_ids).long()
+    if part.dim() == 1:
+        edges = _device_blocks(edge_index, part.numel(), part, k, p, blocksize, False, 0)
+        if edges is not None:
+            return edges
     src, dst = (torch.as_tensor(t).cpu() for t in edge_index)
-    part = torch.as_tensor(partition_ids).cpu().long()
+    part = part.cpu()
     mapping = torch.as_tensor(np.asarray(new_id_mapping)).long()
     ps, pd = part[src.long()], part[dst.long()]
     # sorted by (partition of source, partition of destination, source, destination)
@@ -153,6 +170,18 @@ def generate_new_edges_optimized(edge_index, k: int, partition_ids, p: float, bl
     return torch.cat([piece.to(device) for piece in pieces], dim=1)
 
 
+def _device_blocks(edge_index, num_nodes: int, partition: Optional[Tensor], k: int, p, block: int, by_source: bool,
+                   sub_seq_len: int) -> Optional[Tensor]:
+    """The generator's result from the kernels: pair by pair, or sorted by source (stable) with ``by_source``, ids
+    moved past the per-rank token slots for ``sub_seq_len`` > 0.  ``partition`` None: contiguous equal ranges.
+    None when the edges are not on a GPU or some pair of partitions keeps its original edges."""
+    if not _on_device(edge_index) or not (0 < num_nodes < 2 ** 31 - 1 and 1 <= k <= 8192 and 1 <= block <= 32768):
+        return None
+    if partition is not None:
+        partition = partition.to(edge_index.device).contiguous()
+    return _cabi.native().blocks(edge_index.contiguous(), num_nodes, partition, k, float(p), block, by_source, sub_seq_len)
+
+
 _partitioner: Optional[Callable[[Tensor, int, int], Tensor]] = None
 
 
@@ -175,10 +204,25 @@ def reformat_graph(edge_index: Tensor, k: int, block_size: int, beta_coeffi="1",
     = the old node id at every new position).  The order of edges with equal source is not specified
     (the reference uses a non-stable ``argsort``; a stable sort is used here)."""
     num_nodes = int(edge_index.max().item()) + 1 if edge_index.numel() else 0   # dgl.graph((src, dst)).num_nodes()
+    edges, sorted_indices = _reformat(edge_index, k, block_size, partition_ids, num_nodes, 0)
+    return edges, torch.arange(num_nodes) if sorted_indices is None else sorted_indices
+
+
+def _reformat(edge_index: Tensor, k: int, block_size: int, partition_ids, num_nodes: int, sub_seq_len: int):
+    """``reformat_graph`` of a graph of known size, its result's ids adjusted for ``sub_seq_len`` > 0; None instead
+    of ``sorted_indices`` where the nodes keep their numbers (contiguous partitions)."""
+    if partition_ids is None and _partitioner is None:
+        edges = _device_blocks(edge_index, num_nodes, None, k, 1, block_size, True, sub_seq_len)
+        if edges is not None:
+            return edges, None
     if partition_ids is None:
         fn = _partitioner or contiguous_partition
         partition_ids = fn(edge_index, num_nodes, k)
     partition_ids = torch.as_tensor(partition_ids).cpu().long()
+    if partition_ids.dim() == 1 and partition_ids.numel() == num_nodes:
+        edges = _device_blocks(edge_index, num_nodes, partition_ids, k, 1, block_size, True, sub_seq_len)
+        if edges is not None:
+            return edges, torch.argsort(partition_ids, stable=True)
     new_id_mapping = np.empty(num_nodes, dtype=np.int64)
     current = 0
     part_np = partition_ids.numpy()
@@ -190,7 +234,29 @@ def reformat_graph(edge_index: Tensor, k: int, block_size: int, beta_coeffi="1",
                                                   new_id_mapping=new_id_mapping)
     sorted_indices = torch.argsort(torch.from_numpy(new_id_mapping))
     by_source = torch.argsort(new_edge_index[0], stable=True)
-    return new_edge_index[:, by_source], sorted_indices
+    edges = new_edge_index[:, by_source]
+    return adjust_edge_index_nomerge(edges, sub_seq_len) if sub_seq_len > 0 else edges, sorted_indices
+
+
+def _device_batch(x: Tensor, y: Tensor, idx_batch: Tensor, edge_index: Tensor, N: int, k: int, block_size: int,
+                  graphormer: bool, reorder: bool, lo: int, hi: int, per_rank: int):
+    """Rows ``lo`` .. ``hi`` of the batch and its edges from the kernels (one process, or several without
+    ``reorder``)."""
+    native = _cabi.native()
+    n = idx_batch.shape[0]
+    sub_seq_len = per_rank if graphormer else 0
+    edge_index, idx_batch = edge_index.contiguous(), idx_batch.contiguous()
+    if not reorder:
+        x_i, y_i, edges = native.batch(edge_index, idx_batch, N, graphormer, sub_seq_len, [x, y], lo, hi)
+        return x_i, y_i, edges
+    edges = native.batch(edge_index, idx_batch, N, graphormer, 0, [], 0, 0)[0]
+    edges, order = _reformat(edges, k, block_size, None, n + 1 if graphormer else n, sub_seq_len)
+    if order is not None:
+        if graphormer:   # position 0 is the global token: not a row of x
+            order = order[order != 0] - 1
+        idx_batch = idx_batch[order.to(idx_batch.device)]
+    rows = idx_batch[lo:hi]
+    return native.gather_rows(x, rows), native.gather_rows(y, rows), edges
 
 
 # ---- one training batch of the node-level loops (gt_sp/utils.py:409-520) ------------------------------
@@ -205,12 +271,25 @@ def get_batch_reorder_blockize(args, x: Tensor, y: Tensor, idx_batch: Tensor, re
     world = get_sequence_parallel_world_size() if sequence_parallel_is_initialized() else 1
     rank = get_sequence_parallel_rank() if sequence_parallel_is_initialized() else 0
     seq_length = args.seq_len
+    n = idx_batch.shape[0]
+    reorder = bool(getattr(args, "reorder", False))
+    if (n > 0 and _on_device(edge_index, idx_batch) and N > 0 and not (reorder and world > 1) and
+            (rest_split_sizes is not None if n < seq_length else seq_length % world == 0) and
+            all(t.device == edge_index.device and t.is_contiguous() and not t.requires_grad and t.dim() == d and
+                t.shape[0] == N for t, d in ((x, 2), (y, 1)))):
+        per_rank = max(rest_split_sizes) if n < seq_length else seq_length // world
+        x_i, y_i, edge_index_i = _device_batch(x, y, idx_batch, edge_index, N, k, block_size, args.model == "graphormer",
+                                               reorder, min(rank * per_rank, n), min((rank + 1) * per_rank, n), per_rank)
+        last_batch_flag(n < seq_length)
+        if n < seq_length:
+            x_i, y_i = pad_2d(x_i, per_rank), pad_y(y_i, per_rank)
+        return x_i, y_i, edge_index_i, None
     x_i, y_i = x[idx_batch], y[idx_batch]
     edge_index_i = gen_sub_edge_index(edge_index, idx_batch, N)
     graphormer = args.model == "graphormer"
     if graphormer:
         edge_index_i = fix_edge_index(edge_index_i, idx_batch.shape[0])
-    if getattr(args, "reorder", False):
+    if reorder:
         if world > 1:
             src_rank, group = get_sequence_parallel_src_rank(), get_sequence_parallel_group()
             if dist.get_rank() == src_rank:
