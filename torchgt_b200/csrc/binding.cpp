@@ -238,12 +238,13 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
   variable_list apply(variable_list&& grads) override {
     if (!grads[0].defined()) return variable_list(4);
     const at::Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack();
-    const at::Tensor out_ = with_dbias ? out.unpack(shared_from_this()) : at::Tensor();
+    const bool want_dbias = with_dbias && task_should_compute_output(3);
+    const at::Tensor out_ = want_dbias ? out.unpack(shared_from_this()) : at::Tensor();
     const at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard guard(q_.device());
     const at::Tensor dout = grads[0].contiguous();
     at::Tensor dq = at::empty_like(q_), dk = at::empty_like(k_), dv = at::empty_like(v_), dbias;
-    if (with_dbias) dbias = at::empty_like(bias_);
+    if (want_dbias) dbias = at::empty_like(bias_);
     attention_backward(*graph, dout, q_, k_, v_, bias_, out_, z, dq, dk, dv, dbias, int(q_.size(1)), int(q_.size(2)),
                        dtype);
     return {dq, dk, dv, dbias};
@@ -258,6 +259,10 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
 at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in,
                      const std::optional<at::Tensor>& bias_in, const std::shared_ptr<Graph>& graph) {
   const at::Tensor bias = bias_in.has_value() ? *bias_in : at::Tensor();
+  // the node has no forward-mode formula: refuse a dual tensor rather than drop its tangent
+  for (const at::Tensor* t : {&q_in, &k_in, &v_in, &bias})
+    TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(*t),
+                                "sparse_graph_attention does not support forward-mode AD");
   const at::Tensor q = q_in.contiguous(), k = k_in.contiguous(), v = v_in.contiguous();
   const int heads = int(q.size(1)), head_dim = int(q.size(2));
   const int dtype = q.scalar_type() == at::kFloat ? TGT_F32 : TGT_BF16;
