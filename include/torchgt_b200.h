@@ -458,6 +458,14 @@ TGT_API int tgt_layer_norm_bwd(const float* dy, const float* x, const float* gam
                                size_t scratch_bytes, void* stream);
 
 /*
+ * Product of a narrow nn.Linear over many rows, full fp32 products and sums: c [rows, cols] = a [rows, reduce] w^T +
+ * bias for w [cols, reduce] and bias [cols] (may be NULL).  reduce and cols must be multiples of 4, at most 1024
+ * (TGT_ERR_UNSUPPORTED otherwise), all pointers 16-byte aligned (models/graphormer_dist_node_level.py:241-245,281-286).
+ */
+TGT_API int tgt_linear_rows(const float* a, const float* w, const float* bias, int64_t rows, int reduce, int cols,
+                            float* c, void* stream);
+
+/*
  * Weight and bias gradient of a narrow nn.Linear over many rows, fp32: dw [out_features, in_features] =
  * dy^T x and db [out_features] (may be NULL) = column sums of dy, for dy [rows, out_features] and x [rows,
  * in_features] — the backward of the models' projections and FFN layers (models/graphormer_dist_node_level.py:

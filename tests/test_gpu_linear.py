@@ -72,3 +72,79 @@ def test_linear_wgrad_argument_errors_come_back_as_codes():
     assert lib.tgt_linear_wgrad_scratch_bytes(8, 64, 42, ctypes.byref(nb)) == 3
     assert lib.tgt_linear_wgrad(t.data_ptr(), t.data_ptr(), 8, 64, 64, None, None, None, 0, None) == 1   # INVALID
     assert lib.tgt_linear_wgrad(t.data_ptr(), t.data_ptr(), 8, 64, 64, t.data_ptr(), None, None, 0, None) == 4   # WORKSPACE
+
+
+@pytest.fixture(params=[False, True], ids=["fp32", "tf32"])
+def tf32(request):
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = request.param
+    yield request.param
+    torch.backends.cuda.matmul.allow_tf32 = before
+
+
+@pytest.mark.parametrize("in_features,out_features", [(64, 64), (64, 128), (128, 64), (64, 40), (192, 4), (64, 100)])
+@pytest.mark.parametrize("rows", [1, 1025, 4097, 40000])
+def test_forward_and_input_gradient_match_fp64(rows, in_features, out_features, tf32):
+    """Both tile heights, partial tiles of rows and columns, one and several reduction chunks."""
+    from torchgt_b200.linear import linear
+    gen = torch.Generator().manual_seed(rows + in_features + 3 * out_features)
+    x = torch.randn(rows, in_features, generator=gen).cuda().requires_grad_()
+    w = torch.randn(out_features, in_features, generator=gen).cuda().requires_grad_()
+    b = torch.randn(out_features, generator=gen).cuda().requires_grad_()
+    dy = torch.randn(rows, out_features, generator=gen).cuda()
+    y = linear(x, w, b)
+    grads = torch.autograd.grad(y, (x, w, b), dy)
+    x64, w64, b64 = (t.detach().double().requires_grad_() for t in (x, w, b))
+    y64 = torch.nn.functional.linear(x64, w64, b64)
+    refs = (y64, *torch.autograd.grad(y64, (x64, w64, b64), dy.double()))
+    # fp32: at most 192 products per sum, each sum's error below 192 * 2^-24 of its largest partial sum; tf32 operands
+    # are rounded to 11 bits (2^-11 each)
+    for got, ref, library in zip((y, *grads), refs, (tf32, tf32, False, False)):
+        assert got.shape == ref.shape and _err(got.detach(), ref.detach()) < (2e-3 if library else TOL)
+    with torch.no_grad():
+        assert _err(linear(x, w, b), y64.detach()) < (2e-3 if tf32 else TOL)
+        assert _err(linear(x, w, None), torch.nn.functional.linear(x64, w64).detach()) < (2e-3 if tf32 else TOL)
+
+
+@pytest.mark.parametrize("rows,reduce,cols", [(1, 4, 4), (33, 100, 44), (31, 1024, 68), (50001, 68, 200)])
+def test_row_kernel_at_the_edges_of_its_tiles(rows, reduce, cols):
+    """Reductions and columns that end inside a chunk, with and without a bias, through the C entry."""
+    from torchgt_b200 import _cabi
+    gen = torch.Generator().manual_seed(rows + reduce)
+    x, w, b = (torch.randn(*s, generator=gen).cuda() for s in ((rows, reduce), (cols, reduce), (cols,)))
+    for bias in (b, None):
+        y = torch.full((rows, cols), float("nan"), device="cuda")
+        _cabi.check(_cabi.load().tgt_linear_rows(x.data_ptr(), w.data_ptr(), None if bias is None else b.data_ptr(), rows,
+                                                 reduce, cols, y.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        ref = torch.nn.functional.linear(x.double(), w.double(), None if bias is None else b.double())
+        assert _err(y, ref) < TOL
+
+
+def test_linear_takes_every_call_that_f_linear_takes():
+    """Views off a 16-byte boundary, transposed inputs and weights, leading dimensions, no rows, other widths,
+    infinities, torch.func and second-order gradients."""
+    from torchgt_b200.linear import linear
+    F = torch.nn.functional
+    torch.manual_seed(5)
+    w, b = torch.randn(64, 64, device="cuda"), torch.randn(64, device="cuda")
+    base = torch.randn(2000 * 64 + 1, device="cuda")
+    calls = [(base[1:].view(2000, 64), w, b), (torch.randn(64, 2000, device="cuda").t(), w.t(), b),
+             (torch.randn(2, 30, 50, 64, device="cuda"), w, b), (torch.randn(64, device="cuda"), w, b),
+             (torch.empty(0, 64, device="cuda"), w, b), (torch.randn(9, 100, device="cuda"), torch.randn(47, 100, device="cuda"), None)]
+    for args in calls:
+        x = args[0].detach().requires_grad_()
+        y, ref = linear(x, *args[1:]), F.linear(args[0].double(), *(None if t is None else t.double() for t in args[1:]))
+        assert y.shape == ref.shape and (ref.numel() == 0 or _err(y.detach(), ref) < TOL)
+        dx, = torch.autograd.grad(y.sum(), x)
+        assert dx.shape == x.shape
+    x = torch.randn(4000, 64, device="cuda")
+    x[3, 7], x[11, 0] = float("inf"), float("nan")
+    y, ref = linear(x, w, b), F.linear(x, w, b)
+    assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isinf(), ref.isinf())
+    z = torch.randn(6, 5, 64, device="cuda")
+    assert _err(torch.func.vmap(lambda t: linear(t, w, b))(z), F.linear(z.double(), w.double(), b.double())) < 2e-3
+    x = torch.randn(8, 64, device="cuda", requires_grad=True)
+    w2 = w.clone().requires_grad_()
+    g, = torch.autograd.grad(linear(x, w2, b).sum(), x, create_graph=True)
+    dw, = torch.autograd.grad((g * g).sum(), w2)
+    assert _err(dw, (2 * 8 * w.double().sum(0)).expand(64, 64)) < 2e-3

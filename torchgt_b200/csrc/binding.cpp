@@ -325,4 +325,5 @@ PYBIND11_MODULE(_native, m) {
       .def("poll", &Graph::poll);
   m.def("attention", &attention);
   bind_batching(m);
+  bind_dense(m);
 }

@@ -92,5 +92,6 @@ void attention_backward(Graph& g, const at::Tensor& dout, const at::Tensor& q, c
                         int dtype);
 
 void bind_batching(pybind11::module_& m);   // binding_batch.cpp
+void bind_dense(pybind11::module_& m);      // binding_dense.cpp
 
 }  // namespace tgt_host

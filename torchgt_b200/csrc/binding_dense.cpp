@@ -1,0 +1,126 @@
+// Autograd node of the narrow linear layer (torchgt_b200/linear.py): forward and parameter gradients as this library's
+// kernels, issued without a trip through Python.
+#include "binding.h"
+
+#include <ATen/Context.h>
+#include <ATen/TensorSubclassLikeUtils.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <pybind11/stl.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/utils/pybind.h>
+
+namespace tgt_host {
+namespace {
+
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+bool aligned(const at::Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+
+// contiguous, and copied when it is a view that starts off a 16-byte boundary (the kernels move 16 bytes at a time)
+at::Tensor kernel_ready(const at::Tensor& t) {
+  at::Tensor c = t.contiguous();
+  return aligned(c) ? c : c.clone();
+}
+
+// a plain fp32 CUDA tensor, not a functorch wrapper, a dual number, a fake or a lazily negated view
+bool plain(const at::Tensor& t, const at::Device& device) {
+  return t.defined() && !at::isTensorSubclassLike(t) && t.is_cuda() && t.layout() == at::kStrided &&
+         t.scalar_type() == at::kFloat && t.device() == device && !torch::autograd::isFwGradDefined(t) && !t.is_neg();
+}
+
+// The caller allowed TF32 products: the forward product is then the library's, which has the tensor cores for it.
+// Without it products are full fp32 and this library's kernel is the faster one.
+bool tf32_allowed() {
+  return at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) ==
+         at::Float32Precision::TF32;
+}
+
+struct NarrowLinearBackward : public torch::autograd::Node {
+  SavedVariable x, weight;
+  bool has_bias = false;
+
+  variable_list apply(variable_list&& grads) override {
+    if (!grads[0].defined()) return variable_list(3);
+    const at::Tensor x_ = x.unpack(), w_ = weight.unpack();
+    const c10::cuda::CUDAGuard guard(x_.device());
+    at::Tensor dx, dw, db;
+    const bool recorded = at::GradMode::is_enabled();     // a second-order gradient is wanted: dx as a recorded product
+    if (task_should_compute_output(0) && recorded) dx = at::matmul(grads[0], w_);
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const int64_t out = w_.size(0), in = w_.size(1);
+    const at::Tensor dy = kernel_ready(grads[0]);
+    const int64_t rows = dy.numel() / out;
+    if (task_should_compute_output(0) && !recorded) dx = at::mm(dy.view({rows, out}), w_).view(x_.sizes());
+    if (task_should_compute_output(1) || (has_bias && task_should_compute_output(2))) {
+      const at::Tensor xc = kernel_ready(x_);
+      size_t bytes = 0;
+      check(tgt_linear_wgrad_scratch_bytes(rows, int(in), int(out), &bytes));
+      const at::Tensor scratch = at::empty({int64_t(bytes < 16 ? 16 : bytes)}, dy.options().dtype(at::kByte));
+      dw = at::empty({out, in}, dy.options());
+      if (has_bias) db = at::empty({out}, dy.options());
+      check(tgt_linear_wgrad(fptr(dy), fptr(xc), rows, int(in), int(out), fptr(dw), has_bias ? fptr(db) : nullptr,
+                             scratch.data_ptr(), scratch.numel(), stream_of(dy)));
+    }
+    return {dx, dw, db};
+  }
+  std::string name() const override { return "NarrowLinearBackward"; }
+  void release_variables() override {
+    x.reset_data();
+    weight.reset_data();
+  }
+};
+
+// The shapes of the kernels: whole 64-wide inputs, outputs in fours.  Everything else is the ATen operator.
+bool eligible(const at::Tensor& x, const at::Tensor& w, const at::Tensor& bias) {
+  if (!x.defined() || at::isTensorSubclassLike(x) || !plain(x, x.device()) || !plain(w, x.device())) return false;
+  if (w.dim() != 2 || x.dim() < 1 || x.size(-1) != w.size(1) || x.numel() == 0) return false;
+  const int64_t in = w.size(1), out = w.size(0);
+  if (in % 64 != 0 || in < 64 || in > 1024 || out % 4 != 0 || out < 4 || out > 1024) return false;
+  return !bias.defined() || (plain(bias, x.device()) && bias.dim() == 1 && bias.size(0) == out);
+}
+
+at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<at::Tensor>& bias_in) {
+  const at::Tensor bias = bias_in.has_value() ? *bias_in : at::Tensor();
+  if (!eligible(x, w, bias)) return at::linear(x, w, bias_in);
+  const c10::cuda::CUDAGuard guard(x.device());
+  // With a bias the library runs a second kernel, so this one is ahead from the smallest sizes on (64 x 64, device time
+  // here and there: 1,024 rows 3.8 and 5.8 us, 4,097 rows 4.0 and 6.8 us); up to a thousand rows the library's rounding
+  // is kept, the calls being bound by the host.  Without a bias the library's product is one kernel too and wins in the
+  // middle (8,192 rows 6.6 and 4.7 us, 37,609 rows 17.8 and 10.5 us); this one is ahead on long lists (320,000 rows 78
+  // and 95 us).
+  const int64_t rows = x.numel() / w.size(1);
+  const bool library = tf32_allowed() || rows < (bias.defined() ? 1024 : 200000);
+  const bool record = torch::autograd::compute_requires_grad(x, w, bias);
+  at::Tensor y;
+  if (library && !record) return at::linear(x, w, bias_in);
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    if (library) {
+      y = at::linear(x, w, bias_in);
+    } else {
+      auto sizes = x.sizes().vec();
+      sizes.back() = w.size(0);
+      y = at::empty(sizes, x.options());
+      const at::Tensor xc = kernel_ready(x), wc = kernel_ready(w), bc = bias.defined() ? kernel_ready(bias) : bias;
+      check(tgt_linear_rows(fptr(xc), fptr(wc), bc.defined() ? fptr(bc) : nullptr, rows, int(w.size(1)), int(w.size(0)),
+                            fptr(y), stream_of(x)));
+    }
+  }
+  if (record) {
+    auto node = std::shared_ptr<NarrowLinearBackward>(new NarrowLinearBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, w, bias));
+    node->has_bias = bias.defined();
+    node->x = SavedVariable(x, false);
+    node->weight = SavedVariable(w, false);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+}  // namespace
+
+void bind_dense(pybind11::module_& m) { m.def("linear", &linear); }
+
+}  // namespace tgt_host

@@ -1,24 +1,23 @@
-"""``Linear``: ``torch.nn.Linear`` with the same parameters and ``state_dict`` keys whose backward takes the
-weight and bias gradients from ``csrc/linear_wgrad.cu`` when the layer is narrow and the rows are many (the
-models' 64 x 64 projections and FFN layers over 64,000 to 870,000 rows: a product with a 64 x 64 result and a
-reduction over every row, which a library GEMM runs on a few CTAs).  The forward product and the input
-gradient stay library GEMMs; CPU tensors, other dtypes, inputs that are not a multiple of 64 wide and outputs
-that are not a multiple of 4 wide take ``torch.nn.functional.linear`` end to end."""
+"""``Linear``: ``torch.nn.Linear`` with the same parameters and ``state_dict`` keys for narrow fp32 layers over many
+rows (the models' 64 x 64 projections and FFN layers over 4,000 to 870,000 rows).  The node is in
+``csrc/binding_dense.cpp``: the forward runs ``csrc/linear_rows.cu`` when products are full fp32 (a library GEMM runs
+them as an FMA kernel for wide outputs plus a pass that adds the bias) and the library's tensor-core GEMM when the
+caller allows TF32; the input gradient is the library's product; weight and bias gradients run
+``csrc/linear_wgrad.cu`` (a product with a 64 x 64 result and a reduction over every row, which a library GEMM runs on
+a few CTAs).  CPU tensors, other dtypes, inputs that are not a multiple of 64 wide and outputs that are not a multiple
+of 4 wide are ``torch.nn.functional.linear``, and so is whatever is traced, compiled, autocast or transformed by
+``torch.func``."""
 from __future__ import annotations
 
 import ctypes
 
 import torch
 from torch.nn import functional as F
+from torch.overrides import has_torch_function_variadic
 
 from . import _cabi
 
 _scratch_bytes: dict = {}
-
-
-def supported(x: torch.Tensor, in_features: int, out_features: int) -> bool:
-    return (x.is_cuda and x.dtype == torch.float32 and in_features % 64 == 0 and out_features % 4 == 0 and
-            64 <= in_features <= 1024 and 4 <= out_features <= 1024)
 
 
 def _aligned(t: torch.Tensor) -> torch.Tensor:
@@ -48,29 +47,16 @@ def wgrad(dy: torch.Tensor, x: torch.Tensor, with_bias: bool = True):
     return dw, db
 
 
-class _LinearFn(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, bias):
-        ctx.save_for_backward(x, weight)
-        ctx.has_bias = bias is not None
-        return F.linear(x, weight, bias)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x, weight = ctx.saved_tensors
-        dy2 = dy.contiguous().view(-1, weight.shape[0])
-        dx = (dy2 @ weight).view(x.shape) if ctx.needs_input_grad[0] else None
-        dw = db = None
-        if ctx.needs_input_grad[1] or (ctx.has_bias and ctx.needs_input_grad[2]):
-            dw, db = wgrad(dy2, x.contiguous().view(-1, weight.shape[1]), ctx.has_bias)
-        return dx, dw, db
+def _plain_call(x, weight, bias) -> bool:
+    """No tracer, compiler, autocast or tensor subclass wants to see ``F.linear`` itself."""
+    return not (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch.is_autocast_enabled("cuda") or
+                has_torch_function_variadic(x, weight, bias))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias) -> torch.Tensor:
     """``F.linear(x, weight, bias)``."""
-    if supported(x, weight.shape[1], weight.shape[0]) and torch.is_grad_enabled() and (
-            weight.requires_grad or x.requires_grad):
-        return _LinearFn.apply(x, weight, bias)
+    if x.is_cuda and _plain_call(x, weight, bias):
+        return _cabi.native().linear(x, weight, bias)
     return F.linear(x, weight, bias)
 
 
