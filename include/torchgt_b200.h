@@ -452,10 +452,20 @@ TGT_API int tgt_pull_out_proj(void* const* peer_slots, size_t slot_bytes, const 
  */
 TGT_API int tgt_layer_norm_fwd(const float* x, const float* gamma, const float* beta, float eps, int64_t rows,
                                int hidden, float* y, float* stats, void* stream);
+/*
+ * As tgt_layer_norm_fwd on x + residual (both [rows, hidden]); sum (may be NULL) receives x + residual.  With residual
+ * NULL (and sum NULL) it is tgt_layer_norm_fwd.
+ */
+TGT_API int tgt_add_layer_norm_fwd(const float* x, const float* residual, const float* gamma, const float* beta, float eps,
+                                   int64_t rows, int hidden, float* sum, float* y, float* stats, void* stream);
 TGT_API int tgt_layer_norm_bwd_scratch_bytes(int64_t rows, int hidden, size_t* bytes);
 TGT_API int tgt_layer_norm_bwd(const float* dy, const float* x, const float* gamma, const float* stats,
                                int64_t rows, int hidden, float* dx, float* dgamma, float* dbeta, void* scratch,
                                size_t scratch_bytes, void* stream);
+/* As tgt_layer_norm_bwd, with dsum [rows, hidden] (may be NULL) added to dx: the gradient of the residual stream. */
+TGT_API int tgt_add_layer_norm_bwd(const float* dy, const float* dsum, const float* x, const float* gamma,
+                                   const float* stats, int64_t rows, int hidden, float* dx, float* dgamma, float* dbeta,
+                                   void* scratch, size_t scratch_bytes, void* stream);
 
 /*
  * Product of a narrow nn.Linear over many rows, full fp32 products and sums: c [rows, cols] = a [rows, reduce] w^T +

@@ -110,3 +110,45 @@ def test_layer_norm_and_linear_accept_views_that_start_off_a_16_byte_boundary():
     tol = 2e-3 if torch.backends.cuda.matmul.allow_tf32 else 1e-5
     assert _close(y, ref.detach().cpu(), tol)[0]
     assert _close(xa.grad, xd.grad.cpu(), tol)[0]
+
+
+@pytest.mark.parametrize("hidden", [4, 24, 64, 512])
+@pytest.mark.parametrize("rows", [1, 257, 4099])
+@pytest.mark.parametrize("use", ["both", "norm", "sum"])
+def test_residual_addition_inside_the_norm_gives_the_bits_of_the_two_operations(rows, hidden, use):
+    from torchgt_b200.layer_norm import LayerNorm, add_layer_norm
+    gen = torch.Generator().manual_seed(rows + hidden)
+    x, r, dy, ds = (torch.randn(rows, hidden, generator=gen).cuda() for _ in range(4))
+    norm = LayerNorm(hidden).cuda()
+    with torch.no_grad():
+        norm.weight.copy_(torch.randn(hidden, generator=gen).cuda())
+
+    def run(fused):
+        norm.zero_grad()
+        a, b = x.clone().requires_grad_(), r.clone().requires_grad_()
+        y, s = add_layer_norm(a, b, norm) if fused else (norm(a + b), None)
+        if not fused:
+            s = a + b
+        outs = {"both": ((y, dy), (s, ds)), "norm": ((y, dy),), "sum": ((s, ds),)}[use]
+        torch.autograd.backward([o for o, _ in outs], [g for _, g in outs])
+        return [y, s, a.grad, b.grad, norm.weight.grad, norm.bias.grad]
+
+    for got, want in zip(run(True), run(False)):
+        assert (got is None and want is None) or torch.equal(got, want)
+    with torch.no_grad():
+        y, s = add_layer_norm(x, r, norm, want_sum=False)
+        assert s is None and torch.equal(y, norm(x + r))
+
+
+def test_residual_addition_leaves_hooked_and_uncovered_norms_to_their_own_call():
+    from torchgt_b200.layer_norm import LayerNorm, add_layer_norm
+    norm = LayerNorm(64).cuda()
+    x, r = torch.randn(9, 64, device="cuda"), torch.randn(9, 64, device="cuda")
+    seen = []
+    handle = norm.register_forward_hook(lambda m, args, out: seen.append(args[0]))
+    y, s = add_layer_norm(x, r, norm)
+    assert len(seen) == 1 and torch.equal(seen[0], x + r) and torch.equal(s, x + r)
+    handle.remove()
+    assert torch.equal(add_layer_norm(x, r, norm)[0], y)
+    wide = LayerNorm(64).cuda().double()
+    assert torch.equal(add_layer_norm(x.double(), r.double(), wide)[0], wide(x.double() + r.double()))

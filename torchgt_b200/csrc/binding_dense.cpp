@@ -1,5 +1,5 @@
-// Autograd node of the narrow linear layer (torchgt_b200/linear.py): forward and parameter gradients as this library's
-// kernels, issued without a trip through Python.
+// Autograd nodes of the narrow linear layer (torchgt_b200/linear.py) and of LayerNorm (torchgt_b200/layer_norm.py):
+// this library's kernels, issued without a trip through Python.
 #include "binding.h"
 
 #include <ATen/Context.h>
@@ -119,8 +119,104 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<
   return y;
 }
 
+// ---- LayerNorm, with the residual addition in front of it ------------------------------------------------------
+// Outputs: the normalised rows and, with a residual, x + residual.
+struct LayerNormRowsBackward : public torch::autograd::Node {
+  SavedVariable normalised, weight;   // the norm's input: x, or the output x + residual
+  at::Tensor stats;
+  bool with_residual = false;
+
+  variable_list apply(variable_list&& grads) override {
+    const at::Tensor ds = with_residual ? grads[1] : at::Tensor();
+    if (!grads[0].defined()) return {ds, ds, at::Tensor(), at::Tensor()};   // only x + residual was used
+    const at::Tensor x = with_residual ? normalised.unpack(shared_from_this()) : normalised.unpack();
+    const at::Tensor w = weight.unpack();
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard guard(x.device());
+    const at::Tensor dy = kernel_ready(grads[0]), xc = kernel_ready(x), wc = kernel_ready(w);
+    const at::Tensor dsum = ds.defined() ? kernel_ready(ds) : ds;
+    const int64_t hidden = w.numel(), rows = x.numel() / hidden;
+    const at::Tensor dx = at::empty(x.sizes(), dy.options());
+    const at::Tensor dgamma = at::empty(w.sizes(), dy.options()), dbeta = at::empty(w.sizes(), dy.options());
+    size_t bytes = 0;
+    check(tgt_layer_norm_bwd_scratch_bytes(rows, int(hidden), &bytes));
+    const at::Tensor scratch = at::empty({int64_t(bytes < 16 ? 16 : bytes)}, dy.options().dtype(at::kByte));
+    check(tgt_add_layer_norm_bwd(fptr(dy), dsum.defined() ? fptr(dsum) : nullptr, fptr(xc), fptr(wc), fptr(stats), rows,
+                                 int(hidden), fptr(dx), fptr(dgamma), fptr(dbeta), scratch.data_ptr(), scratch.numel(),
+                                 stream_of(dy)));
+    return {dx, with_residual ? dx : at::Tensor(), dgamma, dbeta};
+  }
+  std::string name() const override { return "LayerNormRowsBackward"; }
+  void release_variables() override {
+    normalised.reset_data();
+    weight.reset_data();
+    stats.reset();
+  }
+};
+
+bool norm_eligible(const at::Tensor& x, const at::Tensor& residual, const at::Tensor& w, const at::Tensor& b) {
+  if (!x.defined() || at::isTensorSubclassLike(x)) return false;
+  const at::Device device = x.device();
+  if (!plain(x, device) || !plain(w, device) || !plain(b, device)) return false;
+  const int64_t hidden = w.numel();
+  if (w.dim() != 1 || b.dim() != 1 || b.numel() != hidden || x.dim() < 1 || x.size(-1) != hidden || x.numel() == 0 ||
+      hidden % 4 != 0 || hidden < 4 || hidden > 512)
+    return false;
+  return !residual.defined() || (plain(residual, device) && residual.sizes() == x.sizes());
+}
+
+// {norm of x (+ residual), x + residual or nothing}; the sum is left out when nobody wants it
+std::pair<at::Tensor, std::optional<at::Tensor>> add_layer_norm(const at::Tensor& x,
+                                                                const std::optional<at::Tensor>& residual_in,
+                                                                const at::Tensor& w, const at::Tensor& b, double eps,
+                                                                bool want_sum) {
+  const at::Tensor residual = residual_in.has_value() ? *residual_in : at::Tensor();
+  if (!norm_eligible(x, residual, w, b)) {
+    const at::Tensor s = residual.defined() ? x + residual : x;
+    return {at::layer_norm(s, w.sizes(), w, b, eps), residual.defined() ? std::optional<at::Tensor>(s) : std::nullopt};
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  const bool record = torch::autograd::compute_requires_grad(x, residual, w, b);
+  const int64_t hidden = w.numel(), rows = x.numel() / hidden;
+  at::Tensor y, sum, stats;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const at::Tensor xc = kernel_ready(x), wc = kernel_ready(w), bc = kernel_ready(b);
+    const at::Tensor rc = residual.defined() ? kernel_ready(residual) : residual;
+    y = at::empty(x.sizes(), x.options());
+    if (residual.defined() && (want_sum || record)) sum = at::empty(x.sizes(), x.options());
+    if (record) stats = at::empty({rows, 2}, x.options());
+    check(tgt_add_layer_norm_fwd(fptr(xc), rc.defined() ? fptr(rc) : nullptr, fptr(wc), fptr(bc), float(eps), rows,
+                                 int(hidden), sum.defined() ? fptr(sum) : nullptr, fptr(y), record ? fptr(stats) : nullptr,
+                                 stream_of(x)));
+  }
+  if (record) {
+    auto node = std::shared_ptr<LayerNormRowsBackward>(new LayerNormRowsBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, residual, w, b));
+    node->with_residual = residual.defined();
+    node->stats = stats;
+    node->weight = SavedVariable(w, false);
+    if (residual.defined()) {
+      torch::autograd::set_history(variable_list{y, sum}, node);
+      node->normalised = SavedVariable(sum, true);
+    } else {
+      torch::autograd::set_history(y, node);
+      node->normalised = SavedVariable(x, false);
+    }
+  }
+  return {y, sum.defined() ? std::optional<at::Tensor>(sum) : std::nullopt};
+}
+
+at::Tensor layer_norm(const at::Tensor& x, const at::Tensor& w, const at::Tensor& b, double eps) {
+  return add_layer_norm(x, std::nullopt, w, b, eps, false).first;
+}
+
 }  // namespace
 
-void bind_dense(pybind11::module_& m) { m.def("linear", &linear); }
+void bind_dense(pybind11::module_& m) {
+  m.def("linear", &linear);
+  m.def("layer_norm", &layer_norm);
+  m.def("add_layer_norm", &add_layer_norm);
+}
 
 }  // namespace tgt_host

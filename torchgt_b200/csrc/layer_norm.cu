@@ -3,7 +3,10 @@
 // 293-311: self_attention_norm before the projections, ffn_norm after the residual; final_ln :395) and the
 // backward half of the fused LayerNorm + projection kernel.  With rows this short a row is a few lanes of
 // one warp: LPR lanes hold a row as 16-byte pieces, 32 / LPR rows per warp, everything in registers, one
-// read of the input and one write of the result (forward), two reads and one write (backward).  The
+// read of the input and one write of the result (forward), two reads and one write (backward).  The residual
+// addition in front of the norm is part of both: x + r is formed in registers, kept for the residual stream and
+// normalised (two reads and two writes, where an addition of its own and the norm make three and two), and the gradient
+// that comes down the residual stream is added to the norm's own: one pass and one launch less each way.  The
 // parameter gradients are summed per thread over the rows it walks, then per CTA in shared memory, then
 // over the CTAs by a second small kernel in a fixed order: no atomics, bitwise reproducible.
 #include <type_traits>
@@ -25,8 +28,10 @@ __device__ __forceinline__ float row_sum(float x) {
 
 struct LnFwdParams {
   const float* x;
+  const float* residual;   // added to x first; may be null
   const float* gamma;
   const float* beta;
+  float* sum;      // x + residual; may be null
   float* y;
   float2* stats;   // [rows] mean, 1 / sqrt(var + eps); may be null
   int64_t rows;
@@ -60,6 +65,11 @@ __global__ void __launch_bounds__(kLnThreads) layer_norm_fwd_kernel(const LnFwdP
       const int c = l + j * LPR;
       v[j] = live && c < pieces ? __ldg(reinterpret_cast<const float4*>(p.x + row * p.hidden) + c)
                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (p.residual != nullptr && live && c < pieces) {
+        const float4 r = __ldg(reinterpret_cast<const float4*>(p.residual + row * p.hidden) + c);
+        v[j].x += r.x; v[j].y += r.y; v[j].z += r.z; v[j].w += r.w;
+        if (p.sum != nullptr) reinterpret_cast<float4*>(p.sum + row * p.hidden)[c] = v[j];
+      }
       s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
     }
     const float mean = row_sum<LPR>(s) * inv_h;
@@ -93,6 +103,7 @@ __global__ void __launch_bounds__(kLnThreads) layer_norm_fwd_kernel(const LnFwdP
 
 struct LnBwdParams {
   const float* dy;
+  const float* dsum;   // gradient of the normalised input from elsewhere, added to dx; may be null
   const float* x;
   const float* gamma;
   const float2* stats;
@@ -155,6 +166,10 @@ __global__ void __launch_bounds__(kLnThreads) layer_norm_bwd_kernel(const LnBwdP
           o.y = st.y * (g[j].y - c1 - xh[j].y * c2);
           o.z = st.y * (g[j].z - c1 - xh[j].z * c2);
           o.w = st.y * (g[j].w - c1 - xh[j].w * c2);
+          if (p.dsum != nullptr) {
+            const float4 e = __ldg(reinterpret_cast<const float4*>(p.dsum + row * p.hidden) + c);
+            o.x += e.x; o.y += e.y; o.z += e.z; o.w += e.w;
+          }
           reinterpret_cast<float4*>(p.dx + row * p.hidden)[c] = o;
         }
       }
@@ -229,7 +244,13 @@ bool ln_dispatch(int lpr, int pieces, F&& f) {
 }  // namespace tgt
 
 extern "C" int tgt_layer_norm_fwd(const float* x, const float* gamma, const float* beta, float eps,
-                                  int64_t rows, int hidden, float* y, float* stats, void* stream_) {
+                                  int64_t rows, int hidden, float* y, float* stats, void* stream) {
+  return tgt_add_layer_norm_fwd(x, nullptr, gamma, beta, eps, rows, hidden, nullptr, y, stats, stream);
+}
+
+extern "C" int tgt_add_layer_norm_fwd(const float* x, const float* residual, const float* gamma, const float* beta,
+                                      float eps, int64_t rows, int hidden, float* sum, float* y, float* stats,
+                                      void* stream_) {
   using namespace tgt;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   int lpr = 0, pieces = 0;
@@ -239,10 +260,11 @@ extern "C" int tgt_layer_norm_fwd(const float* x, const float* gamma, const floa
   TGT_CHECK_ARG(rows >= 0, "rows must be >= 0");
   if (rows == 0) return TGT_OK;
   TGT_CHECK_ARG(x && gamma && beta && y, "x, gamma, beta and y must not be null");
-  TGT_CHECK_ARG(aligned16(x) && aligned16(gamma) && aligned16(beta) && aligned16(y) &&
+  TGT_CHECK_ARG(sum == nullptr || residual != nullptr, "sum without a residual");
+  TGT_CHECK_ARG(aligned16(x) && aligned16(residual) && aligned16(gamma) && aligned16(beta) && aligned16(sum) && aligned16(y) &&
                     (reinterpret_cast<uintptr_t>(stats) & 7u) == 0,
                 "tensors must be 16-byte aligned (stats 8-byte)");
-  LnFwdParams p{x, gamma, beta, y, reinterpret_cast<float2*>(stats), rows, hidden, eps};
+  LnFwdParams p{x, residual, gamma, beta, sum, y, reinterpret_cast<float2*>(stats), rows, hidden, eps};
   const int grid = ln_grid(rows, lpr);
   const bool built = ln_dispatch(lpr, pieces, [&](auto L, auto P) {
     layer_norm_fwd_kernel<decltype(L)::value, decltype(P)::value><<<grid, kLnThreads, 0, stream>>>(p);
@@ -266,7 +288,14 @@ extern "C" int tgt_layer_norm_bwd_scratch_bytes(int64_t rows, int hidden, size_t
 
 extern "C" int tgt_layer_norm_bwd(const float* dy, const float* x, const float* gamma, const float* stats,
                                   int64_t rows, int hidden, float* dx, float* dgamma, float* dbeta,
-                                  void* scratch, size_t scratch_bytes, void* stream_) {
+                                  void* scratch, size_t scratch_bytes, void* stream) {
+  return tgt_add_layer_norm_bwd(dy, nullptr, x, gamma, stats, rows, hidden, dx, dgamma, dbeta, scratch, scratch_bytes,
+                                stream);
+}
+
+extern "C" int tgt_add_layer_norm_bwd(const float* dy, const float* dsum, const float* x, const float* gamma,
+                                      const float* stats, int64_t rows, int hidden, float* dx, float* dgamma,
+                                      float* dbeta, void* scratch, size_t scratch_bytes, void* stream_) {
   using namespace tgt;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   int lpr = 0, pieces = 0;
@@ -281,14 +310,14 @@ extern "C" int tgt_layer_norm_bwd(const float* dy, const float* x, const float* 
     return TGT_OK;
   }
   TGT_CHECK_ARG(dy && x && gamma && stats && dx, "dy, x, gamma, stats and dx must not be null");
-  TGT_CHECK_ARG(aligned16(dy) && aligned16(x) && aligned16(gamma) && aligned16(dx) && aligned16(scratch) &&
+  TGT_CHECK_ARG(aligned16(dy) && aligned16(dsum) && aligned16(x) && aligned16(gamma) && aligned16(dx) && aligned16(scratch) &&
                     (reinterpret_cast<uintptr_t>(stats) & 7u) == 0,
                 "tensors must be 16-byte aligned (stats 8-byte)");
   const int grid = ln_grid(rows, lpr);
   const size_t need = size_t(grid) * 2 * size_t(hidden) * sizeof(float);
   if (scratch == nullptr || scratch_bytes < need)
     return set_error(TGT_ERR_WORKSPACE, "scratch holds %zu bytes, %zu needed", scratch_bytes, need);
-  LnBwdParams p{dy, x, gamma, reinterpret_cast<const float2*>(stats), dx, static_cast<float*>(scratch), rows, hidden};
+  LnBwdParams p{dy, dsum, x, gamma, reinterpret_cast<const float2*>(stats), dx, static_cast<float*>(scratch), rows, hidden};
   const bool built = ln_dispatch(lpr, pieces, [&](auto L, auto P) {
     layer_norm_bwd_kernel<decltype(L)::value, decltype(P)::value><<<grid, kLnThreads, 0, stream>>>(p);
   });

@@ -18,7 +18,7 @@ from torch.nn import functional as F
 
 from .attn_module import CoreAttention
 from .gt_sp.initialize import get_sequence_parallel_group, sequence_parallel_is_initialized
-from .layer_norm import LayerNorm
+from .layer_norm import LayerNorm, add_layer_norm
 from .linear import Linear
 from .gt_sp.layer import DistributedAttentionNoMerge
 
@@ -121,8 +121,8 @@ class EncoderLayer(nn.Module):
         y = self._fused_attention_half(x, attn_bias, edge_index, attn_type)
         if y is None:
             y = self.self_attention(self.self_attention_norm(x), attn_bias, edge_index, attn_type=attn_type)
-        x = x + self.self_attention_dropout(y)
-        y = self.ffn(self.ffn_norm(x))
+        normed, x = add_layer_norm(x, self.self_attention_dropout(y), self.ffn_norm)
+        y = self.ffn(normed)
         return x + self.ffn_dropout(y)
 
 

@@ -19,7 +19,7 @@ from torch.nn import functional as F
 from .attn_module import CoreAttentionQKV as CoreAttention  # (q, k, v) order, as models/gt_dist_node_level.py:83
 from .gt_sp.gt_layer import DistributedAttention, DistributedAttentionNodeLevel, _SeqGather
 from .gt_sp.initialize import get_sequence_parallel_group, sequence_parallel_is_initialized
-from .layer_norm import LayerNorm
+from .layer_norm import LayerNorm, add_layer_norm
 from .linear import Linear
 
 
@@ -84,9 +84,9 @@ class EncoderLayer(nn.Module):
     def forward(self, x, attn_bias=None, mask=None, edge_index=None, attn_type=None):
         y = self.self_attention(x, attn_bias, mask=mask, edge_index=edge_index, attn_type=attn_type)
         y = self.O(self.self_attention_dropout(y))
-        x = self.layer_norm1(x + y)
+        x, _ = add_layer_norm(x, y, self.layer_norm1, want_sum=False)
         y = self.FFN_layer2(self.self_attention_dropout(F.relu(self.FFN_layer1(y))))
-        return self.layer_norm2(x + y)
+        return add_layer_norm(x, y, self.layer_norm2, want_sum=False)[0]
 
 
 class MLPReadout(nn.Module):
