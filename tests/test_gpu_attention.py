@@ -447,3 +447,34 @@ def test_dependent_launches_change_no_bit(heads, head_dim, dtype, with_bias):
     _check_against_closed_form(q.to(dtype).float(), k.to(dtype).float(), v.to(dtype).float(), ei,
                                dout.to(dtype).float(), bias, {n_: t for n_, t in base.items() if n_ != "dbias"},
                                TOL_F32 if dtype == torch.float32 else TOL_BF16)
+
+
+@pytest.mark.parametrize("heads,dtype", [(8, torch.float32), (1, torch.float32), (8, torch.bfloat16)])
+@pytest.mark.parametrize("rows,edges", [(200_003, 37), (200_003, 3000), (513, 1)])
+def test_rows_far_beyond_the_edges_are_zero_filled(heads, dtype, rows, edges):
+    """Many more rows than the tiles' blocks look at by themselves: extra blocks, the last partial share, gaps of every
+    alignment.  The rows that edges touch are compared on the compacted graph, every other row is exactly 0."""
+    gen = torch.Generator().manual_seed(rows + edges)
+    used = torch.randperm(rows, generator=gen)[:300].sort().values
+    local = torch.randint(0, used.numel(), (2, edges), generator=gen)
+    q, k, v, dout = (torch.randn(used.numel(), heads, 8, generator=gen).to(dtype).float() for _ in range(4))
+    spread = []
+    for t in (q, k, v, dout):
+        big = torch.randn(rows, heads, 8, generator=gen)
+        big[used] = t
+        spread.append(big)
+    junk = [torch.full((rows, heads, 8), float("nan"), device="cuda", dtype=dtype) for _ in range(6)]
+    del junk                                                   # the allocator hands these blocks out again
+    res = _run_cuda(*spread[:3], used[local], spread[3], dtype=dtype)
+    others = torch.ones(rows, dtype=torch.bool)
+    others[used] = False
+    for name, t in res.items():
+        assert torch.count_nonzero(t.cpu()[others]) == 0, name
+    got = {name: t.cpu()[used] for name, t in res.items()}
+    ref_out, _ = sao.forward_closed_form(q, k, v, local)
+    refs = dict(zip(("dq", "dk", "dv"), sao.backward_closed_form(q, k, v, local, dout)[:3]), out=ref_out)
+    tol = TOL_F32 if dtype == torch.float32 else TOL_BF16
+    for name, ref in refs.items():
+        # rows with a single in-edge have gradients that cancel to about 1e-7 of their operands
+        err = np.abs(got[name].double().numpy() - ref).max()
+        assert err < tol * float(np.abs(ref).max()) + 1e-5, (name, err)

@@ -17,8 +17,16 @@
 // also crosses the tile boundary the CTA writes its sum to a per-tile carry in global memory and
 // counts itself in on the row's arrival counter; the CTA that arrives last adds the carries in tile
 // order and finishes the row (nobody waits for anybody).  Every sum has a fixed order whichever CTA
-// does it: no floating-point atomics, bitwise reproducible results.  Rows without edges are
-// zero-filled by the group that walks the gap.
+// does it: no floating-point atomics, bitwise reproducible results.
+//
+// Rows without edges are zero-filled.  The few between two rows of a range are filled by the group that walks over
+// them; aligned blocks of kGapRows rows that are empty as a whole are looked for by the first CTAs, 4,096 rows each, two
+// words of ptr[] per block.  Left to the walking group, the padding behind the graphs of a padded batch is one serial
+// chain of stores: 16 graphs padded to 20,000 rows (320,000 rows, half of them empty, gaps of up to 18,000, 8 heads of
+// 8) took 485 us forward, 192 us dQ and 475 us dK/dV per layer and take 59, 60 and 136.
+// What batches without empty rows pay for it decides who looks: CTAs of their own behind the tiles' hold up the launch
+// of the call's next kernel (64K step + 1.4 %), an equal share for every CTA costs each of them a round trip to memory
+// (one-head 512K step + 2.3 %).
 #pragma once
 
 #include <type_traits>
@@ -91,6 +99,7 @@ struct SegWalk {
   int n_edges;
   int ge;          // edges per lane group per tile (multiple of kGeStep, <= GE_MAX)
   int n_tiles;
+  int gap_ctas;    // CTAs that look for rows without edges (fill_gaps)
   float* gcarry;   // [n_tiles][2][gridDim.y * G * NACC] cross-tile partial sums
   int* tile_done;  // [gridDim.y][n_tiles] arrivals per row that crosses tiles, indexed by the tile it
                    // starts in; zero when the kernel starts.  Null: a second kernel finishes those rows
@@ -182,6 +191,39 @@ __device__ __forceinline__ float fast_exp(float x) {
 
 template <int G, class Policy>
 __device__ __forceinline__ void finish_row(const SegWalk& w, const Policy& pol, float* s_part, int tile);
+
+constexpr int kGapRows = 8;   // rows of an aligned block that fill_gaps fills when it is empty as a whole
+
+// Zero-fills the rows strictly between `before` and `after`, which have no edges, except the whole aligned blocks.
+template <class Policy>
+__device__ __forceinline__ void zero_gap(const Policy& pol, int before, int after) {
+  for (int r = before + 1; r < after; ++r) {
+    if (r % kGapRows == 0 && after - r >= kGapRows) r = after / kGapRows * kGapRows;   // behind the last whole block
+    if (r < after) pol.zero_row(r);
+  }
+}
+
+// The first CTAs of the grid test kGapShare rows each, whole blocks of kGapRows, and zero-fill the empty ones.
+constexpr int kGapShare = 4096;
+template <int G, class Policy>
+__device__ __forceinline__ void fill_gaps(const SegWalk& w, const Policy& pol) {
+  const int lane = threadIdx.x % 32;
+  constexpr int kRounds = kGapShare / (kBlockThreads * kGapRows);   // of 32 blocks per warp
+  const int64_t row0 = int64_t(blockIdx.x) * kGapShare + threadIdx.x / 32 * (kRounds * 32 * kGapRows);
+  bool empty[kRounds];
+#pragma unroll
+  for (int i = 0; i < kRounds; ++i) {
+    const int64_t row = row0 + (32 * i + lane) * kGapRows;
+    empty[i] = row + kGapRows <= w.n_rows && __ldg(w.ptr + row) == __ldg(w.ptr + row + kGapRows);
+  }
+#pragma unroll
+  for (int i = 0; i < kRounds; ++i) {
+    const unsigned mask = __ballot_sync(0xffffffffu, empty[i]);
+    if (mask == 0) continue;
+    for (int r = lane / G; r < 32 * kGapRows; r += 32 / G)
+      if (mask >> (r / kGapRows) & 1) pol.zero_row(int(row0) + 32 * i * kGapRows + r);
+  }
+}
 
 // The walk.  Policy supplies:
 //   static constexpr int NACC;                     accumulators per lane
@@ -277,7 +319,7 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
             }
           }
           head_pending = false;
-          for (int r = cur + 1; r < row[u]; ++r) pol.zero_row(r);
+          zero_gap(pol, cur, row[u]);
           cur = row[u];
           own = true;
 #pragma unroll
@@ -311,9 +353,9 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
     } else {
       pol.finalize(cur, acc);
     }
-    if (t0 + gend == w.n_edges)  // this group owns the last edge: rows after it have no edges
-      for (int r = cur + 1; r < w.n_rows; ++r) pol.zero_row(r);
+    if (t0 + gend == w.n_edges) zero_gap(pol, cur, w.n_rows);  // this group owns the last edge
   }
+  if (blockIdx.x < w.gap_ctas) fill_gaps<G, Policy>(w, pol);
   __syncthreads();
 
   // ---- stitch rows that cross group boundaries, in group order
@@ -564,6 +606,13 @@ struct TilePlan {
 };
 TilePlan plan_tiles(int64_t n_edges, const HeadSplit& hs, int nacc, int ctas_per_sm);
 
+// CTAs of a walk kernel in x: one per tile, and more where there are over kGapShare rows per tile.
+inline int gap_ctas(int64_t n_rows) { return int((n_rows + kGapShare - 1) / kGapShare); }
+inline unsigned walk_ctas(const TilePlan& tp, int64_t n_rows) {
+  const int gaps = gap_ctas(n_rows);
+  return unsigned(gaps > tp.n_tiles ? gaps : tp.n_tiles);
+}
+
 // Shared-memory bytes walk_tile needs (indices + carries), as the kernels declare them.
 template <int G, int NACC>
 struct TileSmem {
@@ -586,6 +635,12 @@ struct TileSmem {
 // The call every walk kernel makes.
 template <int G, class Policy>
 __device__ __forceinline__ void walk_tile_in(TileSmem<G, Policy::NACC>& sm, const SegWalk& w, const Policy& pol) {
+  if (blockIdx.x >= w.n_tiles) {     // launched for its share of the empty rows only
+    release_dependents();
+    dependent_wait();                // the rows may be what the previous kernel of the call works on
+    fill_gaps<G, Policy>(w, pol);
+    return;
+  }
   walk_tile<G, Policy>(w, pol, sm.idx.other, sm.idx.seg, sm.idx.perm, sm.carry, sm.carry_row, sm.part, sm.finish);
 }
 

@@ -83,7 +83,7 @@ void fill_walk(SegWalk* w, const tgt_layout& L, const TilePlan& tp, float* carry
                bool need_perm) {
   w->ptr = L.ptr; w->other = L.other; w->perm = L.perm; w->seg = L.seg;
   w->n_rows = int(L.n_rows); w->n_edges = int(L.n_edges);
-  w->ge = tp.ge; w->n_tiles = tp.n_tiles;
+  w->ge = tp.ge; w->n_tiles = tp.n_tiles; w->gap_ctas = gap_ctas(L.n_rows);
   w->gcarry = carry;
   w->tile_done = counters;
   w->need_perm = need_perm;
@@ -276,20 +276,20 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
     // pass A that derives the row statistics itself (and leaves them in scratch for pass B)
     fill_walk(&p.walk, *by_dst, sc.plan_a_fused, reinterpret_cast<float*>(base + sc.carry_a), counters_a,
               bias != nullptr);
-    const dim3 grid(sc.plan_a_fused.n_tiles, hs.groups);
+    const dim3 grid(walk_ctas(sc.plan_a_fused, n_rows), hs.groups);
     built = bwd::launch_dq_fused(p, dtype, hs, grid, second_kernel, link, stream);
-    link = second_kernel && grid.x > 1 ? kLinkAfterStitch : kLinkWalk;
+    link = second_kernel && p.walk.n_tiles > 1 ? kLinkAfterStitch : kLinkWalk;
   } else if (passes & 2) {
     // pass A with per-edge dbias: uses the statistics of the pre-pass (stage 1)
     fill_walk(&p.walk, *by_dst, sc.plan_a, reinterpret_cast<float*>(base + sc.carry_a), counters_a, true);
-    const dim3 grid(sc.plan_a.n_tiles, hs.groups);
+    const dim3 grid(walk_ctas(sc.plan_a, n_rows), hs.groups);
     built = bwd::launch_dq(p, dtype, hs, grid, second_kernel, link, stream);
-    link = second_kernel && grid.x > 1 ? kLinkAfterStitch : kLinkWalk;
+    link = second_kernel && p.walk.n_tiles > 1 ? kLinkAfterStitch : kLinkWalk;
   }
   if (built && (passes & 4)) {
     fill_walk(&p.walk, *by_src, sc.plan_b, reinterpret_cast<float*>(base + sc.carry_b), counters_b,
               bias != nullptr);
-    const dim3 grid(sc.plan_b.n_tiles, hsb.groups);
+    const dim3 grid(walk_ctas(sc.plan_b, n_rows), hsb.groups);
     built = bwd::launch_dkv(p, dtype, hsb, grid, second_kernel_b, link, stream);
   }
   if (!built) return set_error(TGT_ERR_UNSUPPORTED, "no kernel is built for this head layout");

@@ -141,8 +141,8 @@ bool launch_dq_fused(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 gr
   return dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
     launch_chained(bwd_dq_fused_kernel<typename S::T, S::W, S::LPH, S::G>, grid, kBlockThreads, stream, link, p);
-    if (second_kernel && grid.x > 1)
-      launch_chained(bwd_dq_fused_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, grid, kBlockThreads, stream, kLinkStitch, p);
+    if (second_kernel && p.walk.n_tiles > 1)
+      launch_chained(bwd_dq_fused_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(p.walk.n_tiles, grid.y), kBlockThreads, stream, kLinkStitch, p);
   });
 }
 

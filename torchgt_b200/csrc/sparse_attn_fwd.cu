@@ -246,7 +246,7 @@ extern "C" int tgt_sparse_attn_fwd_strided(const void* q, int64_t q_row_bytes, c
   p.inv_scale = 1.0f / sqrtf(float(head_dim));
   p.walk.ptr = L.ptr; p.walk.other = L.other; p.walk.perm = L.perm; p.walk.seg = L.seg;
   p.walk.n_rows = int(L.n_rows); p.walk.n_edges = int(L.n_edges);
-  p.walk.ge = tp.ge; p.walk.n_tiles = tp.n_tiles;
+  p.walk.ge = tp.ge; p.walk.n_tiles = tp.n_tiles; p.walk.gap_ctas = gap_ctas(L.n_rows);
   p.walk.gcarry = static_cast<float*>(scratch);
   const bool second_kernel = stitch_in_second_kernel(hs.g);
   p.walk.tile_done = second_kernel ? nullptr : reinterpret_cast<int*>(static_cast<char*>(scratch) + tp.carry_bytes);
@@ -254,12 +254,12 @@ extern "C" int tgt_sparse_attn_fwd_strided(const void* q, int64_t q_row_bytes, c
   if (tp.n_tiles > 1 && !second_kernel)
     TGT_CHECK_CUDA(cudaMemsetAsync(p.walk.tile_done, 0, tp.counter_bytes, stream));
 
-  const dim3 grid(tp.n_tiles, hs.groups);
+  const dim3 grid(walk_ctas(tp, L.n_rows), hs.groups);
   const bool built = dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
     fwd_kernel<typename S::T, S::W, S::LPH, S::G><<<grid, kBlockThreads, 0, stream>>>(p);
     if (second_kernel && tp.n_tiles > 1)
-      launch_chained(fwd_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, grid, kBlockThreads, stream, kLinkStitch, p);
+      launch_chained(fwd_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(p.walk.n_tiles, grid.y), kBlockThreads, stream, kLinkStitch, p);
   });
   if (!built) return set_error(TGT_ERR_UNSUPPORTED, "no kernel is built for this head layout");
   TGT_CHECK_CUDA(cudaGetLastError());
