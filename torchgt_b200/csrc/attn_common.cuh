@@ -26,7 +26,9 @@
 // 8) took 485 us forward, 192 us dQ and 475 us dK/dV per layer and take 59, 60 and 136.
 // What batches without empty rows pay for it decides who looks: CTAs of their own behind the tiles' hold up the launch
 // of the call's next kernel (64K step + 1.4 %), an equal share for every CTA costs each of them a round trip to memory
-// (one-head 512K step + 2.3 %).
+// (one-head 512K step + 2.3 %), testing in front of the walk changes its registers (64K step + 4.6 %) and behind the
+// stitching its occupancy.  Between the walk and the stitching it costs 0.7 % (64K step with bias gradient 160.3 -> 161.4
+// us, one-head 512K step 304.0 -> 306.1) or nothing (870K, forward alone).
 #pragma once
 
 #include <type_traits>
