@@ -478,3 +478,18 @@ def test_rows_far_beyond_the_edges_are_zero_filled(heads, dtype, rows, edges):
         # rows with a single in-edge have gradients that cancel to about 1e-7 of their operands
         err = np.abs(got[name].double().numpy() - ref).max()
         assert err < tol * float(np.abs(ref).max()) + 1e-5, (name, err)
+
+
+def test_forward_mode_is_refused_and_only_asked_gradients_are_computed():
+    import torch.autograd.forward_ad as fwd
+    from torchgt_b200 import SparseGraph, sparse_graph_attention
+    ei = random_graph(3, 50, 4.0).cuda()
+    q, k, v = (torch.randn(50, 8, 8, device="cuda", requires_grad=True) for _ in range(3))
+    bias = torch.zeros(ei.shape[1], device="cuda", requires_grad=True)
+    graph = SparseGraph(ei, 50)
+    with fwd.dual_level(), pytest.raises(RuntimeError):
+        sparse_graph_attention(fwd.make_dual(q, torch.ones_like(q)), k, v, graph)
+    both = torch.autograd.grad(sparse_graph_attention(q, k, v, graph, bias).sum(), (q, k, v, bias))
+    some = torch.autograd.grad(sparse_graph_attention(q, k, v, graph, bias).sum(), (q, k, v))
+    for a, b in zip(some, both):
+        assert (a - b).abs().max() <= TOL_F32 * float(b.abs().max()) + 1e-6   # the passes differ in their sums' order
