@@ -493,3 +493,27 @@ def test_forward_mode_is_refused_and_only_asked_gradients_are_computed():
     some = torch.autograd.grad(sparse_graph_attention(q, k, v, graph, bias).sum(), (q, k, v))
     for a, b in zip(some, both):
         assert (a - b).abs().max() <= TOL_F32 * float(b.abs().max()) + 1e-6   # the passes differ in their sums' order
+
+
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_a_traced_call_runs_again_on_other_inputs(with_bias):
+    """The traced function computes, forward and backward, what the function computes: the same kernels, the same bits."""
+    from torchgt_b200 import SparseGraph, sparse_graph_attention
+    ei = random_graph(5, 60, 4.0).cuda()
+    graph = SparseGraph(ei, 60)
+
+    def inputs():
+        return [torch.randn(60, 8, 8, device="cuda", requires_grad=True) for _ in range(3)] + (
+            [torch.randn(ei.shape[1], device="cuda", requires_grad=True)] if with_bias else [])
+
+    call = lambda q, k, v, bias=None: 2 * sparse_graph_attention(q, k, v, graph, bias)
+    traced = torch.jit.trace(call, tuple(inputs()), check_trace=False)
+    for _ in range(2):
+        args = inputs()
+        want, got = call(*args), traced(*args)
+        assert torch.equal(got, want)
+        dout = torch.randn_like(want)
+        for a, b in zip(torch.autograd.grad(got, args, dout), torch.autograd.grad(want, args, dout)):
+            assert torch.equal(a, b)
+        with torch.no_grad():
+            assert torch.equal(traced(*args), want)

@@ -4,6 +4,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <pybind11/stl.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/utils/pybind.h>
 
@@ -200,6 +201,8 @@ int bias_heads(const at::Tensor& bias) {
   return bias.defined() ? (bias.dim() == 1 ? 1 : int(bias.size(1))) : 0;
 }
 
+int dtype_of(const at::Tensor& q) { return q.scalar_type() == at::kFloat ? TGT_F32 : TGT_BF16; }
+
 at::Tensor scratch(Graph& g, int heads, int head_dim, int dtype, int phase, const at::Tensor& like) {
   return at::empty({int64_t(g.scratch_bytes(heads, head_dim, dtype, phase))}, like.options().dtype(at::kByte));
 }
@@ -265,7 +268,7 @@ at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::T
                                 "sparse_graph_attention does not support forward-mode AD");
   const at::Tensor q = q_in.contiguous(), k = k_in.contiguous(), v = v_in.contiguous();
   const int heads = int(q.size(1)), head_dim = int(q.size(2));
-  const int dtype = q.scalar_type() == at::kFloat ? TGT_F32 : TGT_BF16;
+  const int dtype = dtype_of(q);
   const c10::cuda::CUDAGuard guard(q.device());
   at::Tensor out, z;
   {
@@ -290,6 +293,29 @@ at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::T
     if (node->with_dbias) node->out = SavedVariable(out, true);
   }
   return out;
+}
+
+// The two passes without an autograd node, for callers that keep one of their own (torchgt_b200/sparse_attn.py).
+std::pair<at::Tensor, at::Tensor> forward_pass(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                                               const std::optional<at::Tensor>& bias, const std::shared_ptr<Graph>& graph) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  const int heads = int(q.size(1)), head_dim = int(q.size(2));
+  at::Tensor out = at::empty_like(q), z = at::empty({q.size(0), heads}, q.options().dtype(at::kFloat));
+  attention_forward(*graph, q, k, v, bias.value_or(at::Tensor()), out, z, heads, head_dim, dtype_of(q));
+  return {out, z};
+}
+
+std::vector<std::optional<at::Tensor>> backward_pass(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k,
+                                                     const at::Tensor& v, const std::optional<at::Tensor>& bias,
+                                                     const at::Tensor& out, const at::Tensor& z,
+                                                     const std::shared_ptr<Graph>& graph, bool want_dbias) {
+  const c10::cuda::CUDAGuard guard(q.device());
+  const at::Tensor bias_ = bias.value_or(at::Tensor());
+  at::Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dbias;
+  if (want_dbias) dbias = at::empty_like(bias_);
+  attention_backward(*graph, dout.contiguous(), q, k, v, bias_, out, z, dq, dk, dv, dbias, int(q.size(1)),
+                     int(q.size(2)), dtype_of(q));
+  return {dq, dk, dv, want_dbias ? std::optional<at::Tensor>(dbias) : std::nullopt};
 }
 
 }  // namespace
@@ -324,6 +350,8 @@ PYBIND11_MODULE(_native, m) {
       .def("has_by_src", &Graph::has_by_src)
       .def("poll", &Graph::poll);
   m.def("attention", &attention);
+  m.def("attention_forward", &forward_pass);
+  m.def("attention_backward", &backward_pass);
   bind_batching(m);
   bind_dense(m);
 }

@@ -38,6 +38,24 @@ def _scratch(graph: SparseGraph, heads: int, head_dim: int, dtype: int, phase: i
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
+class _TracedAttention(torch.autograd.Function):
+    """The call as ``torch.jit.trace`` has to see it: one operation that a traced module calls again.  The native
+    node cannot be recorded; the tracer would keep its output's allocation and nothing that fills it."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, bias, graph: SparseGraph):
+        out, z = _cabi.native().attention_forward(q, k, v, bias, graph.native)
+        ctx.graph = graph
+        ctx.save_for_backward(q, k, v, bias, out, z)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        q, k, v, bias, out, z = ctx.saved_tensors
+        want_dbias = bias is not None and ctx.needs_input_grad[3]
+        return (*_cabi.native().attention_backward(dout, q, k, v, bias, out, z, ctx.graph.native, want_dbias), None)
+
+
 def _heads_fit_one_group(heads: int, head_dim: int, dtype: torch.dtype) -> bool:
     row_bytes = heads * head_dim * (4 if dtype == torch.float32 else 2)
     return row_bytes <= 512 and (heads & (heads - 1)) == 0
@@ -77,4 +95,6 @@ def sparse_graph_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
         bias = bias.contiguous()
         if graph.n_edges == 0:
             bias = None  # nothing to add the (empty) bias to
+    if torch.jit.is_tracing():
+        return _TracedAttention.apply(q.contiguous(), k.contiguous(), v.contiguous(), bias, graph)
     return _cabi.native().attention(q, k, v, bias, graph.native)
