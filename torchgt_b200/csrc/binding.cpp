@@ -3,6 +3,7 @@
 
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/core/LegacyTypeDispatch.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
 #include <torch/csrc/autograd/functions/utils.h>
@@ -318,6 +319,17 @@ std::vector<std::optional<at::Tensor>> backward_pass(const at::Tensor& dout, con
   return {dq, dk, dv, want_dbias ? std::optional<at::Tensor>(dbias) : std::nullopt};
 }
 
+// into[i] <- of[i] in one multi-tensor copy.  The caller drops the sources right away, so their memory, which may belong
+// to another stream, is marked as in use on this one (for memory of this stream that is a comparison).
+void take_gradients(const std::vector<at::Tensor>& into, const std::vector<at::Tensor>& of) {
+  const at::NoGradGuard no_grad;
+  at::_foreach_copy_(into, of);
+  for (const at::Tensor& t : of)
+    if (t.is_cuda())
+      c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(),
+                                                    at::cuda::getCurrentCUDAStream(t.device().index()));
+}
+
 }  // namespace
 }  // namespace tgt_host
 
@@ -349,6 +361,7 @@ PYBIND11_MODULE(_native, m) {
       .def("by_src", &Graph::by_src)
       .def("has_by_src", &Graph::has_by_src)
       .def("poll", &Graph::poll);
+  m.def("take_gradients", &take_gradients);
   m.def("attention", &attention);
   m.def("attention_forward", &forward_pass);
   m.def("attention_backward", &backward_pass);
