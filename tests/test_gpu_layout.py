@@ -161,3 +161,83 @@ def test_device_side_batch_edges_on_the_reference_golden_ring():
         n, sub = int(g[f"rand{i}_n"]), int(g[f"rand{i}_sub"])
         got = prepare_edges(torch.from_numpy(g[f"rand{i}_in"]).cuda(), n, None, True, sub, 0)
         assert np.array_equal(got.cpu().numpy().astype(np.int64), g[f"rand{i}_adjusted"]), i
+
+
+def test_a_graph_is_asked_by_one_thread_while_the_first_backward_builds_its_source_layout():
+    """The backward runs on autograd's own thread and builds the layout there; other threads poll, check and ask for the
+    layouts of the same graph meanwhile."""
+    import threading
+    from torchgt_b200 import SparseGraph, sparse_graph_attention
+    ei = random_graph(8, 300, 5.0)
+    bad = ei.clone()
+    bad[0, 3] = 300
+    q = torch.randn(300, 8, 8, device="cuda", requires_grad=True)
+    for edges, wrong in ((ei.cuda(), False), (bad.cuda(), True)):
+        for _ in range(20):
+            graph, stop, failures, reported = SparseGraph(edges, 300), threading.Event(), [], []
+
+            def ask():
+                from torchgt_b200 import _cabi
+                while not stop.is_set():
+                    try:
+                        graph.poll()
+                        graph.check()
+                        graph.native.has_by_src()
+                        graph.by_dst.verified
+                    except _cabi.TgtError:
+                        reported.append(True)
+                    except Exception as e:
+                        failures.append(e)
+
+            threads = [threading.Thread(target=ask) for _ in range(3)]
+            for t in threads:
+                t.start()
+            try:
+                out = sparse_graph_attention(q, q, q, graph)
+                out.sum().backward()
+            except Exception as e:
+                if not wrong:
+                    failures.append(e)
+            finally:
+                stop.set()
+                for t in threads:
+                    t.join()
+            assert not failures, failures
+            assert bool(reported) <= wrong
+            if not wrong:
+                graph.check()
+                assert graph.by_dst.verified and graph.by_src.verified
+                for lay, group_by in ((graph.by_dst, 1), (graph.by_src, 0)):
+                    ptr, other, perm = elo.segment_layout(ei.numpy(), 300, group_by)
+                    assert np.array_equal(lay.ptr.cpu().numpy(), ptr) and np.array_equal(lay.perm.cpu().numpy(), perm)
+            else:
+                with pytest.raises(Exception, match="outside"):
+                    graph.check()
+
+
+def test_other_threads_run_while_a_layout_check_waits_for_the_gpu():
+    import threading
+    import time
+    from torchgt_b200 import SparseGraph
+    ei = random_graph(8, 300, 5.0).cuda()
+    SparseGraph(ei, 300).check()                      # everything is loaded
+    stop, ticks = threading.Event(), []
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.001)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(400_000_000)                # about 0.2 s of the GPU
+        graph = SparseGraph(ei, 300)
+        before = time.perf_counter()
+        graph.check()
+        after = time.perf_counter()
+    finally:
+        stop.set()
+        thread.join()
+    assert after - before > 0.05
+    assert sum(before < t < after for t in ticks) >= 10

@@ -121,9 +121,11 @@ Layout::Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by_) : gr
     slot_ = check_words().take(edge_index.device().index());
     if (slot_ >= 0) {
       const auto w = check_words().at(slot_);
-      check_cuda(cudaMemcpyAsync(w.host, bad_index.data_ptr(), 4, cudaMemcpyDeviceToHost,
-                                 static_cast<cudaStream_t>(stream)), "cudaMemcpyAsync");
-      check_cuda(cudaEventRecord(w.event, static_cast<cudaStream_t>(stream)), "cudaEventRecord");
+      cudaError_t e = cudaMemcpyAsync(w.host, bad_index.data_ptr(), 4, cudaMemcpyDeviceToHost,
+                                      static_cast<cudaStream_t>(stream));
+      if (e == cudaSuccess) e = cudaEventRecord(w.event, static_cast<cudaStream_t>(stream));
+      if (e != cudaSuccess) check_words().give_back(slot_);   // no destructor runs after a throw
+      check_cuda(e, "copy of the range check's result");
     }
   }
 }
@@ -138,28 +140,48 @@ void Layout::settle(bool bad) {
     check_words().give_back(slot_);
     slot_ = -1;
   }
-  if (bad)
+}
+
+bool Layout::settled() const {
+  if (state_ == kBad)
     throw TgtFailure(TGT_ERR_INDEX_RANGE, "edge_index holds a node id outside [0, " + std::to_string(c.n_rows) + ")");
+  return state_ == kGood;
 }
 
 void Layout::poll() {
-  if (state_ == kGood) return;
-  if (state_ == kBad) settle(true);
-  if (slot_ < 0 || capturing(ptr)) return;
+  std::lock_guard<std::mutex> lock(mutex_);
+  if (settled() || slot_ < 0 || capturing(ptr)) return;
   const auto w = check_words().at(slot_);
   const cudaError_t e = cudaEventQuery(w.event);
-  if (e == cudaSuccess) return settle(*static_cast<volatile int32_t*>(w.host) != 0);
+  if (e == cudaSuccess) {
+    settle(*static_cast<volatile int32_t*>(w.host) != 0);
+    settled();
+    return;
+  }
   if (e != cudaErrorNotReady) check_cuda(e, "cudaEventQuery");
   cudaGetLastError();
 }
 
 void Layout::verify() {
-  if (state_ == kGood) return;
-  if (state_ == kBad) settle(true);
-  if (slot_ < 0) return settle(bad_index.item<int32_t>() != 0);
-  const auto w = check_words().at(slot_);
-  check_cuda(cudaEventSynchronize(w.event), "cudaEventSynchronize");
-  settle(*static_cast<volatile int32_t*>(w.host) != 0);
+  int slot;
+  {
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (settled()) return;
+    slot = slot_;
+  }
+  // waits without the lock; while the state is pending the word and its event belong to this layout, and whoever
+  // settles it first is believed
+  bool bad = false;
+  CheckWords::Word w;
+  if (slot < 0) {
+    bad = bad_index.item<int32_t>() != 0;
+  } else {
+    w = check_words().at(slot);
+    check_cuda(cudaEventSynchronize(w.event), "cudaEventSynchronize");
+  }
+  std::lock_guard<std::mutex> lock(mutex_);
+  if (state_ == kPending) settle(slot < 0 ? bad : *static_cast<volatile int32_t*>(w.host) != 0);
+  settled();
 }
 
 Graph::Graph(const at::Tensor& edge_index, int64_t rows)
@@ -167,17 +189,23 @@ Graph::Graph(const at::Tensor& edge_index, int64_t rows)
       by_dst_(std::make_shared<Layout>(edge_index, rows, 1)) {}
 
 std::shared_ptr<Layout> Graph::by_src() {
+  at::Tensor done;   // outlives the lock: a tensor that Python has seen takes the interpreter lock on its way out
   std::lock_guard<std::mutex> lock(mutex_);
   if (!by_src_) {
     by_src_ = std::make_shared<Layout>(edge_index_, n_rows, 0);
-    edge_index_.reset();
+    done = std::move(edge_index_);
   }
+  return by_src_;
+}
+
+std::shared_ptr<Layout> Graph::built_by_src() {
+  std::lock_guard<std::mutex> lock(mutex_);   // an autograd thread may be building it
   return by_src_;
 }
 
 void Graph::poll() {
   by_dst_->poll();
-  if (by_src_) by_src_->poll();
+  if (const auto by_src = built_by_src()) by_src->poll();
 }
 
 size_t Graph::scratch_bytes(int heads, int head_dim, int dtype, int phase) {
@@ -345,10 +373,10 @@ PYBIND11_MODULE(_native, m) {
     }
   });
   py::class_<Layout, std::shared_ptr<Layout>>(m, "Layout")
-      .def(py::init<const at::Tensor&, int64_t, int>())
-      .def("poll", &Layout::poll)
-      .def("verify", &Layout::verify)
-      .def_property_readonly("verified", &Layout::verified)
+      .def(py::init<const at::Tensor&, int64_t, int>(), Unlocked())
+      .def("poll", &Layout::poll, Unlocked())
+      .def("verify", &Layout::verify, Unlocked())
+      .def_property_readonly("verified", py::cpp_function(&Layout::verified, Unlocked()))
       .def_readonly("ptr", &Layout::ptr)
       .def_readonly("other", &Layout::other)
       .def_readonly("perm", &Layout::perm)
@@ -356,15 +384,15 @@ PYBIND11_MODULE(_native, m) {
       .def_readonly("bad_index", &Layout::bad_index)
       .def_readonly("group_by", &Layout::group_by);
   py::class_<Graph, std::shared_ptr<Graph>>(m, "Graph")
-      .def(py::init<const at::Tensor&, int64_t>())
+      .def(py::init<const at::Tensor&, int64_t>(), Unlocked())
       .def("by_dst", &Graph::by_dst)
-      .def("by_src", &Graph::by_src)
-      .def("has_by_src", &Graph::has_by_src)
-      .def("poll", &Graph::poll);
-  m.def("take_gradients", &take_gradients);
-  m.def("attention", &attention);
-  m.def("attention_forward", &forward_pass);
-  m.def("attention_backward", &backward_pass);
+      .def("by_src", &Graph::by_src, Unlocked())
+      .def("has_by_src", &Graph::has_by_src, Unlocked())
+      .def("poll", &Graph::poll, Unlocked());
+  m.def("take_gradients", &take_gradients, Unlocked());
+  m.def("attention", &attention, Unlocked());
+  m.def("attention_forward", &forward_pass, Unlocked());
+  m.def("attention_backward", &backward_pass, Unlocked());
   bind_batching(m);
   bind_dense(m);
 }

@@ -24,10 +24,7 @@ Words read_back(const int64_t* device, int n, const at::Tensor& like) {
     throw TgtFailure(TGT_ERR_CUDA, "cudaHostAlloc failed");
   const auto stream = static_cast<cudaStream_t>(stream_of(like));
   cudaError_t e = cudaMemcpyAsync(pinned, device, size_t(n) * 8, cudaMemcpyDeviceToHost, stream);
-  if (e == cudaSuccess) {
-    pybind11::gil_scoped_release release;
-    e = cudaStreamSynchronize(stream);
-  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) throw TgtFailure(TGT_ERR_CUDA, cudaGetErrorString(e));
   Words w{};
   for (int i = 0; i < n; ++i) w.v[i] = pinned[i];
@@ -95,12 +92,12 @@ std::optional<at::Tensor> blocks(const at::Tensor& edge_index, int64_t n_nodes, 
 }  // namespace
 
 void bind_batching(pybind11::module_& m) {
-  m.def("batch", &batch);
-  m.def("blocks", &blocks);
+  m.def("batch", &batch, Unlocked());
+  m.def("blocks", &blocks, Unlocked());
   m.def("gather_rows", [](const at::Tensor& x, const at::Tensor& idx) {
     const c10::cuda::CUDAGuard guard(x.device());
     return gather_rows(x, idx);
-  });
+  }, Unlocked());
 }
 
 }  // namespace tgt_host

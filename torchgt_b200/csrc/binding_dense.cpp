@@ -214,9 +214,9 @@ at::Tensor layer_norm(const at::Tensor& x, const at::Tensor& w, const at::Tensor
 }  // namespace
 
 void bind_dense(pybind11::module_& m) {
-  m.def("linear", &linear);
-  m.def("layer_norm", &layer_norm);
-  m.def("add_layer_norm", &add_layer_norm);
+  m.def("linear", &linear, Unlocked());
+  m.def("layer_norm", &layer_norm, Unlocked());
+  m.def("add_layer_norm", &add_layer_norm, Unlocked());
 }
 
 }  // namespace tgt_host
