@@ -517,3 +517,14 @@ def test_a_traced_call_runs_again_on_other_inputs(with_bias):
             assert torch.equal(a, b)
         with torch.no_grad():
             assert torch.equal(traced(*args), want)
+
+
+def test_an_error_inside_the_backward_keeps_its_class_and_code():
+    from torchgt_b200 import SparseGraph, _cabi, sparse_graph_attention
+    ei = random_graph(3, 50, 4.0).cuda()
+    q, k, v = (torch.randn(50, 8, 8, device="cuda", requires_grad=True) for _ in range(3))
+    out = sparse_graph_attention(q, k, v, SparseGraph(ei, 50))
+    off_by_one = torch.randn(out.numel() + 1, device="cuda")[1:].view_as(out)   # the kernels take 16-byte aligned tensors
+    with pytest.raises(_cabi.TgtError, match="aligned") as info:
+        out.backward(off_by_one)
+    assert info.value.code == 1                                                 # TGT_ERR_INVALID

@@ -6,12 +6,37 @@
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <pybind11/stl.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/utils/pybind.h>
 
 namespace py = pybind11;
 
 namespace tgt_host {
+
+namespace {
+// torchgt_b200._cabi.TgtError; kept for the life of the process
+PyObject* tgt_error(const TgtFailure& e, PyObject** type) {
+  static py::object* error = new py::object(py::module_::import("torchgt_b200._cabi").attr("TgtError"));
+  *type = error->ptr();
+  return (*error)(e.code, e.message).release().ptr();
+}
+}  // namespace
+
+void set_python_error(const TgtFailure& e) {
+  PyObject* type = nullptr;
+  PyObject* value = tgt_error(e, &type);
+  PyErr_SetObject(type, value);
+  Py_DECREF(value);
+}
+
+void throw_python_error(const TgtFailure& e) {
+  const py::gil_scoped_acquire gil;
+  set_python_error(e);
+  python_error error;
+  error.persist();
+  throw error;
+}
 
 void* stream_of(const at::Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
@@ -268,6 +293,9 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
   bool with_dbias = false;   // the statistics of the forward's output are read only then, so only then is it kept
 
   variable_list apply(variable_list&& grads) override {
+    return reporting([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
     if (!grads[0].defined()) return variable_list(4);
     const at::Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack();
     const bool want_dbias = with_dbias && task_should_compute_output(3);
@@ -363,13 +391,11 @@ void take_gradients(const std::vector<at::Tensor>& into, const std::vector<at::T
 
 PYBIND11_MODULE(_native, m) {
   using namespace tgt_host;
-  static py::object tgt_error = py::module_::import("torchgt_b200._cabi").attr("TgtError");
-  tgt_error.inc_ref();
   py::register_exception_translator([](std::exception_ptr p) {
     try {
       if (p) std::rethrow_exception(p);
     } catch (const TgtFailure& e) {
-      PyErr_SetObject(tgt_error.ptr(), tgt_error(e.code, e.message).ptr());
+      set_python_error(e);
     }
   });
   py::class_<Layout, std::shared_ptr<Layout>>(m, "Layout")

@@ -34,6 +34,20 @@ inline void check(int code) {
   if (code != TGT_OK) throw TgtFailure(code, tgt_last_error());
 }
 
+void set_python_error(const TgtFailure& e);                   // with the interpreter lock
+[[noreturn]] void throw_python_error(const TgtFailure& e);    // without
+
+// What a backward node runs in: an exception leaves it through PyTorch's engine, which hands on Python's exceptions as
+// they are and makes a plain RuntimeError of anything else.
+template <class F>
+auto reporting(F&& f) -> decltype(f()) {
+  try {
+    return f();
+  } catch (const TgtFailure& e) {
+    throw_python_error(e);
+  }
+}
+
 // Every entry that allocates, launches, waits or takes a mutex runs without the interpreter lock: other Python threads
 // (loaders, a prefetch) go on, and a thread that holds one of the mutexes never waits for one that holds the interpreter.
 using Unlocked = pybind11::call_guard<pybind11::gil_scoped_release>;

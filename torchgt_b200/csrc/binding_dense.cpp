@@ -42,6 +42,9 @@ struct NarrowLinearBackward : public torch::autograd::Node {
   bool has_bias = false;
 
   variable_list apply(variable_list&& grads) override {
+    return reporting([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
     if (!grads[0].defined()) return variable_list(3);
     const at::Tensor x_ = x.unpack(), w_ = weight.unpack();
     const c10::cuda::CUDAGuard guard(x_.device());
@@ -127,6 +130,9 @@ struct LayerNormRowsBackward : public torch::autograd::Node {
   bool with_residual = false;
 
   variable_list apply(variable_list&& grads) override {
+    return reporting([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
     const at::Tensor ds = with_residual ? grads[1] : at::Tensor();
     if (!grads[0].defined()) return {ds, ds, at::Tensor(), at::Tensor()};   // only x + residual was used
     const at::Tensor x = with_residual ? normalised.unpack(shared_from_this()) : normalised.unpack();
