@@ -528,3 +528,24 @@ def test_an_error_inside_the_backward_keeps_its_class_and_code():
     with pytest.raises(_cabi.TgtError, match="aligned") as info:
         out.backward(off_by_one)
     assert info.value.code == 1                                                 # TGT_ERR_INVALID
+
+
+def test_saved_tensor_hooks_see_everything_the_backward_keeps():
+    """Offloading what is saved to the host leaves the gradients' bits as they are."""
+    from torchgt_b200 import SparseGraph, sparse_graph_attention
+    ei = random_graph(3, 50, 4.0).cuda()
+    q, k, v = (torch.randn(50, 8, 8, device="cuda", requires_grad=True) for _ in range(3))
+    bias = torch.randn(ei.shape[1], device="cuda", requires_grad=True)
+    graph = SparseGraph(ei, 50)
+    want = torch.autograd.grad(sparse_graph_attention(q, k, v, graph, bias).square().sum(), (q, k, v, bias))
+    shapes = []
+
+    def pack(t):
+        shapes.append(tuple(t.shape))
+        return t.detach().cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        out = sparse_graph_attention(q, k, v, graph, bias)
+    assert sorted(shapes) == sorted([(50, 8, 8)] * 4 + [(50, 8), (ei.shape[1],)])   # q, k, v, out; sums of weights; bias
+    for a, b in zip(torch.autograd.grad(out.square().sum(), (q, k, v, bias)), want):
+        assert torch.equal(a, b)

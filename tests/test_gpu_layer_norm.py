@@ -152,3 +152,25 @@ def test_residual_addition_leaves_hooked_and_uncovered_norms_to_their_own_call()
     assert torch.equal(add_layer_norm(x, r, norm)[0], y)
     wide = LayerNorm(64).cuda().double()
     assert torch.equal(add_layer_norm(x.double(), r.double(), wide)[0], wide(x.double() + r.double()))
+
+
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_saved_tensor_hooks_see_everything_the_backward_keeps(with_residual):
+    """Offloading what is saved to the host leaves the gradients' bits as they are."""
+    from torchgt_b200.layer_norm import LayerNorm, add_layer_norm
+    norm = LayerNorm(64).cuda()
+    x, r = (torch.randn(37, 64, device="cuda", requires_grad=True) for _ in range(2))
+    inputs = [x, norm.weight, norm.bias] + ([r] if with_residual else [])
+    call = lambda: add_layer_norm(x, r, norm)[0] if with_residual else norm(x)
+    want = torch.autograd.grad(call().square().sum(), inputs)
+    shapes = []
+
+    def pack(t):
+        shapes.append(tuple(t.shape))
+        return t.detach().cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        y = call()
+    assert sorted(shapes) == sorted([(37, 64), (64,), (37, 2)])      # the norm's input, its weight, mean and deviation
+    for a, b in zip(torch.autograd.grad(y.square().sum(), inputs), want):
+        assert torch.equal(a, b)

@@ -287,8 +287,7 @@ using torch::autograd::variable_list;
 
 struct SparseGraphAttentionBackward : public torch::autograd::Node {
   std::shared_ptr<Graph> graph;
-  SavedVariable q, k, v, bias, out;
-  at::Tensor z;
+  SavedVariable q, k, v, bias, out, z;
   int dtype = 0;
   bool with_dbias = false;   // the statistics of the forward's output are read only then, so only then is it kept
 
@@ -297,7 +296,7 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
   }
   variable_list backward(const variable_list& grads) {
     if (!grads[0].defined()) return variable_list(4);
-    const at::Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack();
+    const at::Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack(), z_ = z.unpack();
     const bool want_dbias = with_dbias && task_should_compute_output(3);
     const at::Tensor out_ = want_dbias ? out.unpack(shared_from_this()) : at::Tensor();
     const at::AutoDispatchBelowADInplaceOrView below;
@@ -305,14 +304,14 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
     const at::Tensor dout = grads[0].contiguous();
     at::Tensor dq = at::empty_like(q_), dk = at::empty_like(k_), dv = at::empty_like(v_), dbias;
     if (want_dbias) dbias = at::empty_like(bias_);
-    attention_backward(*graph, dout, q_, k_, v_, bias_, out_, z, dq, dk, dv, dbias, int(q_.size(1)), int(q_.size(2)),
+    attention_backward(*graph, dout, q_, k_, v_, bias_, out_, z_, dq, dk, dv, dbias, int(q_.size(1)), int(q_.size(2)),
                        dtype);
     return {dq, dk, dv, dbias};
   }
   std::string name() const override { return "SparseGraphAttentionBackward"; }
   void release_variables() override {
     q.reset_data(); k.reset_data(); v.reset_data(); bias.reset_data(); out.reset_data();
-    z.reset();
+    z.reset_data();
   }
 };
 
@@ -345,7 +344,7 @@ at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::T
     node->k = SavedVariable(k, false);
     node->v = SavedVariable(v, false);
     node->bias = SavedVariable(bias, false);
-    node->z = z;
+    node->z = SavedVariable(z, false);
     torch::autograd::set_history(out, node);
     if (node->with_dbias) node->out = SavedVariable(out, true);
   }

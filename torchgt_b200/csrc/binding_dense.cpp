@@ -125,8 +125,7 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<
 // ---- LayerNorm, with the residual addition in front of it ------------------------------------------------------
 // Outputs: the normalised rows and, with a residual, x + residual.
 struct LayerNormRowsBackward : public torch::autograd::Node {
-  SavedVariable normalised, weight;   // the norm's input: x, or the output x + residual
-  at::Tensor stats;
+  SavedVariable normalised, weight, stats;   // the norm's input: x, or the output x + residual
   bool with_residual = false;
 
   variable_list apply(variable_list&& grads) override {
@@ -136,7 +135,7 @@ struct LayerNormRowsBackward : public torch::autograd::Node {
     const at::Tensor ds = with_residual ? grads[1] : at::Tensor();
     if (!grads[0].defined()) return {ds, ds, at::Tensor(), at::Tensor()};   // only x + residual was used
     const at::Tensor x = with_residual ? normalised.unpack(shared_from_this()) : normalised.unpack();
-    const at::Tensor w = weight.unpack();
+    const at::Tensor w = weight.unpack(), stats_ = stats.unpack();
     const at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard guard(x.device());
     const at::Tensor dy = kernel_ready(grads[0]), xc = kernel_ready(x), wc = kernel_ready(w);
@@ -147,7 +146,7 @@ struct LayerNormRowsBackward : public torch::autograd::Node {
     size_t bytes = 0;
     check(tgt_layer_norm_bwd_scratch_bytes(rows, int(hidden), &bytes));
     const at::Tensor scratch = at::empty({int64_t(bytes < 16 ? 16 : bytes)}, dy.options().dtype(at::kByte));
-    check(tgt_add_layer_norm_bwd(fptr(dy), dsum.defined() ? fptr(dsum) : nullptr, fptr(xc), fptr(wc), fptr(stats), rows,
+    check(tgt_add_layer_norm_bwd(fptr(dy), dsum.defined() ? fptr(dsum) : nullptr, fptr(xc), fptr(wc), fptr(stats_), rows,
                                  int(hidden), fptr(dx), fptr(dgamma), fptr(dbeta), scratch.data_ptr(), scratch.numel(),
                                  stream_of(dy)));
     return {dx, with_residual ? dx : at::Tensor(), dgamma, dbeta};
@@ -156,7 +155,7 @@ struct LayerNormRowsBackward : public torch::autograd::Node {
   void release_variables() override {
     normalised.reset_data();
     weight.reset_data();
-    stats.reset();
+    stats.reset_data();
   }
 };
 
@@ -200,7 +199,7 @@ std::pair<at::Tensor, std::optional<at::Tensor>> add_layer_norm(const at::Tensor
     auto node = std::shared_ptr<LayerNormRowsBackward>(new LayerNormRowsBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x, residual, w, b));
     node->with_residual = residual.defined();
-    node->stats = stats;
+    node->stats = SavedVariable(stats, false);
     node->weight = SavedVariable(w, false);
     if (residual.defined()) {
       torch::autograd::set_history(variable_list{y, sum}, node);
