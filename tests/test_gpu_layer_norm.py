@@ -174,3 +174,44 @@ def test_saved_tensor_hooks_see_everything_the_backward_keeps(with_residual):
     assert sorted(shapes) == sorted([(37, 64), (64,), (37, 2)])      # the norm's input, its weight, mean and deviation
     for a, b in zip(torch.autograd.grad(y.square().sum(), inputs), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("shape", [(3, 64), (2, 17, 96)])
+@pytest.mark.parametrize("outputs", ["norm", "sum", "both", "alone"])
+def test_second_order_gradients(shape, outputs):
+    """A gradient penalty against torch's norm in 64 bits, through the norm and through the residual stream.  Tolerance:
+    about ten roundings of 6e-8 per value, sums over up to 96 columns and three nested means: 1e-5 of the largest value."""
+    from torchgt_b200.layer_norm import LayerNorm, add_layer_norm
+    gen = torch.Generator().manual_seed(shape[-1])
+    x, r, a, b = (torch.randn(shape, generator=gen, dtype=torch.float64) for _ in range(4))
+    w, c = torch.rand(shape[-1], generator=gen, dtype=torch.float64) + 0.5, torch.randn(shape[-1], generator=gen, dtype=torch.float64)
+
+    def penalty(call, x, r, a, b, norm):
+        y, s = call(x, r, norm)
+        terms = {"norm": [y * a], "sum": [s.square() * b], "both": [y.sin() * a, s.square() * b], "alone": [y.sin() * a]}[outputs]
+        first = torch.autograd.grad(sum(t.sum() for t in terms), (x, r, norm.weight), create_graph=True, allow_unused=True)
+        kept = [g for g in first if g is not None]
+        wrt = (x, r, norm.weight)
+        second = torch.autograd.grad(sum(g.square().sum() for g in kept) + kept[0].sin().sum(), wrt, allow_unused=True)
+        return [*first, *second]
+
+    def torch_call(x, r, norm):
+        s = x if outputs == "alone" else x + r
+        return norm(s), s
+
+    def own_call(x, r, norm):
+        return (norm(x), x) if outputs == "alone" else add_layer_norm(x, r, norm)
+
+    results = []
+    for call, norm, device, dtype in ((torch_call, torch.nn.LayerNorm(shape[-1]), "cpu", torch.float64),
+                                      (own_call, LayerNorm(shape[-1]), "cuda", torch.float32)):
+        norm = norm.to(device, dtype)
+        with torch.no_grad():
+            norm.weight.copy_(w)
+            norm.bias.copy_(c)
+        xs = [t.to(device, dtype) for t in (x, r, a, b)]
+        results.append(penalty(call, xs[0].requires_grad_(), xs[1].requires_grad_(), xs[2], xs[3], norm))
+    for got, want in zip(results[1], results[0]):
+        assert (got is None) == (want is None)
+        if want is not None:
+            assert float((got.double().cpu() - want).abs().max()) <= 1e-5 * float(want.abs().max()) + 1e-12

@@ -127,6 +127,18 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<
 struct LayerNormRowsBackward : public torch::autograd::Node {
   SavedVariable normalised, weight, stats;   // the norm's input: x, or the output x + residual
   bool with_residual = false;
+  double eps = 0;
+
+  // With create_graph the gradient is itself differentiated: the formula as recorded operations.
+  variable_list recorded(const at::Tensor& dy, const at::Tensor& ds, const at::Tensor& x, const at::Tensor& w) {
+    const int64_t hidden = w.numel();
+    const at::Tensor d = x - x.mean(-1, true), rstd = (d * d).mean(-1, true).add(eps).rsqrt(), xhat = d * rstd;
+    const at::Tensor g = dy * w;
+    at::Tensor dx = rstd * (g - g.mean(-1, true) - xhat * (g * xhat).mean(-1, true));
+    if (ds.defined()) dx = dx + ds;
+    return {dx, with_residual ? dx : at::Tensor(), (dy * xhat).reshape({-1, hidden}).sum(0),
+            dy.reshape({-1, hidden}).sum(0)};
+  }
 
   variable_list apply(variable_list&& grads) override {
     return reporting([&] { return backward(grads); });
@@ -136,6 +148,7 @@ struct LayerNormRowsBackward : public torch::autograd::Node {
     if (!grads[0].defined()) return {ds, ds, at::Tensor(), at::Tensor()};   // only x + residual was used
     const at::Tensor x = with_residual ? normalised.unpack(shared_from_this()) : normalised.unpack();
     const at::Tensor w = weight.unpack(), stats_ = stats.unpack();
+    if (at::GradMode::is_enabled()) return recorded(grads[0], ds, x, w);
     const at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard guard(x.device());
     const at::Tensor dy = kernel_ready(grads[0]), xc = kernel_ready(x), wc = kernel_ready(w);
@@ -199,6 +212,7 @@ std::pair<at::Tensor, std::optional<at::Tensor>> add_layer_norm(const at::Tensor
     auto node = std::shared_ptr<LayerNormRowsBackward>(new LayerNormRowsBackward(), torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(x, residual, w, b));
     node->with_residual = residual.defined();
+    node->eps = eps;
     node->stats = SavedVariable(stats, false);
     node->weight = SavedVariable(w, false);
     if (residual.defined()) {
