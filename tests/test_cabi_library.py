@@ -67,3 +67,17 @@ def test_check_raises_with_the_library_message(lib):
     from torchgt_b200 import _cabi
     with pytest.raises(_cabi.TgtError, match="TGT_ERR_INVALID"):
         _cabi.check(lib.tgt_debug_set_tile_edges(-5))
+
+
+def test_the_batch_dispatch_sends_no_size_the_kernels_refuse(lib):
+    """gen_sub_edge_index and get_batch_reorder_blockize pick the device path by the limits of the C entries."""
+    from torchgt_b200.gt_sp import batching
+    n, limit = ctypes.c_size_t(), batching._MAX_CANDIDATES
+    for edges, nodes in ((0, 1), (limit - 11, 10), (limit - 10, 10), (10, limit - 11), (10, limit - 10), (2 ** 31, 1), (2 ** 40, 2 ** 30)):
+        accepted = lib.tgt_subgraph_workspace_bytes(edges, nodes, ctypes.byref(n)) == 0
+        assert batching._subgraph_fits(edges, nodes, 1) == accepted, (edges, nodes)
+    for batch in (0, batching._MAX_BATCH - 1, batching._MAX_BATCH):
+        # refused on n_idx, or accepted up to the null pointers behind it
+        assert lib.tgt_subgraph_count(None, 0, 10, None, batch, None, 0, None, None) == 1
+        assert batching._subgraph_fits(0, 10, batch) == (b"n_idx" not in lib.tgt_last_error())
+    assert not batching._subgraph_fits(0, 0, 1)

@@ -80,3 +80,17 @@ def test_training_batch(model, reorder, features, dtype):
             assert got[3] is None and get_last_batch_flag() == flag
             for a, b in zip(got[:3], want[:3]):
                 assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
+
+
+def test_lists_the_kernels_cannot_number_take_the_pytorch_formulation(monkeypatch):
+    from torchgt_b200.gt_sp import batching
+    edges, perm = _graph(5, 300, 2000)
+    want = batching.gen_sub_edge_index(edges, perm[:200], 300)
+    monkeypatch.setattr(batching, "_MAX_CANDIDATES", 2300)
+    monkeypatch.setattr(batching._cabi, "native", None)          # the kernels are out of reach
+    assert torch.equal(batching.gen_sub_edge_index(edges.cuda(), perm[:200].cuda(), 300).cpu(), want)
+    args = types.SimpleNamespace(seq_len=200, model="graphormer", reorder=False)
+    x, y = torch.randn(300, 4), torch.arange(300)
+    want = batching.get_batch_reorder_blockize(args, x, y, perm[:200], None, "cpu", edges, 300, 4, 8)
+    got = batching.get_batch_reorder_blockize(args, x.cuda(), y.cuda(), perm[:200].cuda(), None, "cuda", edges.cuda(), 300, 4, 8)
+    assert all(torch.equal(a.cpu(), b) for a, b in zip(got[:3], want[:3]))

@@ -70,13 +70,21 @@ def _on_device(edge_index, *ids) -> bool:
             all(t.device == edge_index.device and t.dtype == torch.int64 and t.dim() == 1 for t in ids))
 
 
+_MAX_CANDIDATES, _MAX_BATCH = 2 ** 31 - 2048, 2 ** 30    # the sub-graph kernels number edges and nodes in 32 bits
+
+
+def _subgraph_fits(n_edges: int, n_nodes: int, n_batch: int) -> bool:
+    """Do the sub-graph kernels take these sizes?  (Larger lists take the PyTorch formulation.)"""
+    return 0 < n_nodes and n_edges + n_nodes < _MAX_CANDIDATES and n_batch < _MAX_BATCH
+
+
 # ---- induced sub-graph of a batch (gt_sp/utils.py:202-215) --------------------------------------------
 def gen_sub_edge_index(edge_index: Tensor, idx_batch: Tensor, N: int) -> Tensor:
     """Edges among the nodes ``idx_batch`` of the whole graph, renumbered by position in ``idx_batch``:
     existing self loops are dropped, one self loop per node is added, and the kept columns keep their
     order (original edges first, then the self loops in node-id order)."""
     idx_batch = idx_batch.to(edge_index.device)
-    if _on_device(edge_index, idx_batch) and N > 0:
+    if _on_device(edge_index, idx_batch) and _subgraph_fits(edge_index.shape[1], N, idx_batch.shape[0]):
         return _cabi.native().batch(edge_index.contiguous(), idx_batch.contiguous(), N, False, 0, [], 0, 0)[0]
     src, dst = edge_index[0], edge_index[1]
     keep = src != dst                                              # remove_self_loops
@@ -273,7 +281,8 @@ def get_batch_reorder_blockize(args, x: Tensor, y: Tensor, idx_batch: Tensor, re
     seq_length = args.seq_len
     n = idx_batch.shape[0]
     reorder = bool(getattr(args, "reorder", False))
-    if (n > 0 and _on_device(edge_index, idx_batch) and N > 0 and not (reorder and world > 1) and
+    if (n > 0 and _on_device(edge_index, idx_batch) and _subgraph_fits(edge_index.shape[1], N, n) and
+            not (reorder and world > 1) and
             (rest_split_sizes is not None if n < seq_length else seq_length % world == 0) and
             all(t.device == edge_index.device and t.is_contiguous() and not t.requires_grad and t.dim() == d and
                 t.shape[0] == N for t, d in ((x, 2), (y, 1)))):
