@@ -87,10 +87,29 @@ def test_lists_the_kernels_cannot_number_take_the_pytorch_formulation(monkeypatc
     edges, perm = _graph(5, 300, 2000)
     want = batching.gen_sub_edge_index(edges, perm[:200], 300)
     monkeypatch.setattr(batching, "_MAX_CANDIDATES", 2300)
-    monkeypatch.setattr(batching._cabi, "native", None)          # the kernels are out of reach
+    no_kernels = types.SimpleNamespace(plain=lambda tensors: True)
+    monkeypatch.setattr(batching._cabi, "native", lambda: no_kernels)
     assert torch.equal(batching.gen_sub_edge_index(edges.cuda(), perm[:200].cuda(), 300).cpu(), want)
     args = types.SimpleNamespace(seq_len=200, model="graphormer", reorder=False)
     x, y = torch.randn(300, 4), torch.arange(300)
     want = batching.get_batch_reorder_blockize(args, x, y, perm[:200], None, "cpu", edges, 300, 4, 8)
     got = batching.get_batch_reorder_blockize(args, x.cuda(), y.cuda(), perm[:200].cuda(), None, "cuda", edges.cuda(), 300, 4, 8)
     assert all(torch.equal(a.cpu(), b) for a, b in zip(got[:3], want[:3]))
+
+
+def test_a_traced_sub_graph_runs_again_on_other_batches():
+    from torchgt_b200.gt_sp.batching import gen_sub_edge_index
+    edges, perm = _graph(5, 300, 2000)
+    edges, perm = edges.cuda(), perm.cuda()
+    traced = torch.jit.trace(lambda e, i: gen_sub_edge_index(e, i, 300), (edges, perm[:200]), check_trace=False)
+    for idx in (perm[100:], perm[:50]):
+        assert torch.equal(traced(edges, idx), gen_sub_edge_index(edges, idx, 300))
+
+
+def test_features_with_a_pending_conjugation():
+    from torchgt_b200.gt_sp.batching import get_batch_reorder_blockize
+    edges, perm = _graph(5, 300, 2000)
+    x, y = torch.randn(300, 4, dtype=torch.complex64), torch.arange(300)
+    args = types.SimpleNamespace(seq_len=200, model="graphormer", reorder=False)
+    got = get_batch_reorder_blockize(args, x.cuda().conj(), y.cuda(), perm[:200].cuda(), None, "cuda", edges.cuda(), 300, 4, 8)
+    assert torch.equal(got[0].cpu(), x[perm[:200]].conj())

@@ -2,6 +2,7 @@
 // the launches.
 #include "binding.h"
 
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/utils/pybind.h>
@@ -91,7 +92,16 @@ std::optional<at::Tensor> blocks(const at::Tensor& edge_index, int64_t n_nodes, 
 
 }  // namespace
 
+// strided tensors whose memory is theirs to read: no wrapper of a transform, no dispatch mode above, no pending
+// conjugation or negation
+bool plain(const std::vector<at::Tensor>& tensors) {
+  for (const at::Tensor& t : tensors)
+    if (at::isTensorSubclassLike(t) || t.layout() != at::kStrided || t.is_conj() || t.is_neg()) return false;
+  return true;
+}
+
 void bind_batching(pybind11::module_& m) {
+  m.def("plain", &plain);
   m.def("batch", &batch, Unlocked());
   m.def("blocks", &blocks, Unlocked());
   m.def("gather_rows", [](const at::Tensor& x, const at::Tensor& idx) {

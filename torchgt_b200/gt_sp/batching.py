@@ -25,6 +25,7 @@ import numpy as np
 import torch
 import torch.distributed as dist
 from torch import Tensor
+from torch.overrides import has_torch_function_variadic
 
 from .. import _cabi
 from .initialize import (get_sequence_parallel_group, get_sequence_parallel_rank, get_sequence_parallel_src_rank,
@@ -63,11 +64,19 @@ def random_split_idx(data_y, frac_train: float, frac_valid: float, frac_test: fl
     return {"train": torch.tensor(all_idx[:a]), "valid": torch.tensor(all_idx[a:b]), "test": torch.tensor(all_idx[b:])}
 
 
+def _kernels_may_take(*tensors) -> bool:
+    """Nobody records or intercepts the operations on these CUDA tensors, and their memory holds their values: a
+    tracer would keep the allocation of a result and not the kernel that fills it."""
+    return not (torch.compiler.is_compiling() or torch.jit.is_tracing() or has_torch_function_variadic(*tensors)) and \
+        _cabi.native().plain(tensors)
+
+
 def _on_device(edge_index, *ids) -> bool:
     """Can the kernels take this edge list and these id lists?"""
     return (isinstance(edge_index, Tensor) and edge_index.is_cuda and edge_index.dtype == torch.int64 and
             edge_index.dim() == 2 and edge_index.shape[0] == 2 and
-            all(t.device == edge_index.device and t.dtype == torch.int64 and t.dim() == 1 for t in ids))
+            all(t.device == edge_index.device and t.dtype == torch.int64 and t.dim() == 1 for t in ids) and
+            _kernels_may_take(edge_index, *ids))
 
 
 _MAX_CANDIDATES, _MAX_BATCH = 2 ** 31 - 2048, 2 ** 30    # the sub-graph kernels number edges and nodes in 32 bits
@@ -285,7 +294,7 @@ def get_batch_reorder_blockize(args, x: Tensor, y: Tensor, idx_batch: Tensor, re
             not (reorder and world > 1) and
             (rest_split_sizes is not None if n < seq_length else seq_length % world == 0) and
             all(t.device == edge_index.device and t.is_contiguous() and not t.requires_grad and t.dim() == d and
-                t.shape[0] == N for t, d in ((x, 2), (y, 1)))):
+                t.shape[0] == N for t, d in ((x, 2), (y, 1))) and _kernels_may_take(x, y)):
         per_rank = max(rest_split_sizes) if n < seq_length else seq_length // world
         x_i, y_i, edge_index_i = _device_batch(x, y, idx_batch, edge_index, N, k, block_size, args.model == "graphormer",
                                                reorder, min(rank * per_rank, n), min((rank + 1) * per_rank, n), per_rank)
