@@ -113,3 +113,23 @@ def test_features_with_a_pending_conjugation():
     args = types.SimpleNamespace(seq_len=200, model="graphormer", reorder=False)
     got = get_batch_reorder_blockize(args, x.cuda().conj(), y.cuda(), perm[:200].cuda(), None, "cuda", edges.cuda(), 300, 4, 8)
     assert torch.equal(got[0].cpu(), x[perm[:200]].conj())
+
+
+def test_block_generator_with_ids_outside_the_nodes_and_the_partitions():
+    """What numpy's indexing makes of them: negative ids count from the end, a partition that no edge mentions may lie
+    beyond k, an id beyond the nodes is an error."""
+    from torchgt_b200.gt_sp.batching import contiguous_partition, generate_new_edges_optimized
+    edges, _ = _graph(11, 200, 900)
+    part = contiguous_partition(edges, 200, 4)
+    mapping = np.arange(200)
+    negative, alone, beyond = edges.clone(), part.clone(), edges.clone()
+    negative[0, :50] -= 200
+    edges_without_7 = edges[:, (edges != 7).all(0)]
+    alone[7] = 4
+    for e, p in ((negative, part), (edges_without_7, alone)):
+        want = generate_new_edges_optimized(e, 4, p, 1, 8, mapping)
+        assert torch.equal(generate_new_edges_optimized(e.cuda(), 4, p, 1, 8, mapping).cpu(), want)
+    beyond[1, 5] = 200
+    for e in (beyond, beyond.cuda()):
+        with pytest.raises(IndexError):
+            generate_new_edges_optimized(e, 4, part, 1, 8, mapping)

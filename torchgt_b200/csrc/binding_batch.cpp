@@ -69,7 +69,9 @@ std::vector<at::Tensor> batch(const at::Tensor& edge_index, const at::Tensor& id
   return out;
 }
 
-// The block generator's edges, or None where some pair of partitions keeps its original edges (or there are 2^31 blocks).
+// The block generator's edges, or None where the numpy formulation has to answer: some pair of partitions keeps its
+// original edges, an id lies outside the nodes or the partitions (it counts from the end, has no edges, or is an
+// error), or there are 2^31 blocks.
 std::optional<at::Tensor> blocks(const at::Tensor& edge_index, int64_t n_nodes, const std::optional<at::Tensor>& partition,
                                  int k, double p, int64_t block, bool by_source, int64_t sub_seq_len) {
   const c10::cuda::CUDAGuard guard(edge_index.device());
@@ -80,8 +82,7 @@ std::optional<at::Tensor> blocks(const at::Tensor& edge_index, int64_t n_nodes, 
   check(tgt_blocks_plan(ids(edge_index), edge_index.size(1), n_nodes, partition.has_value() ? ids(*partition) : nullptr, k,
                         p, block, ws.data_ptr(), ws.numel(), &result, stream_of(edge_index)));
   const Words w = read_back(result, 4, edge_index);
-  if (w.v[3] != 0) bad_id(n_nodes);
-  if (w.v[2] != 0 || w.v[0] >= (int64_t(1) << 31) - 1) return std::nullopt;   // blocks are numbered in 32 bits
+  if (w.v[2] != 0 || w.v[3] != 0 || w.v[0] >= (int64_t(1) << 31) - 1) return std::nullopt;
   at::Tensor out = at::empty({2, w.v[0] * block * block}, edge_index.options());
   check(tgt_blocks_list_bytes(w.v[0], &need));
   at::Tensor list = bytes_like(edge_index, need);

@@ -191,7 +191,8 @@ def _device_blocks(edge_index, num_nodes: int, partition: Optional[Tensor], k: i
                    sub_seq_len: int) -> Optional[Tensor]:
     """The generator's result from the kernels: pair by pair, or sorted by source (stable) with ``by_source``, ids
     moved past the per-rank token slots for ``sub_seq_len`` > 0.  ``partition`` None: contiguous equal ranges.
-    None when the edges are not on a GPU or some pair of partitions keeps its original edges."""
+    None when the edges are not on a GPU, some pair of partitions keeps its original edges or an id is not one of
+    0 .. ``num_nodes`` - 1 (a partition's: 0 .. ``k`` - 1)."""
     if not _on_device(edge_index) or not (0 < num_nodes < 2 ** 31 - 1 and 1 <= k <= 8192 and 1 <= block <= 32768):
         return None
     if partition is not None:
