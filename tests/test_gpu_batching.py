@@ -133,3 +133,20 @@ def test_block_generator_with_ids_outside_the_nodes_and_the_partitions():
     for e in (beyond, beyond.cuda()):
         with pytest.raises(IndexError):
             generate_new_edges_optimized(e, 4, part, 1, 8, mapping)
+
+
+def test_threads_that_build_batches_leave_no_pinned_memory_behind():
+    import threading
+    from torchgt_b200.gt_sp.batching import gen_sub_edge_index
+    edges, perm = _graph(5, 300, 2000)
+    edges, idx, results = edges.cuda(), perm[:200].cuda(), []
+    results.append(gen_sub_edge_index(edges, idx, 300))
+    before = torch.cuda.host_memory_stats()
+    for _ in range(100):
+        thread = threading.Thread(target=lambda: results.append(gen_sub_edge_index(edges, idx, 300)))
+        thread.start()
+        thread.join()
+    after = torch.cuda.host_memory_stats()
+    assert all(torch.equal(r, results[0]) for r in results) and len(results) == 101
+    assert after["active_requests.allocated"] >= before["active_requests.allocated"] + 100    # each call asked the pool,
+    assert after["num_host_alloc"] == before["num_host_alloc"]                                  # which had what it needs

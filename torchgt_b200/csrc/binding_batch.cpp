@@ -19,12 +19,11 @@ at::Tensor bytes_like(const at::Tensor& t, size_t n) {
 // The first `n` result words of a pass, on the host (waits for the pass).
 struct Words { int64_t v[4]; };
 Words read_back(const int64_t* device, int n, const at::Tensor& like) {
-  // one small pinned buffer per thread: no page is pinned per call and nothing is shared between threads
-  thread_local int64_t* pinned = nullptr;
-  if (pinned == nullptr && cudaHostAlloc(reinterpret_cast<void**>(&pinned), sizeof(Words), cudaHostAllocPortable) != cudaSuccess)
-    throw TgtFailure(TGT_ERR_CUDA, "cudaHostAlloc failed");
+  // from PyTorch's pool of pinned memory: nothing is pinned per call, nor kept by a thread that has ended
+  const at::Tensor host = at::empty({4}, at::TensorOptions().dtype(at::kLong).pinned_memory(true));
+  const int64_t* pinned = host.const_data_ptr<int64_t>();
   const auto stream = static_cast<cudaStream_t>(stream_of(like));
-  cudaError_t e = cudaMemcpyAsync(pinned, device, size_t(n) * 8, cudaMemcpyDeviceToHost, stream);
+  cudaError_t e = cudaMemcpyAsync(host.data_ptr(), device, size_t(n) * 8, cudaMemcpyDeviceToHost, stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) throw TgtFailure(TGT_ERR_CUDA, cudaGetErrorString(e));
   Words w{};
