@@ -174,6 +174,7 @@ bool Layout::settled() const {
 }
 
 void Layout::poll() {
+  if (state_.load(std::memory_order_acquire) == kGood) return;   // every call but a graph's first few
   std::lock_guard<std::mutex> lock(mutex_);
   if (settled() || slot_ < 0 || capturing(ptr)) return;
   const auto w = check_words().at(slot_);
@@ -218,19 +219,15 @@ std::shared_ptr<Layout> Graph::by_src() {
   std::lock_guard<std::mutex> lock(mutex_);
   if (!by_src_) {
     by_src_ = std::make_shared<Layout>(edge_index_, n_rows, 0);
+    built_.store(by_src_.get(), std::memory_order_release);
     done = std::move(edge_index_);
   }
   return by_src_;
 }
 
-std::shared_ptr<Layout> Graph::built_by_src() {
-  std::lock_guard<std::mutex> lock(mutex_);   // an autograd thread may be building it
-  return by_src_;
-}
-
 void Graph::poll() {
   by_dst_->poll();
-  if (const auto by_src = built_by_src()) by_src->poll();
+  if (Layout* by_src = built_.load(std::memory_order_acquire)) by_src->poll();
 }
 
 size_t Graph::scratch_bytes(int heads, int head_dim, int dtype, int phase) {
@@ -399,9 +396,9 @@ PYBIND11_MODULE(_native, m) {
   });
   py::class_<Layout, std::shared_ptr<Layout>>(m, "Layout")
       .def(py::init<const at::Tensor&, int64_t, int>(), Unlocked())
-      .def("poll", &Layout::poll, Unlocked())
+      .def("poll", &Layout::poll)   // waits for nothing, and nobody waits for the interpreter under its mutex
       .def("verify", &Layout::verify, Unlocked())
-      .def_property_readonly("verified", py::cpp_function(&Layout::verified, Unlocked()))
+      .def_property_readonly("verified", &Layout::verified)
       .def_readonly("ptr", &Layout::ptr)
       .def_readonly("other", &Layout::other)
       .def_readonly("perm", &Layout::perm)
@@ -412,8 +409,8 @@ PYBIND11_MODULE(_native, m) {
       .def(py::init<const at::Tensor&, int64_t>(), Unlocked())
       .def("by_dst", &Graph::by_dst)
       .def("by_src", &Graph::by_src, Unlocked())
-      .def("has_by_src", &Graph::has_by_src, Unlocked())
-      .def("poll", &Graph::poll, Unlocked());
+      .def("has_by_src", &Graph::has_by_src)
+      .def("poll", &Graph::poll);
   m.def("take_gradients", &take_gradients, Unlocked());
   m.def("attention", &attention, Unlocked());
   m.def("attention_forward", &forward_pass, Unlocked());

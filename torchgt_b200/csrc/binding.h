@@ -12,6 +12,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
 
+#include <atomic>
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -48,7 +49,7 @@ auto reporting(F&& f) -> decltype(f()) {
   }
 }
 
-// Every entry that allocates, launches, waits or takes a mutex runs without the interpreter lock: other Python threads
+// Every entry that allocates, launches, waits or takes a mutex others allocate under runs without the interpreter lock: other Python threads
 // (loaders, a prefetch) go on, and a thread that holds one of the mutexes never waits for one that holds the interpreter.
 using Unlocked = pybind11::call_guard<pybind11::gil_scoped_release>;
 
@@ -68,10 +69,7 @@ class Layout {
 
   void poll();     // throws if the build is known to have seen a bad node id; never waits
   void verify();   // waits for the build first
-  bool verified() {
-    std::lock_guard<std::mutex> lock(mutex_);
-    return state_ == kGood;
-  }
+  bool verified() const { return state_ == kGood; }
 
   tgt_layout c{};
   at::Tensor ptr, other, perm, seg, bad_index;
@@ -82,7 +80,7 @@ class Layout {
   void settle(bool bad);
   bool settled() const;   // throws if the build saw a bad id
   std::mutex mutex_;      // of the two below: calls come from Python's threads and from autograd's
-  State state_ = kPending;
+  std::atomic<State> state_{kPending};
   int slot_ = -1;   // pinned word and event of a pending check (-1: none, the device word is read instead)
 };
 
@@ -92,17 +90,17 @@ class Graph {
   Graph(const at::Tensor& edge_index, int64_t n_rows);
   std::shared_ptr<Layout> by_dst() const { return by_dst_; }
   std::shared_ptr<Layout> by_src();
-  bool has_by_src() { return built_by_src() != nullptr; }
+  bool has_by_src() const { return built_ != nullptr; }
   void poll();
   // bytes of scratch the attention kernels need (asked from the library once per shape and phase)
   size_t scratch_bytes(int heads, int head_dim, int dtype, int phase);
   int64_t n_rows, n_edges;
 
  private:
-  std::shared_ptr<Layout> built_by_src();   // null before its first use
   std::mutex mutex_;
   at::Tensor edge_index_;   // kept until by_src is built
   std::shared_ptr<Layout> by_dst_, by_src_;
+  std::atomic<Layout*> built_{nullptr};   // by_src_ once it is there, for whoever must not wait for its construction
   struct Need { int heads, head_dim, dtype, phase; size_t bytes; };
   std::vector<Need> needs_;
 };
