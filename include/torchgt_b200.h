@@ -99,10 +99,12 @@ TGT_API int tgt_debug_set_lane_mode(int mode);
 TGT_API int tgt_debug_set_dependent_launch(int links);
 
 /*
- * Bytes of device workspace tgt_edge_layout_build needs.
+ * Bytes of device workspace tgt_edge_layout_build needs (enough for tgt_edge_layout_build_i32 as well, which
+ * is content with the 4 bytes per edge less of tgt_edge_layout_sizes_i32).
  * Replaces nothing in the reference (the reference keeps edges as an unsorted COO list).
  */
 TGT_API int tgt_edge_layout_sizes(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes);
+TGT_API int tgt_edge_layout_sizes_i32(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes);
 
 /*
  * Build one segment layout from the COO edge list the reference's batch packing produces

@@ -241,3 +241,48 @@ def test_other_threads_run_while_a_layout_check_waits_for_the_gpu():
         thread.join()
     assert after - before > 0.05
     assert sum(before < t < after for t in ticks) >= 10
+
+
+@pytest.mark.parametrize("n_edges", [1, 64, 65, 5000])
+def test_an_int32_list_needs_no_workspace_for_a_narrow_copy(n_edges):
+    """Its build fits the smaller size, to the byte, and gives the arrays of the int64 list."""
+    import ctypes
+    from torchgt_b200 import _cabi
+    lib, n_rows = _cabi.load(), 300
+    wide, narrow = ctypes.c_size_t(), ctypes.c_size_t()
+    _cabi.check(lib.tgt_edge_layout_sizes(n_rows, n_edges, ctypes.byref(wide)))
+    _cabi.check(lib.tgt_edge_layout_sizes_i32(n_rows, n_edges, ctypes.byref(narrow)))
+    assert wide.value - narrow.value == (4 * n_edges + 255) // 256 * 256
+    edges = torch.randint(0, n_rows, (2, n_edges), generator=torch.Generator().manual_seed(n_edges))
+    i32 = edges.int().cuda()
+    workspace = torch.full((narrow.value + 4096,), 171, dtype=torch.uint8, device="cuda")
+    ptr = torch.empty(n_rows + 1, dtype=torch.int32, device="cuda")
+    other, perm, seg = (torch.empty(n_edges, dtype=torch.int32, device="cuda") for _ in range(3))
+    for group_by in (0, 1):
+        args = (i32.data_ptr(), n_edges, n_rows, group_by, ptr.data_ptr(), other.data_ptr(), perm.data_ptr(), seg.data_ptr(),
+                workspace.data_ptr())
+        assert lib.tgt_edge_layout_build_i32(*args, narrow.value - 1, None, None) == 4     # TGT_ERR_WORKSPACE
+        torch.cuda.synchronize()
+        _cabi.check(lib.tgt_edge_layout_build_i32(*args, narrow.value, None, torch.cuda.current_stream().cuda_stream))
+        assert (workspace[narrow.value:] == 171).all()
+        want = elo.segment_layout(edges.numpy(), n_rows, group_by)
+        for got, ref in zip((ptr, other, perm), want):
+            assert np.array_equal(got.cpu().numpy().astype(np.int64), ref)
+
+
+def test_a_graph_from_an_int32_list_allocates_no_narrow_copy():
+    import ctypes
+    from torchgt_b200 import _cabi
+    from torchgt_b200.graph import SparseGraph
+    n_rows, n_edges = 1000, 4_000_000
+    edges = torch.randint(0, n_rows, (2, n_edges), dtype=torch.int32, device="cuda")
+    need = ctypes.c_size_t()
+    _cabi.check(_cabi.load().tgt_edge_layout_sizes_i32(n_rows, n_edges, ctypes.byref(need)))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    graph = SparseGraph(edges, n_rows)
+    graph.check()
+    # other, perm, seg and the workspace; a megabyte of rounding per allocation is below the 16 MB of a copy
+    assert torch.cuda.max_memory_allocated() - before < 3 * 4 * n_edges + need.value + (6 << 20)

@@ -57,6 +57,7 @@ SIGNATURES = {
     "tgt_last_error": (c_char_p, []),
     "tgt_debug_set_tile_edges": (c_int, [c_int]),
     "tgt_edge_layout_sizes": (c_int, [c_int64, c_int64, POINTER(c_size_t)]),
+    "tgt_edge_layout_sizes_i32": (c_int, [c_int64, c_int64, POINTER(c_size_t)]),
     "tgt_edge_layout_build": (c_int, [c_void_p, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "tgt_edge_layout_build_i32": (c_int, [c_void_p, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p,

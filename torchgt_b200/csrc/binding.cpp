@@ -117,7 +117,7 @@ CheckWords& check_words() {
 Layout::Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by_) : group_by(group_by_) {
   const int64_t n_edges = edge_index.size(1);
   size_t ws = 0;
-  check(tgt_edge_layout_sizes(n_rows, n_edges, &ws));
+  check((edge_index.scalar_type() == at::kLong ? tgt_edge_layout_sizes : tgt_edge_layout_sizes_i32)(n_rows, n_edges, &ws));
   const c10::cuda::CUDAGuard guard(edge_index.device());
   const auto i32 = edge_index.options().dtype(at::kInt);
   ptr = at::empty({n_rows + 1}, i32);

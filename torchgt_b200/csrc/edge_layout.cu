@@ -82,7 +82,8 @@ struct Workspace {
   size_t keys, iota, narrow, flag, cub, total, cub_bytes;
 };
 
-int plan_workspace(int64_t n_rows, int64_t n_edges, Workspace* w) {
+// `wide`: the list is int64, and a narrow copy of it is made (extract_keys_kernel).
+int plan_workspace(int64_t n_rows, int64_t n_edges, bool wide, Workspace* w) {
   size_t sort_bytes = 0;
   if (n_edges > 0) {
     cudaError_t e = cub::DeviceRadixSort::SortPairs(
@@ -96,7 +97,7 @@ int plan_workspace(int64_t n_rows, int64_t n_edges, Workspace* w) {
   size_t off = 0;
   w->keys = off; off += e4;
   w->iota = off; off += e4;
-  w->narrow = off; off += e4;
+  w->narrow = off; off += wide ? e4 : 0;
   w->flag = off; off += 256;
   w->cub = off;
   w->cub_bytes = round_up(sort_bytes, 256) + 256;
@@ -105,24 +106,17 @@ int plan_workspace(int64_t n_rows, int64_t n_edges, Workspace* w) {
   return TGT_OK;
 }
 
-}  // namespace
-}  // namespace tgt
-
-extern "C" int tgt_edge_layout_sizes(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes) {
-  using namespace tgt;
+int workspace_size(int64_t n_rows, int64_t n_edges, bool wide, size_t* workspace_bytes) {
   TGT_CHECK_ARG(n_rows >= 0 && n_edges >= 0, "n_rows and n_edges must be >= 0");
   TGT_CHECK_ARG(n_rows < (int64_t(1) << 31) - 1 && n_edges < (int64_t(1) << 31) - 1,
                 "n_rows and n_edges must fit in int32");
   TGT_CHECK_ARG(workspace_bytes, "null output pointer");
   Workspace w;
-  const int rc = plan_workspace(n_rows, n_edges, &w);
+  const int rc = plan_workspace(n_rows, n_edges, wide, &w);
   if (rc != TGT_OK) return rc;
   *workspace_bytes = w.total;
   return TGT_OK;
 }
-
-namespace tgt {
-namespace {
 
 // The build for endpoint type I (int64: the reference's edge_index as is; int32: lists prepared on
 // the device by tgt_edge_prepare, half the upload and half the reads).
@@ -142,7 +136,7 @@ int build_layout(const I* edge_index, int64_t n_edges, int64_t n_rows, int group
   TGT_CHECK_ARG(aligned16(edge_index) && aligned16(workspace), "pointers must be 16-byte aligned");
 
   Workspace w;
-  int rc = plan_workspace(n_rows, n_edges, &w);
+  int rc = plan_workspace(n_rows, n_edges, sizeof(I) == 8, &w);
   if (rc != TGT_OK) return rc;
   if (workspace_bytes < w.total)
     return set_error(TGT_ERR_WORKSPACE, "workspace holds %zu bytes, %zu needed", workspace_bytes,
@@ -252,6 +246,14 @@ __global__ void edge_prepare_kernel(const PrepareParams p) {
 
 }  // namespace
 }  // namespace tgt
+
+extern "C" int tgt_edge_layout_sizes(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes) {
+  return tgt::workspace_size(n_rows, n_edges, true, workspace_bytes);
+}
+
+extern "C" int tgt_edge_layout_sizes_i32(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes) {
+  return tgt::workspace_size(n_rows, n_edges, false, workspace_bytes);
+}
 
 extern "C" int tgt_edge_layout_build(const int64_t* edge_index, int64_t n_edges, int64_t n_rows,
                                      int group_by, int32_t* ptr, int32_t* other, int32_t* perm,
