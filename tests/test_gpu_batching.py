@@ -82,6 +82,31 @@ def test_training_batch(model, reorder, features, dtype):
                 assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
 
 
+@pytest.mark.parametrize("model", ["graphormer", "gt"])
+@pytest.mark.parametrize("nodes,rest", [(1000, None), (777, [300, 300, 177, 0]), (250, [250, 0, 0, 0])])
+def test_every_rank_takes_its_slice(model, nodes, rest, monkeypatch):
+    """Slices that start inside the batch, end with it, or are empty, as four ranks take them (no collective is part of it)."""
+    from torchgt_b200.gt_sp import batching
+    n = 3001
+    edges, perm = _graph(21, n, 25000)
+    x, y, idx = torch.randn(n, 6), torch.arange(n), perm[:nodes]
+    args = types.SimpleNamespace(seq_len=1000, model=model, reorder=False)
+    monkeypatch.setattr(batching, "sequence_parallel_is_initialized", lambda: True)
+    monkeypatch.setattr(batching, "get_sequence_parallel_world_size", lambda: 4)
+    taken = []
+    device_batch = batching._device_batch
+    monkeypatch.setattr(batching, "_device_batch", lambda *a: (taken.append(a[-3:-1]), device_batch(*a))[1])
+    for rank in range(4):
+        monkeypatch.setattr(batching, "get_sequence_parallel_rank", lambda: rank)
+        want = batching.get_batch_reorder_blockize(args, x, y, idx, rest, "cpu", edges, n, 4, 8)
+        got = batching.get_batch_reorder_blockize(args, x.cuda(), y.cuda(), idx.cuda(), rest, "cuda", edges.cuda(), n, 4, 8)
+        assert len(taken) == rank + 1
+        for a, b in zip(got[:3], want[:3]):
+            assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
+    if rest is not None:
+        assert taken[-1] == (nodes, nodes)
+
+
 def test_lists_the_kernels_cannot_number_take_the_pytorch_formulation(monkeypatch):
     from torchgt_b200.gt_sp import batching
     edges, perm = _graph(5, 300, 2000)
