@@ -279,8 +279,8 @@ def epoch_benchmark(rank, world, dev, workload="64k"):
         out = model(x, None, graph, attn_type="sparse")
         loss = F.nll_loss(out, y)
         if reducer is not None:
-            reducer.prepare()                   # gradients accumulate straight into one flat buffer
-            loss.backward()                     # its all-reduce starts when the last gradient has arrived
+            reducer.prepare()
+            loss.backward()                     # the last gradient's hook moves all into one flat buffer and reduces it
             reducer.synchronize()
         else:
             opt.zero_grad(set_to_none=True)
