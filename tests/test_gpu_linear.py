@@ -148,3 +148,30 @@ def test_linear_takes_every_call_that_f_linear_takes():
     g, = torch.autograd.grad(linear(x, w2, b).sum(), x, create_graph=True)
     dw, = torch.autograd.grad((g * g).sum(), w2)
     assert _err(dw, (2 * 8 * w.double().sum(0)).expand(64, 64)) < 2e-3
+
+
+# either side of every line of the rule: rows, reduction, columns, bias
+@pytest.mark.parametrize("rows,reduce,cols,bias,own", [
+    (1023, 64, 64, True, False), (1024, 64, 64, True, True), (32768, 64, 28, True, False), (32767, 64, 28, True, True),
+    (32768, 64, 32, True, True), (8191, 128, 64, True, True), (8192, 128, 64, True, False), (32768, 128, 64, True, True),
+    (4097, 192, 64, True, False), (4097, 512, 512, True, False), (65535, 64, 64, False, False), (65536, 64, 64, False, True),
+    (65536, 128, 64, False, False), (65536, 64, 28, False, False)])
+def test_full_fp32_products_take_the_kernel_that_is_ahead(rows, reduce, cols, bias, own):
+    """Bit for bit the library's product, or the row kernel's; both within the bound of a fp32 sum of 64-bit values."""
+    from torchgt_b200 import _cabi
+    from torchgt_b200.linear import linear
+    gen = torch.Generator().manual_seed(rows + reduce + cols)
+    x, w, b = (torch.randn(*s, generator=gen).cuda() for s in ((rows, reduce), (cols, reduce), (cols,)))
+    b = b if bias else None
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    try:
+        with torch.no_grad():
+            y, library = linear(x, w, b), torch.nn.functional.linear(x, w, b)
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = before
+    kernel = torch.empty_like(y)
+    _cabi.check(_cabi.load().tgt_linear_rows(x.data_ptr(), w.data_ptr(), b.data_ptr() if bias else None, rows, reduce, cols,
+                                             kernel.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(y, kernel if own else library)
+    assert _err(y, torch.nn.functional.linear(x.double(), w.double(), b.double() if bias else None)) < TOL

@@ -31,7 +31,6 @@ bool plain(const at::Tensor& t, const at::Device& device) {
 }
 
 // The caller allowed TF32 products: the forward product is then the library's, which has the tensor cores for it.
-// Without it products are full fp32 and this library's kernel is the faster one.
 bool tf32_allowed() {
   return at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) ==
          at::Float32Precision::TF32;
@@ -84,17 +83,29 @@ bool eligible(const at::Tensor& x, const at::Tensor& w, const at::Tensor& bias) 
   return !bias.defined() || (plain(bias, x.device()) && bias.dim() == 1 && bias.size(0) == out);
 }
 
+// Is linear_rows.cu ahead of the library's fp32 product?  Device time of both at reductions of 64 to 1024, 4 to 1024
+// columns and 1,100 to 320,000 rows (us here / there); up to a thousand rows the library's rounding is kept, the calls
+// being bound by the host.
+//   64 in, with a bias (the library runs a second kernel for it): ahead everywhere, 64 x 64 5.1 / 7.3 at 4,097 rows, 11.2 /
+//     12.3 at 16,384, 77.8 / 173 at 320,000, 64 x 256 272 / 679; not with few columns of its 64-wide tile in use on long
+//     lists: 64 x 4 8.7 / 9.3 at 16,384 rows but 18.9 / 16.4 at 65,536 (64 x 40: 19.1 / 29.3).
+//   128 in, with a bias: 128 x 64 7.0 / 9.1 at 4,097 rows, 17.9 / 14.9 at 16,384, 35.8 / 42.6 at 65,536.
+//   64 in, no bias: 64 x 64 11.7 / 7.8 at 16,384 rows, 20.1 / 21.1 at 65,536, 76.5 / 87.1 at 320,000.
+//   Longer reductions, or 128 without a bias: behind (256 x 256 26.5 / 20.7 at 4,097 rows, 512 x 512 4091 / 3623 and
+//     1024 x 1024 16602 / 12243 at 320,000) or ahead by a little on long lists only.
+bool rows_kernel_ahead(int64_t rows, int64_t in, int64_t out, bool bias) {
+  if (rows < 1024 || in > 128) return false;
+  if (!bias) return in == 64 && out >= 32 && rows >= 65536;
+  if (in == 128 && rows >= 8192 && rows < 32768) return false;
+  return out >= 32 || rows < 32768;
+}
+
 at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<at::Tensor>& bias_in) {
   const at::Tensor bias = bias_in.has_value() ? *bias_in : at::Tensor();
   if (!eligible(x, w, bias)) return at::linear(x, w, bias_in);
   const c10::cuda::CUDAGuard guard(x.device());
-  // With a bias the library runs a second kernel, so this one is ahead from the smallest sizes on (64 x 64, device time
-  // here and there: 1,024 rows 3.8 and 5.8 us, 4,097 rows 4.0 and 6.8 us); up to a thousand rows the library's rounding
-  // is kept, the calls being bound by the host.  Without a bias the library's product is one kernel too and wins in the
-  // middle (8,192 rows 6.6 and 4.7 us, 37,609 rows 17.8 and 10.5 us); this one is ahead on long lists (320,000 rows 78
-  // and 95 us).
   const int64_t rows = x.numel() / w.size(1);
-  const bool library = tf32_allowed() || rows < (bias.defined() ? 1024 : 200000);
+  const bool library = tf32_allowed() || !rows_kernel_ahead(rows, w.size(1), w.size(0), bias.defined());
   const bool record = torch::autograd::compute_requires_grad(x, w, bias);
   at::Tensor y;
   if (library && !record) return at::linear(x, w, bias_in);
