@@ -27,8 +27,10 @@
 // What batches without empty rows pay for it decides who looks: CTAs of their own behind the tiles' hold up the launch
 // of the call's next kernel (64K step + 1.4 %), an equal share for every CTA costs each of them a round trip to memory
 // (one-head 512K step + 2.3 %), testing in front of the walk changes its registers (64K step + 4.6 %) and behind the
-// stitching its occupancy.  Between the walk and the stitching it costs 0.7 % (64K step with bias gradient 160.3 -> 161.4
-// us, one-head 512K step 304.0 -> 306.1) or nothing (870K, forward alone).
+// stitching its occupancy.  Loading the tested words with the tile's indices gains nothing (one-head 512K step 307.9 us
+// against 306.3), and as a function that is not inlined it costs the walk its registers (322 us; 64K step 172 against 162).
+// Between the walk and the stitching the search is free (without it 308.6 against 308.2); what is left, 303.9 -> 307.2 us
+// for the one-head 512K step and 160.5 -> 161.3 for the 64K step with bias gradient, is zero_gap's longer code in the walk.
 #pragma once
 
 #include <type_traits>
