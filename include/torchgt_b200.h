@@ -490,6 +490,37 @@ TGT_API int tgt_linear_wgrad_scratch_bytes(int64_t rows, int in_features, int ou
 TGT_API int tgt_linear_wgrad(const float* dy, const float* x, int64_t rows, int in_features, int out_features,
                              float* dw, float* db, void* scratch, size_t scratch_bytes, void* stream);
 
+/*
+ * The input gradient of the same layer: dx [rows, in_features] = dy [rows, out_features] w for w [out_features,
+ * in_features], full fp32 products and sums.  Both widths multiples of 4, at most 1024 (TGT_ERR_UNSUPPORTED otherwise),
+ * pointers 16-byte aligned.
+ */
+TGT_API int tgt_linear_input_grad(const float* dy, const float* w, int64_t rows, int out_features, int in_features,
+                                  float* dx, void* stream);
+
+/*
+ * The same three for up to three layers of equal shape: products of one input (tgt_linear_rows_multi: c[i] = a w[i]^T +
+ * bias[i]), the sum of their input gradients (dx = sum_i dy[i] w[i]) and their parameters' gradients, each in one pass over
+ * what the layers share.  w, bias, dy, c, dw and db are host arrays of `count` device pointers; bias[i] and db[i] may be
+ * NULL.  With one product, c = act(a w^T + bias) + add; pre receives a w^T + bias, both [rows, cols] and NULL where they
+ * are not wanted.  tgt_linear_input_grad_multi multiplies dx by the derivative of `act` at gate [rows, in_features], the
+ * activation's input, or for TGT_ACT_RELU its result (models/graphormer_dist_node_level.py:236-245,281-286).
+ */
+#define TGT_ACT_NONE 0
+#define TGT_ACT_RELU 1
+#define TGT_ACT_GELU 2
+TGT_API int tgt_linear_rows_multi(const float* a, const float* const* w, const float* const* bias, int count,
+                                  int64_t rows, int reduce, int cols, int act, float* pre, const float* add,
+                                  float* const* c, void* stream);
+TGT_API int tgt_linear_input_grad_multi(const float* const* dy, const float* const* w, int count, int64_t rows,
+                                        int out_features, int in_features, int act, const float* gate, float* dx,
+                                        void* stream);
+TGT_API int tgt_linear_wgrad_multi_scratch_bytes(int count, int64_t rows, int in_features, int out_features,
+                                                 size_t* bytes);
+TGT_API int tgt_linear_wgrad_multi(const float* const* dy, const float* x, int count, int64_t rows, int in_features,
+                                   int out_features, float* const* dw, float* const* db, void* scratch,
+                                   size_t scratch_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,150 @@
+"""Products and parameter gradients of the narrow linear layers on the tensor cores, at the edges of their tiles, against
+fp64.  Three bf16 pieces carry 24 bits of an operand, the dropped piece products stay below 2^-23 of a product, and sums are
+fp32 over chains of at most 1024 products: relative 2-norm errors stay below 1024^0.5 * 2^-23 < 4e-6; what is measured is 7e-8
+to 5e-7."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+TOL = 4e-6
+
+
+def _lib():
+    from torchgt_b200 import _cabi
+    return _cabi
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+def _rand(seed, *shapes):
+    gen = torch.Generator().manual_seed(seed)
+    return [torch.randn(*s, generator=gen).cuda() for s in shapes]
+
+
+def _rel(got, ref):
+    return float((got.double() - ref).norm() / ref.norm().clamp_min(1e-30))
+
+
+def _array(tensors):
+    return (ctypes.c_void_p * len(tensors))(*[None if t is None else t.data_ptr() for t in tensors])
+
+
+def _act(name, t):
+    return {"none": lambda v: v, "relu": torch.relu, "gelu": torch.nn.functional.gelu}[name](t)
+
+
+ACTS = {"none": 0, "relu": 1, "gelu": 2}
+
+
+@pytest.mark.parametrize("count", [1, 3])
+@pytest.mark.parametrize("rows,reduce,cols", [
+    (1, 64, 64), (4064, 64, 64), (8064, 64, 64), (8065, 64, 64), (8192, 64, 64), (20001, 64, 64), (38017, 64, 40),
+    (9000, 128, 64), (9000, 64, 128), (9000, 68, 100), (9000, 4, 4), (2049, 64, 1024), (8200, 384, 64), (8200, 448, 64),
+    (8200, 1024, 8)])
+def test_products_and_input_gradients(rows, reduce, cols, count):
+    c = _lib()
+    x, = _rand(rows + reduce, (rows, reduce))
+    w, b = _rand(cols, (count, cols, reduce), (count, cols))
+    w, b = list(w.contiguous().unbind(0)), list(b.contiguous().unbind(0))
+    y = [torch.full((rows, cols), float("nan"), device="cuda") for _ in range(count)]
+    c.check(c.load().tgt_linear_rows_multi(x.data_ptr(), _array(w), _array(b), count, rows, reduce, cols, 0, None, None,
+                                           _array(y), _stream()))
+    for i in range(count):
+        assert _rel(y[i], x.double() @ w[i].double().t() + b[i].double()) < TOL
+    dx = torch.full((rows, reduce), float("nan"), device="cuda")
+    c.check(c.load().tgt_linear_input_grad_multi(_array(y), _array(w), count, rows, cols, reduce, 0, None, dx.data_ptr(),
+                                                 _stream()))
+    assert _rel(dx, sum(y[i].double() @ w[i].double() for i in range(count))) < TOL
+    again = torch.empty_like(dx)
+    c.check(c.load().tgt_linear_input_grad_multi(_array(y), _array(w), count, rows, cols, reduce, 0, None, again.data_ptr(),
+                                                 _stream()))
+    assert torch.equal(dx, again)
+
+
+@pytest.mark.parametrize("act", ["relu", "gelu"])
+@pytest.mark.parametrize("rows", [33, 8065])
+def test_activation_residual_and_gate(rows, act):
+    c = _lib()
+    x, w, b, add, dy = _rand(rows, (rows, 64), (128, 64), (128,), (rows, 128), (rows, 64))
+    pre, y = torch.empty(rows, 128, device="cuda"), torch.empty(rows, 128, device="cuda")
+    c.check(c.load().tgt_linear_rows_multi(x.data_ptr(), _array([w]), _array([b]), 1, rows, 64, 128, ACTS[act],
+                                           pre.data_ptr(), add.data_ptr(), _array([y]), _stream()))
+    z = x.double() @ w.double().t() + b.double()
+    assert _rel(pre, z) < TOL and _rel(y, _act(act, z) + add.double()) < TOL
+    gate = torch.relu(pre) if act == "relu" else pre
+    w2, = _rand(1, (64, 128))
+    dx = torch.empty(rows, 128, device="cuda")
+    c.check(c.load().tgt_linear_input_grad_multi(_array([dy]), _array([w2]), 1, rows, 64, 128, ACTS[act], gate.data_ptr(),
+                                                 dx.data_ptr(), _stream()))
+    leaf = pre.double().requires_grad_()
+    ref, = torch.autograd.grad(_act(act, leaf), leaf, dy.double() @ w2.double())
+    assert _rel(dx, ref) < TOL
+
+
+@pytest.mark.parametrize("count", [1, 2, 3])
+@pytest.mark.parametrize("rows,inp,out", [(1, 64, 64), (63, 64, 64), (64, 64, 64), (65, 64, 4), (9473, 64, 64),
+                                          (20001, 128, 64), (20001, 64, 100), (150001, 64, 64)])
+def test_parameter_gradients(rows, inp, out, count):
+    c = _lib()
+    x, = _rand(rows + inp, (rows, inp))
+    dy = list(_rand(out, (count, rows, out))[0].unbind(0))
+    dw = [torch.full((out, inp), float("nan"), device="cuda") for _ in range(count)]
+    db = [torch.full((out,), float("nan"), device="cuda") for _ in range(count - 1)] + [None]
+    need = ctypes.c_size_t()
+    c.check(c.load().tgt_linear_wgrad_multi_scratch_bytes(count, rows, inp, out, ctypes.byref(need)))
+    scratch = torch.full((need.value + 512,), 171, dtype=torch.uint8, device="cuda")
+    c.check(c.load().tgt_linear_wgrad_multi(_array(dy), x.data_ptr(), count, rows, inp, out, _array(dw), _array(db),
+                                            scratch.data_ptr(), need.value, _stream()))
+    assert (scratch[need.value:] == 171).all()
+    for i in range(count):
+        assert _rel(dw[i], dy[i].double().t() @ x.double()) < TOL
+        assert db[i] is None or _rel(db[i], dy[i].double().sum(0)) < TOL
+
+
+def test_values_that_are_not_finite_and_sums_past_the_range():
+    """They come out as fp32 FMAs give them: infinities and NaN where those belong, and nowhere else."""
+    c = _lib()
+    rows = 9000
+    x, w = _rand(3, (rows, 64), (64, 64))
+    x[5, 3], x[700, 1], x[8999] = float("inf"), float("nan"), 3e38
+    w[9, 2] = float("-inf")
+    y = torch.empty(rows, 64, device="cuda")
+    c.check(c.load().tgt_linear_rows(x.data_ptr(), w.data_ptr(), None, rows, 64, 64, y.data_ptr(), _stream()))
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    ref = x @ w.t()
+    torch.backends.cuda.matmul.allow_tf32 = before
+    assert torch.equal(y.isnan()[:8999], ref.isnan()[:8999]) and torch.equal(y.isinf()[:8999], ref.isinf()[:8999])
+    assert not y[8999].isfinite().all()
+    fine = ref.isfinite() & y.isfinite()
+    fine[8999] = False
+    assert _rel(y[fine], (x.double() @ w.double().t())[fine]) < TOL
+    dy, = _rand(4, (rows, 64))
+    x[8999] = 0
+    need = ctypes.c_size_t()
+    c.check(c.load().tgt_linear_wgrad_scratch_bytes(rows, 64, 64, ctypes.byref(need)))
+    scratch, dw = torch.empty(need.value, dtype=torch.uint8, device="cuda"), torch.empty(64, 64, device="cuda")
+    c.check(c.load().tgt_linear_wgrad(dy.data_ptr(), x.data_ptr(), rows, 64, 64, dw.data_ptr(), None, scratch.data_ptr(),
+                                      need.value, _stream()))
+    assert dw[:, 3].isinf().all() and dw[:, 1].isnan().all()
+    rest = [i for i in range(64) if i not in (1, 3)]
+    assert _rel(dw[:, rest], (dy.double().t() @ x.double())[:, rest]) < TOL
+
+
+def test_arguments_the_calls_refuse():
+    c = _lib()
+    lib = c.load()
+    t = torch.randn(8, 64, device="cuda")
+    one = _array([t])
+    assert lib.tgt_linear_rows_multi(t.data_ptr(), one, one, 4, 8, 64, 64, 0, None, None, one, None) == 1
+    assert lib.tgt_linear_rows_multi(t.data_ptr(), one, one, 1, 8, 62, 64, 0, None, None, one, None) == 3
+    assert lib.tgt_linear_rows_multi(t.data_ptr(), one, one, 1, 8, 64, 64, 7, None, None, one, None) == 1
+    assert lib.tgt_linear_input_grad_multi(one, one, 1, 8, 64, 64, 1, None, t.data_ptr(), None) == 1     # a gate is missing
+    assert lib.tgt_linear_input_grad(t.data_ptr() + 4, t.data_ptr(), 8, 64, 64, t.data_ptr(), None) == 1
+    n = ctypes.c_size_t()
+    assert lib.tgt_linear_wgrad_multi_scratch_bytes(4, 8, 64, 64, ctypes.byref(n)) == 1

@@ -121,6 +121,14 @@ SIGNATURES = {
     "tgt_add_layer_norm_bwd": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_void_p,
                                        c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     "tgt_linear_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p]),
+    "tgt_linear_input_grad": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p]),
+    "tgt_linear_rows_multi": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_int, c_void_p, c_void_p,
+                                      c_void_p, c_void_p]),
+    "tgt_linear_input_grad_multi": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_int, c_void_p, c_void_p,
+                                            c_void_p]),
+    "tgt_linear_wgrad_multi_scratch_bytes": (c_int, [c_int, c_int64, c_int, c_int, POINTER(c_size_t)]),
+    "tgt_linear_wgrad_multi": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                                       c_size_t, c_void_p]),
     "tgt_linear_wgrad_scratch_bytes": (c_int, [c_int64, c_int, c_int, POINTER(c_size_t)]),
     "tgt_linear_wgrad": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t,
                                  c_void_p]),

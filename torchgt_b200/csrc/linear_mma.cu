@@ -1,0 +1,297 @@
+// fp32 products of long matrices with small ones on the tensor cores, for the forward and the input gradient of narrow
+// linear layers over many rows (models/graphormer_dist_node_level.py:241-245,281-286,
+// models/gt_dist_node_level.py:189-193,232-236: 64 x 64 to 128 x 64 over 8,000 to 870,000 rows).
+//
+// A tile is 128 rows x 64 columns.  A CTA keeps its columns' weights as bf16 pieces in shared memory (tensor_core.cuh) and
+// walks row tiles: 256 threads split the rows' values on their way from registers into shared memory, one thread issues
+// the products, and while they run the next rows are on their way in and the tile before is finished from the other half
+// of the tensor memory.  CTAs of the same rows are neighbours in the grid, so a second column tile or a second layer finds
+// the rows in the L2.
+//
+// 320,000 rows of 64 x 64: 48 us against 80 for the FMA kernel that was here and 92 for the library's input gradient (a
+// copy of the same bytes: 25); 64 x 128: 78 against 143 and 138; 128 x 64: 79 against 151 and 134; 64,001 rows: 18 against
+// 25 and 27.  Sums stored row by row straight from tensor memory, without the blocks in shared memory, and without the
+// second half: 59 us.  Relative error against 64 bits 7e-8 (FMA 1.1e-7, library 1.5e-7), 128 long 1.2e-7 (1.5e-7, 2.0e-7).
+#include "linear_rows.cuh"
+#include "tensor_core.cuh"
+
+namespace tgt {
+namespace {
+
+constexpr int kThreads = 256, kWarps = kThreads / 32;
+constexpr int kRows = 128, kCols = 64;     // of a tile: M and N of one product
+constexpr int kChunk = 64;                 // reduction elements staged at a time
+constexpr int kPieceA = kRows * 128;       // bytes of one piece of a tile of A
+constexpr int kPieceW = kCols * 128;
+constexpr int kTmemCols = 4 * kCols;       // two tiles' large and small products
+constexpr int kMostSmem = 227 * 1024;
+
+struct SplitGemm : LinearRows {
+  int col_tiles;                    // per output
+  int kept;                         // chunks of the weights in shared memory: all, or one
+};
+
+// Finished sums on their way out: 32 rows x 16 columns per warp, 16-byte pieces in an order that keeps rows' equal pieces
+// in different banks.
+constexpr int kBlockCols = 16, kBlockBytes = 32 * kBlockCols * 4;
+__device__ __forceinline__ int block_offset(int row, int piece) { return row * 64 + ((piece ^ (row / 2)) & 3) * 16; }
+
+// An infinity or NaN among the operands, or a sum past the range of fp32: the pieces' sum says no more than that.  The
+// values of this row that are not finite (16 of them in the warp's block) are summed again from the operands themselves.
+__device__ __noinline__ void sum_again(const SplitGemm& p, int out, int64_t row, int col, uint8_t* block, int lane) {
+  for (int x = 0; x < 16; ++x) {
+    float* v = reinterpret_cast<float*>(block + block_offset(lane, x / 4)) + x % 4;
+    if (fabsf(*v) < __int_as_float(0x7f800000) || row >= p.rows || col + x >= p.cols) continue;
+    float s = 0.f;
+    for (int src = 0; src < p.sources; ++src) {
+      const float* a = p.a[src] + row * p.red;
+      const float* w = p.w[p.sources > 1 ? src : out] + (p.transposed ? int64_t(col + x) : int64_t(col + x) * p.red);
+      for (int k = 0; k < p.red; ++k) s = fmaf(__ldg(a + k), __ldg(w + int64_t(k) * (p.transposed ? p.cols : 1)), s);
+    }
+    *v = s;
+  }
+}
+
+// Shared memory of a CTA, from a 1,024-byte boundary on: pieces of a chunk of A, pieces of `kept` chunks of the weights,
+// one block of finished sums per warp, the barrier and the tensor memory's address.
+inline int split_gemm_smem(int kept) { return 3 * kPieceA + kept * 3 * kPieceW + kWarps * kBlockBytes + 16; }
+
+__global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_constant__ SplitGemm p) {
+  extern __shared__ __align__(1024) uint8_t s_raw[];
+  const int src_chunks = (p.red + kChunk - 1) / kChunk, chunks = src_chunks * p.sources;
+  const uint32_t s_a = tc::smem_address(s_raw);
+  const uint32_t s_w = s_a + 3 * kPieceA;
+  uint8_t* const s_block = s_raw + 3 * kPieceA + p.kept * 3 * kPieceW + threadIdx.x / 32 * kBlockBytes;
+  uint64_t* const s_done = reinterpret_cast<uint64_t*>(s_raw + 3 * kPieceA + p.kept * 3 * kPieceW + kWarps * kBlockBytes);
+  uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(s_done + 1);
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int across = p.col_tiles * p.outputs;               // neighbours in the grid read the same rows of A
+  const int tile_col = blockIdx.x % across;
+  const int out = tile_col / p.col_tiles, c0 = tile_col % p.col_tiles * kCols;
+  const int walkers = gridDim.x / across;
+  const int64_t tiles = (p.rows + kRows - 1) / kRows;
+
+  if (warp == 0) tc::allocate<kTmemCols>(s_tmem);
+  if (tid == 32) tc::barrier_init(s_done);
+
+  const int q = 4 * (tid % 16), r0 = tid / 16;              // this thread's four reduction elements and first row
+  float4 next[kRows / 16];
+  auto load = [&](int64_t tile, int chunk) {
+    const int src = chunk / src_chunks, k = chunk % src_chunks * kChunk + q;
+    const float* a = p.a[src];
+#pragma unroll
+    for (int i = 0; i < kRows / 16; ++i) {
+      const int64_t row = tile * kRows + r0 + 16 * i;
+      next[i] = row < p.rows && k < p.red ? __ldg(reinterpret_cast<const float4*>(a + row * p.red + k))
+                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  int64_t tile = blockIdx.x / across;
+  load(tile, 0);
+  auto stage_weights = [&](int chunk, int slot) {
+    const int src = chunk / src_chunks, k0 = chunk % src_chunks * kChunk;
+    const float* w = p.w[p.sources > 1 ? src : out];
+#pragma unroll 4
+    for (int u = tid; u < kCols * 16; u += kThreads) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      int n, k;
+      if (!p.transposed) {
+        n = u / 16; k = 4 * (u % 16);
+        if (c0 + n < p.cols && k0 + k < p.red)
+          v = __ldg(reinterpret_cast<const float4*>(w + int64_t(c0 + n) * p.red + k0 + k));
+      } else {
+        n = u % kCols; k = 4 * (u / kCols);
+        if (c0 + n < p.cols && k0 + k < p.red) {
+          const float* f = w + int64_t(k0 + k) * p.cols + c0 + n;
+          v = make_float4(__ldg(f), __ldg(f + p.cols), __ldg(f + 2 * p.cols), __ldg(f + 3 * p.cols));
+        }
+      }
+      tc::store4(s_w + slot * (3 * kPieceW), kPieceW, tc::tile_offset(n, k), tc::split4(v));
+    }
+  };
+  if (p.kept == chunks)                                     // once; a long reduction's weights come along with its rows
+    for (int chunk = 0; chunk < chunks; ++chunk) stage_weights(chunk, chunk);
+  tc::fence_before_barrier();
+  __syncthreads();
+  tc::fence_after_barrier();
+  const uint32_t tmem = *s_tmem;
+  uint32_t phase = 0;
+  bool ok = true;
+
+  // sums of a tile -> C: a warp finishes 32 rows x 32 columns, 16 columns at a time through its block of shared memory, so
+  // that the stores are runs of 64 bytes per row
+  auto finish = [&](int64_t of, uint32_t sums) {
+    const int64_t row0 = of * kRows + warp % 4 * 32;
+    sums += (uint32_t(warp % 4 * 32) << 16) + warp / 4 * 32;
+#pragma unroll 1
+    for (int j = 0; j < 32; j += kBlockCols) {
+      uint32_t big[16], small[16];
+      tc::read16(sums + j, big);
+      tc::read16(sums + kCols + j, small);
+      tc::reads_done();
+      const int col = c0 + warp / 4 * 32 + j;
+      float size = 0.f;
+#pragma unroll
+      for (int x = 0; x < 16; x += 4) {
+        const float4 v = make_float4(__uint_as_float(big[x]) + __uint_as_float(small[x]),
+                                     __uint_as_float(big[x + 1]) + __uint_as_float(small[x + 1]),
+                                     __uint_as_float(big[x + 2]) + __uint_as_float(small[x + 2]),
+                                     __uint_as_float(big[x + 3]) + __uint_as_float(small[x + 3]));
+        size += (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w));
+        *reinterpret_cast<float4*>(s_block + block_offset(lane, x / 4)) = v;
+      }
+      if (!(size < __int_as_float(0x7f800000))) sum_again(p, out, row0 + lane, col, s_block, lane);
+      __syncwarp();
+      const int my_col = col + 4 * (lane % 4);
+      if (my_col < p.cols) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = lane / 4 + 8 * i;
+          float4 v = *reinterpret_cast<const float4*>(s_block + block_offset(r, lane % 4));
+          if (!ok) v.x = __int_as_float(0x7fffffff);
+          if (row0 + r < p.rows) finish_values(p, out, row0 + r, my_col, v);
+        }
+      }
+      __syncwarp();
+    }
+  };
+
+  // A tile's products run under the finishing of the tile before, whose sums lie in the other half of the tensor memory.
+  int64_t before = -1;
+  uint32_t sums = tmem;
+  for (; tile < tiles; tile += walkers) {
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+#pragma unroll
+      for (int i = 0; i < kRows / 16; ++i)
+        tc::store4(s_a, kPieceA, tc::tile_offset(r0 + 16 * i, q), tc::split4(next[i]));
+      if (p.kept < chunks) stage_weights(chunk, 0);
+      tc::publish_operands();
+      tc::fence_before_barrier();                           // everybody has read the sums of two tiles ago
+      ok = __syncthreads_and(ok);
+      if (!ok) goto finished;
+      if (tid == 0) {
+        tc::fence_after_barrier();
+        const uint32_t w = s_w + (p.kept < chunks ? 0 : chunk * (3 * kPieceW));
+#pragma unroll
+        for (int k = 0; k < kChunk / 16; ++k) {
+          const uint64_t a1 = tc::k_major(s_a + 32 * k), a2 = tc::k_major(s_a + kPieceA + 32 * k),
+                         a3 = tc::k_major(s_a + 2 * kPieceA + 32 * k);
+          const uint64_t w1 = tc::k_major(w + 32 * k), w2 = tc::k_major(w + kPieceW + 32 * k),
+                         w3 = tc::k_major(w + 2 * kPieceW + 32 * k);
+          constexpr uint32_t both = tc::instruction(kRows, 2 * kCols, false, false),
+                             one = tc::instruction(kRows, kCols, false, false);
+          tc::multiply(sums, a1, w1, both, chunk + k > 0);       // a1 w1 | a1 w2
+          tc::multiply(sums + kCols, a2, w1, one, true);
+          tc::multiply(sums + kCols, a2, w2, one, true);
+          tc::multiply(sums + kCols, a1, w3, one, true);
+          tc::multiply(sums + kCols, a3, w1, one, true);
+        }
+        tc::commit(s_done);
+      }
+      // the next step's rows arrive under the products and the stores
+      const bool last = chunk + 1 == chunks;
+      const int64_t next_tile = last ? tile + walkers : tile;
+      if (next_tile < tiles) load(next_tile, last ? 0 : chunk + 1);
+      if (chunk == 0 && before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
+      ok = tc::wait(s_done, phase) && ok;
+      phase ^= 1;
+    }
+    tc::fence_after_barrier();
+    before = tile;
+    sums = tmem + (sums == tmem ? 2 * kCols : 0);
+  }
+finished:
+  if (before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
+  tc::fence_before_barrier();
+  __syncthreads();
+  if (warp == 0) tc::release<kTmemCols>(tmem);
+}
+
+int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
+  SplitGemm p;
+  static_cast<LinearRows&>(p) = of;
+  const int chunks = (p.red + kChunk - 1) / kChunk * p.sources;
+  p.kept = split_gemm_smem(chunks) <= kMostSmem ? chunks : 1;
+  const int smem = split_gemm_smem(p.kept);
+  const int rc = allow_shared_memory<split_gemm_kernel>(kMostSmem);
+  if (rc != TGT_OK) return rc;
+  p.col_tiles = (p.cols + kCols - 1) / kCols;
+  const int64_t tiles = (p.rows + kRows - 1) / kRows;
+  const int resident = 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
+  const int across = p.col_tiles * p.outputs;
+  int64_t walkers = int64_t(sm_count()) * resident / across;
+  if (walkers < 1) walkers = 1;
+  if (walkers > tiles) walkers = tiles;
+  split_gemm_kernel<<<unsigned(walkers * across), kThreads, smem, stream>>>(p);
+  TGT_CHECK_CUDA(cudaGetLastError());
+  return TGT_OK;
+}
+
+bool shape_supported(int reduce, int cols) {
+  return reduce >= 4 && reduce % 4 == 0 && reduce <= 1024 && cols >= 4 && cols % 4 == 0 && cols <= 1024;
+}
+
+}  // namespace
+}  // namespace tgt
+
+extern "C" int tgt_linear_rows(const float* a, const float* w, const float* bias, int64_t rows, int reduce, int cols,
+                               float* c, void* stream) {
+  return tgt_linear_rows_multi(a, &w, &bias, 1, rows, reduce, cols, TGT_ACT_NONE, nullptr, nullptr, &c, stream);
+}
+
+extern "C" int tgt_linear_rows_multi(const float* a, const float* const* w, const float* const* bias, int count, int64_t rows,
+                                     int reduce, int cols, int act, float* pre, const float* add, float* const* c,
+                                     void* stream_) {
+  using namespace tgt;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  TGT_CHECK_ARG(rows >= 0, "rows must be >= 0");
+  TGT_CHECK_ARG(count >= 1 && count <= kMostProducts, "count must be 1 to %d", kMostProducts);
+  TGT_CHECK_ARG(act == TGT_ACT_NONE || act == TGT_ACT_RELU || act == TGT_ACT_GELU, "act is none of TGT_ACT_*");
+  TGT_CHECK_ARG(count == 1 || (act == TGT_ACT_NONE && !pre && !add), "act, pre and add are for one product");
+  if (!shape_supported(reduce, cols))
+    return set_error(TGT_ERR_UNSUPPORTED, "reduce=%d cols=%d: both must be multiples of 4, at most 1024", reduce, cols);
+  if (rows == 0) return TGT_OK;
+  TGT_CHECK_ARG(a && w && bias && c, "a, w, bias and c must not be null");
+  TGT_CHECK_ARG(aligned16(a) && aligned16(pre) && aligned16(add), "tensors must be 16-byte aligned");
+  LinearRows p{};
+  p.a[0] = a;
+  for (int i = 0; i < count; ++i) {
+    TGT_CHECK_ARG(w[i] && c[i], "a, w and c must not be null");
+    TGT_CHECK_ARG(aligned16(w[i]) && aligned16(bias[i]) && aligned16(c[i]), "tensors must be 16-byte aligned");
+    p.w[i] = w[i]; p.bias[i] = bias[i]; p.c[i] = c[i];
+  }
+  p.rows = rows; p.red = reduce; p.cols = cols; p.sources = 1; p.outputs = count;
+  p.act = act; p.pre = pre; p.add = add;
+  return few_rows(rows, cols * count) ? linear_few_rows(p, stream) : launch_split_gemm(p, stream);
+}
+
+extern "C" int tgt_linear_input_grad(const float* dy, const float* w, int64_t rows, int out_features, int in_features,
+                                     float* dx, void* stream) {
+  return tgt_linear_input_grad_multi(&dy, &w, 1, rows, out_features, in_features, TGT_ACT_NONE, nullptr, dx, stream);
+}
+
+extern "C" int tgt_linear_input_grad_multi(const float* const* dy, const float* const* w, int count, int64_t rows,
+                                           int out_features, int in_features, int act, const float* gate, float* dx,
+                                           void* stream_) {
+  using namespace tgt;
+  TGT_CHECK_ARG(rows >= 0, "rows must be >= 0");
+  TGT_CHECK_ARG(count >= 1 && count <= kMostProducts, "count must be 1 to %d", kMostProducts);
+  TGT_CHECK_ARG(act == TGT_ACT_NONE || act == TGT_ACT_RELU || act == TGT_ACT_GELU, "act is none of TGT_ACT_*");
+  TGT_CHECK_ARG((act == TGT_ACT_NONE) == (gate == nullptr) || rows == 0, "act and gate disagree");
+  if (!shape_supported(out_features, in_features))
+    return set_error(TGT_ERR_UNSUPPORTED, "out_features=%d in_features=%d: both must be multiples of 4, at most 1024",
+                     out_features, in_features);
+  if (rows == 0) return TGT_OK;
+  TGT_CHECK_ARG(dy && w && dx, "dy, w and dx must not be null");
+  TGT_CHECK_ARG(aligned16(dx) && aligned16(gate), "tensors must be 16-byte aligned");
+  LinearRows p{};
+  for (int i = 0; i < count; ++i) {
+    TGT_CHECK_ARG(dy[i] && w[i], "dy, w and dx must not be null");
+    TGT_CHECK_ARG(aligned16(dy[i]) && aligned16(w[i]), "tensors must be 16-byte aligned");
+    p.a[i] = dy[i]; p.w[i] = w[i];
+  }
+  p.c[0] = dx;
+  p.rows = rows; p.red = out_features; p.cols = in_features; p.sources = count; p.outputs = 1; p.transposed = true;
+  p.gate_act = act; p.gate = gate;
+  return launch_split_gemm(p, static_cast<cudaStream_t>(stream_));
+}

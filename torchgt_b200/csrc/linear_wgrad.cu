@@ -1,117 +1,205 @@
 // Weight and bias gradient of a narrow nn.Linear over many rows: dW[o][i] = sum_r dY[r][o] X[r][i],
 // db[o] = sum_r dY[r][o], fp32.  The graph transformers' projections are 64 x 64 (128 x 64 for the node
 // encoder) over 64,000 to 870,000 rows (models/graphormer_dist_node_level.py:241-245,281-286,343: linear_q/k/v,
-// output_layer, the two FFN layers, node_encoder): a product with a tiny result and a very long reduction,
-// which a library GEMM runs split over a few CTAs (66 us at 64,001 rows, plus 25 us for the bias sum).
-// Here every CTA walks its share of the rows in chunks staged in shared memory and keeps a 64 x 64 tile of
-// dW in registers (8 x 8 per thread, fp32 FMA); the CTAs' tiles are then added in a fixed order by a second
-// kernel.  No atomics: results are bitwise reproducible.
-#include "tgt_common.cuh"
+// output_layer, the two FFN layers, node_encoder): a product with a tiny result and a very long reduction.
+//
+// Every CTA walks its share of the rows in chunks of 64, splits both operands into three bf16 pieces on their way into
+// shared memory (tensor_core.cuh) and keeps a 64 x 64 tile of dW in tensor memory; dY and X are both read as they lie,
+// rows being the reduction.  Tensor cores round a running sum towards zero at every step, so the large products are
+// drained after every chunk and added in fp32 registers; the small ones, 2^-8 of them, stay till the end.  The CTAs'
+// tiles are then added in a fixed order by a second kernel.  No atomics: results are bitwise reproducible.
+//
+// 320,000 rows of 64 x 64: 58 us with the sums, 75 for the FMA kernel that was here (a copy of the same bytes: 25); 64 x
+// 128 and 128 x 64: 91 against 130; 64,001 rows of 64 x 64: 25.6 against 27.6; one CTA per SM: 79 us.  Relative error against
+// 64 bits at 320,000 rows 1.5e-7, the FMA kernel's 4.4e-7.
+#include "tensor_core.cuh"
 
 namespace tgt {
 namespace {
 
-constexpr int kWgThreads = 64;
-constexpr int kWgTile = 64;        // outputs and inputs per tile
-constexpr int kWgChunk = 32;       // rows staged at a time
+constexpr int kMostGrads = 3;                   // products that share x
+constexpr int kWgTile = 64;                     // outputs and inputs per tile
+constexpr int kWgThreads = 256;
+constexpr int kWgChunk = 64;                    // rows staged at a time
+constexpr int kWgPiece = kWgChunk * 128;        // bytes of one piece of a chunk, 64 columns wide
+constexpr int kWgTmemCols = 256;
 
 struct WgradParams {
-  const float* dy;   // [rows, out]
-  const float* x;    // [rows, in]
-  float* partial;    // [gridDim.x][out * in + out]
+  const float* dy[kMostGrads];   // [rows, out]
+  const float* x;                // [rows, in]
+  float* partial;                // [gridDim.x][count][out * in + out]
   int64_t rows;
-  int in, out;
+  int in, out, count;
 };
 
-// 16 bytes global -> shared without passing through registers; bytes = 0 fills the destination with zeros
-__device__ __forceinline__ void copy_async_16(void* smem_dst, const void* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(smem_dst))),
-               "l"(src), "r"(bytes)
-               : "memory");
+// One element summed again from the operands (this CTA's rows): where the pieces' sum is not finite it says no more.
+__device__ __noinline__ float exact_sum(const WgradParams& p, const float* dy, int o, int i) {
+  float s = 0.f;
+  const int64_t chunks = (p.rows + kWgChunk - 1) / kWgChunk;
+  for (int64_t chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x)
+    for (int64_t r = chunk * kWgChunk; r < min((chunk + 1) * kWgChunk, p.rows); ++r)
+      s = fmaf(__ldg(dy + r * p.out + o), __ldg(p.x + r * p.in + i), s);
+  return s;
 }
 
-// Two warps per CTA; thread (ty, tx) of the 8 x 8 grid owns outputs {4 ty .. 4 ty + 3, 32 + 4 ty .. 32 + 4 ty + 3}
-// x inputs {4 tx .. 4 tx + 3, 32 + 4 tx .. 32 + 4 tx + 3}: per staged row four 16-byte shared-memory reads (two of
-// them the same address for the eight lanes of a quarter warp, two contiguous over them) feed 64 FMAs, so the
-// FMA pipe, not shared memory, sets the pace.  Chunks of 32 rows are double-buffered with asynchronous copies.
-__global__ void __launch_bounds__(kWgThreads) linear_wgrad_kernel(const WgradParams p) {
-  __shared__ __align__(16) float s_dy[2][kWgChunk][kWgTile];
-  __shared__ __align__(16) float s_x[2][kWgChunk][kWgTile];
-  const int tid = threadIdx.x;
-  const int ty = tid / 8, tx = tid % 8;
-  const int tiles_in = p.in / kWgTile;
-  const int o0 = (blockIdx.y / tiles_in) * kWgTile, i0 = (blockIdx.y % tiles_in) * kWgTile;
-  float acc[8][8];
+__global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __grid_constant__ WgradParams p) {
+  extern __shared__ __align__(1024) uint8_t s_base[];
+  const uint32_t s_dy = tc::smem_address(s_base);            // [2][dy's pieces, x's pieces]
+  uint64_t* const s_done = reinterpret_cast<uint64_t*>(s_base + 12 * kWgPiece);
+  uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(s_done + 2);
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  const int tiles_in = (p.in + 63) / 64;
+  const int tile = blockIdx.y / p.count, which = blockIdx.y % p.count;    // neighbours read the same rows of x
+  const int o0 = tile / tiles_in * 64, i0 = tile % tiles_in * 64;
+  const float* const from = p.dy[which];
+  const int64_t chunks = (p.rows + kWgChunk - 1) / kWgChunk;
+  if (warp == 0) tc::allocate<kWgTmemCols>(s_tmem);
+  if (tid == 32) {
+    tc::barrier_init(s_done);
+    tc::barrier_init(s_done + 1);
+  }
+
+  const int q = 4 * (tid % 16), r0 = tid / 16;
+  float4 dy[kWgChunk / 16], x[kWgChunk / 16];
+  auto load = [&](int64_t chunk) {
 #pragma unroll
-  for (int a = 0; a < 8; ++a)
-#pragma unroll
-    for (int b = 0; b < 8; ++b) acc[a][b] = 0.f;
-  float bias_acc = 0.f;          // thread tid sums column o0 + tid of dY
-  const int64_t n_chunks = (p.rows + kWgChunk - 1) / kWgChunk;
-  auto stage = [&](int64_t chunk, int buf) {
-#pragma unroll
-    for (int j = 0; j < kWgChunk * 16 / kWgThreads; ++j) {
-      const int u = tid + j * kWgThreads;            // 512 pieces of 16 bytes per operand: 32 rows x 16
-      const int r = u / 16, c4 = u % 16;
-      const int64_t row = chunk * kWgChunk + r;
-      const bool live = row < p.rows;
-      const int64_t from = live ? row : 0;
-      const bool col = o0 + 4 * c4 < p.out;          // the last tile of outputs may be narrower than 64
-      copy_async_16(&s_dy[buf][r][4 * c4], p.dy + from * p.out + (col ? o0 + 4 * c4 : 0), live && col ? 16 : 0);
-      copy_async_16(&s_x[buf][r][4 * c4], p.x + from * p.in + i0 + 4 * c4, live ? 16 : 0);
+    for (int i = 0; i < kWgChunk / 16; ++i) {
+      const int64_t row = chunk * kWgChunk + r0 + 16 * i;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      dy[i] = row < p.rows && o0 + q < p.out ? __ldg(reinterpret_cast<const float4*>(from + row * p.out + o0 + q)) : zero;
+      x[i] = row < p.rows && i0 + q < p.in ? __ldg(reinterpret_cast<const float4*>(p.x + row * p.in + i0 + q)) : zero;
     }
   };
-  if (int64_t(blockIdx.x) < n_chunks) stage(blockIdx.x, 0);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  int buf = 0;
-  for (int64_t chunk = blockIdx.x; chunk < n_chunks; chunk += gridDim.x, buf ^= 1) {
-    if (chunk + gridDim.x < n_chunks) stage(chunk + gridDim.x, buf ^ 1);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");     // this chunk's copies have landed
-    __syncthreads();
-#pragma unroll 4
-    for (int r = 0; r < kWgChunk; ++r) {
-      const float4 a0 = *reinterpret_cast<const float4*>(&s_dy[buf][r][4 * ty]);
-      const float4 a1 = *reinterpret_cast<const float4*>(&s_dy[buf][r][32 + 4 * ty]);
-      const float4 b0 = *reinterpret_cast<const float4*>(&s_x[buf][r][4 * tx]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&s_x[buf][r][32 + 4 * tx]);
-      const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+  float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+  float main_sum[32];     // of warps 0, 1, 4 and 5: row 32 (warp % 4) + lane, columns 32 (warp / 4) ..
 #pragma unroll
-      for (int a = 0; a < 8; ++a)
+  for (int j = 0; j < 32; ++j) main_sum[j] = 0.f;
+  int64_t chunk = blockIdx.x;
+  if (chunk < chunks) load(chunk);
+  tc::fence_before_barrier();
+  __syncthreads();
+  tc::fence_after_barrier();
+  const uint32_t tmem = *s_tmem;
+  const uint32_t mine = tmem + (uint32_t(warp % 4 * 32) << 16) + warp / 4 * 32;
+  bool ok = true;
+  // A chunk's products run under the split of the next one (two buffers) and under the draining of the last one's large
+  // products (two places in tensor memory).  Waits alternate over two barriers.
+  auto drain = [&](int n) {                        // large products of this CTA's n-th chunk, counted from 0
+    ok = tc::wait(s_done + n % 2, n / 2 % 2) && ok;
+    tc::fence_after_barrier();
+    if (warp % 4 < 2) {
 #pragma unroll
-        for (int b = 0; b < 8; ++b) acc[a][b] = fmaf(av[a], bv[b], acc[a][b]);
+      for (int j = 0; j < 32; j += 16) {
+        uint32_t v[16];
+        tc::read16(mine + n % 2 * 64 + j, v);
+        tc::reads_done();
+#pragma unroll
+        for (int a = 0; a < 16; ++a) main_sum[j + a] += __uint_as_float(v[a]);
+      }
     }
-    if (i0 == 0) {
-#pragma unroll 8
-      for (int r = 0; r < kWgChunk; ++r) bias_acc += s_dy[buf][r][tid];
-    }
-    __syncthreads();                                 // the next iteration's copies overwrite this buffer
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  float* out = p.partial + int64_t(blockIdx.x) * (int64_t(p.out) * p.in + p.out);
+  };
+  int n = 0;
+  for (; chunk < chunks; chunk += gridDim.x, ++n) {
+    const uint32_t b_dy = s_dy + n % 2 * (6 * kWgPiece), b_x = b_dy + 3 * kWgPiece;
 #pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int o = o0 + (a < 4 ? 4 * ty + a : 32 + 4 * ty + a - 4);
-    if (o >= p.out) continue;
-    *reinterpret_cast<float4*>(out + int64_t(o) * p.in + i0 + 4 * tx) = make_float4(acc[a][0], acc[a][1], acc[a][2], acc[a][3]);
-    *reinterpret_cast<float4*>(out + int64_t(o) * p.in + i0 + 32 + 4 * tx) = make_float4(acc[a][4], acc[a][5], acc[a][6], acc[a][7]);
+    for (int i = 0; i < kWgChunk / 16; ++i) {
+      tc::store4(b_dy, kWgPiece, tc::tile_offset(r0 + 16 * i, q), tc::split4(dy[i]));
+      tc::store4(b_x, kWgPiece, tc::tile_offset(r0 + 16 * i, q), tc::split4(x[i]));
+      bias.x += dy[i].x; bias.y += dy[i].y; bias.z += dy[i].z; bias.w += dy[i].w;
+    }
+    tc::publish_operands();
+    tc::fence_before_barrier();
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    if (tid == 0) {
+      tc::fence_after_barrier();
+      constexpr uint32_t one = tc::instruction(128, 64, true, true);
+#pragma unroll
+      for (int k = 0; k < kWgChunk / 16; ++k) {
+        const uint64_t dy12 = tc::mn_major(b_dy + 2048 * k, kWgPiece), dy23 = tc::mn_major(b_dy + kWgPiece + 2048 * k, kWgPiece);
+        const uint64_t x1 = tc::mn_major(b_x + 2048 * k, kWgPiece), x2 = tc::mn_major(b_x + kWgPiece + 2048 * k, kWgPiece),
+                       x3 = tc::mn_major(b_x + 2 * kWgPiece + 2048 * k, kWgPiece);
+        // lanes 0..63 | 64..127 of columns 0..63 or 64..127: dy1 x1 | dy2 x1 (not used), afresh in every chunk, of columns
+        // 128..191: dy1 x2 + dy1 x3 + dy2 x1 | dy2 x2 + dy2 x3 + dy3 x1
+        tc::multiply(tmem + n % 2 * 64, dy12, x1, one, k > 0);
+        tc::multiply(tmem + 128, dy12, x2, one, n + k > 0);
+        tc::multiply(tmem + 128, dy12, x3, one, true);
+        tc::multiply(tmem + 128, dy23, x1, one, true);
+      }
+      tc::commit(s_done + n % 2);
+    }
+    if (chunk + gridDim.x < chunks) load(chunk + gridDim.x);
+    if (n > 0) drain(n - 1);
   }
-  if (i0 == 0 && o0 + tid < p.out) out[int64_t(p.out) * p.in + o0 + tid] = bias_acc;
+  if (n > 0) drain(n - 1);
+  // the small products of lanes 64..127 go to the warps that hold the same rows of the large ones
+  __syncthreads();
+  float* const s_small = reinterpret_cast<float*>(s_base);       // [64][65]
+  float4* const s_bias = reinterpret_cast<float4*>(s_base + 64 * 65 * 4);   // [16][16]
+  const bool any = int64_t(blockIdx.x) < chunks;
+  if (warp % 4 >= 2 && any) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 16) {
+      uint32_t v[16];
+      tc::read16(mine + 128 + j, v);
+      tc::reads_done();
+#pragma unroll
+      for (int a = 0; a < 16; ++a) s_small[(warp % 4 * 32 - 64 + lane) * 65 + warp / 4 * 32 + j + a] = __uint_as_float(v[a]);
+    }
+  }
+  s_bias[r0 * 16 + tid % 16] = bias;
+  __syncthreads();
+  float* out = p.partial + (int64_t(blockIdx.x) * p.count + which) * (int64_t(p.out) * p.in + p.out);
+  if (warp % 4 < 2) {
+    const int row = warp % 4 * 32 + lane;
+#pragma unroll
+    for (int j = 0; j < 32; j += 16) {
+      uint32_t v[16];
+      if (any) tc::read16(mine + 128 + j, v);
+      tc::reads_done();
+#pragma unroll
+      for (int a = 0; a < 16; a += 4) {
+        const int col = warp / 4 * 32 + j + a;
+        if (o0 + row >= p.out || i0 + col >= p.in) continue;
+        float f[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          f[b] = any ? main_sum[j + a + b] + (__uint_as_float(v[a + b]) + s_small[row * 65 + col + b]) : 0.f;
+          if (!(fabsf(f[b]) < __int_as_float(0x7f800000))) f[b] = exact_sum(p, from, o0 + row, i0 + col + b);
+          if (!ok) f[b] = __int_as_float(0x7fffffff);
+        }
+        *reinterpret_cast<float4*>(out + int64_t(o0 + row) * p.in + i0 + col) = make_float4(f[0], f[1], f[2], f[3]);
+      }
+      __syncwarp();
+    }
+  }
+  if (i0 == 0 && tid < 64 && o0 + tid < p.out) {
+    float s = 0.f;
+    for (int r = 0; r < 16; ++r) s += reinterpret_cast<const float*>(s_bias)[r * 64 + tid];
+    out[int64_t(p.out) * p.in + o0 + tid] = s;
+  }
+  tc::fence_before_barrier();
+  __syncthreads();
+  if (warp == 0) tc::release<kWgTmemCols>(tmem);
 }
 
-// dw[j] = sum over CTAs of partial[cta][j], db likewise (db may be null); sum_partials: fixed association.
-__global__ void __launch_bounds__(kPartialSumThreads) linear_wgrad_sum_kernel(const float* __restrict__ partial,
-                                                                              int ctas, int n_w, int n_b,
-                                                                              float* __restrict__ dw,
-                                                                              float* __restrict__ db) {
+struct WgradSumParams {
+  const float* partial;
+  float* dw[kMostGrads];
+  float* db[kMostGrads];         // may be null
+  int ctas, count, n_w, n_b;
+};
+
+// dw[j] = sum over CTAs of partial[cta][j], db likewise; sum_partials: fixed association.
+__global__ void __launch_bounds__(kPartialSumThreads) linear_wgrad_sum_kernel(const __grid_constant__ WgradSumParams p) {
   __shared__ float s_part[16][32];
-  const int i = blockIdx.x * 32 + threadIdx.x % 32;
-  const bool live = i < n_w + n_b;
-  const float s = sum_partials(partial, ctas, int64_t(n_w) + n_b, i, live, s_part);
+  const int i = blockIdx.x * 32 + threadIdx.x % 32, each = p.n_w + p.n_b;
+  const bool live = i < p.count * each;
+  const float s = sum_partials(p.partial, p.ctas, int64_t(p.count) * each, i, live, s_part);
   if (threadIdx.x < 32 && live) {
-    if (i < n_w) dw[i] = s;
-    else if (db != nullptr) db[i - n_w] = s;
+    const int which = i / each, j = i % each;
+    if (j < p.n_w) p.dw[which][j] = s;
+    else if (p.db[which] != nullptr) p.db[which][j - p.n_w] = s;
   }
 }
 
@@ -121,11 +209,12 @@ bool wgrad_supported(int in, int out) {
   return in >= kWgTile && in % kWgTile == 0 && in <= 1024 && out >= 4 && out % 4 == 0 && out <= 1024;
 }
 int wgrad_out_tiles(int out) { return (out + kWgTile - 1) / kWgTile; }
+constexpr int kWgSmem = 12 * kWgPiece + 32;     // two buffers, two barriers and the tensor memory's address
 
-int wgrad_grid(int64_t rows, int in, int out) {
-  const int tiles = (in / kWgTile) * wgrad_out_tiles(out);
+int wgrad_grid(int64_t rows, int in, int out, int count) {
+  const int tiles = (in / kWgTile) * wgrad_out_tiles(out) * count;
   const int64_t chunks = (rows + kWgChunk - 1) / kWgChunk;
-  int64_t g = int64_t(sm_count()) * 4 / tiles;     // about four CTAs (of two warps) per SM over all tiles
+  int64_t g = int64_t(sm_count()) * 2 / tiles;     // the two CTAs an SM holds, over all tiles
   if (g < 1) g = 1;
   if (g > chunks) g = chunks < 1 ? 1 : chunks;
   return int(g);
@@ -135,43 +224,68 @@ int wgrad_grid(int64_t rows, int in, int out) {
 }  // namespace tgt
 
 extern "C" int tgt_linear_wgrad_scratch_bytes(int64_t rows, int in_features, int out_features, size_t* bytes) {
+  return tgt_linear_wgrad_multi_scratch_bytes(1, rows, in_features, out_features, bytes);
+}
+
+extern "C" int tgt_linear_wgrad_multi_scratch_bytes(int count, int64_t rows, int in_features, int out_features, size_t* bytes) {
   using namespace tgt;
   TGT_CHECK_ARG(bytes != nullptr, "bytes is null");
   TGT_CHECK_ARG(rows >= 0, "rows must be >= 0");
+  TGT_CHECK_ARG(count >= 1 && count <= kMostGrads, "count must be 1 to %d", kMostGrads);
   if (!wgrad_supported(in_features, out_features))
     return set_error(TGT_ERR_UNSUPPORTED, "in_features=%d out_features=%d: in_features must be a multiple of 64, out_features of 4, both at most 1024",
                      in_features, out_features);
-  *bytes = size_t(wgrad_grid(rows, in_features, out_features)) *
+  *bytes = size_t(wgrad_grid(rows, in_features, out_features, count)) * count *
            (size_t(in_features) * out_features + out_features) * sizeof(float);
   return TGT_OK;
 }
 
 extern "C" int tgt_linear_wgrad(const float* dy, const float* x, int64_t rows, int in_features, int out_features,
-                                float* dw, float* db, void* scratch, size_t scratch_bytes, void* stream_) {
+                                float* dw, float* db, void* scratch, size_t scratch_bytes, void* stream) {
+  return tgt_linear_wgrad_multi(&dy, x, 1, rows, in_features, out_features, &dw, &db, scratch, scratch_bytes, stream);
+}
+
+extern "C" int tgt_linear_wgrad_multi(const float* const* dy, const float* x, int count, int64_t rows, int in_features,
+                                      int out_features, float* const* dw, float* const* db, void* scratch,
+                                      size_t scratch_bytes, void* stream_) {
   using namespace tgt;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
   TGT_CHECK_ARG(rows >= 0, "rows must be >= 0");
+  TGT_CHECK_ARG(count >= 1 && count <= kMostGrads, "count must be 1 to %d", kMostGrads);
   if (!wgrad_supported(in_features, out_features))
     return set_error(TGT_ERR_UNSUPPORTED, "in_features=%d out_features=%d: in_features must be a multiple of 64, out_features of 4, both at most 1024",
                      in_features, out_features);
-  TGT_CHECK_ARG(dw != nullptr, "dw must not be null");
+  TGT_CHECK_ARG(dy && dw && db, "dy, dw and db must not be null");
   const size_t n_w = size_t(in_features) * out_features;
+  WgradParams p{};
+  WgradSumParams q{};
+  for (int i = 0; i < count; ++i) {
+    TGT_CHECK_ARG(dw[i] != nullptr, "dw must not be null");
+    TGT_CHECK_ARG(rows == 0 || (dy[i] && x), "dy and x must not be null");
+    TGT_CHECK_ARG(aligned16(dy[i]) && aligned16(dw[i]), "tensors must be 16-byte aligned");
+    p.dy[i] = dy[i];
+    q.dw[i] = dw[i]; q.db[i] = db[i];
+  }
   if (rows == 0) {
-    TGT_CHECK_CUDA(cudaMemsetAsync(dw, 0, n_w * sizeof(float), stream));
-    if (db != nullptr) TGT_CHECK_CUDA(cudaMemsetAsync(db, 0, size_t(out_features) * sizeof(float), stream));
+    for (int i = 0; i < count; ++i) {
+      TGT_CHECK_CUDA(cudaMemsetAsync(dw[i], 0, n_w * sizeof(float), stream));
+      if (db[i] != nullptr) TGT_CHECK_CUDA(cudaMemsetAsync(db[i], 0, size_t(out_features) * sizeof(float), stream));
+    }
     return TGT_OK;
   }
-  TGT_CHECK_ARG(dy && x, "dy and x must not be null");
-  TGT_CHECK_ARG(aligned16(dy) && aligned16(x) && aligned16(dw) && aligned16(scratch), "tensors must be 16-byte aligned");
-  const int grid = wgrad_grid(rows, in_features, out_features);
-  const size_t need = size_t(grid) * (n_w + out_features) * sizeof(float);
+  TGT_CHECK_ARG(aligned16(x) && aligned16(scratch), "tensors must be 16-byte aligned");
+  const int grid = wgrad_grid(rows, in_features, out_features, count);
+  const size_t need = size_t(grid) * count * (n_w + out_features) * sizeof(float);
   if (scratch == nullptr || scratch_bytes < need)
     return set_error(TGT_ERR_WORKSPACE, "scratch holds %zu bytes, %zu needed", scratch_bytes, need);
-  WgradParams p{dy, x, static_cast<float*>(scratch), rows, in_features, out_features};
-  const dim3 g(grid, (in_features / kWgTile) * wgrad_out_tiles(out_features));
-  linear_wgrad_kernel<<<g, kWgThreads, 0, stream>>>(p);
-  const int n = int(n_w) + out_features;
-  linear_wgrad_sum_kernel<<<(n + 31) / 32, kPartialSumThreads, 0, stream>>>(p.partial, grid, int(n_w), out_features, dw, db);
+  const int rc = allow_shared_memory<linear_wgrad_kernel>(kWgSmem);
+  if (rc != TGT_OK) return rc;
+  p.x = x; p.partial = static_cast<float*>(scratch); p.rows = rows; p.in = in_features; p.out = out_features; p.count = count;
+  const dim3 g(grid, (in_features / kWgTile) * wgrad_out_tiles(out_features) * count);
+  linear_wgrad_kernel<<<g, kWgThreads, kWgSmem, stream>>>(p);
+  q.partial = p.partial; q.ctas = grid; q.count = count; q.n_w = int(n_w); q.n_b = out_features;
+  const int n = count * (q.n_w + q.n_b);
+  linear_wgrad_sum_kernel<<<(n + 31) / 32, kPartialSumThreads, 0, stream>>>(q);
   TGT_CHECK_CUDA(cudaGetLastError());
   return TGT_OK;
 }

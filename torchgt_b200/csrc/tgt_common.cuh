@@ -39,6 +39,22 @@ int current_device();
 // B200).  Grids and tile plans are sized from it.
 int sm_count();
 
+#ifdef __CUDACC__
+// Lets Kernel have up to `bytes` of dynamic shared memory: a property of the function on a device, set once for each
+// (by several threads at the same time is harmless).
+template <auto Kernel>
+inline int allow_shared_memory(int bytes) {
+  static bool allowed[kMaxDevices] = {};
+  const int dev = current_device();
+  if (dev < 0) return TGT_ERR_CUDA;
+  if (!__atomic_load_n(&allowed[dev], __ATOMIC_ACQUIRE)) {
+    TGT_CHECK_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    __atomic_store_n(&allowed[dev], true, __ATOMIC_RELEASE);
+  }
+  return TGT_OK;
+}
+#endif
+
 inline size_t round_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // ---- programmatic dependent launch ----------------------------------------------------------------
