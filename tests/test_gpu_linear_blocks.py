@@ -1,0 +1,163 @@
+"""The projections of one input as one node and the feed-forward block as one node against the modules in fp64, and the
+calls that have to go through the modules."""
+import pytest
+import torch
+from torch import nn
+
+pytestmark = pytest.mark.gpu
+
+# 2-norm, relative: chains of two products of at most 192 terms, each sum within 192^0.5 * 2^-23 of itself
+TOL = 4e-6
+
+
+@pytest.fixture(autouse=True)
+def full_fp32():
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    yield
+    torch.backends.cuda.matmul.allow_tf32 = before
+
+
+def _rel(got, ref):
+    return float((got.detach().double() - ref.detach()).norm() / ref.detach().norm().clamp_min(1e-30))
+
+
+def _layers(n, inp, out, bias=True):
+    from torchgt_b200.linear import Linear
+    return [Linear(inp, out, bias=bias).cuda() for _ in range(n)]
+
+
+def _double(module):
+    ref = nn.Linear(module.in_features, module.out_features, bias=module.bias is not None).cuda().double()
+    ref.load_state_dict({k: v.double() for k, v in module.state_dict().items()})
+    return ref
+
+
+def _compare(outs, refs, x, x64, modules, modules64, extra=(), extra64=()):
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    dy = [torch.randn(o.shape, generator=gen, device="cuda") for o in outs]
+    leaves = [x, *extra, *(p for m in modules for p in m.parameters())]
+    leaves64 = [x64, *extra64, *(p for m in modules64 for p in m.parameters())]
+    for got, ref in zip(outs, refs):
+        assert got.shape == ref.shape and _rel(got, ref) < TOL
+    got = torch.autograd.grad(outs, leaves, dy)
+    ref = torch.autograd.grad(refs, leaves64, [d.double() for d in dy])
+    for g, r in zip(got, ref):
+        assert g.shape == r.shape and _rel(g, r) < TOL
+
+
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("shape,out", [((1023, 64), 64), ((1024, 64), 64), ((3, 700, 64), 64), ((1, 2689, 64), 64), ((30001, 128), 64), ((9000, 64), 100)])
+def test_three_projections(shape, out, bias):
+    from torchgt_b200.linear import linear3
+    torch.manual_seed(shape[-2])
+    layers = _layers(3, shape[-1], out, bias)
+    x = torch.randn(shape, device="cuda").requires_grad_()
+    y = linear3(x, *layers)
+    if x.numel() // shape[-1] >= 1024:
+        assert "NarrowLinear3" in y[0].grad_fn.name() and y[0].grad_fn is y[2].grad_fn
+    x64, layers64 = x.detach().double().requires_grad_(), [_double(m) for m in layers]
+    _compare(y, [m(x64) for m in layers64], x, x64, layers, layers64)
+    with torch.no_grad():
+        assert all(torch.equal(a, b.detach()) for a, b in zip(linear3(x, *layers), y))
+
+
+@pytest.mark.parametrize("act", ["relu", "gelu"])
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("shape,mid", [((1023, 64), 64), ((1024, 64), 64), ((1, 2000, 64), 128), ((20001, 64), 128), ((9000, 128), 64)])
+def test_feed_forward(shape, mid, residual, act):
+    from torchgt_b200.linear import feed_forward
+    torch.manual_seed(shape[-2] + mid)
+    layers = _layers(1, shape[-1], mid) + _layers(1, mid, shape[-1])
+    x = torch.randn(shape, device="cuda").requires_grad_()
+    r = torch.randn(shape, device="cuda").requires_grad_() if residual else None
+    y = feed_forward(x, *layers, act, r)
+    if x.numel() // shape[-1] >= 1024:
+        assert "FeedForward" in y.grad_fn.name()
+    x64, layers64 = x.detach().double().requires_grad_(), [_double(m) for m in layers]
+    r64 = r.detach().double().requires_grad_() if residual else None
+    fn = torch.relu if act == "relu" else nn.functional.gelu
+    ref = layers64[1](fn(layers64[0](x64)))
+    _compare([y], [ref + r64 if residual else ref], x, x64, layers, layers64, [r] if residual else [], [r64] if residual else [])
+    with torch.no_grad():
+        assert torch.equal(feed_forward(x, *layers, act, r), y.detach())
+
+
+def test_a_missing_gradient_and_gradients_nobody_wants():
+    from torchgt_b200.linear import feed_forward, linear3
+    torch.manual_seed(0)
+    layers = _layers(3, 64, 64)
+    x = torch.randn(1500, 64, device="cuda").requires_grad_()
+    q, k, v = linear3(x, *layers)
+    (q.sum() + 2 * v.sum()).backward()
+    assert layers[1].weight.grad is None or not layers[1].weight.grad.any()
+    ref = (layers[0].weight.detach().double().sum(0) + 2 * layers[2].weight.detach().double().sum(0)).expand(1500, 64)
+    assert _rel(x.grad, ref) < TOL
+    layers[0].weight.requires_grad_(False)
+    layers[0].bias.requires_grad_(False)
+    y = feed_forward(x.detach(), layers[0], layers[1], "relu")
+    layers[1].weight.grad = None
+    y.sum().backward()
+    assert layers[1].weight.grad is not None
+
+
+def test_second_order_gradients():
+    from torchgt_b200.linear import feed_forward, linear3
+    torch.manual_seed(1)
+    layers = _layers(3, 64, 64)
+    layers64 = [_double(m) for m in layers]
+    x = torch.randn(1100, 64, device="cuda").requires_grad_()
+    x64 = x.detach().double().requires_grad_()
+    for act, fn in (("relu", torch.relu), ("gelu", nn.functional.gelu)):
+        y, ref = feed_forward(x, layers[0], layers[1], act, x), x64 + layers64[1](fn(layers64[0](x64)))
+        got, want = [], []
+        for out, leaf, w, into in ((y, x, layers[0].weight, got), (ref, x64, layers64[0].weight, want)):
+            g, = torch.autograd.grad((out * out).sum(), leaf, create_graph=True)
+            into.extend(torch.autograd.grad((g * g).sum(), [leaf, w]))
+        assert all(_rel(a, b) < 1e-5 for a, b in zip(got, want))
+    g, = torch.autograd.grad(sum(t.sum() for t in linear3(x, *layers)), x, create_graph=True)
+    dw, = torch.autograd.grad((g * g).sum(), layers[1].weight)
+    total = sum(m.weight.detach().double().sum(0) for m in layers)
+    assert _rel(dw, (2 * 1100 * total).expand(64, 64)) < 1e-5
+
+
+def test_infinities_and_nan_pass_as_through_the_modules():
+    from torchgt_b200.linear import feed_forward, linear3
+    torch.manual_seed(2)
+    layers = _layers(3, 64, 64)
+    for rows in (1300, 9000):
+        x = torch.randn(rows, 64, device="cuda")
+        x[3, 7], x[11, 0] = float("inf"), float("nan")
+        with torch.no_grad():
+            refs = [nn.functional.linear(x, m.weight, m.bias) for m in layers]
+            outs = linear3(x, *layers)
+            for act, fn in (("relu", torch.relu), ("gelu", nn.functional.gelu)):
+                outs = [*outs, feed_forward(x, layers[0], layers[1], act)]
+                refs.append(nn.functional.linear(fn(refs[0]), layers[1].weight, layers[1].bias))
+        for y, ref in zip(outs, refs):
+            assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isinf(), ref.isinf())
+
+
+def test_layers_that_differ_and_observed_modules_are_called_one_by_one():
+    from torchgt_b200.linear import Linear, feed_forward, linear3, passes_through
+    torch.manual_seed(3)
+    a, b = _layers(2, 64, 64)
+    c = Linear(64, 128).cuda()
+    x = torch.randn(10, 64, device="cuda")
+    outs = linear3(x, a, b, c)
+    assert [tuple(o.shape) for o in outs] == [(10, 64), (10, 64), (10, 128)]
+    seen = []
+    handle = a.register_forward_hook(lambda m, i, o: seen.append(m))
+    linear3(x, a, b, b)
+    assert seen == [a] and feed_forward(x, a, b, "relu") is None
+    handle.remove()
+    assert feed_forward(x, a, b, "relu") is not None
+    assert feed_forward(x, Linear(64, 64, bias=False).cuda(), b, "relu") is None
+    y = feed_forward(x, Linear(64, 44).cuda(), Linear(44, 64).cuda(), "gelu", x)       # no kernel: 44 wide in between
+    assert y.shape == x.shape
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert feed_forward(x, a, b, "relu") is None and linear3(x, a, b, b)[0].dtype == torch.bfloat16
+    z = torch.func.vmap(lambda t: linear3(t, a, b, b)[1])(torch.randn(3, 5, 64, device="cuda"))
+    assert z.shape == (3, 5, 64)
+    drop = nn.Dropout(0.1).train()
+    assert not passes_through(drop) and passes_through(drop.eval()) and passes_through(nn.Dropout(0.0).train())

@@ -145,6 +145,233 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<
   return y;
 }
 
+// ---- three layers of one input: the query, key and value projections ---------------------------------------------
+// Parameter gradients of up to three layers of one input, in one pass over it; db[i] may be null.
+void parameter_gradients(const std::vector<at::Tensor>& dy, const at::Tensor& x, int64_t rows, int64_t in, int64_t out,
+                         const std::vector<at::Tensor*>& dw, const std::vector<at::Tensor*>& db) {
+  const int n = int(dy.size());
+  size_t bytes = 0;
+  check(tgt_linear_wgrad_multi_scratch_bytes(n, rows, int(in), int(out), &bytes));
+  const at::Tensor scratch = at::empty({int64_t(bytes < 16 ? 16 : bytes)}, x.options().dtype(at::kByte));
+  const float* from[3];
+  float *w[3], *b[3];
+  for (int i = 0; i < n; ++i) {
+    from[i] = fptr(dy[i]);
+    *dw[i] = at::empty({out, in}, x.options());
+    w[i] = fptr(*dw[i]);
+    if (db[i] != nullptr) *db[i] = at::empty({out}, x.options());
+    b[i] = db[i] != nullptr ? fptr(*db[i]) : nullptr;
+  }
+  check(tgt_linear_wgrad_multi(from, fptr(x), n, rows, int(in), int(out), w, b, scratch.data_ptr(), scratch.numel(),
+                               stream_of(x)));
+}
+
+struct NarrowLinear3Backward : public torch::autograd::Node {
+  SavedVariable x, weight[3];
+  bool has_bias = false;
+
+  variable_list apply(variable_list&& grads) override {
+    return reporting([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
+    variable_list result(7);
+    const at::Tensor x_ = x.unpack();
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const bool want_dx = task_should_compute_output(0), recorded = at::GradMode::is_enabled();
+    std::vector<at::Tensor> dy, w, dy_p;
+    std::vector<at::Tensor*> dw, db;
+    for (int i = 0; i < 3; ++i) {
+      if (!grads[i].defined()) continue;
+      const at::Tensor w_ = weight[i].unpack();
+      if (want_dx && recorded) {       // a second-order gradient is wanted: dx as recorded products
+        const at::Tensor d = at::matmul(grads[i], w_);
+        result[0] = result[0].defined() ? result[0] + d : d;
+      }
+      const at::AutoDispatchBelowADInplaceOrView below;
+      dy.push_back(kernel_ready(grads[i]));
+      w.push_back(kernel_ready(w_));
+      if (!task_should_compute_output(1 + 2 * i) && !(has_bias && task_should_compute_output(2 + 2 * i))) continue;
+      dy_p.push_back(dy.back());
+      dw.push_back(&result[1 + 2 * i]);
+      db.push_back(has_bias ? &result[2 + 2 * i] : nullptr);
+    }
+    if (dy.empty()) return result;
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const int64_t out = w[0].size(0), in = w[0].size(1), rows = x_.numel() / in;
+    if (want_dx && !recorded) {
+      const float *from[3], *by[3];
+      for (size_t i = 0; i < dy.size(); ++i) {
+        from[i] = fptr(dy[i]);
+        by[i] = fptr(w[i]);
+      }
+      result[0] = at::empty(x_.sizes(), dy[0].options());
+      check(tgt_linear_input_grad_multi(from, by, int(dy.size()), rows, int(out), int(in), TGT_ACT_NONE, nullptr,
+                                        fptr(result[0]), stream_of(x_)));
+    }
+    if (!dy_p.empty()) parameter_gradients(dy_p, kernel_ready(x_), rows, in, out, dw, db);
+    return result;
+  }
+  std::string name() const override { return "NarrowLinear3Backward"; }
+  void release_variables() override {
+    x.reset_data();
+    for (SavedVariable& w : weight) w.reset_data();
+  }
+};
+
+// Shorter inputs keep the library's rounding, as the single layer does (rows_kernel_ahead).
+constexpr int64_t kBlockRows = 1024;
+
+// {x w_i^T + b_i}
+std::vector<at::Tensor> linear3(const at::Tensor& x, const std::vector<at::Tensor>& w,
+                                const std::vector<std::optional<at::Tensor>>& bias_in) {
+  TORCH_CHECK(w.size() == 3 && bias_in.size() == 3, "linear3 takes three layers");
+  std::vector<at::Tensor> bias;
+  bool together = true;
+  for (int i = 0; i < 3; ++i) {
+    bias.push_back(bias_in[i].has_value() ? *bias_in[i] : at::Tensor());
+    together = together && eligible(x, w[i], bias[i]) && w[i].sizes() == w[0].sizes() && bias[i].defined() == bias[0].defined();
+  }
+  if (!together || x.numel() / w[0].size(1) < kBlockRows)
+    return {tgt_host::linear(x, w[0], bias_in[0]), tgt_host::linear(x, w[1], bias_in[1]), tgt_host::linear(x, w[2], bias_in[2])};
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t out = w[0].size(0), in = w[0].size(1), rows = x.numel() / in;
+  variable_list y;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const at::Tensor xc = kernel_ready(x);
+    auto sizes = x.sizes().vec();
+    sizes.back() = out;
+    std::vector<at::Tensor> kept;      // copies, while the launch needs them
+    const float *by[3], *b[3];
+    float* c[3];
+    for (int i = 0; i < 3; ++i) {
+      kept.push_back(kernel_ready(w[i]));
+      by[i] = fptr(kept.back());
+      if (bias[i].defined()) kept.push_back(kernel_ready(bias[i]));
+      b[i] = bias[i].defined() ? fptr(kept.back()) : nullptr;
+      y.push_back(at::empty(sizes, x.options()));
+      c[i] = fptr(y[i]);
+    }
+    check(tgt_linear_rows_multi(fptr(xc), by, b, 3, rows, int(in), int(out), TGT_ACT_NONE, nullptr, nullptr, c, stream_of(x)));
+  }
+  if (torch::autograd::compute_requires_grad(x, w[0], w[1], w[2], bias[0], bias[1], bias[2])) {
+    auto node = std::shared_ptr<NarrowLinear3Backward>(new NarrowLinear3Backward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, w[0], bias[0], w[1], bias[1], w[2], bias[2]));
+    node->has_bias = bias[0].defined();
+    node->x = SavedVariable(x, false);
+    for (int i = 0; i < 3; ++i) node->weight[i] = SavedVariable(w[i], false);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
+// ---- feed-forward block: act(x w1^T + b1) w2^T + b2 (+ residual) ---------------------------------------------------
+struct FeedForwardBackward : public torch::autograd::Node {
+  SavedVariable x, w1, b1, w2, hidden, gate;   // gate: the activation's input (relu: its result says enough)
+  int act = TGT_ACT_NONE;
+  bool with_residual = false;
+
+  variable_list apply(variable_list&& grads) override {
+    return reporting([&] { return backward(grads); });
+  }
+  // With create_graph the gradient is itself differentiated: the block's formula as recorded operations.
+  variable_list recorded(const at::Tensor& dy, const at::Tensor& x_, const at::Tensor& w1_, const at::Tensor& w2_) {
+    const at::Tensor z = at::linear(x_, w1_, b1.unpack());
+    const at::Tensor h = act == TGT_ACT_RELU ? at::relu(z) : at::gelu(z);
+    const at::Tensor dh = at::matmul(dy, w2_);
+    const at::Tensor dz = act == TGT_ACT_RELU ? dh * (z > 0).to(dh.scalar_type()) : at::gelu_backward(dh, z);
+    auto flat = [](const at::Tensor& t) { return t.reshape({-1, t.size(-1)}); };
+    return {at::matmul(dz, w1_), at::matmul(flat(dz).t(), flat(x_)), flat(dz).sum(0), at::matmul(flat(dy).t(), flat(h)),
+            flat(dy).sum(0), with_residual ? dy : at::Tensor()};
+  }
+  variable_list backward(const variable_list& grads) {
+    variable_list result(6);
+    if (!grads[0].defined()) return result;
+    const at::Tensor x_ = x.unpack(), w1_ = w1.unpack(), w2_ = w2.unpack();
+    if (at::GradMode::is_enabled()) return recorded(grads[0], x_, w1_, w2_);
+    if (with_residual) result[5] = grads[0];
+    const at::Tensor h = hidden.unpack(), gate_ = act == TGT_ACT_RELU ? h : gate.unpack();
+    const c10::cuda::CUDAGuard guard(x_.device());
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const at::Tensor dy = kernel_ready(grads[0]), w2c = kernel_ready(w2_), hc = kernel_ready(h), gc = kernel_ready(gate_);
+    const int64_t in = w1_.size(1), mid = w1_.size(0), out = w2_.size(0), rows = x_.numel() / in;
+    if (task_should_compute_output(3) || task_should_compute_output(4))
+      parameter_gradients({dy}, hc, rows, mid, out, {&result[3]}, {&result[4]});
+    const bool first = task_should_compute_output(1) || task_should_compute_output(2);
+    if (!first && !task_should_compute_output(0)) return result;
+    const at::Tensor dz = at::empty(h.sizes(), h.options());
+    const float *from = fptr(dy), *by = fptr(w2c);
+    check(tgt_linear_input_grad_multi(&from, &by, 1, rows, int(out), int(mid), act, fptr(gc), fptr(dz), stream_of(x_)));
+    if (first) parameter_gradients({dz}, kernel_ready(x_), rows, in, mid, {&result[1]}, {&result[2]});
+    if (task_should_compute_output(0)) {
+      const at::Tensor w1c = kernel_ready(w1_);
+      result[0] = at::empty(x_.sizes(), dz.options());
+      check(tgt_linear_input_grad(fptr(dz), fptr(w1c), rows, int(mid), int(in), fptr(result[0]), stream_of(x_)));
+    }
+    return result;
+  }
+  std::string name() const override { return "FeedForwardBackward"; }
+  void release_variables() override {
+    for (SavedVariable* v : {&x, &w1, &b1, &w2, &hidden, &gate}) v->reset_data();
+  }
+};
+
+bool feed_forward_eligible(const at::Tensor& x, const at::Tensor& w1, const at::Tensor& b1, const at::Tensor& w2,
+                           const at::Tensor& b2, const at::Tensor& residual) {
+  if (!b1.defined() || !b2.defined() || !eligible(x, w1, b1) || x.numel() / w1.size(1) < kBlockRows ||
+      !plain(w2, x.device()) || !plain(b2, x.device())) return false;
+  if (w2.dim() != 2 || w2.size(1) != w1.size(0) || b2.dim() != 1 || b2.size(0) != w2.size(0)) return false;
+  const int64_t mid = w2.size(1), out = w2.size(0);
+  if (mid % 64 != 0 || mid > 1024 || out % 4 != 0 || out < 4 || out > 1024) return false;
+  return !residual.defined() || (plain(residual, x.device()) && out == w1.size(1) && residual.sizes() == x.sizes());
+}
+
+at::Tensor feed_forward(const at::Tensor& x, const at::Tensor& w1, const at::Tensor& b1, const at::Tensor& w2,
+                        const at::Tensor& b2, const std::string& activation, const std::optional<at::Tensor>& residual_in) {
+  const at::Tensor residual = residual_in.has_value() ? *residual_in : at::Tensor();
+  const int act = activation == "relu" ? TGT_ACT_RELU : TGT_ACT_GELU;
+  if (!feed_forward_eligible(x, w1, b1, w2, b2, residual)) {
+    const at::Tensor z = tgt_host::linear(x, w1, b1);
+    const at::Tensor y = tgt_host::linear(act == TGT_ACT_RELU ? at::relu(z) : at::gelu(z), w2, b2);
+    return residual.defined() ? residual + y : y;
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t in = w1.size(1), mid = w1.size(0), out = w2.size(0), rows = x.numel() / in;
+  const bool record = torch::autograd::compute_requires_grad(x, w1, b1, w2, b2, residual);
+  at::Tensor y, h, z;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const at::Tensor xc = kernel_ready(x), w1c = kernel_ready(w1), b1c = kernel_ready(b1), w2c = kernel_ready(w2),
+                     b2c = kernel_ready(b2), rc = residual.defined() ? kernel_ready(residual) : residual;
+    auto sizes = x.sizes().vec();
+    sizes.back() = mid;
+    h = at::empty(sizes, x.options());
+    if (record && act == TGT_ACT_GELU) z = at::empty(sizes, x.options());
+    sizes.back() = out;
+    y = at::empty(sizes, x.options());
+    const float *by = fptr(w1c), *b = fptr(b1c);
+    float* c = fptr(h);
+    check(tgt_linear_rows_multi(fptr(xc), &by, &b, 1, rows, int(in), int(mid), act, fptr(z), nullptr, &c, stream_of(x)));
+    by = fptr(w2c); b = fptr(b2c); c = fptr(y);
+    check(tgt_linear_rows_multi(fptr(h), &by, &b, 1, rows, int(mid), int(out), TGT_ACT_NONE, nullptr,
+                                rc.defined() ? fptr(rc) : nullptr, &c, stream_of(x)));
+  }
+  if (record) {
+    auto node = std::shared_ptr<FeedForwardBackward>(new FeedForwardBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(x, w1, b1, w2, b2, residual));
+    node->act = act;
+    node->with_residual = residual.defined();
+    node->x = SavedVariable(x, false);
+    node->w1 = SavedVariable(w1, false);
+    node->b1 = SavedVariable(b1, false);
+    node->w2 = SavedVariable(w2, false);
+    node->hidden = SavedVariable(h, false);
+    node->gate = SavedVariable(z, false);
+    torch::autograd::set_history(y, node);
+  }
+  return y;
+}
+
 // ---- LayerNorm, with the residual addition in front of it ------------------------------------------------------
 // Outputs: the normalised rows and, with a residual, x + residual.
 struct LayerNormRowsBackward : public torch::autograd::Node {
@@ -257,6 +484,8 @@ at::Tensor layer_norm(const at::Tensor& x, const at::Tensor& w, const at::Tensor
 
 void bind_dense(pybind11::module_& m) {
   m.def("linear", &linear, Unlocked());
+  m.def("linear3", &linear3, Unlocked());
+  m.def("feed_forward", &feed_forward, Unlocked());
   m.def("layer_norm", &layer_norm, Unlocked());
   m.def("add_layer_norm", &add_layer_norm, Unlocked());
 }

@@ -19,7 +19,7 @@ from torch.nn import functional as F
 from .attn_module import CoreAttention
 from .gt_sp.initialize import get_sequence_parallel_group, sequence_parallel_is_initialized
 from .layer_norm import LayerNorm, add_layer_norm
-from .linear import Linear
+from .linear import Linear, feed_forward, linear3, passes_through, unobserved
 from .gt_sp.layer import DistributedAttentionNoMerge
 
 
@@ -67,17 +67,18 @@ class MultiHeadAttention(nn.Module):
     def forward(self, x, attn_bias=None, edge_index=None, attn_type=None, mask=None):
         b = x.size(0)
         use_sp = sequence_parallel_is_initialized() if self.sequence_parallel is None else self.sequence_parallel
+        if not use_sp:  # single process without a sequence-parallel group: the layer would only pass through
+            q, k, v = (t.view(b, -1, self.num_heads, self.att_size)
+                       for t in linear3(x, self.linear_q, self.linear_k, self.linear_v))
+            return self.output_layer(self.dist_attn.local_attn(q, k, v, attn_bias, edge_index, attn_type))
         q = self.linear_q(x).view(b, -1, self.num_heads, self.att_size)
         # the exchange of q starts now and runs under the next two projections; k follows under v's
-        pending = self.dist_attn.start_exchange(q, attn_bias, edge_index, attn_type) if use_sp else None
+        pending = self.dist_attn.start_exchange(q, attn_bias, edge_index, attn_type)
         k = self.linear_k(x).view(b, -1, self.num_heads, self.att_size)
         if pending is not None:
             pending.add(k)
         v = self.linear_v(x).view(b, -1, self.num_heads, self.att_size)
-        if use_sp:
-            ctx = self.dist_attn(q, k, v, attn_bias, edge_index, attn_type, pending=pending)
-        else:  # single process without a sequence-parallel group: the layer would only pass through
-            ctx = self.dist_attn.local_attn(q, k, v, attn_bias, edge_index, attn_type)
+        ctx = self.dist_attn(q, k, v, attn_bias, edge_index, attn_type, pending=pending)
         return self.output_layer(ctx)
 
 
@@ -122,6 +123,11 @@ class EncoderLayer(nn.Module):
         if y is None:
             y = self.self_attention(self.self_attention_norm(x), attn_bias, edge_index, attn_type=attn_type)
         normed, x = add_layer_norm(x, self.self_attention_dropout(y), self.ffn_norm)
+        if passes_through(self.ffn_dropout) and unobserved(self.ffn, FeedForwardNetwork) and \
+                unobserved(self.ffn.gelu, nn.GELU) and self.ffn.gelu.approximate == "none":
+            y = feed_forward(normed, self.ffn.layer1, self.ffn.layer2, "gelu", x)
+            if y is not None:
+                return y
         y = self.ffn(normed)
         return x + self.ffn_dropout(y)
 

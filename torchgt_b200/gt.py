@@ -20,7 +20,7 @@ from .attn_module import CoreAttentionQKV as CoreAttention  # (q, k, v) order, a
 from .gt_sp.gt_layer import DistributedAttention, DistributedAttentionNodeLevel, _SeqGather
 from .gt_sp.initialize import get_sequence_parallel_group, sequence_parallel_is_initialized
 from .layer_norm import LayerNorm, add_layer_norm
-from .linear import Linear
+from .linear import Linear, feed_forward, linear3, passes_through
 
 
 def _init_params(module: nn.Module, n_layers: int) -> None:
@@ -50,18 +50,21 @@ class MultiHeadAttention(nn.Module):
 
     def forward(self, x, attn_bias=None, mask=None, edge_index=None, attn_type=None):
         b = x.size(0)
-        use_sp = sequence_parallel_is_initialized()
+        if not sequence_parallel_is_initialized():  # without a group the layer would only pass through
+            q, k, v = (t.view(b, -1, self.num_heads, self.att_size)
+                       for t in linear3(x, self.linear_q, self.linear_k, self.linear_v))
+            return self._checked(x, self.dist_attn.local_attn(q, k, v, attn_bias, edge_index, attn_type))
         q = self.linear_q(x).view(b, -1, self.num_heads, self.att_size)
         # the exchange of q starts now and runs under the next two projections; k follows under v's
-        pending = self.dist_attn.start_exchange(q, attn_bias, edge_index, attn_type) if use_sp else None
+        pending = self.dist_attn.start_exchange(q, attn_bias, edge_index, attn_type)
         k = self.linear_k(x).view(b, -1, self.num_heads, self.att_size)
         if pending is not None:
             pending.add(k)
         v = self.linear_v(x).view(b, -1, self.num_heads, self.att_size)
-        if use_sp:
-            out = self.dist_attn(q, k, v, attn_bias, edge_index, attn_type, pending=pending)
-        else:  # single process without a sequence-parallel group: the layer would only pass through
-            out = self.dist_attn.local_attn(q, k, v, attn_bias, edge_index, attn_type)
+        return self._checked(x, self.dist_attn(q, k, v, attn_bias, edge_index, attn_type, pending=pending))
+
+    @staticmethod
+    def _checked(x, out):
         if out.size() != x.size():
             raise RuntimeError(f"attention returned {tuple(out.size())} for an input of {tuple(x.size())}")
         return out
@@ -85,7 +88,8 @@ class EncoderLayer(nn.Module):
         y = self.self_attention(x, attn_bias, mask=mask, edge_index=edge_index, attn_type=attn_type)
         y = self.O(self.self_attention_dropout(y))
         x, _ = add_layer_norm(x, y, self.layer_norm1, want_sum=False)
-        y = self.FFN_layer2(self.self_attention_dropout(F.relu(self.FFN_layer1(y))))
+        z = feed_forward(y, self.FFN_layer1, self.FFN_layer2, "relu") if passes_through(self.self_attention_dropout) else None
+        y = self.FFN_layer2(self.self_attention_dropout(F.relu(self.FFN_layer1(y)))) if z is None else z
         return add_layer_norm(x, y, self.layer_norm2, want_sum=False)[0]
 
 

@@ -13,6 +13,7 @@ import ctypes
 
 import torch
 from torch.nn import functional as F
+from torch.nn.modules import module as _module
 from torch.overrides import has_torch_function_variadic
 
 from . import _cabi
@@ -65,3 +66,35 @@ class Linear(torch.nn.Linear):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         return linear(x, self.weight, self.bias)
+
+
+def unobserved(module: torch.nn.Module, kind: type) -> bool:
+    """``module`` is a plain ``kind`` whose call nobody observes through module hooks."""
+    if type(module) is not kind or "forward" in module.__dict__:
+        return False
+    return not any((module._forward_hooks, module._forward_pre_hooks, module._backward_hooks, module._backward_pre_hooks,
+                    _module._global_forward_hooks, _module._global_forward_pre_hooks, _module._global_backward_hooks,
+                    _module._global_backward_pre_hooks))
+
+
+def linear3(x: torch.Tensor, a: torch.nn.Module, b: torch.nn.Module, c: torch.nn.Module):
+    """``a(x), b(x), c(x)``: one node that reads ``x`` once each way where the three are plain layers of equal shape."""
+    layers = (a, b, c)
+    if x.is_cuda and all(unobserved(m, Linear) and _plain_call(x, m.weight, m.bias) for m in layers):
+        return _cabi.native().linear3(x, [m.weight for m in layers], [m.bias for m in layers])
+    return a(x), b(x), c(x)
+
+
+def feed_forward(x: torch.Tensor, first: torch.nn.Module, second: torch.nn.Module, activation: str, residual=None):
+    """``(residual +) second(act(first(x)))`` with ``activation`` "relu" or "gelu" (exact), one node whose activation is
+    part of the products' kernels, or None where the caller has to go through the modules."""
+    if not (x.is_cuda and unobserved(first, Linear) and unobserved(second, Linear) and first.bias is not None and
+            second.bias is not None and _plain_call(x, first.weight, first.bias) and
+            not has_torch_function_variadic(second.weight, second.bias, residual)):
+        return None
+    return _cabi.native().feed_forward(x, first.weight, first.bias, second.weight, second.bias, activation, residual)
+
+
+def passes_through(dropout: torch.nn.Module) -> bool:
+    """``dropout`` returns its input as it is, and nobody observes the call."""
+    return unobserved(dropout, torch.nn.Dropout) and (not dropout.training or dropout.p == 0.0)
