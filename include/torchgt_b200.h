@@ -521,6 +521,20 @@ TGT_API int tgt_linear_wgrad_multi(const float* const* dy, const float* x, int c
                                    int out_features, float* const* dw, float* const* db, void* scratch,
                                    size_t scratch_bytes, void* stream);
 
+/*
+ * Sum of the embedding vectors of every row's integer features: out [rows, hidden] = sum_f table[ids[row][f]] for table
+ * [n_table, hidden] fp32 and ids [rows, features] int64 (models/gt_dist_graph_level.py:345), and its gradient: dtable
+ * [n_table, hidden], fixed summation order, zero in row padding_idx (none: -1).  hidden 32, 64 or 128, fewer than 2^26
+ * rows on either side and fewer than 2^31 - 1 pairs (TGT_ERR_UNSUPPORTED otherwise).  An id outside the table is a failed
+ * device assertion in the forward, as it is in torch.nn.Embedding; the gradient counts it for row 0.
+ */
+TGT_API int tgt_embedding_sum(const float* table, int64_t n_table, int hidden, const int64_t* ids, int64_t rows,
+                              int features, float* out, void* stream);
+TGT_API int tgt_embedding_sum_grad_scratch_bytes(int64_t n_table, int hidden, int64_t rows, int features, size_t* bytes);
+TGT_API int tgt_embedding_sum_grad(const float* dout, const int64_t* ids, int64_t rows, int features, int64_t n_table,
+                                   int hidden, int64_t padding_idx, float* dtable, void* scratch, size_t scratch_bytes,
+                                   void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -129,6 +129,10 @@ SIGNATURES = {
     "tgt_linear_wgrad_multi_scratch_bytes": (c_int, [c_int, c_int64, c_int, c_int, POINTER(c_size_t)]),
     "tgt_linear_wgrad_multi": (c_int, [c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p,
                                        c_size_t, c_void_p]),
+    "tgt_embedding_sum": (c_int, [c_void_p, c_int64, c_int, c_void_p, c_int64, c_int, c_void_p, c_void_p]),
+    "tgt_embedding_sum_grad_scratch_bytes": (c_int, [c_int64, c_int, c_int64, c_int, POINTER(c_size_t)]),
+    "tgt_embedding_sum_grad": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int64, c_int, c_int64, c_void_p, c_void_p,
+                                       c_size_t, c_void_p]),
     "tgt_linear_wgrad_scratch_bytes": (c_int, [c_int64, c_int, c_int, POINTER(c_size_t)]),
     "tgt_linear_wgrad": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t,
                                  c_void_p]),

@@ -372,6 +372,72 @@ at::Tensor feed_forward(const at::Tensor& x, const at::Tensor& w1, const at::Ten
   return y;
 }
 
+// ---- sum of embedding vectors ---------------------------------------------------------------------------------------
+struct EmbeddingSumBackward : public torch::autograd::Node {
+  SavedVariable ids;
+  int64_t n_table = 0, hidden = 0, padding = -1;
+
+  variable_list apply(variable_list&& grads) override {
+    return reporting([&] { return backward(grads); });
+  }
+  variable_list backward(const variable_list& grads) {
+    if (!grads[0].defined()) return variable_list(1);
+    const at::Tensor ids_ = ids.unpack();
+    if (at::GradMode::is_enabled()) {      // a second-order gradient is wanted: the library's recorded operation
+      auto sizes = ids_.sizes().vec();
+      sizes.push_back(hidden);
+      return {at::embedding_dense_backward(grads[0].unsqueeze(-2).expand(sizes), ids_, n_table, padding, false)};
+    }
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard guard(ids_.device());
+    const at::Tensor dy = kernel_ready(grads[0]), ic = ids_.contiguous();
+    const int64_t features = ids_.size(-1), rows = ids_.numel() / features;
+    size_t bytes = 0;
+    check(tgt_embedding_sum_grad_scratch_bytes(n_table, int(hidden), rows, int(features), &bytes));
+    const at::Tensor scratch = at::empty({int64_t(bytes)}, dy.options().dtype(at::kByte));
+    const at::Tensor dtable = at::empty({n_table, hidden}, dy.options());
+    check(tgt_embedding_sum_grad(fptr(dy), static_cast<const int64_t*>(ptr(ic)), rows, int(features), n_table, int(hidden),
+                                 padding, fptr(dtable), scratch.data_ptr(), scratch.numel(), stream_of(dy)));
+    return {dtable};
+  }
+  std::string name() const override { return "EmbeddingSumBackward"; }
+  void release_variables() override { ids.reset_data(); }
+};
+
+// embedding(ids).sum(-2)
+at::Tensor embedding_sum(const at::Tensor& table, const at::Tensor& ids, int64_t padding) {
+  constexpr int64_t kMost = int64_t(1) << 26;
+  const bool own = ids.defined() && table.defined() && !at::isTensorSubclassLike(ids) && plain(table, ids.device()) &&
+                   ids.is_cuda() && ids.layout() == at::kStrided && ids.scalar_type() == at::kLong && ids.dim() >= 1 &&
+                   ids.numel() > 0 && table.dim() == 2 &&
+                   (table.size(1) == 32 || table.size(1) == 64 || table.size(1) == 128) && table.size(0) >= 1 &&
+                   table.size(0) < kMost && ids.size(-1) <= 1024 && ids.numel() / ids.size(-1) < kMost &&
+                   ids.numel() < (int64_t(1) << 31) - 1;
+  if (!own) return at::embedding(table, ids, padding).sum(-2);
+  const c10::cuda::CUDAGuard guard(table.device());
+  const int64_t features = ids.size(-1), rows = ids.numel() / features, hidden = table.size(1);
+  at::Tensor out;
+  {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const at::Tensor tc = kernel_ready(table), ic = ids.contiguous();
+    auto sizes = ids.sizes().vec();
+    sizes.back() = hidden;
+    out = at::empty(sizes, table.options());
+    check(tgt_embedding_sum(fptr(tc), table.size(0), int(hidden), static_cast<const int64_t*>(ptr(ic)), rows, int(features),
+                            fptr(out), stream_of(table)));
+  }
+  if (torch::autograd::compute_requires_grad(table)) {
+    auto node = std::shared_ptr<EmbeddingSumBackward>(new EmbeddingSumBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(table));
+    node->ids = SavedVariable(ids, false);
+    node->n_table = table.size(0);
+    node->hidden = hidden;
+    node->padding = padding;
+    torch::autograd::set_history(out, node);
+  }
+  return out;
+}
+
 // ---- LayerNorm, with the residual addition in front of it ------------------------------------------------------
 // Outputs: the normalised rows and, with a residual, x + residual.
 struct LayerNormRowsBackward : public torch::autograd::Node {
@@ -485,6 +551,7 @@ at::Tensor layer_norm(const at::Tensor& x, const at::Tensor& w, const at::Tensor
 void bind_dense(pybind11::module_& m) {
   m.def("linear", &linear, Unlocked());
   m.def("linear3", &linear3, Unlocked());
+  m.def("embedding_sum", &embedding_sum, Unlocked());
   m.def("feed_forward", &feed_forward, Unlocked());
   m.def("layer_norm", &layer_norm, Unlocked());
   m.def("add_layer_norm", &add_layer_norm, Unlocked());

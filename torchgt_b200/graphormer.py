@@ -19,7 +19,7 @@ from torch.nn import functional as F
 from .attn_module import CoreAttention
 from .gt_sp.initialize import get_sequence_parallel_group, sequence_parallel_is_initialized
 from .layer_norm import LayerNorm, add_layer_norm
-from .linear import Linear, feed_forward, linear3, passes_through, unobserved
+from .linear import Linear, embedding_sum, feed_forward, linear3, passes_through, unobserved
 from .gt_sp.layer import DistributedAttentionNoMerge
 
 
@@ -186,7 +186,7 @@ class GraphNodeFeature(nn.Module):
 
     def forward(self, batched_data):
         x = batched_data.x
-        h = (self.atom_encoder(x).sum(dim=-2) + self.in_degree_encoder(batched_data.in_degree) +
+        h = (embedding_sum(self.atom_encoder, x) + self.in_degree_encoder(batched_data.in_degree) +
              self.out_degree_encoder(batched_data.out_degree))
         token = self.graph_token.weight.unsqueeze(0).expand(x.size(0), -1, -1)
         return torch.cat([token, h], dim=1)

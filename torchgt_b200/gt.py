@@ -20,7 +20,7 @@ from .attn_module import CoreAttentionQKV as CoreAttention  # (q, k, v) order, a
 from .gt_sp.gt_layer import DistributedAttention, DistributedAttentionNodeLevel, _SeqGather
 from .gt_sp.initialize import get_sequence_parallel_group, sequence_parallel_is_initialized
 from .layer_norm import LayerNorm, add_layer_norm
-from .linear import Linear, feed_forward, linear3, passes_through
+from .linear import Linear, embedding_sum, feed_forward, linear3, passes_through
 
 
 def _init_params(module: nn.Module, n_layers: int) -> None:
@@ -160,7 +160,7 @@ class GTGraphLevel(nn.Module):
     def forward(self, batched_data, perturb=None, attn_type=None):
         """batched_data.x: int64 [b, s/p, F]; batched_data.edge_index: [2, E] over the b * s flattened rows
         of the gathered batch (or a ``SparseGraph``); returns [b, output_dim]."""
-        h = self.input_dropout(self.embedding_h(batched_data.x).sum(dim=-2))
+        h = self.input_dropout(embedding_sum(self.embedding_h, batched_data.x))
         edge_index = batched_data.edge_index
         for layer in self.layers:
             h = layer(h, edge_index=edge_index, attn_type=attn_type)

@@ -98,3 +98,12 @@ def feed_forward(x: torch.Tensor, first: torch.nn.Module, second: torch.nn.Modul
 def passes_through(dropout: torch.nn.Module) -> bool:
     """``dropout`` returns its input as it is, and nobody observes the call."""
     return unobserved(dropout, torch.nn.Dropout) and (not dropout.training or dropout.p == 0.0)
+
+
+def embedding_sum(embedding: torch.nn.Module, ids: torch.Tensor) -> torch.Tensor:
+    """``embedding(ids).sum(dim=-2)``; the gathered vectors are never stored (csrc/embedding_sum.cu)."""
+    if (ids.is_cuda and unobserved(embedding, torch.nn.Embedding) and embedding.max_norm is None and not embedding.sparse and
+            not embedding.scale_grad_by_freq and _plain_call(ids, embedding.weight, None)):
+        padding = -1 if embedding.padding_idx is None else embedding.padding_idx
+        return _cabi.native().embedding_sum(embedding.weight, ids, padding)
+    return embedding(ids).sum(dim=-2)
