@@ -3,22 +3,25 @@
 // models/gt_dist_node_level.py:189-193,232-236: 64 x 64 to 128 x 64 over 8,000 to 870,000 rows).
 //
 // A tile is 128 rows x 64 columns.  A CTA keeps its columns' weights as bf16 pieces in shared memory (tensor_core.cuh) and
-// walks row tiles: 256 threads split the rows' values on their way from registers into shared memory, one thread issues
+// walks row tiles: 256 threads split the rows' values on their way from registers into shared memory, a ninth warp issues
 // the products, and while they run the next rows are on their way in and the tile before is finished from the other half
 // of the tensor memory.  CTAs of the same rows are neighbours in the grid, so a second column tile or a second layer finds
 // the rows in the L2.
 //
-// 320,000 rows of 64 x 64: 48 us against 80 for the FMA kernel that was here and 92 for the library's input gradient (a
-// copy of the same bytes: 25); 64 x 128: 78 against 143 and 138; 128 x 64: 79 against 151 and 134; 64,001 rows: 18 against
-// 25 and 27.  Sums stored row by row straight from tensor memory, without the blocks in shared memory, and without the
-// second half: 59 us.  Relative error against 64 bits 7e-8 (FMA 1.1e-7, library 1.5e-7), 128 long 1.2e-7 (1.5e-7, 2.0e-7).
+// us back to back, here | FMA kernel that was here | library's input gradient: 320,000 rows of 64 x 64 43 | 75 | 87 (a copy of
+// the same bytes: 25), 64 x 128 74 | 139 | 132, 128 x 64 75 | 144 | 127, three layers of 64 x 64 105 forward and 110 back; 64,001
+// rows 12 | 19 | 18.  Sums stored row by row straight from tensor memory, without the blocks in shared memory, and without
+// the second half: + 11 us; with a worker issuing the products and a general finish for every call: + 4 us.  Issue slots are
+// half busy with the split; 16 warps per SM hold the registers.
+// Relative error against 64 bits 7e-8 (FMA 1.1e-7, library 1.5e-7), 128 long 1.2e-7 (1.5e-7, 2.0e-7).
 #include "linear_rows.cuh"
 #include "tensor_core.cuh"
 
 namespace tgt {
 namespace {
 
-constexpr int kThreads = 256, kWarps = kThreads / 32;
+constexpr int kWarps = 8, kWorkers = 32 * kWarps;   // split, load and finish; one warp more issues the products
+constexpr int kThreads = kWorkers + 32;
 constexpr int kRows = 128, kCols = 64;     // of a tile: M and N of one product
 constexpr int kChunk = 64;                 // reduction elements staged at a time
 constexpr int kPieceA = kRows * 128;       // bytes of one piece of a tile of A
@@ -56,6 +59,7 @@ __device__ __noinline__ void sum_again(const SplitGemm& p, int out, int64_t row,
 // one block of finished sums per warp, the barrier and the tensor memory's address.
 inline int split_gemm_smem(int kept) { return 3 * kPieceA + kept * 3 * kPieceW + kWarps * kBlockBytes + 16; }
 
+template <bool PLAIN>   // nothing but a bias is added to the sums
 __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_constant__ SplitGemm p) {
   extern __shared__ __align__(1024) uint8_t s_raw[];
   const int src_chunks = (p.red + kChunk - 1) / kChunk, chunks = src_chunks * p.sources;
@@ -74,25 +78,31 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
   if (warp == 0) tc::allocate<kTmemCols>(s_tmem);
   if (tid == 32) tc::barrier_init(s_done);
 
-  const int q = 4 * (tid % 16), r0 = tid / 16;              // this thread's four reduction elements and first row
+  const int q = 4 * (tid % 16), r0 = tid / 16;              // a worker's four reduction elements and first row
   float4 next[kRows / 16];
   auto load = [&](int64_t tile, int chunk) {
-    const int src = chunk / src_chunks, k = chunk % src_chunks * kChunk + q;
-    const float* a = p.a[src];
+    const int src = src_chunks == 1 ? chunk : chunk / src_chunks;
+    const int k = (src_chunks == 1 ? 0 : chunk % src_chunks * kChunk) + q;
+    const int64_t row = tile * kRows + r0;
+    const float* a = p.a[src] + row * p.red + k;
+    const int64_t step = int64_t(16) * p.red;
+    if (tile * kRows + kRows <= p.rows && k < p.red) {
 #pragma unroll
-    for (int i = 0; i < kRows / 16; ++i) {
-      const int64_t row = tile * kRows + r0 + 16 * i;
-      next[i] = row < p.rows && k < p.red ? __ldg(reinterpret_cast<const float4*>(a + row * p.red + k))
-                                          : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < kRows / 16; ++i, a += step) next[i] = __ldg(reinterpret_cast<const float4*>(a));
+    } else {
+#pragma unroll
+      for (int i = 0; i < kRows / 16; ++i, a += step)
+        next[i] = row + 16 * i < p.rows && k < p.red ? __ldg(reinterpret_cast<const float4*>(a))
+                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
   int64_t tile = blockIdx.x / across;
-  load(tile, 0);
+  if (warp < kWarps) load(tile, 0);
   auto stage_weights = [&](int chunk, int slot) {
     const int src = chunk / src_chunks, k0 = chunk % src_chunks * kChunk;
     const float* w = p.w[p.sources > 1 ? src : out];
 #pragma unroll 4
-    for (int u = tid; u < kCols * 16; u += kThreads) {
+    for (int u = tid; u < kCols * 16; u += kWorkers) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       int n, k;
       if (!p.transposed) {
@@ -109,8 +119,9 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
       tc::store4(s_w + slot * (3 * kPieceW), kPieceW, tc::tile_offset(n, k), tc::split4(v));
     }
   };
-  if (p.kept == chunks)                                     // once; a long reduction's weights come along with its rows
+  if (p.kept == chunks && warp < kWarps)                    // once; a long reduction's weights come along with its rows
     for (int chunk = 0; chunk < chunks; ++chunk) stage_weights(chunk, chunk);
+  if (warp < kWarps) tc::publish_operands();
   tc::fence_before_barrier();
   __syncthreads();
   tc::fence_after_barrier();
@@ -144,12 +155,21 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
       __syncwarp();
       const int my_col = col + 4 * (lane % 4);
       if (my_col < p.cols) {
+        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (PLAIN && p.bias[out] != nullptr) b = __ldg(reinterpret_cast<const float4*>(p.bias[out] + my_col));
+        float* c = p.c[out] + (row0 + lane / 4) * p.cols + my_col;
+        const int left = int(min(p.rows - row0, int64_t(32)));        // of the warp's rows
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int r = lane / 4 + 8 * i;
           float4 v = *reinterpret_cast<const float4*>(s_block + block_offset(r, lane % 4));
           if (!ok) v.x = __int_as_float(0x7fffffff);
-          if (row0 + r < p.rows) finish_values(p, out, row0 + r, my_col, v);
+          if (r >= left) continue;
+          if (PLAIN) {
+            *reinterpret_cast<float4*>(c + int64_t(8 * i) * p.cols) = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+          } else {
+            finish_values(p, out, row0 + r, my_col, v);
+          }
         }
       }
       __syncwarp();
@@ -157,51 +177,62 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
   };
 
   // A tile's products run under the finishing of the tile before, whose sums lie in the other half of the tensor memory.
-  int64_t before = -1;
   uint32_t sums = tmem;
-  for (; tile < tiles; tile += walkers) {
-    for (int chunk = 0; chunk < chunks; ++chunk) {
+  if (warp == kWarps) {
+    for (; tile < tiles; tile += walkers) {
+      for (int chunk = 0; chunk < chunks; ++chunk) {
+        if (!__syncthreads_and(true)) goto finished;        // the workers' pieces are in place
+        if (lane == 0) {
+          tc::fence_after_barrier();
+          const uint32_t w = s_w + (p.kept < chunks ? 0 : chunk * (3 * kPieceW));
 #pragma unroll
-      for (int i = 0; i < kRows / 16; ++i)
-        tc::store4(s_a, kPieceA, tc::tile_offset(r0 + 16 * i, q), tc::split4(next[i]));
-      if (p.kept < chunks) stage_weights(chunk, 0);
-      tc::publish_operands();
-      tc::fence_before_barrier();                           // everybody has read the sums of two tiles ago
-      ok = __syncthreads_and(ok);
-      if (!ok) goto finished;
-      if (tid == 0) {
-        tc::fence_after_barrier();
-        const uint32_t w = s_w + (p.kept < chunks ? 0 : chunk * (3 * kPieceW));
-#pragma unroll
-        for (int k = 0; k < kChunk / 16; ++k) {
-          const uint64_t a1 = tc::k_major(s_a + 32 * k), a2 = tc::k_major(s_a + kPieceA + 32 * k),
-                         a3 = tc::k_major(s_a + 2 * kPieceA + 32 * k);
-          const uint64_t w1 = tc::k_major(w + 32 * k), w2 = tc::k_major(w + kPieceW + 32 * k),
-                         w3 = tc::k_major(w + 2 * kPieceW + 32 * k);
-          constexpr uint32_t both = tc::instruction(kRows, 2 * kCols, false, false),
-                             one = tc::instruction(kRows, kCols, false, false);
-          tc::multiply(sums, a1, w1, both, chunk + k > 0);       // a1 w1 | a1 w2
-          tc::multiply(sums + kCols, a2, w1, one, true);
-          tc::multiply(sums + kCols, a2, w2, one, true);
-          tc::multiply(sums + kCols, a1, w3, one, true);
-          tc::multiply(sums + kCols, a3, w1, one, true);
+          for (int k = 0; k < kChunk / 16; ++k) {
+            const uint64_t a1 = tc::k_major(s_a + 32 * k), a2 = tc::k_major(s_a + kPieceA + 32 * k),
+                           a3 = tc::k_major(s_a + 2 * kPieceA + 32 * k);
+            const uint64_t w1 = tc::k_major(w + 32 * k), w2 = tc::k_major(w + kPieceW + 32 * k),
+                           w3 = tc::k_major(w + 2 * kPieceW + 32 * k);
+            constexpr uint32_t both = tc::instruction(kRows, 2 * kCols, false, false),
+                               one = tc::instruction(kRows, kCols, false, false);
+            tc::multiply(sums, a1, w1, both, chunk + k > 0);     // a1 w1 | a1 w2
+            tc::multiply(sums + kCols, a2, w1, one, true);
+            tc::multiply(sums + kCols, a2, w2, one, true);
+            tc::multiply(sums + kCols, a1, w3, one, true);
+            tc::multiply(sums + kCols, a3, w1, one, true);
+          }
+          tc::commit(s_done);
         }
-        tc::commit(s_done);
+        __syncwarp();
       }
-      // the next step's rows arrive under the products and the stores
-      const bool last = chunk + 1 == chunks;
-      const int64_t next_tile = last ? tile + walkers : tile;
-      if (next_tile < tiles) load(next_tile, last ? 0 : chunk + 1);
-      if (chunk == 0 && before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
-      ok = tc::wait(s_done, phase) && ok;
-      phase ^= 1;
+      sums = tmem + (sums == tmem ? 2 * kCols : 0);
     }
-    tc::fence_after_barrier();
-    before = tile;
-    sums = tmem + (sums == tmem ? 2 * kCols : 0);
+  } else {
+    int64_t before = -1;
+    for (; tile < tiles; tile += walkers) {
+      for (int chunk = 0; chunk < chunks; ++chunk) {
+#pragma unroll
+        for (int i = 0; i < kRows / 16; ++i)
+          tc::store4(s_a, kPieceA, tc::tile_offset(r0 + 16 * i, q), tc::split4(next[i]));
+        if (p.kept < chunks) stage_weights(chunk, 0);
+        tc::publish_operands();
+        tc::fence_before_barrier();                         // everybody has read the sums of two tiles ago
+        ok = __syncthreads_and(ok);
+        if (!ok) goto give_up;
+        // the next step's rows arrive under the products and the stores
+        const bool last = chunk + 1 == chunks;
+        const int64_t next_tile = last ? tile + walkers : tile;
+        if (next_tile < tiles) load(next_tile, last ? 0 : chunk + 1);
+        if (chunk == 0 && before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
+        ok = tc::wait(s_done, phase) && ok;
+        phase ^= 1;
+      }
+      tc::fence_after_barrier();
+      before = tile;
+      sums = tmem + (sums == tmem ? 2 * kCols : 0);
+    }
+  give_up:
+    if (before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
   }
 finished:
-  if (before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
   tc::fence_before_barrier();
   __syncthreads();
   if (warp == 0) tc::release<kTmemCols>(tmem);
@@ -213,7 +244,9 @@ int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
   const int chunks = (p.red + kChunk - 1) / kChunk * p.sources;
   p.kept = split_gemm_smem(chunks) <= kMostSmem ? chunks : 1;
   const int smem = split_gemm_smem(p.kept);
-  const int rc = allow_shared_memory<split_gemm_kernel>(kMostSmem);
+  const bool plain = p.act == TGT_ACT_NONE && p.pre == nullptr && p.gate_act == TGT_ACT_NONE && p.add == nullptr;
+  const int rc = plain ? allow_shared_memory<split_gemm_kernel<true>>(kMostSmem)
+                       : allow_shared_memory<split_gemm_kernel<false>>(kMostSmem);
   if (rc != TGT_OK) return rc;
   p.col_tiles = (p.cols + kCols - 1) / kCols;
   const int64_t tiles = (p.rows + kRows - 1) / kRows;
@@ -222,7 +255,8 @@ int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
   int64_t walkers = int64_t(sm_count()) * resident / across;
   if (walkers < 1) walkers = 1;
   if (walkers > tiles) walkers = tiles;
-  split_gemm_kernel<<<unsigned(walkers * across), kThreads, smem, stream>>>(p);
+  if (plain) split_gemm_kernel<true><<<unsigned(walkers * across), kThreads, smem, stream>>>(p);
+  else split_gemm_kernel<false><<<unsigned(walkers * across), kThreads, smem, stream>>>(p);
   TGT_CHECK_CUDA(cudaGetLastError());
   return TGT_OK;
 }

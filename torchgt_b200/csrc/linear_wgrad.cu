@@ -9,8 +9,8 @@
 // drained after every chunk and added in fp32 registers; the small ones, 2^-8 of them, stay till the end.  The CTAs'
 // tiles are then added in a fixed order by a second kernel.  No atomics: results are bitwise reproducible.
 //
-// 320,000 rows of 64 x 64: 58 us with the sums, 75 for the FMA kernel that was here (a copy of the same bytes: 25); 64 x
-// 128 and 128 x 64: 91 against 130; 64,001 rows of 64 x 64: 25.6 against 27.6; one CTA per SM: 79 us.  Relative error against
+// us back to back with the sums, here | FMA kernel that was here: 320,000 rows of 64 x 64 50 | 66 (a copy of the same bytes:
+// 25), 64 x 128 and 128 x 64 80 | 121, three gradients of one input 110; 64,001 rows 18 | 19, three 29.  Relative error against
 // 64 bits at 320,000 rows 1.5e-7, the FMA kernel's 4.4e-7.
 #include "tensor_core.cuh"
 
@@ -61,13 +61,18 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
 
   const int q = 4 * (tid % 16), r0 = tid / 16;
   float4 dy[kWgChunk / 16], x[kWgChunk / 16];
+  const bool has_dy = o0 + q < p.out, has_x = i0 + q < p.in;
   auto load = [&](int64_t chunk) {
+    const int64_t row = chunk * kWgChunk + r0;
+    const float *a = from + row * p.out + o0 + q, *b = p.x + row * p.in + i0 + q;
+    const int64_t step_a = int64_t(16) * p.out, step_b = int64_t(16) * p.in;
+    const bool whole = (chunk + 1) * kWgChunk <= p.rows;
 #pragma unroll
-    for (int i = 0; i < kWgChunk / 16; ++i) {
-      const int64_t row = chunk * kWgChunk + r0 + 16 * i;
+    for (int i = 0; i < kWgChunk / 16; ++i, a += step_a, b += step_b) {
+      const bool live = whole || row + 16 * i < p.rows;
       const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      dy[i] = row < p.rows && o0 + q < p.out ? __ldg(reinterpret_cast<const float4*>(from + row * p.out + o0 + q)) : zero;
-      x[i] = row < p.rows && i0 + q < p.in ? __ldg(reinterpret_cast<const float4*>(p.x + row * p.in + i0 + q)) : zero;
+      dy[i] = live && has_dy ? __ldg(reinterpret_cast<const float4*>(a)) : zero;
+      x[i] = live && has_x ? __ldg(reinterpret_cast<const float4*>(b)) : zero;
     }
   };
   float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -111,7 +116,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
     tc::fence_before_barrier();
     ok = __syncthreads_and(ok);
     if (!ok) break;
-    if (tid == 0) {
+    if (tid == 64) {                                 // of a warp that does not drain
       tc::fence_after_barrier();
       constexpr uint32_t one = tc::instruction(128, 64, true, true);
 #pragma unroll
