@@ -47,7 +47,7 @@ def _compare(outs, refs, x, x64, modules, modules64, extra=(), extra64=()):
 
 
 @pytest.mark.parametrize("bias", [True, False])
-@pytest.mark.parametrize("shape,out", [((1023, 64), 64), ((1024, 64), 64), ((3, 700, 64), 64), ((1, 2689, 64), 64), ((30001, 128), 64), ((9000, 64), 100)])
+@pytest.mark.parametrize("shape,out", [((1023, 64), 64), ((1024, 64), 64), ((3, 700, 64), 64), ((1, 2689, 64), 64), ((30001, 128), 64), ((10300, 64), 100)])
 def test_three_projections(shape, out, bias):
     from torchgt_b200.linear import linear3
     torch.manual_seed(shape[-2])
@@ -64,7 +64,7 @@ def test_three_projections(shape, out, bias):
 
 @pytest.mark.parametrize("act", ["relu", "gelu"])
 @pytest.mark.parametrize("residual", [True, False])
-@pytest.mark.parametrize("shape,mid", [((1023, 64), 64), ((1024, 64), 64), ((1, 2000, 64), 128), ((20001, 64), 128), ((9000, 128), 64)])
+@pytest.mark.parametrize("shape,mid", [((1023, 64), 64), ((1024, 64), 64), ((1, 2000, 64), 128), ((20001, 64), 128), ((10300, 128), 64)])
 def test_feed_forward(shape, mid, residual, act):
     from torchgt_b200.linear import feed_forward
     torch.manual_seed(shape[-2] + mid)
@@ -125,7 +125,7 @@ def test_infinities_and_nan_pass_as_through_the_modules():
     from torchgt_b200.linear import feed_forward, linear3
     torch.manual_seed(2)
     layers = _layers(3, 64, 64)
-    for rows in (1300, 9000):
+    for rows in (1300, 10300):
         x = torch.randn(rows, 64, device="cuda")
         x[3, 7], x[11, 0] = float("inf"), float("nan")
         with torch.no_grad():

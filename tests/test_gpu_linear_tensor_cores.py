@@ -43,9 +43,9 @@ ACTS = {"none": 0, "relu": 1, "gelu": 2}
 
 @pytest.mark.parametrize("count", [1, 3])
 @pytest.mark.parametrize("rows,reduce,cols", [
-    (1, 64, 64), (4064, 64, 64), (8064, 64, 64), (8065, 64, 64), (8192, 64, 64), (20001, 64, 64), (38017, 64, 40),
-    (9000, 128, 64), (9000, 64, 128), (9000, 68, 100), (9000, 4, 4), (2049, 64, 1024), (8200, 384, 64), (8200, 448, 64),
-    (8200, 1024, 8)])
+    (1, 64, 64), (4064, 64, 64), (10112, 64, 64), (10113, 64, 64), (10240, 64, 64), (20001, 64, 64), (38017, 64, 40),
+    (10300, 128, 64), (10300, 64, 128), (10300, 68, 100), (10300, 4, 4), (2049, 64, 1024), (10300, 384, 64), (10300, 448, 64),
+    (10300, 1024, 8)])
 def test_products_and_input_gradients(rows, reduce, cols, count):
     c = _lib()
     x, = _rand(rows + reduce, (rows, reduce))
@@ -67,7 +67,7 @@ def test_products_and_input_gradients(rows, reduce, cols, count):
 
 
 @pytest.mark.parametrize("act", ["relu", "gelu"])
-@pytest.mark.parametrize("rows", [33, 8065])
+@pytest.mark.parametrize("rows", [33, 10113])
 def test_activation_residual_and_gate(rows, act):
     c = _lib()
     x, w, b, add, dy = _rand(rows, (rows, 64), (128, 64), (128,), (rows, 128), (rows, 64))
@@ -109,9 +109,9 @@ def test_parameter_gradients(rows, inp, out, count):
 def test_values_that_are_not_finite_and_sums_past_the_range():
     """They come out as fp32 FMAs give them: infinities and NaN where those belong, and nowhere else."""
     c = _lib()
-    rows = 9000
+    rows = 10300
     x, w = _rand(3, (rows, 64), (64, 64))
-    x[5, 3], x[700, 1], x[8999] = float("inf"), float("nan"), 3e38
+    x[5, 3], x[700, 1], x[10299] = float("inf"), float("nan"), 3e38
     w[9, 2] = float("-inf")
     y = torch.empty(rows, 64, device="cuda")
     c.check(c.load().tgt_linear_rows(x.data_ptr(), w.data_ptr(), None, rows, 64, 64, y.data_ptr(), _stream()))
@@ -119,13 +119,13 @@ def test_values_that_are_not_finite_and_sums_past_the_range():
     torch.backends.cuda.matmul.allow_tf32 = False
     ref = x @ w.t()
     torch.backends.cuda.matmul.allow_tf32 = before
-    assert torch.equal(y.isnan()[:8999], ref.isnan()[:8999]) and torch.equal(y.isinf()[:8999], ref.isinf()[:8999])
-    assert not y[8999].isfinite().all()
+    assert torch.equal(y.isnan()[:10299], ref.isnan()[:10299]) and torch.equal(y.isinf()[:10299], ref.isinf()[:10299])
+    assert not y[10299].isfinite().all()
     fine = ref.isfinite() & y.isfinite()
-    fine[8999] = False
+    fine[10299] = False
     assert _rel(y[fine], (x.double() @ w.double().t())[fine]) < TOL
     dy, = _rand(4, (rows, 64))
-    x[8999] = 0
+    x[10299] = 0
     need = ctypes.c_size_t()
     c.check(c.load().tgt_linear_wgrad_scratch_bytes(rows, 64, 64, ctypes.byref(need)))
     scratch, dw = torch.empty(need.value, dtype=torch.uint8, device="cuda"), torch.empty(64, 64, device="cuda")

@@ -36,9 +36,10 @@ bool tf32_allowed() {
          at::Float32Precision::TF32;
 }
 
-// From here on linear_mma.cu is ahead of the library's fp32 product for the input gradient (us a call): 64 x 64 11.2 / 10.2
-// at 4,097 rows, 18.4 / 26.6 at 64,001, 47 / 92 at 320,000; 128 x 64 14.4 / 10.3, 26.7 / 36.9, 78 / 134.
-constexpr int64_t kInputGradRows = 8192;
+// From here on linear_mma.cu is ahead of the library's fp32 product for the input gradient (us back to back, here / library):
+// 64 x 64 6.3 / 4.5 at 8,192 rows, 6.4 / 7.2 at 16,384, 12.3 / 18.5 at 64,001, 43 / 87 at 320,000; 128 outputs 9.0 / 6.2, 9.0 /
+// 10.1, 17.6 / 28.3, 74 / 127.
+constexpr int64_t kInputGradRows = 12288;
 
 struct NarrowLinearBackward : public torch::autograd::Node {
   SavedVariable x, weight;

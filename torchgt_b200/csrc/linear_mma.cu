@@ -244,7 +244,7 @@ int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
   const int chunks = (p.red + kChunk - 1) / kChunk * p.sources;
   p.kept = split_gemm_smem(chunks) <= kMostSmem ? chunks : 1;
   const int smem = split_gemm_smem(p.kept);
-  const bool plain = p.act == TGT_ACT_NONE && p.pre == nullptr && p.gate_act == TGT_ACT_NONE && p.add == nullptr;
+  const bool plain = is_plain(p);
   const int rc = plain ? allow_shared_memory<split_gemm_kernel<true>>(kMostSmem)
                        : allow_shared_memory<split_gemm_kernel<false>>(kMostSmem);
   if (rc != TGT_OK) return rc;

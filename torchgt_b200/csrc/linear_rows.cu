@@ -37,6 +37,7 @@ __device__ __forceinline__ float pair_sum(uint64_t v) {
 // 4 tx .. 4 tx + 3 and 32 + 4 tx .. 32 + 4 tx + 3
 __device__ __forceinline__ int lr_slot(int c) { return (c % 32) / 4 + 8 * (4 * (c / 32) + c % 4); }
 
+template <bool PLAIN>   // nothing but a bias is added to the sums
 __global__ void __launch_bounds__(kLrThreads, 4) linear_rows_kernel(const __grid_constant__ LinearRows p) {
   constexpr int TM = kLrRows / 16, BM = kLrRows;
   extern __shared__ __align__(16) float s_mem[];
@@ -68,6 +69,22 @@ __global__ void __launch_bounds__(kLrThreads, 4) linear_rows_kernel(const __grid
     }
   };
 
+  float4 b[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int col = c0 + 32 * h + 4 * tx;
+    b[h] = p.bias[out] != nullptr && col < p.cols ? __ldg(reinterpret_cast<const float4*>(p.bias[out] + col))
+                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float* const c = p.c[out];
+  auto finish = [&](int64_t row, int col, const float4& v) {
+    if (PLAIN) {
+      const float4& add = col < c0 + 32 ? b[0] : b[1];
+      *reinterpret_cast<float4*>(c + row * p.cols + col) = make_float4(v.x + add.x, v.y + add.y, v.z + add.z, v.w + add.w);
+    } else {
+      finish_values(p, out, row, col, v);
+    }
+  };
   uint64_t acc[TM][8];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
@@ -110,8 +127,8 @@ __global__ void __launch_bounds__(kLrThreads, 4) linear_rows_kernel(const __grid
         for (int h = 0; h < 2; ++h) {
           const int col = c0 + 32 * h + 4 * tx;
           if (row < p.rows && col < p.cols)
-            finish_values(p, out, row, col, make_float4(pair_sum(acc[i][4 * h]), pair_sum(acc[i][4 * h + 1]),
-                                                        pair_sum(acc[i][4 * h + 2]), pair_sum(acc[i][4 * h + 3])));
+            finish(row, col, make_float4(pair_sum(acc[i][4 * h]), pair_sum(acc[i][4 * h + 1]),
+                                         pair_sum(acc[i][4 * h + 2]), pair_sum(acc[i][4 * h + 3])));
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] = 0;
@@ -130,13 +147,17 @@ __global__ void __launch_bounds__(kLrThreads, 4) linear_rows_kernel(const __grid
 int linear_few_rows(const LinearRows& p, cudaStream_t stream) {
   const int col_tiles = (p.cols + kLrTile - 1) / kLrTile, chunks = (p.red + kLrTile - 1) / kLrTile;
   const int smem = (2 * kLrRows + kLrTile * (chunks > 1 ? 2 : 1)) * kLrPitch * int(sizeof(float));
-  const int rc = allow_shared_memory<linear_rows_kernel>((2 * kLrRows + 2 * kLrTile) * kLrPitch * int(sizeof(float)));
+  constexpr int kMost = (2 * kLrRows + 2 * kLrTile) * kLrPitch * int(sizeof(float));
+  const bool plain = is_plain(p);
+  const int rc = plain ? allow_shared_memory<linear_rows_kernel<true>>(kMost) : allow_shared_memory<linear_rows_kernel<false>>(kMost);
   if (rc != TGT_OK) return rc;
   const int64_t tiles = (p.rows + kLrRows - 1) / kLrRows;
   int64_t ctas = int64_t(sm_count()) * 4 / (col_tiles * p.outputs);
   if (ctas < 1) ctas = 1;
   if (ctas > tiles) ctas = tiles;
-  linear_rows_kernel<<<dim3(unsigned(ctas), col_tiles, p.outputs), kLrThreads, smem, stream>>>(p);
+  const dim3 grid(unsigned(ctas), col_tiles, p.outputs);
+  if (plain) linear_rows_kernel<true><<<grid, kLrThreads, smem, stream>>>(p);
+  else linear_rows_kernel<false><<<grid, kLrThreads, smem, stream>>>(p);
   TGT_CHECK_CUDA(cudaGetLastError());
   return TGT_OK;
 }

@@ -219,7 +219,9 @@ constexpr int kWgSmem = 12 * kWgPiece + 32;     // two buffers, two barriers and
 int wgrad_grid(int64_t rows, int in, int out, int count) {
   const int tiles = (in / kWgTile) * wgrad_out_tiles(out) * count;
   const int64_t chunks = (rows + kWgChunk - 1) / kWgChunk;
-  int64_t g = int64_t(sm_count()) * 2 / tiles;     // the two CTAs an SM holds, over all tiles
+  // The two CTAs an SM holds, over all tiles; one where that leaves them a chunk or two each, so that the sums have half as
+  // many tiles to read (16,384 rows of 64 x 64: 12.7 us, with 256 CTAs 14.8)
+  int64_t g = int64_t(sm_count()) * (chunks * tiles > 4 * int64_t(sm_count()) ? 2 : 1) / tiles;
   if (g < 1) g = 1;
   if (g > chunks) g = chunks < 1 ? 1 : chunks;
   return int(g);
