@@ -121,6 +121,34 @@ def test_second_order_gradients():
     assert _rel(dw, (2 * 1100 * total).expand(64, 64)) < 1e-5
 
 
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("block", ["linear", "linear3"])
+def test_second_order_gradients_through_the_parameters_gradients(block, bias):
+    """What is built on dW and db reaches the input, the weights and the gradient that came in; dW has the same bits as without
+    create_graph."""
+    from torchgt_b200.linear import linear3
+    torch.manual_seed(6)
+    layers = _layers(3, 64, 64, bias)
+    x = (0.3 * torch.randn(1100, 64, device="cuda")).requires_grad_()
+    x64, layers64 = x.detach().double().requires_grad_(), [_double(m) for m in layers]
+    got, want = [], []
+    for leaf, mods, into in ((x, layers, got), (x64, layers64, want)):
+        if block == "linear":
+            loss = (mods[0](leaf) ** 2).sum()
+            mods = mods[:1]
+        else:
+            q, k, v = linear3(leaf, *mods) if leaf is x else [m(leaf) for m in mods]
+            loss = (q * k).sum() + (v * v * v).sum()
+        params = [p for m in mods for p in m.parameters()]
+        first = torch.autograd.grad(loss, params, create_graph=True)
+        assert all(g.requires_grad for g in first)
+        if leaf is x:
+            assert all(torch.equal(a, b) for a, b in zip(first, torch.autograd.grad(loss, params, retain_graph=True)))
+        into.extend(torch.autograd.grad(sum((g * g).sum() for g in first), [leaf, *params]))
+    # chains of four products of at most 1,100 terms of mixed sign
+    assert all(_rel(a, b) < 2e-5 for a, b in zip(got, want))
+
+
 def test_infinities_and_nan_pass_as_through_the_modules():
     from torchgt_b200.linear import feed_forward, linear3
     torch.manual_seed(2)

@@ -41,6 +41,41 @@ bool tf32_allowed() {
 // 10.1, 17.6 / 28.3, 74 / 127.
 constexpr int64_t kInputGradRows = 12288;
 
+// dW = dY^T X and db = the sum of dY's rows where the gradient is itself differentiated (create_graph): the kernel's values,
+// with what the two formulas' derivatives are as operations that can be recorded again.
+struct ParameterGradientsBackward : public torch::autograd::Node {
+  SavedVariable dy, x;
+
+  variable_list apply(variable_list&& grads) override {
+    const at::Tensor dy_ = dy.unpack(), x_ = x.unpack();
+    variable_list result(2);
+    if (grads[0].defined()) {
+      if (task_should_compute_output(0)) result[0] = at::matmul(x_, grads[0].t());
+      if (task_should_compute_output(1)) result[1] = at::matmul(dy_, grads[0]);
+    }
+    if (grads.size() > 1 && grads[1].defined() && task_should_compute_output(0)) {
+      const at::Tensor rows = grads[1].expand_as(dy_);
+      result[0] = result[0].defined() ? result[0] + rows : rows;
+    }
+    return result;
+  }
+  std::string name() const override { return "ParameterGradientsBackward"; }
+  void release_variables() override {
+    dy.reset_data();
+    x.reset_data();
+  }
+};
+
+// db may be undefined
+void record_parameter_gradients(const at::Tensor& dw, const at::Tensor& db, const at::Tensor& dy, const at::Tensor& x) {
+  if (!torch::autograd::compute_requires_grad(dy, x)) return;
+  auto node = std::shared_ptr<ParameterGradientsBackward>(new ParameterGradientsBackward(), torch::autograd::deleteNode);
+  node->set_next_edges(torch::autograd::collect_next_edges(dy, x));
+  node->dy = SavedVariable(dy, false);
+  node->x = SavedVariable(x, false);
+  torch::autograd::set_history(db.defined() ? variable_list{dw, db} : variable_list{dw}, node);
+}
+
 struct NarrowLinearBackward : public torch::autograd::Node {
   SavedVariable x, weight;
   bool has_bias = false;
@@ -53,11 +88,17 @@ struct NarrowLinearBackward : public torch::autograd::Node {
     const at::Tensor x_ = x.unpack(), w_ = weight.unpack();
     const c10::cuda::CUDAGuard guard(x_.device());
     at::Tensor dx, dw, db;
-    const bool recorded = at::GradMode::is_enabled();     // a second-order gradient is wanted: dx as a recorded product
+    const bool recorded = at::GradMode::is_enabled();     // a second-order gradient is wanted
     if (task_should_compute_output(0) && recorded) dx = at::matmul(grads[0], w_);
+    kernels(grads[0], x_, w_, recorded, dx, dw, db);
+    if (recorded && dw.defined()) record_parameter_gradients(dw, db, grads[0], x_);
+    return {dx, dw, db};
+  }
+  void kernels(const at::Tensor& dy_, const at::Tensor& x_, const at::Tensor& w_, bool recorded, at::Tensor& dx, at::Tensor& dw,
+               at::Tensor& db) {
     const at::AutoDispatchBelowADInplaceOrView below;
     const int64_t out = w_.size(0), in = w_.size(1);
-    const at::Tensor dy = kernel_ready(grads[0]);
+    const at::Tensor dy = kernel_ready(dy_);
     const int64_t rows = dy.numel() / out;
     if (task_should_compute_output(0) && !recorded) {
       if (tf32_allowed() || rows < kInputGradRows) {
@@ -78,7 +119,6 @@ struct NarrowLinearBackward : public torch::autograd::Node {
       check(tgt_linear_wgrad(fptr(dy), fptr(xc), rows, int(in), int(out), fptr(dw), has_bias ? fptr(db) : nullptr,
                              scratch.data_ptr(), scratch.numel(), stream_of(dy)));
     }
-    return {dx, dw, db};
   }
   std::string name() const override { return "NarrowLinearBackward"; }
   void release_variables() override {
@@ -175,16 +215,23 @@ struct NarrowLinear3Backward : public torch::autograd::Node {
     return reporting([&] { return backward(grads); });
   }
   variable_list backward(const variable_list& grads) {
-    variable_list result(7);
     const at::Tensor x_ = x.unpack();
+    const bool recorded = at::GradMode::is_enabled();      // a second-order gradient is wanted
+    variable_list result = kernels(grads, x_, recorded);
+    for (int i = 0; recorded && i < 3; ++i)
+      if (result[1 + 2 * i].defined()) record_parameter_gradients(result[1 + 2 * i], result[2 + 2 * i], grads[i], x_);
+    return result;
+  }
+  variable_list kernels(const variable_list& grads, const at::Tensor& x_, bool recorded) {
+    variable_list result(7);
     const c10::cuda::CUDAGuard guard(x_.device());
-    const bool want_dx = task_should_compute_output(0), recorded = at::GradMode::is_enabled();
+    const bool want_dx = task_should_compute_output(0);
     std::vector<at::Tensor> dy, w, dy_p;
     std::vector<at::Tensor*> dw, db;
     for (int i = 0; i < 3; ++i) {
       if (!grads[i].defined()) continue;
       const at::Tensor w_ = weight[i].unpack();
-      if (want_dx && recorded) {       // a second-order gradient is wanted: dx as recorded products
+      if (want_dx && recorded) {
         const at::Tensor d = at::matmul(grads[i], w_);
         result[0] = result[0].defined() ? result[0] + d : d;
       }
