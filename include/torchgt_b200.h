@@ -503,7 +503,7 @@ TGT_API int tgt_linear_input_grad(const float* dy, const float* w, int64_t rows,
  * bias[i]), the sum of their input gradients (dx = sum_i dy[i] w[i]) and their parameters' gradients, each in one pass over
  * what the layers share.  w, bias, dy, c, dw and db are host arrays of `count` device pointers; bias[i] and db[i] may be
  * NULL.  With one product, c = act(a w^T + bias) + add; pre receives a w^T + bias, both [rows, cols] and NULL where they
- * are not wanted.  tgt_linear_input_grad_multi multiplies dx by the derivative of `act` at gate [rows, in_features], the
+ * are not wanted.  add and gate must not overlap what is written.  tgt_linear_input_grad_multi multiplies dx by the derivative of `act` at gate [rows, in_features], the
  * activation's input, or for TGT_ACT_RELU its result (models/graphormer_dist_node_level.py:236-245,281-286).
  */
 #define TGT_ACT_NONE 0

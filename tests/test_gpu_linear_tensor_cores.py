@@ -45,7 +45,7 @@ ACTS = {"none": 0, "relu": 1, "gelu": 2}
 @pytest.mark.parametrize("rows,reduce,cols", [
     (1, 64, 64), (4064, 64, 64), (10112, 64, 64), (10113, 64, 64), (10240, 64, 64), (20001, 64, 64), (38017, 64, 40),
     (10300, 128, 64), (10300, 64, 128), (10300, 68, 100), (10300, 4, 4), (2049, 64, 1024), (10300, 384, 64), (10300, 448, 64),
-    (10300, 1024, 8)])
+    (10300, 832, 64), (10300, 1024, 8)])
 def test_products_and_input_gradients(rows, reduce, cols, count):
     c = _lib()
     x, = _rand(rows + reduce, (rows, reduce))
@@ -66,20 +66,58 @@ def test_products_and_input_gradients(rows, reduce, cols, count):
     assert torch.equal(dx, again)
 
 
+@pytest.mark.parametrize("signs", ["mixed", "one"])
+@pytest.mark.parametrize("reduce,count", [(64, 3), (128, 1), (192, 1), (132, 2), (128, 3), (448, 1), (448, 3), (1024, 1), (1024, 3)])
+def test_long_reductions_are_no_further_off_than_sums_rounded_to_nearest(reduce, count, signs):
+    """Tensor cores round a running sum towards zero at each of its steps of 16: where all products have one sign that adds up.
+    With at most 128 products per running sum the loss is below 8 steps of 2^-23 of the sum, and 24 such sums are added with
+    rounding to nearest: below 1e-6 + 24^0.5 * 2^-24 in all.  With mixed signs it averages out and has to stay below the error
+    of the library's fp32 product."""
+    c = _lib()
+    rows, cols = 10300, 64
+    x, = _rand(reduce, (rows, reduce))
+    dy = list(_rand(count, (count, rows, reduce))[0].unbind(0))
+    w = list(_rand(reduce + count, (count, reduce, cols))[0].unbind(0))
+    if signs == "one":
+        x, dy, w = x.abs(), [t.abs() for t in dy], [t.abs() for t in w]
+    y, dx = torch.empty(rows, cols, device="cuda"), torch.empty(rows, cols, device="cuda")
+    wt = w[0].t().contiguous()
+    c.check(c.load().tgt_linear_rows(x.data_ptr(), wt.data_ptr(), None, rows, reduce, cols, y.data_ptr(), _stream()))
+    c.check(c.load().tgt_linear_input_grad_multi(_array(dy), _array(w), count, rows, reduce, cols, 0, None, dx.data_ptr(),
+                                                 _stream()))
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    library = x @ w[0], sum(d @ v for d, v in zip(dy, w))
+    torch.backends.cuda.matmul.allow_tf32 = before
+    refs = x.double() @ w[0].double(), sum(d.double() @ v.double() for d, v in zip(dy, w))
+    for got, near, ref in zip((y, dx), library, refs):
+        assert _rel(got, ref) < (_rel(near, ref) if signs == "mixed" else 1.3e-6)
+
+
 @pytest.mark.parametrize("act", ["relu", "gelu"])
 @pytest.mark.parametrize("rows", [33, 10113])
 def test_activation_residual_and_gate(rows, act):
+    _follow_a_sum(rows, act, 64)
+
+
+@pytest.mark.parametrize("act", ["relu", "gelu"])
+@pytest.mark.parametrize("reduce", [388, 832])      # two and three launches
+def test_activation_residual_and_gate_after_a_sum_in_parts(reduce, act):
+    _follow_a_sum(10113, act, reduce)
+
+
+def _follow_a_sum(rows, act, reduce):
     c = _lib()
-    x, w, b, add, dy = _rand(rows, (rows, 64), (128, 64), (128,), (rows, 128), (rows, 64))
+    x, w, b, add, dy = _rand(rows, (rows, reduce), (128, reduce), (128,), (rows, 128), (rows, reduce))
     pre, y = torch.empty(rows, 128, device="cuda"), torch.empty(rows, 128, device="cuda")
-    c.check(c.load().tgt_linear_rows_multi(x.data_ptr(), _array([w]), _array([b]), 1, rows, 64, 128, ACTS[act],
+    c.check(c.load().tgt_linear_rows_multi(x.data_ptr(), _array([w]), _array([b]), 1, rows, reduce, 128, ACTS[act],
                                            pre.data_ptr(), add.data_ptr(), _array([y]), _stream()))
     z = x.double() @ w.double().t() + b.double()
     assert _rel(pre, z) < TOL and _rel(y, _act(act, z) + add.double()) < TOL
     gate = torch.relu(pre) if act == "relu" else pre
-    w2, = _rand(1, (64, 128))
+    w2, = _rand(1, (reduce, 128))
     dx = torch.empty(rows, 128, device="cuda")
-    c.check(c.load().tgt_linear_input_grad_multi(_array([dy]), _array([w2]), 1, rows, 64, 128, ACTS[act], gate.data_ptr(),
+    c.check(c.load().tgt_linear_input_grad_multi(_array([dy]), _array([w2]), 1, rows, reduce, 128, ACTS[act], gate.data_ptr(),
                                                  dx.data_ptr(), _stream()))
     leaf = pre.double().requires_grad_()
     ref, = torch.autograd.grad(_act(act, leaf), leaf, dy.double() @ w2.double())

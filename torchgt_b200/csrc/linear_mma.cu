@@ -8,12 +8,19 @@
 // of the tensor memory.  CTAs of the same rows are neighbours in the grid, so a second column tile or a second layer finds
 // the rows in the L2.
 //
-// us back to back, here | FMA kernel that was here | library's input gradient: 320,000 rows of 64 x 64 43 | 75 | 87 (a copy of
-// the same bytes: 25), 64 x 128 74 | 139 | 132, 128 x 64 75 | 144 | 127, three layers of 64 x 64 105 forward and 110 back; 64,001
+// Tensor cores round a running sum towards zero at every step, so an error of one sign grows with the sum's length.  One
+// running sum of the large products therefore takes at most two chunks of 64; a tile has up to three of them side by side,
+// added in fp32 on the way out, and longer reductions are several launches, each adding to what the one before has written.
+//
+// us back to back, here | FMA kernel that was here | library's input gradient: 320,000 rows of 64 x 64 42 | 75 | 87 (a copy of
+// the same bytes: 25), 64 x 128 69 | 139 | 132, 128 x 64 70 | 144 | 127, three layers of 64 x 64 99 forward and 106 back; 64,001
 // rows 12 | 19 | 18.  Sums stored row by row straight from tensor memory, without the blocks in shared memory, and without
 // the second half: + 11 us; with a worker issuing the products and a general finish for every call: + 4 us.  Issue slots are
 // half busy with the split; 16 warps per SM hold the registers.
-// Relative error against 64 bits 7e-8 (FMA 1.1e-7, library 1.5e-7), 128 long 1.2e-7 (1.5e-7, 2.0e-7).
+// Relative error against 64 bits, normal operands: 64 long 7e-8 (FMA 1.1e-7, library 1.5e-7), 128 long 1.2e-7 (1.5e-7, 2.0e-7),
+// 1024 long 1.2e-7 (4.1e-7, 5.7e-7; with one running sum 1.0e-6), three gradients 64 long 7.6e-8 (library 1.5e-7, one running
+// sum 1.7e-7); operands of one sign, 128 long 1.8e-7 (9e-8, 1.7e-7), 1024 long 1.6e-7 (2.5e-7, 4.9e-7; 2.2e-6).  Six chunks at
+// most are one launch because their weights fit shared memory; 1024 x 1024 over 8,192 rows in three launches 282 us.
 #include "linear_rows.cuh"
 #include "tensor_core.cuh"
 
@@ -26,13 +33,16 @@ constexpr int kRows = 128, kCols = 64;     // of a tile: M and N of one product
 constexpr int kChunk = 64;                 // reduction elements staged at a time
 constexpr int kPieceA = kRows * 128;       // bytes of one piece of a tile of A
 constexpr int kPieceW = kCols * 128;
-constexpr int kTmemCols = 4 * kCols;       // two tiles' large and small products
-constexpr int kMostSmem = 227 * 1024;
+constexpr int kMostSums = 3;               // running sums of large products per tile, of at most two chunks each
+constexpr int kMostChunks = 2 * kMostSums; // of one launch; the weights' pieces of all of them are kept
 
 struct SplitGemm : LinearRows {
   int col_tiles;                    // per output
-  int kept;                         // chunks of the weights in shared memory: all, or one
+  int first, chunks;                // the part of the reduction this launch sums, in chunks (sources one after the other)
+  int big_sums;                     // of two chunks each, the last perhaps of one
 };
+// Tensor memory of a CTA: for each of two tiles the first sum of large products, the sum of small ones, more sums of large ones
+constexpr int tile_columns(bool more) { return (more ? 1 + kMostSums : 2) * kCols; }
 
 // Finished sums on their way out: 32 rows x 16 columns per warp, 16-byte pieces in an order that keeps rows' equal pieces
 // in different banks.
@@ -42,31 +52,37 @@ __device__ __forceinline__ int block_offset(int row, int piece) { return row * 6
 // An infinity or NaN among the operands, or a sum past the range of fp32: the pieces' sum says no more than that.  The
 // values of this row that are not finite (16 of them in the warp's block) are summed again from the operands themselves.
 __device__ __noinline__ void sum_again(const SplitGemm& p, int out, int64_t row, int col, uint8_t* block, int lane) {
+  const int src_chunks = (p.red + kChunk - 1) / kChunk;
   for (int x = 0; x < 16; ++x) {
     float* v = reinterpret_cast<float*>(block + block_offset(lane, x / 4)) + x % 4;
     if (fabsf(*v) < __int_as_float(0x7f800000) || row >= p.rows || col + x >= p.cols) continue;
     float s = 0.f;
-    for (int src = 0; src < p.sources; ++src) {
+    for (int chunk = p.first; chunk < p.first + p.chunks; ++chunk) {
+      const int src = chunk / src_chunks, k0 = chunk % src_chunks * kChunk, k1 = min(k0 + kChunk, p.red);
       const float* a = p.a[src] + row * p.red;
       const float* w = p.w[p.sources > 1 ? src : out] + (p.transposed ? int64_t(col + x) : int64_t(col + x) * p.red);
-      for (int k = 0; k < p.red; ++k) s = fmaf(__ldg(a + k), __ldg(w + int64_t(k) * (p.transposed ? p.cols : 1)), s);
+      for (int k = k0; k < k1; ++k) s = fmaf(__ldg(a + k), __ldg(w + int64_t(k) * (p.transposed ? p.cols : 1)), s);
     }
     *v = s;
   }
 }
 
-// Shared memory of a CTA, from a 1,024-byte boundary on: pieces of a chunk of A, pieces of `kept` chunks of the weights,
-// one block of finished sums per warp, the barrier and the tensor memory's address.
-inline int split_gemm_smem(int kept) { return 3 * kPieceA + kept * 3 * kPieceW + kWarps * kBlockBytes + 16; }
+// Shared memory of a CTA, from a 1,024-byte boundary on: pieces of a chunk of A, pieces of the chunks of the weights, one block
+// of finished sums per warp, the barrier and the tensor memory's address.
+__host__ __device__ inline int split_gemm_smem(int chunks) {
+  return 3 * kPieceA + chunks * 3 * kPieceW + kWarps * kBlockBytes + 16;
+}
+static_assert(3 * kPieceA + kMostChunks * 3 * kPieceW + kWarps * kBlockBytes + 16 <= 227 * 1024, "one CTA per SM");
+static_assert(2 * (3 * kPieceA + 2 * 3 * kPieceW + kWarps * kBlockBytes + 16 + 1024) <= 228 * 1024, "two with two chunks");
 
-template <bool PLAIN>   // nothing but a bias is added to the sums
-__global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_constant__ SplitGemm p) {
+template <bool PLAIN, bool LONG>   // nothing but a bias is added to the sums; more than two chunks
+__global__ void __launch_bounds__(kThreads, LONG ? 1 : 2) split_gemm_kernel(const __grid_constant__ SplitGemm p) {
   extern __shared__ __align__(1024) uint8_t s_raw[];
-  const int src_chunks = (p.red + kChunk - 1) / kChunk, chunks = src_chunks * p.sources;
+  const int src_chunks = (p.red + kChunk - 1) / kChunk;
   const uint32_t s_a = tc::smem_address(s_raw);
   const uint32_t s_w = s_a + 3 * kPieceA;
-  uint8_t* const s_block = s_raw + 3 * kPieceA + p.kept * 3 * kPieceW + threadIdx.x / 32 * kBlockBytes;
-  uint64_t* const s_done = reinterpret_cast<uint64_t*>(s_raw + 3 * kPieceA + p.kept * 3 * kPieceW + kWarps * kBlockBytes);
+  uint8_t* const s_block = s_raw + 3 * kPieceA + p.chunks * 3 * kPieceW + threadIdx.x / 32 * kBlockBytes;
+  uint64_t* const s_done = reinterpret_cast<uint64_t*>(s_raw + split_gemm_smem(p.chunks) - 16);
   uint32_t* const s_tmem = reinterpret_cast<uint32_t*>(s_done + 1);
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int across = p.col_tiles * p.outputs;               // neighbours in the grid read the same rows of A
@@ -75,12 +91,14 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
   const int walkers = gridDim.x / across;
   const int64_t tiles = (p.rows + kRows - 1) / kRows;
 
-  if (warp == 0) tc::allocate<kTmemCols>(s_tmem);
+  constexpr int kHalf = tile_columns(LONG);                 // of the tensor memory: a tile's sums
+  if (warp == 0) tc::allocate<2 * kHalf>(s_tmem);
   if (tid == 32) tc::barrier_init(s_done);
 
   const int q = 4 * (tid % 16), r0 = tid / 16;              // a worker's four reduction elements and first row
   float4 next[kRows / 16];
   auto load = [&](int64_t tile, int chunk) {
+    chunk += p.first;
     const int src = src_chunks == 1 ? chunk : chunk / src_chunks;
     const int k = (src_chunks == 1 ? 0 : chunk % src_chunks * kChunk) + q;
     const int64_t row = tile * kRows + r0;
@@ -98,8 +116,8 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
   };
   int64_t tile = blockIdx.x / across;
   if (warp < kWarps) load(tile, 0);
-  auto stage_weights = [&](int chunk, int slot) {
-    const int src = chunk / src_chunks, k0 = chunk % src_chunks * kChunk;
+  auto stage_weights = [&](int slot) {
+    const int src = (p.first + slot) / src_chunks, k0 = (p.first + slot) % src_chunks * kChunk;
     const float* w = p.w[p.sources > 1 ? src : out];
 #pragma unroll 4
     for (int u = tid; u < kCols * 16; u += kWorkers) {
@@ -119,8 +137,8 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
       tc::store4(s_w + slot * (3 * kPieceW), kPieceW, tc::tile_offset(n, k), tc::split4(v));
     }
   };
-  if (p.kept == chunks && warp < kWarps)                    // once; a long reduction's weights come along with its rows
-    for (int chunk = 0; chunk < chunks; ++chunk) stage_weights(chunk, chunk);
+  if (warp < kWarps)
+    for (int chunk = 0; chunk < p.chunks; ++chunk) stage_weights(chunk);
   if (warp < kWarps) tc::publish_operands();
   tc::fence_before_barrier();
   __syncthreads();
@@ -141,15 +159,20 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
       tc::read16(sums + kCols + j, small);
       tc::reads_done();
       const int col = c0 + warp / 4 * 32 + j;
-      float size = 0.f;
+      float v[16], size = 0.f;
+#pragma unroll
+      for (int x = 0; x < 16; ++x) v[x] = __uint_as_float(big[x]) + __uint_as_float(small[x]);
+#pragma unroll 1
+      for (int more = 1; LONG && more < p.big_sums; ++more) {
+        tc::read16(sums + (1 + more) * kCols + j, big);
+        tc::reads_done();
+#pragma unroll
+        for (int x = 0; x < 16; ++x) v[x] += __uint_as_float(big[x]);
+      }
 #pragma unroll
       for (int x = 0; x < 16; x += 4) {
-        const float4 v = make_float4(__uint_as_float(big[x]) + __uint_as_float(small[x]),
-                                     __uint_as_float(big[x + 1]) + __uint_as_float(small[x + 1]),
-                                     __uint_as_float(big[x + 2]) + __uint_as_float(small[x + 2]),
-                                     __uint_as_float(big[x + 3]) + __uint_as_float(small[x + 3]));
-        size += (fabsf(v.x) + fabsf(v.y)) + (fabsf(v.z) + fabsf(v.w));
-        *reinterpret_cast<float4*>(s_block + block_offset(lane, x / 4)) = v;
+        size += (fabsf(v[x]) + fabsf(v[x + 1])) + (fabsf(v[x + 2]) + fabsf(v[x + 3]));
+        *reinterpret_cast<float4*>(s_block + block_offset(lane, x / 4)) = make_float4(v[x], v[x + 1], v[x + 2], v[x + 3]);
       }
       if (!(size < __int_as_float(0x7f800000))) sum_again(p, out, row0 + lane, col, s_block, lane);
       __syncwarp();
@@ -180,11 +203,11 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
   uint32_t sums = tmem;
   if (warp == kWarps) {
     for (; tile < tiles; tile += walkers) {
-      for (int chunk = 0; chunk < chunks; ++chunk) {
+      for (int chunk = 0; chunk < p.chunks; ++chunk) {
         if (!__syncthreads_and(true)) goto finished;        // the workers' pieces are in place
         if (lane == 0) {
           tc::fence_after_barrier();
-          const uint32_t w = s_w + (p.kept < chunks ? 0 : chunk * (3 * kPieceW));
+          const uint32_t w = s_w + chunk * (3 * kPieceW);
 #pragma unroll
           for (int k = 0; k < kChunk / 16; ++k) {
             const uint64_t a1 = tc::k_major(s_a + 32 * k), a2 = tc::k_major(s_a + kPieceA + 32 * k),
@@ -193,7 +216,12 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
                            w3 = tc::k_major(w + 2 * kPieceW + 32 * k);
             constexpr uint32_t both = tc::instruction(kRows, 2 * kCols, false, false),
                                one = tc::instruction(kRows, kCols, false, false);
-            tc::multiply(sums, a1, w1, both, chunk + k > 0);     // a1 w1 | a1 w2
+            if (!LONG || chunk < 2) {
+              tc::multiply(sums, a1, w1, both, chunk + k > 0);   // a1 w1 | a1 w2
+            } else {
+              tc::multiply(sums + (1 + chunk / 2) * kCols, a1, w1, one, chunk % 2 + k > 0);
+              tc::multiply(sums + kCols, a1, w2, one, true);
+            }
             tc::multiply(sums + kCols, a2, w1, one, true);
             tc::multiply(sums + kCols, a2, w2, one, true);
             tc::multiply(sums + kCols, a1, w3, one, true);
@@ -203,61 +231,76 @@ __global__ void __launch_bounds__(kThreads, 2) split_gemm_kernel(const __grid_co
         }
         __syncwarp();
       }
-      sums = tmem + (sums == tmem ? 2 * kCols : 0);
+      sums = tmem + (sums == tmem ? kHalf : 0);
     }
   } else {
     int64_t before = -1;
     for (; tile < tiles; tile += walkers) {
-      for (int chunk = 0; chunk < chunks; ++chunk) {
+      for (int chunk = 0; chunk < p.chunks; ++chunk) {
 #pragma unroll
         for (int i = 0; i < kRows / 16; ++i)
           tc::store4(s_a, kPieceA, tc::tile_offset(r0 + 16 * i, q), tc::split4(next[i]));
-        if (p.kept < chunks) stage_weights(chunk, 0);
         tc::publish_operands();
         tc::fence_before_barrier();                         // everybody has read the sums of two tiles ago
         ok = __syncthreads_and(ok);
         if (!ok) goto give_up;
         // the next step's rows arrive under the products and the stores
-        const bool last = chunk + 1 == chunks;
+        const bool last = chunk + 1 == p.chunks;
         const int64_t next_tile = last ? tile + walkers : tile;
         if (next_tile < tiles) load(next_tile, last ? 0 : chunk + 1);
-        if (chunk == 0 && before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
+        if (chunk == 0 && before >= 0) finish(before, tmem + (sums == tmem ? kHalf : 0));
         ok = tc::wait(s_done, phase) && ok;
         phase ^= 1;
       }
       tc::fence_after_barrier();
       before = tile;
-      sums = tmem + (sums == tmem ? 2 * kCols : 0);
+      sums = tmem + (sums == tmem ? kHalf : 0);
     }
   give_up:
-    if (before >= 0) finish(before, tmem + (sums == tmem ? 2 * kCols : 0));
+    if (before >= 0) finish(before, tmem + (sums == tmem ? kHalf : 0));
   }
 finished:
   tc::fence_before_barrier();
   __syncthreads();
-  if (warp == 0) tc::release<kTmemCols>(tmem);
+  if (warp == 0) tc::release<2 * kHalf>(tmem);
 }
 
-int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
-  SplitGemm p;
-  static_cast<LinearRows&>(p) = of;
-  const int chunks = (p.red + kChunk - 1) / kChunk * p.sources;
-  p.kept = split_gemm_smem(chunks) <= kMostSmem ? chunks : 1;
-  const int smem = split_gemm_smem(p.kept);
-  const bool plain = is_plain(p);
-  const int rc = plain ? allow_shared_memory<split_gemm_kernel<true>>(kMostSmem)
-                       : allow_shared_memory<split_gemm_kernel<false>>(kMostSmem);
+template <bool PLAIN, bool LONG>
+int launch_part(SplitGemm& p, cudaStream_t stream) {
+  const int rc = allow_shared_memory<split_gemm_kernel<PLAIN, LONG>>(split_gemm_smem(LONG ? kMostChunks : 2));
   if (rc != TGT_OK) return rc;
+  p.big_sums = (p.chunks + 1) / 2;
   p.col_tiles = (p.cols + kCols - 1) / kCols;
   const int64_t tiles = (p.rows + kRows - 1) / kRows;
-  const int resident = 2 * (smem + 1024) <= 228 * 1024 ? 2 : 1;
+  const int resident = LONG ? 1 : 2;               // by shared memory, and tensor memory has 512 columns
   const int across = p.col_tiles * p.outputs;
   int64_t walkers = int64_t(sm_count()) * resident / across;
   if (walkers < 1) walkers = 1;
   if (walkers > tiles) walkers = tiles;
-  if (plain) split_gemm_kernel<true><<<unsigned(walkers * across), kThreads, smem, stream>>>(p);
-  else split_gemm_kernel<false><<<unsigned(walkers * across), kThreads, smem, stream>>>(p);
+  split_gemm_kernel<PLAIN, LONG><<<unsigned(walkers * across), kThreads, split_gemm_smem(p.chunks), stream>>>(p);
   TGT_CHECK_CUDA(cudaGetLastError());
+  return TGT_OK;
+}
+
+int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
+  const int chunks = (of.red + kChunk - 1) / kChunk * of.sources, parts = (chunks + kMostChunks - 1) / kMostChunks;
+  for (int part = 0; part < parts; ++part) {
+    SplitGemm p{};
+    static_cast<LinearRows&>(p) = of;
+    p.first = chunks * part / parts;
+    p.chunks = chunks * (part + 1) / parts - p.first;
+    p.onto = part > 0;
+    if (part + 1 < parts) {            // what follows the sum is for the last part
+      for (const float*& b : p.bias) b = nullptr;
+      p.act = p.gate_act = TGT_ACT_NONE;
+      p.pre = nullptr;
+      p.gate = p.add = nullptr;
+    }
+    const bool plain = is_plain(p);
+    const int rc = p.chunks > 2 ? (plain ? launch_part<true, true>(p, stream) : launch_part<false, true>(p, stream))
+                                : (plain ? launch_part<true, false>(p, stream) : launch_part<false, false>(p, stream));
+    if (rc != TGT_OK) return rc;
+  }
   return TGT_OK;
 }
 

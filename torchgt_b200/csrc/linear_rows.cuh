@@ -25,6 +25,7 @@ struct LinearRows {
   int red, cols;
   int sources, outputs;
   bool transposed;
+  bool onto;                          // c holds part of the sums already, they are added to it
   // what is done to a sum on its way out, all of it for a single output only (null / 0: nothing):
   int act;                            // TGT_ACT_*: c = act(sum + bias); pre (may be null) receives sum + bias
   float* pre;
@@ -35,12 +36,16 @@ struct LinearRows {
 
 // nothing but a bias is added to the sums
 inline bool is_plain(const LinearRows& p) {
-  return p.act == TGT_ACT_NONE && p.pre == nullptr && p.gate_act == TGT_ACT_NONE && p.add == nullptr;
+  return !p.onto && p.act == TGT_ACT_NONE && p.pre == nullptr && p.gate_act == TGT_ACT_NONE && p.add == nullptr;
 }
 
 // four values of a row
 __device__ __forceinline__ void finish_values(const LinearRows& p, int out, int64_t row, int col, float4 v) {
   const int64_t at = row * p.cols + col;
+  if (p.onto) {
+    const float4 c = *reinterpret_cast<const float4*>(p.c[out] + at);
+    v.x += c.x; v.y += c.y; v.z += c.z; v.w += c.w;
+  }
   if (p.bias[out] != nullptr) {
     const float4 b = __ldg(reinterpret_cast<const float4*>(p.bias[out] + col));
     v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
@@ -67,7 +72,7 @@ __device__ __forceinline__ void finish_values(const LinearRows& p, int out, int6
   *reinterpret_cast<float4*>(p.c[out] + at) = v;
 }
 
-// Full fp32 FMAs on tiles of 32 rows (linear_rows.cu): sources == 1, not transposed.
+// Full fp32 FMAs on tiles of 32 rows (linear_rows.cu): sources == 1, not transposed, not onto.
 int linear_few_rows(const LinearRows& p, cudaStream_t stream);
 
 // Tiles of 128 rows x 64 columns that the tensor cores would get; with fewer, the FMA kernel's smaller tiles occupy the
