@@ -522,6 +522,14 @@ TGT_API int tgt_linear_wgrad_multi(const float* const* dy, const float* x, int c
                                    size_t scratch_bytes, void* stream);
 
 /*
+ * A kernel of the products or parameter gradients above whose wait for the tensor cores ran out (about a second) makes its
+ * results NaN and is reported once, as TGT_ERR_CUDA, by the next of these calls on its device or by tgt_products_status,
+ * whichever comes first.  tgt_debug_expire_wait launches a kernel whose wait runs out.
+ */
+TGT_API int tgt_products_status(void);
+TGT_API int tgt_debug_expire_wait(void* stream);
+
+/*
  * Sum of the embedding vectors of every row's integer features: out [rows, hidden] = sum_f table[ids[row][f]] for table
  * [n_table, hidden] fp32 and ids [rows, features] int64 (models/gt_dist_graph_level.py:345), and its gradient: dtable
  * [n_table, hidden], fixed summation order, zero in row padding_idx (none: -1).  hidden 32, 64 or 128, fewer than 2^26

@@ -186,3 +186,24 @@ def test_arguments_the_calls_refuse():
     assert lib.tgt_linear_input_grad(t.data_ptr() + 4, t.data_ptr(), 8, 64, 64, t.data_ptr(), None) == 1
     n = ctypes.c_size_t()
     assert lib.tgt_linear_wgrad_multi_scratch_bytes(4, 8, 64, 64, ctypes.byref(n)) == 1
+
+
+def test_a_wait_that_runs_out_is_reported_once():
+    from torchgt_b200.linear import linear
+    c = _lib()
+    lib = c.load()
+    x, w, y = torch.randn(64, 64, device="cuda"), torch.randn(64, 64, device="cuda"), torch.empty(64, 64, device="cuda")
+    wide = torch.randn(20000, 64, device="cuda")
+
+    def product():
+        return lib.tgt_linear_rows(x.data_ptr(), w.data_ptr(), None, 64, 64, 64, y.data_ptr(), _stream())
+    assert product() == 0 and lib.tgt_products_status() == 0
+    c.check(lib.tgt_debug_expire_wait(_stream()))
+    torch.cuda.synchronize()
+    assert product() == 2 and b"tensor cores" in lib.tgt_last_error()
+    assert product() == 0 and lib.tgt_products_status() == 0
+    c.check(lib.tgt_debug_expire_wait(_stream()))
+    torch.cuda.synchronize()
+    with pytest.raises(c.TgtError):
+        linear(wide, w, w[0])
+    assert _rel(linear(wide, w, w[0]), wide.double() @ w.double().t() + w[0].double()) < 1e-3

@@ -133,6 +133,8 @@ SIGNATURES = {
     "tgt_embedding_sum_grad_scratch_bytes": (c_int, [c_int64, c_int, c_int64, c_int, POINTER(c_size_t)]),
     "tgt_embedding_sum_grad": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int64, c_int, c_int64, c_void_p, c_void_p,
                                        c_size_t, c_void_p]),
+    "tgt_products_status": (c_int, []),
+    "tgt_debug_expire_wait": (c_int, [c_void_p]),
     "tgt_linear_wgrad_scratch_bytes": (c_int, [c_int64, c_int, c_int, POINTER(c_size_t)]),
     "tgt_linear_wgrad": (c_int, [c_void_p, c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_size_t,
                                  c_void_p]),

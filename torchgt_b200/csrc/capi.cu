@@ -2,6 +2,8 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <cstring>
+#include <mutex>
 
 #include "attn_common.cuh"
 
@@ -54,6 +56,32 @@ int sm_count() {
   return n;
 }
 
+int expired_wait_word(int** word) {
+  static std::atomic<int*> words{nullptr};     // of all devices, for good
+  static std::mutex mutex;
+  const int dev = current_device();
+  if (dev < 0) return TGT_ERR_UNSUPPORTED;
+  int* all = words.load(std::memory_order_acquire);
+  if (all == nullptr) {
+    const std::lock_guard<std::mutex> lock(mutex);
+    all = words.load(std::memory_order_relaxed);
+    if (all == nullptr) {
+      // the allocation is not part of a graph that this thread may be capturing
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      TGT_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      const cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&all), kMaxDevices * sizeof(int), cudaHostAllocPortable);
+      TGT_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      TGT_CHECK_CUDA(e);
+      memset(all, 0, kMaxDevices * sizeof(int));
+      words.store(all, std::memory_order_release);
+    }
+  }
+  *word = all + dev;
+  if (__atomic_load_n(*word, __ATOMIC_RELAXED) != 0 && __atomic_exchange_n(*word, 0, __ATOMIC_RELAXED) != 0)
+    return set_error(TGT_ERR_CUDA, "a product launched before waited in vain for the tensor cores; its results are NaN");
+  return TGT_OK;
+}
+
 int check_layout(const tgt_layout* L, const char* name) {
   if (L == nullptr) return set_error(TGT_ERR_INVALID, "%s is null", name);
   if (L->n_rows < 0 || L->n_edges < 0 || L->n_rows >= (int64_t(1) << 31) - 1 ||
@@ -72,6 +100,11 @@ int check_layout(const tgt_layout* L, const char* name) {
 extern "C" int tgt_version(void) { return 101; }
 
 extern "C" const char* tgt_last_error(void) { return tgt::g_error; }
+
+extern "C" int tgt_products_status(void) {
+  int* word = nullptr;
+  return tgt::expired_wait_word(&word);
+}
 
 extern "C" int tgt_debug_set_tile_edges(int edges_per_lane_group) {
   TGT_CHECK_ARG(edges_per_lane_group >= 0, "edges_per_lane_group must be >= 0");

@@ -40,6 +40,7 @@ struct SplitGemm : LinearRows {
   int col_tiles;                    // per output
   int first, chunks;                // the part of the reduction this launch sums, in chunks (sources one after the other)
   int big_sums;                     // of two chunks each, the last perhaps of one
+  int* expired;                     // expired_wait_word
 };
 // Tensor memory of a CTA: for each of two tiles the first sum of large products, the sum of small ones, more sums of large ones
 constexpr int tile_columns(bool more) { return (more ? 1 + kMostSums : 2) * kCols; }
@@ -65,6 +66,19 @@ __device__ __noinline__ void sum_again(const SplitGemm& p, int out, int64_t row,
     }
     *v = s;
   }
+}
+
+// A wait for the products has run out: this CTA's results from `tile` on become NaN.
+__device__ __noinline__ void give_up(const SplitGemm& p, int out, int c0, int64_t tile, int walkers) {
+  if (threadIdx.x == 0) tc::report_expired_wait(p.expired);
+  const float nan = __int_as_float(0x7fffffff);
+  const int col = c0 + 4 * (threadIdx.x % 16);
+  if (col >= p.cols) return;
+  for (; tile * kRows < p.rows; tile += walkers)
+    for (int64_t row = tile * kRows + threadIdx.x / 16; row < min((tile + 1) * kRows, p.rows); row += kWorkers / 16) {
+      *reinterpret_cast<float4*>(p.c[out] + row * p.cols + col) = make_float4(nan, nan, nan, nan);
+      if (p.pre != nullptr) *reinterpret_cast<float4*>(p.pre + row * p.cols + col) = make_float4(nan, nan, nan, nan);
+    }
 }
 
 // Shared memory of a CTA, from a 1,024-byte boundary on: pieces of a chunk of A, pieces of the chunks of the weights, one block
@@ -145,7 +159,8 @@ __global__ void __launch_bounds__(kThreads, LONG ? 1 : 2) split_gemm_kernel(cons
   tc::fence_after_barrier();
   const uint32_t tmem = *s_tmem;
   uint32_t phase = 0;
-  bool ok = true;
+  bool ok = true;                      // no wait of this thread has run out
+  int64_t failed = -1;                 // the first tile of whose products one has
 
   // sums of a tile -> C: a warp finishes 32 rows x 32 columns, 16 columns at a time through its block of shared memory, so
   // that the stores are runs of 64 bytes per row
@@ -185,8 +200,7 @@ __global__ void __launch_bounds__(kThreads, LONG ? 1 : 2) split_gemm_kernel(cons
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const int r = lane / 4 + 8 * i;
-          float4 v = *reinterpret_cast<const float4*>(s_block + block_offset(r, lane % 4));
-          if (!ok) v.x = __int_as_float(0x7fffffff);
+          const float4 v = *reinterpret_cast<const float4*>(s_block + block_offset(r, lane % 4));
           if (r >= left) continue;
           if (PLAIN) {
             *reinterpret_cast<float4*>(c + int64_t(8 * i) * p.cols) = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
@@ -233,6 +247,7 @@ __global__ void __launch_bounds__(kThreads, LONG ? 1 : 2) split_gemm_kernel(cons
       }
       sums = tmem + (sums == tmem ? kHalf : 0);
     }
+    __syncthreads_and(true);
   } else {
     int64_t before = -1;
     for (; tile < tiles; tile += walkers) {
@@ -243,26 +258,34 @@ __global__ void __launch_bounds__(kThreads, LONG ? 1 : 2) split_gemm_kernel(cons
         tc::publish_operands();
         tc::fence_before_barrier();                         // everybody has read the sums of two tiles ago
         ok = __syncthreads_and(ok);
-        if (!ok) goto give_up;
+        if (!ok) {
+          failed = chunk > 0 ? tile : before;
+          goto last;
+        }
         // the next step's rows arrive under the products and the stores
         const bool last = chunk + 1 == p.chunks;
         const int64_t next_tile = last ? tile + walkers : tile;
         if (next_tile < tiles) load(next_tile, last ? 0 : chunk + 1);
         if (chunk == 0 && before >= 0) finish(before, tmem + (sums == tmem ? kHalf : 0));
-        ok = tc::wait(s_done, phase) && ok;
+        ok = tc::wait(s_done, phase);
         phase ^= 1;
       }
       tc::fence_after_barrier();
       before = tile;
       sums = tmem + (sums == tmem ? kHalf : 0);
     }
-  give_up:
-    if (before >= 0) finish(before, tmem + (sums == tmem ? kHalf : 0));
+    if (!__syncthreads_and(ok)) failed = before;
+  last:
+    if (failed >= 0) give_up(p, out, c0, failed, walkers);
+    else if (before >= 0) finish(before, tmem + (sums == tmem ? kHalf : 0));
   }
 finished:
   tc::fence_before_barrier();
   __syncthreads();
-  if (warp == 0) tc::release<2 * kHalf>(tmem);
+  if (warp == 0) {
+    if (failed >= 0) tc::wait(s_done, phase ^ 1);           // products that still run write to the memory given back
+    tc::release<2 * kHalf>(tmem);
+  }
 }
 
 template <bool PLAIN, bool LONG>
@@ -282,7 +305,7 @@ int launch_part(SplitGemm& p, cudaStream_t stream) {
   return TGT_OK;
 }
 
-int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
+int launch_split_gemm(const LinearRows& of, int* expired, cudaStream_t stream) {
   const int chunks = (of.red + kChunk - 1) / kChunk * of.sources, parts = (chunks + kMostChunks - 1) / kMostChunks;
   for (int part = 0; part < parts; ++part) {
     SplitGemm p{};
@@ -290,6 +313,7 @@ int launch_split_gemm(const LinearRows& of, cudaStream_t stream) {
     p.first = chunks * part / parts;
     p.chunks = chunks * (part + 1) / parts - p.first;
     p.onto = part > 0;
+    p.expired = expired;
     if (part + 1 < parts) {            // what follows the sum is for the last part
       for (const float*& b : p.bias) b = nullptr;
       p.act = p.gate_act = TGT_ACT_NONE;
@@ -328,6 +352,9 @@ extern "C" int tgt_linear_rows_multi(const float* a, const float* const* w, cons
   if (!shape_supported(reduce, cols))
     return set_error(TGT_ERR_UNSUPPORTED, "reduce=%d cols=%d: both must be multiples of 4, at most 1024", reduce, cols);
   if (rows == 0) return TGT_OK;
+  int* expired = nullptr;
+  const int rc = expired_wait_word(&expired);
+  if (rc != TGT_OK) return rc;
   TGT_CHECK_ARG(a && w && bias && c, "a, w, bias and c must not be null");
   TGT_CHECK_ARG(aligned16(a) && aligned16(pre) && aligned16(add), "tensors must be 16-byte aligned");
   LinearRows p{};
@@ -339,7 +366,7 @@ extern "C" int tgt_linear_rows_multi(const float* a, const float* const* w, cons
   }
   p.rows = rows; p.red = reduce; p.cols = cols; p.sources = 1; p.outputs = count;
   p.act = act; p.pre = pre; p.add = add;
-  return few_rows(rows, cols * count) ? linear_few_rows(p, stream) : launch_split_gemm(p, stream);
+  return few_rows(rows, cols * count) ? linear_few_rows(p, stream) : launch_split_gemm(p, expired, stream);
 }
 
 extern "C" int tgt_linear_input_grad(const float* dy, const float* w, int64_t rows, int out_features, int in_features,
@@ -359,6 +386,9 @@ extern "C" int tgt_linear_input_grad_multi(const float* const* dy, const float* 
     return set_error(TGT_ERR_UNSUPPORTED, "out_features=%d in_features=%d: both must be multiples of 4, at most 1024",
                      out_features, in_features);
   if (rows == 0) return TGT_OK;
+  int* expired = nullptr;
+  const int rc = expired_wait_word(&expired);
+  if (rc != TGT_OK) return rc;
   TGT_CHECK_ARG(dy && w && dx, "dy, w and dx must not be null");
   TGT_CHECK_ARG(aligned16(dx) && aligned16(gate), "tensors must be 16-byte aligned");
   LinearRows p{};
@@ -370,5 +400,28 @@ extern "C" int tgt_linear_input_grad_multi(const float* const* dy, const float* 
   p.c[0] = dx;
   p.rows = rows; p.red = out_features; p.cols = in_features; p.sources = count; p.outputs = 1; p.transposed = true;
   p.gate_act = act; p.gate = gate;
-  return launch_split_gemm(p, static_cast<cudaStream_t>(stream_));
+  return launch_split_gemm(p, expired, static_cast<cudaStream_t>(stream_));
+}
+
+namespace tgt {
+namespace {
+
+// A wait as the products' kernels have it, for an arrival that never comes.
+__global__ void expire_wait_kernel(int* expired) {
+  __shared__ uint64_t s_bar;
+  tc::barrier_init(&s_bar);
+  if (!tc::wait(&s_bar, 0)) tc::report_expired_wait(expired);
+}
+
+}  // namespace
+}  // namespace tgt
+
+extern "C" int tgt_debug_expire_wait(void* stream) {
+  using namespace tgt;
+  int* expired = nullptr;
+  const int rc = expired_wait_word(&expired);
+  if (rc != TGT_OK) return rc;
+  expire_wait_kernel<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(expired);
+  TGT_CHECK_CUDA(cudaGetLastError());
+  return TGT_OK;
 }

@@ -30,6 +30,7 @@ struct WgradParams {
   float* partial;                // [gridDim.x][count][out * in + out]
   int64_t rows;
   int in, out, count;
+  int* expired;                  // expired_wait_word
 };
 
 // One element summed again from the operands (this CTA's rows): where the pieces' sum is not finite it says no more.
@@ -138,7 +139,8 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
   }
   if (n > 0) drain(n - 1);
   // the small products of lanes 64..127 go to the warps that hold the same rows of the large ones
-  __syncthreads();
+  ok = __syncthreads_and(ok);
+  if (!ok && tid == 0) tc::report_expired_wait(p.expired);
   float* const s_small = reinterpret_cast<float*>(s_base);       // [64][65]
   float4* const s_bias = reinterpret_cast<float4*>(s_base + 64 * 65 * 4);   // [16][16]
   const bool any = int64_t(blockIdx.x) < chunks;
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
   if (i0 == 0 && tid < 64 && o0 + tid < p.out) {
     float s = 0.f;
     for (int r = 0; r < 16; ++r) s += reinterpret_cast<const float*>(s_bias)[r * 64 + tid];
+    if (!ok) s = __int_as_float(0x7fffffff);
     out[int64_t(p.out) * p.in + o0 + tid] = s;
   }
   tc::fence_before_barrier();
@@ -280,12 +283,14 @@ extern "C" int tgt_linear_wgrad_multi(const float* const* dy, const float* x, in
     }
     return TGT_OK;
   }
+  int rc = expired_wait_word(&p.expired);
+  if (rc != TGT_OK) return rc;
   TGT_CHECK_ARG(aligned16(x) && aligned16(scratch), "tensors must be 16-byte aligned");
   const int grid = wgrad_grid(rows, in_features, out_features, count);
   const size_t need = size_t(grid) * count * (n_w + out_features) * sizeof(float);
   if (scratch == nullptr || scratch_bytes < need)
     return set_error(TGT_ERR_WORKSPACE, "scratch holds %zu bytes, %zu needed", scratch_bytes, need);
-  const int rc = allow_shared_memory<linear_wgrad_kernel>(kWgSmem);
+  rc = allow_shared_memory<linear_wgrad_kernel>(kWgSmem);
   if (rc != TGT_OK) return rc;
   p.x = x; p.partial = static_cast<float*>(scratch); p.rows = rows; p.in = in_features; p.out = out_features; p.count = count;
   const dim3 g(grid, (in_features / kWgTile) * wgrad_out_tiles(out_features) * count);

@@ -79,17 +79,26 @@ __device__ __forceinline__ void commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_address(bar))
                : "memory");
 }
-// False when the phase has not completed after about a second, far beyond any product's time.
+// False when the phase has not completed after about a second, far beyond any product's time.  The last look comes after the
+// clock: a CTA that was switched out in between sees what has been done meanwhile.
 __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t phase) {
   const uint32_t address = smem_address(bar);
   const long long start = clock64();
-  do {
+  bool late = false;
+  while (true) {
     uint32_t done;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.b32 %0, 1, 0, p;\n\t}"
                  : "=r"(done) : "r"(address), "r"(phase) : "memory");
     if (done) return true;
-  } while (clock64() - start < (1ll << 31));
-  return false;
+    if (late) return false;
+    late = clock64() - start >= (1ll << 31);
+  }
+}
+// What a kernel does whose wait ran out, besides making its results NaN: the host finds it out at its next call
+// (expired_wait_word).
+__device__ __forceinline__ void report_expired_wait(int* word) {
+  *reinterpret_cast<volatile int*>(word) = 1;
+  __threadfence_system();
 }
 
 // ---- the split ----------------------------------------------------------------------------------------------------

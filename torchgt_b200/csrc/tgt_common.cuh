@@ -39,6 +39,10 @@ int current_device();
 // B200).  Grids and tile plans are sized from it.
 int sm_count();
 
+// The word (pinned host memory, one per device) that kernels of the current device set when a wait of theirs ran out.
+// TGT_ERR_CUDA, and the word cleared, when one has: to be called in front of every launch of such a kernel.
+int expired_wait_word(int** word);
+
 #ifdef __CUDACC__
 // Lets Kernel have up to `bytes` of dynamic shared memory: a property of the function on a device, set once for each
 // (by several threads at the same time is harmless).
