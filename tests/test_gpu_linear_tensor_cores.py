@@ -174,6 +174,33 @@ def test_values_that_are_not_finite_and_sums_past_the_range():
     assert _rel(dw[:, rest], (dy.double().t() @ x.double())[:, rest]) < TOL
 
 
+def test_one_nan_costs_a_small_multiple():
+    """The elements it reaches are summed again by whole blocks; one thread per element took 130 times as long."""
+    c = _lib()
+    rows = 200000
+    dy, x, w = _rand(5, (rows, 64), (rows, 64), (64, 64))
+    need = ctypes.c_size_t()
+    c.check(c.load().tgt_linear_wgrad_scratch_bytes(rows, 64, 64, ctypes.byref(need)))
+    scratch, dw = torch.empty(need.value, dtype=torch.uint8, device="cuda"), torch.empty(64, 64, device="cuda")
+    y, events = torch.empty(rows, 64, device="cuda"), [torch.cuda.Event(enable_timing=True) for _ in range(3)]
+
+    def times():
+        best = [1e9, 1e9]
+        for _ in range(5):
+            events[0].record()
+            c.check(c.load().tgt_linear_wgrad(dy.data_ptr(), x.data_ptr(), rows, 64, 64, dw.data_ptr(), None,
+                                              scratch.data_ptr(), need.value, _stream()))
+            events[1].record()
+            c.check(c.load().tgt_linear_rows(x.data_ptr(), w.data_ptr(), None, rows, 64, 64, y.data_ptr(), _stream()))
+            events[2].record()
+            torch.cuda.synchronize()
+            best = [min(b, events[i].elapsed_time(events[i + 1])) for i, b in enumerate(best)]
+        return best
+    fine = times()
+    x[777, 5] = dy[1234, 7] = float("nan")
+    assert all(slow < 20 * fast for slow, fast in zip(times(), fine))
+
+
 def test_arguments_the_calls_refuse():
     c = _lib()
     lib = c.load()

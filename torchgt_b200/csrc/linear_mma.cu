@@ -50,22 +50,37 @@ constexpr int tile_columns(bool more) { return (more ? 1 + kMostSums : 2) * kCol
 constexpr int kBlockCols = 16, kBlockBytes = 32 * kBlockCols * 4;
 __device__ __forceinline__ int block_offset(int row, int piece) { return row * 64 + ((piece ^ (row / 2)) & 3) * 16; }
 
-// An infinity or NaN among the operands, or a sum past the range of fp32: the pieces' sum says no more than that.  The
-// values of this row that are not finite (16 of them in the warp's block) are summed again from the operands themselves.
-__device__ __noinline__ void sum_again(const SplitGemm& p, int out, int64_t row, int col, uint8_t* block, int lane) {
-  const int src_chunks = (p.red + kChunk - 1) / kChunk;
-  for (int x = 0; x < 16; ++x) {
-    float* v = reinterpret_cast<float*>(block + block_offset(lane, x / 4)) + x % 4;
-    if (fabsf(*v) < __int_as_float(0x7f800000) || row >= p.rows || col + x >= p.cols) continue;
+// An infinity or NaN among the operands, or a sum past the range of fp32: the pieces' sum says no more than that.  The values
+// of such rows (bits of `rows`, counted from row0) that are not finite are summed again from the operands themselves, a row at a
+// time by the whole warp: a lane has one of the 16 columns of the warp's block and every other reduction element.  (320,000 rows
+// of 64 x 64, one row not finite: 43 us, with a thread per row and column after column 200; all rows 2.5 ms and 4.9.)
+template <int UNROLL>
+__device__ __forceinline__ void sum_rows_again(const SplitGemm& p, int out, int64_t row0, uint32_t rows, int col, uint8_t* block) {
+  const int src_chunks = (p.red + kChunk - 1) / kChunk, lane = threadIdx.x % 32;
+  col += lane % 16;
+  __syncwarp();                                             // the block is complete
+  for (; rows != 0; rows &= rows - 1) {
+    const int r = __ffs(rows) - 1;
     float s = 0.f;
-    for (int chunk = p.first; chunk < p.first + p.chunks; ++chunk) {
-      const int src = chunk / src_chunks, k0 = chunk % src_chunks * kChunk, k1 = min(k0 + kChunk, p.red);
-      const float* a = p.a[src] + row * p.red;
-      const float* w = p.w[p.sources > 1 ? src : out] + (p.transposed ? int64_t(col + x) : int64_t(col + x) * p.red);
-      for (int k = k0; k < k1; ++k) s = fmaf(__ldg(a + k), __ldg(w + int64_t(k) * (p.transposed ? p.cols : 1)), s);
-    }
-    *v = s;
+    if (row0 + r < p.rows && col < p.cols)
+#pragma unroll 1
+      for (int chunk = p.first; chunk < p.first + p.chunks; ++chunk) {
+        const int src = chunk / src_chunks, k0 = chunk % src_chunks * kChunk, k1 = min(k0 + kChunk, p.red);
+        const float* a = p.a[src] + (row0 + r) * p.red;
+        const float* w = p.w[p.sources > 1 ? src : out] + (p.transposed ? col : int64_t(col) * p.red);
+        const int step = p.transposed ? p.cols : 1;
+#pragma unroll UNROLL
+        for (int k = k0 + lane / 16; k < k1; k += 2) s = fmaf(__ldg(a + k), __ldg(w + k * step), s);
+      }
+    s += __shfl_xor_sync(~0u, s, 16);
+    float* const v = reinterpret_cast<float*>(block + block_offset(r, lane % 16 / 4)) + lane % 4;
+    if (lane < 16 && !(fabsf(*v) < __int_as_float(0x7f800000)) && row0 + r < p.rows && col < p.cols) *v = s;
   }
+}
+
+// as a call, which costs fewer registers where the finish has need of them itself
+__device__ __noinline__ void sum_rows_again_called(const SplitGemm& p, int out, int64_t row0, uint32_t rows, int col, uint8_t* block) {
+  sum_rows_again<2>(p, out, row0, rows, col, block);
 }
 
 // A wait for the products has run out: this CTA's results from `tile` on become NaN.
@@ -189,7 +204,11 @@ __global__ void __launch_bounds__(kThreads, LONG ? 1 : 2) split_gemm_kernel(cons
         size += (fabsf(v[x]) + fabsf(v[x + 1])) + (fabsf(v[x + 2]) + fabsf(v[x + 3]));
         *reinterpret_cast<float4*>(s_block + block_offset(lane, x / 4)) = make_float4(v[x], v[x + 1], v[x + 2], v[x + 3]);
       }
-      if (!(size < __int_as_float(0x7f800000))) sum_again(p, out, row0 + lane, col, s_block, lane);
+      const uint32_t odd = __ballot_sync(~0u, !(size < __int_as_float(0x7f800000)));
+      if (odd != 0) {
+        if (PLAIN) sum_rows_again<4>(p, out, row0, odd, col, s_block);
+        else sum_rows_again_called(p, out, row0, odd, col, s_block);
+      }
       __syncwarp();
       const int my_col = col + 4 * (lane % 4);
       if (my_col < p.cols) {
