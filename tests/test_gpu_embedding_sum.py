@@ -59,3 +59,16 @@ def test_calls_that_go_through_the_module():
     g, = torch.autograd.grad(y, table.weight, dy, create_graph=True)
     back, = torch.autograd.grad(g.sum(), dy)
     assert torch.allclose(back, torch.full_like(back, 3.0))
+
+
+def test_many_gradients_at_once():
+    from torchgt_b200.linear import embedding_sum
+    torch.manual_seed(8)
+    emb = torch.nn.Embedding(50, 64, padding_idx=0).cuda()
+    ids = torch.randint(0, 50, (7, 3), device="cuda")
+    dy = torch.randn(4, 7, 64, device="cuda")
+    got, = torch.autograd.grad(embedding_sum(emb, ids), emb.weight, dy, is_grads_batched=True)
+    y = emb(ids).sum(-2)
+    for g, d in zip(got, dy):
+        ref, = torch.autograd.grad(y, emb.weight, d, retain_graph=True)
+        assert (g - ref).abs().max() <= 1e-5 * ref.abs().max()

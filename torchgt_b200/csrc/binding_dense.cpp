@@ -431,7 +431,8 @@ struct EmbeddingSumBackward : public torch::autograd::Node {
   variable_list backward(const variable_list& grads) {
     if (!grads[0].defined()) return variable_list(1);
     const at::Tensor ids_ = ids.unpack();
-    if (at::GradMode::is_enabled()) {      // a second-order gradient is wanted: the library's recorded operation
+    // a second-order gradient is wanted, or many gradients at once (is_grads_batched): the library's recorded operation
+    if (at::GradMode::is_enabled() || at::isTensorSubclassLike(grads[0])) {
       auto sizes = ids_.sizes().vec();
       sizes.push_back(hidden);
       return {at::embedding_dense_backward(grads[0].unsqueeze(-2).expand(sizes), ids_, n_table, padding, false)};
