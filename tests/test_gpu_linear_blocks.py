@@ -83,6 +83,44 @@ def test_feed_forward(shape, mid, residual, act):
         assert torch.equal(feed_forward(x, *layers, act, r), y.detach())
 
 
+@pytest.mark.parametrize("tf32,width", [(False, 512), (True, 512), (True, 256)])
+def test_wide_and_tf32_products_of_the_blocks_are_the_librarys(tf32, width):
+    """Where the library is ahead: the same bits, forward and input gradient."""
+    from torchgt_b200.linear import feed_forward, linear3
+    torch.backends.cuda.matmul.allow_tf32 = tf32
+    torch.manual_seed(width)
+    layers = _layers(3, width, width)
+    x, dy = torch.randn(2048, width, device="cuda").requires_grad_(), torch.randn(2048, width, device="cuda")
+    y, z = linear3(x, *layers), feed_forward(x, layers[0], layers[1], "gelu", x)
+    with torch.no_grad():
+        refs = [nn.functional.linear(x, m.weight, m.bias) for m in layers]
+        ref = x + nn.functional.linear(nn.functional.gelu(refs[0]), layers[1].weight, layers[1].bias)
+        dx = dy @ layers[2].weight
+    assert torch.equal(z, ref) and (not tf32 or all(torch.equal(a, b) for a, b in zip(y, refs)))
+    assert torch.equal(torch.autograd.grad(y[2], x, dy)[0], dx)
+
+
+@pytest.mark.parametrize("rows,inp,out,bias", [(1023, 64, 64, True), (12287, 64, 64, False), (12288, 64, 64, False),
+                                               (10112, 256, 64, True), (10113, 256, 64, True), (5000, 384, 128, True),
+                                               (5000, 448, 128, True), (16257, 64, 28, True), (8129, 128, 320, False), (8065, 512, 448, True)])
+@pytest.mark.parametrize("tf32", [False, True])
+def test_both_sides_of_the_lines_between_the_kernels(rows, inp, out, bias, tf32):
+    from torchgt_b200.linear import linear3
+    torch.manual_seed(rows + out)
+    layers = _layers(3, inp, out, bias)
+    x, dy = torch.randn(rows, inp, device="cuda").requires_grad_(), torch.randn(rows, out, device="cuda")
+    x64, layers64 = x.detach().double().requires_grad_(), [_double(m) for m in layers]
+    torch.backends.cuda.matmul.allow_tf32 = tf32
+    for ys, refs, ms in ((linear3(x, *layers), [m(x64) for m in layers64], range(3)), ([layers[0](x)], [layers64[0](x64)], [0])):
+        got = [*ys, *torch.autograd.grad(ys, [x, *(p for i in ms for p in layers[i].parameters())], [dy] * len(ys))]
+        torch.backends.cuda.matmul.allow_tf32 = False
+        want = [*refs, *torch.autograd.grad(refs, [x64, *(p for i in ms for p in layers64[i].parameters())],
+                                            [dy.double()] * len(ys))]
+        torch.backends.cuda.matmul.allow_tf32 = tf32
+        for i, (a, b) in enumerate(zip(got, want)):      # TF32 rounds operands to 11 bits; parameter gradients stay fp32
+            assert _rel(a, b) < (1e-3 if tf32 and i <= len(ys) else TOL)
+
+
 def test_a_missing_gradient_and_gradients_nobody_wants():
     from torchgt_b200.linear import feed_forward, linear3
     torch.manual_seed(0)
@@ -183,6 +221,8 @@ def test_layers_that_differ_and_observed_modules_are_called_one_by_one():
     assert feed_forward(x, Linear(64, 64, bias=False).cuda(), b, "relu") is None
     y = feed_forward(x, Linear(64, 44).cuda(), Linear(44, 64).cuda(), "gelu", x)       # no kernel: 44 wide in between
     assert y.shape == x.shape
+    with pytest.raises(RuntimeError):
+        feed_forward(x, a, b, "tanh")
     with torch.autocast("cuda", dtype=torch.bfloat16):
         assert feed_forward(x, a, b, "relu") is None and linear3(x, a, b, b)[0].dtype == torch.bfloat16
     z = torch.func.vmap(lambda t: linear3(t, a, b, b)[1])(torch.randn(3, 5, 64, device="cuda"))

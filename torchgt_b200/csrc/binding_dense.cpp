@@ -30,16 +30,109 @@ bool plain(const at::Tensor& t, const at::Device& device) {
          t.scalar_type() == at::kFloat && t.device() == device && !torch::autograd::isFwGradDefined(t) && !t.is_neg();
 }
 
-// The caller allowed TF32 products: the forward product is then the library's, which has the tensor cores for it.
+// The caller allowed TF32 products.
 bool tf32_allowed() {
   return at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL) ==
          at::Float32Precision::TF32;
 }
 
-// From here on linear_mma.cu is ahead of the library's fp32 product for the input gradient (us back to back, here / library):
-// 64 x 64 6.3 / 4.5 at 8,192 rows, 6.4 / 7.2 at 16,384, 12.3 / 18.5 at 64,001, 43 / 87 at 320,000; 128 outputs 9.0 / 6.2, 9.0 /
-// 10.1, 17.6 / 28.3, 74 / 127.
-constexpr int64_t kInputGradRows = 12288;
+// ---- which kernel takes a product ------------------------------------------------------------------------------------
+// Device times in us, back to back in a graph: this library's kernels (linear_mma.cu, for few tiles linear_rows.cu) / PyTorch's
+// operations.  Up to a thousand rows the library's rounding is kept: the calls are bound by the host.
+
+// tiles of 128 rows x 64 columns of a result, what the tensor-core kernel's CTAs walk
+int64_t tiles(int64_t rows, int64_t columns) { return (rows + 127) / 128 * ((columns + 63) / 64); }
+// The longest reduction that is one launch of that kernel; longer ones need longer lists: 512 x 512 at 4,097 rows 47.9 / 51.9
+// forward and 48.8 / 43.2 back, at 8,192 79 / 97 and 81 / 83, at 65,536 556 / 744 and 558 / 564; 1024 x 1024 at 1,100 rows 58
+// / 50 and 61 / 44, at 8,192 282 / 358 and 280 / 321.
+constexpr int64_t kOneLaunch = 384;
+constexpr int64_t kManyTiles = 512;
+
+// A single layer's x w^T + b, fp32.  The lines are those of an FMA kernel for every length; between them calls keep the
+// library's rounding although the tensor cores are ahead of it now: 128 x 64 with a bias 18 / 14 at 16,384 rows then, 9.2 /
+// 13.9 now; 64 x 64 without one 11.7 / 7.8 then, 6.5 / 6.9 now, 13 / 20.5 at 65,536; 64 x 4 with a bias 19 / 16 at 65,536
+// then, 10 / 17 now; 256 x 256 with a bias 26.5 / 20.7 at 4,097 then, 14.9 / 19.2 now.  Inside: 64 x 64 with a bias, for which
+// the library runs a second kernel, 3.6 / 5.5 at 1,100 rows, 4.2 / 6.4 at 4,097, 6.3 / 7.5 at 8,192, 13 / 32 at 65,536, 42 /
+// 170 at 320,000; 128 x 64 5.5 / 6.6, 6.1 / 7.6, 18 / 41 and 70 / 215.  TF32: 3.6 / 3.2, 4.2 / 4.5, 6.3 / 3.5, 13 / 10.6, 42 /
+// 34; 512 x 512 556 / 58 at 65,536.
+bool layer_ahead(int64_t rows, int64_t in, int64_t out, bool bias) {
+  if (tf32_allowed() || rows < 1024 || in > 128) return false;
+  if (!bias) return in == 64 && out >= 32 && rows >= 65536;
+  if (in == 128 && rows >= 8192 && rows < 32768) return false;
+  return out >= 32 || rows < 32768;
+}
+
+// Up to 128 wide the blocks keep these kernels also where the library's take less device time, as long as a step is bound by
+// launches, of which they need fewer.  fp32, any length: below 12,288 rows an input gradient of 64 x 64 is 6.2 / 4.4 us on the
+// device, but a feed-forward block of 1,100 rows, forward and back, costs the host 104 us, with the library's input gradients
+// 122.  TF32 allowed: short lists (128 x 128 at 8,192 rows 72 us on the device forward and back, 58 with the library's
+// products, in 8 launches, not 11), and 64 x 64, where the device times are alike.
+bool narrow_or_short(int64_t rows, int64_t in, int64_t out) {
+  return in <= 128 && out <= 128 && (!tf32_allowed() || rows <= 8192 || in * out <= 64 * 64);
+}
+
+// A layer of the feed-forward block, with its activation or residual: 64 x 64 with gelu 4.8 / 7.5 at 1,100 rows, 9.1 / 13.4 at
+// 16,384, 62 / 197 at 320,000; 128 x 64 with a residual 6.9 / 8.1, 11.9 / 16.2, 102 / 251; reductions over 128 from 80 tiles
+// on (256 x 64 9.4 / 8.6 at 1,100 rows, 14.2 / 12.6 at 8,192, 14.7 / 18.1 at 10,240; 256 x 256 14.9 / 19.2 at 4,097).  TF32:
+// 64 x 64 with gelu 4.8 / 5.2, 9.1 / 6.9, 18.4 / 16.3 at 65,536, 62 / 61; 64 x 128 28 / 22 and 115 / 91.
+bool block_layer_ahead(int64_t rows, int64_t in, int64_t out) {
+  if (rows < 1024) return false;
+  if (tf32_allowed()) return narrow_or_short(rows, in, out);
+  return in <= 128 || tiles(rows, out) >= (in > kOneLaunch ? kManyTiles : 80);
+}
+
+// Three products of one input.  fp32: 64 x 64 4.0 / 16.5, 100 / 510 at 320,000; 256 x 256 14.8 / 30 at 1,100, 1,490 / 3,430;
+// 512 x 512 48 / 58 and 1,590 / 2,230 at 65,536.  TF32: 64 x 64 4.0 / 9.6, 8.3 / 10.5 at 8,192, 25 / 32 at 65,536, 100 / 103;
+// 128 x 128 8.2 / 11.4, 14.5 / 18.3 at 8,192, 22.5 / 17.7 at 16,384; 64 x 128 9.9 / 13.2 at 8,192, 191 / 123 at 320,000;
+// 192 x 192 22 / 16 at 4,097.
+bool three_products_ahead(int64_t rows, int64_t in, int64_t out) {
+  return !tf32_allowed() || narrow_or_short(rows, in, out);
+}
+
+// The sum of dy_i w_i, `out` being the reduction, for a single layer or in a block.  fp32, one: 64 x 64 6.2 / 4.4 at 8,192
+// rows, 6.3 / 6.1 at 12,288, 6.4 / 7.1 at 16,384, 12.9 / 19.6 at 65,536, 41 / 87 at 320,000; 128 x 128 8.9 / 6.0 at 4,097, 9.0
+// / 9.5 at 8,192; 256 outputs and 64 inputs 14.8 / 14.5 at 12,288, 37 / 48 at 65,536; 4 outputs 12.4 / 9.2 there.  With the
+// derivative of relu or gelu 64 x 64 8.4 / 6.2 and 10.0 / 6.9 at 8,192, 8.9 / 9.4 and 10.5 / 10.5 at 16,384, 74 / 124 and 87 /
+// 127 at 320,000.  Three: 64 x 64 11.8 / 11.6 at 1,100, 12.0 / 13.7 at 8,192, 106 / 305; 128 x 128 20.1 / 18.6 at 4,097, 20.3 /
+// 30.5 at 8,192; 256 x 256 43.5 / 45.3 at 4,097, 1,860 / 2,520; 512 x 512 137 / 131 at 4,097, 233 / 258 at 8,192, 1,727 / 1,821
+// at 65,536.  TF32: one 12.9 / 10.5 at 65,536; three of 64 x 64 12.0 / 10.7 at 8,192, 12.2 / 13.0 at 16,384, 106 / 164; 128
+// inputs and 64 outputs 12.3 / 12.8 at 8,192, 197 / 199; 128 outputs 65 / 51 at 65,536; 256 inputs 87 / 65.
+bool input_gradient_ahead(int64_t rows, int64_t out, int64_t in, size_t layers, bool block) {
+  const int64_t have = tiles(rows, in);
+  if (block && narrow_or_short(rows, in, out)) return true;
+  if (tf32_allowed()) return layers > 1 && out <= 64 && in <= 128 && have >= 128;
+  if (layers > 1) return out <= 64 || have >= (out > 256 ? kManyTiles : 128);
+  return out >= 32 && (have >= (out > kOneLaunch ? kManyTiles : 128) || (rows >= 12288 && out <= kOneLaunch));
+}
+
+// dx = (sum of dy_i w_i) * act'(at gate), in the shape of `sizes`; gate: the activation's input, of relu its result.  All but w
+// kernel_ready; below autograd.
+at::Tensor input_gradient(const std::vector<at::Tensor>& dy, const std::vector<at::Tensor>& w, at::IntArrayRef sizes,
+                          bool block, int act = TGT_ACT_NONE, const at::Tensor& gate = at::Tensor()) {
+  const int64_t out = w[0].size(0), in = w[0].size(1), rows = dy[0].numel() / out;
+  if (!input_gradient_ahead(rows, out, in, dy.size(), block)) {
+    at::Tensor dx;
+    for (size_t i = 0; i < dy.size(); ++i) {
+      const at::Tensor d = dy[i].view({rows, out});
+      if (i == 0) dx = at::mm(d, w[i]);
+      else dx.addmm_(d, w[i]);
+    }
+    dx = dx.view(sizes);
+    if (act == TGT_ACT_NONE) return dx;
+    return act == TGT_ACT_RELU ? at::threshold_backward(dx, gate, 0) : at::gelu_backward(dx, gate);
+  }
+  std::vector<at::Tensor> kept;
+  const float *from[3], *by[3];
+  for (size_t i = 0; i < dy.size(); ++i) {
+    kept.push_back(kernel_ready(w[i]));
+    from[i] = fptr(dy[i]);
+    by[i] = fptr(kept.back());
+  }
+  const at::Tensor dx = at::empty(sizes, dy[0].options());
+  check(tgt_linear_input_grad_multi(from, by, int(dy.size()), rows, int(out), int(in), act, fptr(gate), fptr(dx),
+                                    stream_of(dx)));
+  return dx;
+}
 
 // dW = dY^T X and db = the sum of dY's rows where the gradient is itself differentiated (create_graph): the kernel's values,
 // with what the two formulas' derivatives are as operations that can be recorded again.
@@ -100,15 +193,7 @@ struct NarrowLinearBackward : public torch::autograd::Node {
     const int64_t out = w_.size(0), in = w_.size(1);
     const at::Tensor dy = kernel_ready(dy_);
     const int64_t rows = dy.numel() / out;
-    if (task_should_compute_output(0) && !recorded) {
-      if (tf32_allowed() || rows < kInputGradRows) {
-        dx = at::mm(dy.view({rows, out}), w_).view(x_.sizes());
-      } else {
-        const at::Tensor wc = kernel_ready(w_);
-        dx = at::empty(x_.sizes(), dy.options());
-        check(tgt_linear_input_grad(fptr(dy), fptr(wc), rows, int(out), int(in), fptr(dx), stream_of(dy)));
-      }
-    }
+    if (task_should_compute_output(0) && !recorded) dx = input_gradient({dy}, {w_}, x_.sizes(), false);
     if (task_should_compute_output(1) || (has_bias && task_should_compute_output(2))) {
       const at::Tensor xc = kernel_ready(x_);
       size_t bytes = 0;
@@ -136,29 +221,12 @@ bool eligible(const at::Tensor& x, const at::Tensor& w, const at::Tensor& bias) 
   return !bias.defined() || (plain(bias, x.device()) && bias.dim() == 1 && bias.size(0) == out);
 }
 
-// Is linear_rows.cu ahead of the library's fp32 product?  Device time of both at reductions of 64 to 1024, 4 to 1024
-// columns and 1,100 to 320,000 rows (us here / there); up to a thousand rows the library's rounding is kept, the calls
-// being bound by the host.
-//   64 in, with a bias (the library runs a second kernel for it): ahead everywhere, 64 x 64 5.1 / 7.3 at 4,097 rows, 11.2 /
-//     12.3 at 16,384, 77.8 / 173 at 320,000, 64 x 256 272 / 679; not with few columns of its 64-wide tile in use on long
-//     lists: 64 x 4 8.7 / 9.3 at 16,384 rows but 18.9 / 16.4 at 65,536 (64 x 40: 19.1 / 29.3).
-//   128 in, with a bias: 128 x 64 7.0 / 9.1 at 4,097 rows, 17.9 / 14.9 at 16,384, 35.8 / 42.6 at 65,536.
-//   64 in, no bias: 64 x 64 11.7 / 7.8 at 16,384 rows, 20.1 / 21.1 at 65,536, 76.5 / 87.1 at 320,000.
-//   Longer reductions, or 128 without a bias: behind (256 x 256 26.5 / 20.7 at 4,097 rows, 512 x 512 4091 / 3623 and
-//     1024 x 1024 16602 / 12243 at 320,000) or ahead by a little on long lists only.
-bool rows_kernel_ahead(int64_t rows, int64_t in, int64_t out, bool bias) {
-  if (rows < 1024 || in > 128) return false;
-  if (!bias) return in == 64 && out >= 32 && rows >= 65536;
-  if (in == 128 && rows >= 8192 && rows < 32768) return false;
-  return out >= 32 || rows < 32768;
-}
-
 at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<at::Tensor>& bias_in) {
   const at::Tensor bias = bias_in.has_value() ? *bias_in : at::Tensor();
   if (!eligible(x, w, bias)) return at::linear(x, w, bias_in);
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t rows = x.numel() / w.size(1);
-  const bool library = tf32_allowed() || !rows_kernel_ahead(rows, w.size(1), w.size(0), bias.defined());
+  const bool library = !layer_ahead(rows, w.size(1), w.size(0), bias.defined());
   const bool record = torch::autograd::compute_requires_grad(x, w, bias);
   at::Tensor y;
   if (library && !record) return at::linear(x, w, bias_in);
@@ -191,6 +259,11 @@ at::Tensor linear(const at::Tensor& x, const at::Tensor& w, const std::optional<
 void parameter_gradients(const std::vector<at::Tensor>& dy, const at::Tensor& x, int64_t rows, int64_t in, int64_t out,
                          const std::vector<at::Tensor*>& dw, const std::vector<at::Tensor*>& db) {
   const int n = int(dy.size());
+  // wider, the tiles of three gradients fill the chip once and a bit (512 x 512 at 8,192 rows 281 us together, 251 one by one)
+  if (n > 1 && in * out > 384 * 384) {
+    for (int i = 0; i < n; ++i) parameter_gradients({dy[i]}, x, rows, in, out, {dw[i]}, {db[i]});
+    return;
+  }
   size_t bytes = 0;
   check(tgt_linear_wgrad_multi_scratch_bytes(n, rows, int(in), int(out), &bytes));
   const at::Tensor scratch = at::empty({int64_t(bytes < 16 ? 16 : bytes)}, x.options().dtype(at::kByte));
@@ -237,7 +310,7 @@ struct NarrowLinear3Backward : public torch::autograd::Node {
       }
       const at::AutoDispatchBelowADInplaceOrView below;
       dy.push_back(kernel_ready(grads[i]));
-      w.push_back(kernel_ready(w_));
+      w.push_back(w_);
       if (!task_should_compute_output(1 + 2 * i) && !(has_bias && task_should_compute_output(2 + 2 * i))) continue;
       dy_p.push_back(dy.back());
       dw.push_back(&result[1 + 2 * i]);
@@ -246,16 +319,7 @@ struct NarrowLinear3Backward : public torch::autograd::Node {
     if (dy.empty()) return result;
     const at::AutoDispatchBelowADInplaceOrView below;
     const int64_t out = w[0].size(0), in = w[0].size(1), rows = x_.numel() / in;
-    if (want_dx && !recorded) {
-      const float *from[3], *by[3];
-      for (size_t i = 0; i < dy.size(); ++i) {
-        from[i] = fptr(dy[i]);
-        by[i] = fptr(w[i]);
-      }
-      result[0] = at::empty(x_.sizes(), dy[0].options());
-      check(tgt_linear_input_grad_multi(from, by, int(dy.size()), rows, int(out), int(in), TGT_ACT_NONE, nullptr,
-                                        fptr(result[0]), stream_of(x_)));
-    }
+    if (want_dx && !recorded) result[0] = input_gradient(dy, w, x_.sizes(), true);
     if (!dy_p.empty()) parameter_gradients(dy_p, kernel_ready(x_), rows, in, out, dw, db);
     return result;
   }
@@ -265,9 +329,6 @@ struct NarrowLinear3Backward : public torch::autograd::Node {
     for (SavedVariable& w : weight) w.reset_data();
   }
 };
-
-// Shorter inputs keep the library's rounding, as the single layer does (rows_kernel_ahead).
-constexpr int64_t kBlockRows = 1024;
 
 // {x w_i^T + b_i}
 std::vector<at::Tensor> linear3(const at::Tensor& x, const std::vector<at::Tensor>& w,
@@ -279,12 +340,15 @@ std::vector<at::Tensor> linear3(const at::Tensor& x, const std::vector<at::Tenso
     bias.push_back(bias_in[i].has_value() ? *bias_in[i] : at::Tensor());
     together = together && eligible(x, w[i], bias[i]) && w[i].sizes() == w[0].sizes() && bias[i].defined() == bias[0].defined();
   }
-  if (!together || x.numel() / w[0].size(1) < kBlockRows)
+  if (!together || x.numel() / w[0].size(1) < 1024)
     return {tgt_host::linear(x, w[0], bias_in[0]), tgt_host::linear(x, w[1], bias_in[1]), tgt_host::linear(x, w[2], bias_in[2])};
   const c10::cuda::CUDAGuard guard(x.device());
   const int64_t out = w[0].size(0), in = w[0].size(1), rows = x.numel() / in;
   variable_list y;
-  {
+  if (!three_products_ahead(rows, in, out)) {
+    const at::AutoDispatchBelowADInplaceOrView below;
+    for (int i = 0; i < 3; ++i) y.push_back(at::linear(x, w[i], bias_in[i]));
+  } else {
     const at::AutoDispatchBelowADInplaceOrView below;
     const at::Tensor xc = kernel_ready(x);
     auto sizes = x.sizes().vec();
@@ -341,21 +405,15 @@ struct FeedForwardBackward : public torch::autograd::Node {
     const at::Tensor h = hidden.unpack(), gate_ = act == TGT_ACT_RELU ? h : gate.unpack();
     const c10::cuda::CUDAGuard guard(x_.device());
     const at::AutoDispatchBelowADInplaceOrView below;
-    const at::Tensor dy = kernel_ready(grads[0]), w2c = kernel_ready(w2_), hc = kernel_ready(h), gc = kernel_ready(gate_);
+    const at::Tensor dy = kernel_ready(grads[0]), hc = kernel_ready(h), gc = kernel_ready(gate_);
     const int64_t in = w1_.size(1), mid = w1_.size(0), out = w2_.size(0), rows = x_.numel() / in;
     if (task_should_compute_output(3) || task_should_compute_output(4))
       parameter_gradients({dy}, hc, rows, mid, out, {&result[3]}, {&result[4]});
     const bool first = task_should_compute_output(1) || task_should_compute_output(2);
     if (!first && !task_should_compute_output(0)) return result;
-    const at::Tensor dz = at::empty(h.sizes(), h.options());
-    const float *from = fptr(dy), *by = fptr(w2c);
-    check(tgt_linear_input_grad_multi(&from, &by, 1, rows, int(out), int(mid), act, fptr(gc), fptr(dz), stream_of(x_)));
+    const at::Tensor dz = input_gradient({dy}, {w2_}, h.sizes(), true, act, gc);
     if (first) parameter_gradients({dz}, kernel_ready(x_), rows, in, mid, {&result[1]}, {&result[2]});
-    if (task_should_compute_output(0)) {
-      const at::Tensor w1c = kernel_ready(w1_);
-      result[0] = at::empty(x_.sizes(), dz.options());
-      check(tgt_linear_input_grad(fptr(dz), fptr(w1c), rows, int(mid), int(in), fptr(result[0]), stream_of(x_)));
-    }
+    if (task_should_compute_output(0)) result[0] = input_gradient({dz}, {w1_}, x_.sizes(), true);
     return result;
   }
   std::string name() const override { return "FeedForwardBackward"; }
@@ -366,17 +424,21 @@ struct FeedForwardBackward : public torch::autograd::Node {
 
 bool feed_forward_eligible(const at::Tensor& x, const at::Tensor& w1, const at::Tensor& b1, const at::Tensor& w2,
                            const at::Tensor& b2, const at::Tensor& residual) {
-  if (!b1.defined() || !b2.defined() || !eligible(x, w1, b1) || x.numel() / w1.size(1) < kBlockRows ||
-      !plain(w2, x.device()) || !plain(b2, x.device())) return false;
+  if (!b1.defined() || !b2.defined() || !eligible(x, w1, b1) || !plain(w2, x.device()) || !plain(b2, x.device()))
+    return false;
   if (w2.dim() != 2 || w2.size(1) != w1.size(0) || b2.dim() != 1 || b2.size(0) != w2.size(0)) return false;
   const int64_t mid = w2.size(1), out = w2.size(0);
+  const int64_t rows = x.numel() / w1.size(1);
   if (mid % 64 != 0 || mid > 1024 || out % 4 != 0 || out < 4 || out > 1024) return false;
+  // one by one otherwise: a node of the library's products would save nothing
+  if (!block_layer_ahead(rows, w1.size(1), mid) || !block_layer_ahead(rows, mid, out)) return false;
   return !residual.defined() || (plain(residual, x.device()) && out == w1.size(1) && residual.sizes() == x.sizes());
 }
 
 at::Tensor feed_forward(const at::Tensor& x, const at::Tensor& w1, const at::Tensor& b1, const at::Tensor& w2,
                         const at::Tensor& b2, const std::string& activation, const std::optional<at::Tensor>& residual_in) {
   const at::Tensor residual = residual_in.has_value() ? *residual_in : at::Tensor();
+  TORCH_CHECK(activation == "relu" || activation == "gelu", "feed_forward knows relu and gelu, not ", activation);
   const int act = activation == "relu" ? TGT_ACT_RELU : TGT_ACT_GELU;
   if (!feed_forward_eligible(x, w1, b1, w2, b2, residual)) {
     const at::Tensor z = tgt_host::linear(x, w1, b1);

@@ -33,9 +33,9 @@ struct WgradParams {
   int* expired;                  // expired_wait_word
 };
 
-// Where a sum of pieces is not finite (an operand is not, or a sum passes the range of fp32) it says no more than that.  The CTA
-// sums its tile again over its rows with FMAs, four outputs x four inputs a thread, and replaces those elements.  (320,000 rows of
-// 64 x 64 with one NaN 180 us, with a thread per element 7.1 ms; 64,001 of 1024 x 1024 12 ms and 0.98 s.)
+// Where a sum of pieces is not finite (an operand is not, or a sum passes the range of fp32) it says no more than that.  The
+// CTA sums its tile again over its rows with FMAs, four outputs x four inputs a thread, and replaces those elements.  (320,000
+// rows of 64 x 64 with one NaN 180 us, with a thread per element 7.1 ms; 64,001 of 1024 x 1024 12 ms and 0.98 s.)
 __device__ __noinline__ void sum_again(const WgradParams& p, const float* dy, int o0, int i0, float* out) {
   const int o = o0 + 4 * (threadIdx.x / 16), i = i0 + 4 * (threadIdx.x % 16);
   if (o >= p.out || i >= p.in) return;

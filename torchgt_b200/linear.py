@@ -1,10 +1,11 @@
 """``Linear``: ``torch.nn.Linear`` with the same parameters and ``state_dict`` keys for narrow fp32 layers over many
 rows (the models' 64 x 64 projections and FFN layers over 4,000 to 870,000 rows), and the blocks the models build of it.  The
 nodes are in ``csrc/binding_dense.cpp``: full fp32 products and input gradients run on the tensor cores from three bf16 pieces
-per value (``csrc/linear_mma.cu``; few rows: ``csrc/linear_rows.cu``), or as the library's GEMM when the caller allows TF32;
-weight and bias gradients run ``csrc/linear_wgrad.cu``.  CPU tensors, other dtypes, inputs that are not a multiple of 64 wide and
-outputs that are not a multiple of 4 wide are ``torch.nn.functional.linear``, and so is whatever is traced, compiled, autocast
-or transformed by ``torch.func``."""
+per value (``csrc/linear_mma.cu``; few rows: ``csrc/linear_rows.cu``), or as the library's GEMM, by rules on rows, widths and
+whether the caller allows TF32 (there, with the times of both sides; with TF32 allowed single layers are the library's, and blocks
+but the narrow ones); weight and bias gradients run ``csrc/linear_wgrad.cu``.  CPU tensors, other dtypes, inputs that are
+not a multiple of 64 wide and outputs that are not a multiple of 4 wide are ``torch.nn.functional.linear``, and so is whatever
+is traced, compiled, autocast or transformed by ``torch.func``."""
 from __future__ import annotations
 
 import ctypes
