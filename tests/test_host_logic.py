@@ -178,3 +178,27 @@ def test_layer_norm_and_linear_modules_are_torch_modules_on_the_cpu():
     y2.sum().backward()
     assert torch.equal(y, y2) and torch.equal(x.grad, x2.grad)
     assert torch.equal(lin.weight.grad, ref_lin.weight.grad) and torch.equal(ln.weight.grad, ref_ln.weight.grad)
+
+
+def test_products_of_fewer_pieces_miss_the_bound_of_the_tensor_core_tests():
+    """fp32 products from three bf16 pieces per value, in fp64: all six kept products stay below the bound the GPU tests use,
+    without a third piece they do not."""
+    gen = torch.Generator().manual_seed(0)
+    a, b = torch.randn(256, 64, generator=gen), torch.randn(64, 64, generator=gen)
+
+    def pieces(x):
+        out = []
+        for _ in range(3):
+            out.append(x.bfloat16().float())
+            x = x - out[-1]
+        return [p.double() for p in out]
+    pa, pb = pieces(a), pieces(b)
+    ref = a.double() @ b.double()
+
+    def err(kept):
+        return float((sum(pa[i] @ pb[j] for i, j in kept) - ref).norm() / ref.norm())
+    six = [(0, 0), (0, 1), (1, 0), (1, 1), (0, 2), (2, 0)]
+    tol = 1e-6      # TOL in test_gpu_linear_tensor_cores.py
+    assert err(six) < tol / 5
+    for without in ([(0, 2)], [(2, 0)], [(0, 2), (2, 0)]):
+        assert err([p for p in six if p not in without]) > 2 * tol

@@ -76,7 +76,7 @@ __device__ __forceinline__ void finish_values(const LinearRows& p, int out, int6
 int linear_few_rows(const LinearRows& p, cudaStream_t stream);
 
 // Tiles of 128 rows x 64 columns that the tensor cores would get; with fewer, the FMA kernel's smaller tiles occupy the
-// chip better (us back to back, FMA / tensor cores, 64 x 64: 4,097 rows 4.3 / 6.3, 8,192 rows 6.0 / 6.5, 16,384 rows 10.7 / 6.5;
+// chip better (us back to back, FMA / tensor cores, 64 x 64: 4,097 rows 4.2 / 6.3, 8,192 rows 6.0 / 6.5, 16,384 rows 10.7 / 6.5;
 // 64 x 128 at 8,192 rows, 128 tiles, 8.9 / 6.6).
 inline bool few_rows(int64_t rows, int cols) { return (rows + 127) / 128 * ((cols + 63) / 64) < 80; }
 

@@ -164,8 +164,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
   if (!ok && tid == 0) tc::report_expired_wait(p.expired);
   float* const s_small = reinterpret_cast<float*>(s_base);       // [64][65]
   float4* const s_bias = reinterpret_cast<float4*>(s_base + 64 * 65 * 4);   // [16][16]
-  const bool any = int64_t(blockIdx.x) < chunks;
-  if (warp % 4 >= 2 && any) {
+  if (warp % 4 >= 2) {                                           // every CTA has a chunk: wgrad_grid
 #pragma unroll
     for (int j = 0; j < 32; j += 16) {
       uint32_t v[16];
@@ -184,7 +183,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
 #pragma unroll
     for (int j = 0; j < 32; j += 16) {
       uint32_t v[16];
-      if (any) tc::read16(mine + 128 + j, v);
+      tc::read16(mine + 128 + j, v);
       tc::reads_done();
 #pragma unroll
       for (int a = 0; a < 16; a += 4) {
@@ -193,7 +192,7 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
         float f[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-          f[b] = any ? main_sum[j + a + b] + (__uint_as_float(v[a + b]) + s_small[row * 65 + col + b]) : 0.f;
+          f[b] = main_sum[j + a + b] + (__uint_as_float(v[a + b]) + s_small[row * 65 + col + b]);
           if (!ok) f[b] = __int_as_float(0x7fffffff);
           again = again || (ok && !(fabsf(f[b]) < __int_as_float(0x7f800000)));
         }
