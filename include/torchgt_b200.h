@@ -470,8 +470,9 @@ TGT_API int tgt_add_layer_norm_bwd(const float* dy, const float* dsum, const flo
                                    void* scratch, size_t scratch_bytes, void* stream);
 
 /*
- * Product of a narrow nn.Linear over many rows, full fp32 products and sums: c [rows, cols] = a [rows, reduce] w^T +
- * bias for w [cols, reduce] and bias [cols] (may be NULL).  reduce and cols must be multiples of 4, at most 1024
+ * Product of a narrow nn.Linear over many rows in fp32 (FMAs over few rows, else six products of three bf16 pieces per
+ * value with fp32 sums: relative error 7e-8 to 1.4e-7, 1.8e-7 with operands of one sign): c [rows, cols] = a [rows, reduce]
+ * w^T + bias for w [cols, reduce] and bias [cols] (may be NULL).  reduce and cols must be multiples of 4, at most 1024
  * (TGT_ERR_UNSUPPORTED otherwise), all pointers 16-byte aligned (models/graphormer_dist_node_level.py:241-245,281-286).
  */
 TGT_API int tgt_linear_rows(const float* a, const float* w, const float* bias, int64_t rows, int reduce, int cols,
@@ -492,7 +493,7 @@ TGT_API int tgt_linear_wgrad(const float* dy, const float* x, int64_t rows, int 
 
 /*
  * The input gradient of the same layer: dx [rows, in_features] = dy [rows, out_features] w for w [out_features,
- * in_features], full fp32 products and sums.  Both widths multiples of 4, at most 1024 (TGT_ERR_UNSUPPORTED otherwise),
+ * in_features], of the same precision.  Both widths multiples of 4, at most 1024 (TGT_ERR_UNSUPPORTED otherwise),
  * pointers 16-byte aligned.
  */
 TGT_API int tgt_linear_input_grad(const float* dy, const float* w, int64_t rows, int out_features, int in_features,

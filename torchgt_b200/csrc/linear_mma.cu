@@ -16,7 +16,7 @@
 // the same bytes: 25), 64 x 128 69 | 139 | 132, 128 x 64 70 | 144 | 127, three layers of 64 x 64 99 forward and 106 back; 64,001
 // rows 12 | 19 | 18.  Sums stored row by row straight from tensor memory, without the blocks in shared memory, and without
 // the second half: + 11 us; with a worker issuing the products and a general finish for every call: + 4 us.  Issue slots are
-// half busy with the split; 16 warps per SM hold the registers.
+// 42 % busy; what is left is the wait for the rows, with the 17 warps per SM that the registers allow.
 // Relative error against 64 bits, normal operands: 64 long 7e-8 (FMA 1.1e-7, library 1.5e-7), 128 long 1.2e-7 (1.5e-7, 2.0e-7),
 // 1024 long 1.2e-7 (4.1e-7, 5.7e-7; with one running sum 1.0e-6), three gradients 64 long 7.6e-8 (library 1.5e-7, one running
 // sum 1.7e-7); operands of one sign, 128 long 1.8e-7 (9e-8, 1.7e-7), 1024 long 1.6e-7 (2.5e-7, 4.9e-7; 2.2e-6).  Six chunks at
