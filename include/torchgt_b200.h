@@ -94,7 +94,7 @@ TGT_API int tgt_debug_set_lane_mode(int mode);
  * the previous kernel drains, then wait for it to complete).  A bit mask: 1 = a walk kernel after the
  * statistics kernel or another walk kernel, 2 = the kernel that finishes cross-tile rows after its walk
  * kernel, 4 = a walk kernel after such a kernel; 0 launches everything one after the other, the default is
- * 1 | 4.  The results are bitwise the same.  Process-wide.
+ * 1 | 2 | 4.  The results are bitwise the same.  Process-wide.
  */
 TGT_API int tgt_debug_set_dependent_launch(int links);
 
@@ -283,7 +283,8 @@ TGT_API int tgt_sparse_attn_bwd(const void* dout, const void* q, const void* k, 
  * a pass A left in the same scratch for the same inputs), 1 = streaming pre-pass that computes the
  * statistics from dO and O — required (in the same or an earlier call) only when dbias is wanted,
  * because dbias needs them per edge before a row is complete.  tgt_sparse_attn_bwd runs 6, or 7 with
- * dbias.  Lets a caller time or overlap the stages; replaces the same reference code.
+ * dbias; where one call runs 2 and 4, dbias is written by pass B, pass A derives the statistics and stage 1
+ * is left out.  Lets a caller time or overlap the stages; replaces the same reference code.
  */
 TGT_API int tgt_sparse_attn_bwd_passes(const void* dout, const void* q, const void* k, const void* v,
                                        const float* bias, int bias_heads, const void* out,

@@ -1,0 +1,99 @@
+"""Rows that cross tiles, and the two routes of the bias gradient.
+
+A row's tiles leave partial sums that a second kernel adds up: up to eight further tiles by one lane group, more by a
+whole CTA.  dbias is written by the pass over the sources when both passes run in one call, by the pass over the
+destinations when the caller runs them one by one."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import TOL_BF16, TOL_F32, rel_err
+from oracle import sparse_attn_oracle as sao
+
+pytestmark = pytest.mark.gpu
+
+GROUP_TILES = 8
+
+
+@pytest.fixture(autouse=True)
+def _own_tiles():
+    from torchgt_b200 import _cabi
+    yield
+    _cabi.check(_cabi.load().tgt_debug_set_tile_edges(0))
+
+
+def _graph_with_rows_of(lengths, n, seed):
+    """Edges whose destinations (and, in a second copy turned round, sources) have exactly `lengths` edges each."""
+    rng = np.random.default_rng(seed)
+    rows = np.concatenate([np.full(m, i) for i, m in enumerate(lengths)])
+    ends = rng.integers(0, n, rows.size)
+    ei = np.concatenate([np.stack([ends, rows]), np.stack([rows, ends])], axis=1)
+    return torch.from_numpy(ei[:, rng.permutation(ei.shape[1])])
+
+
+@pytest.mark.parametrize("heads,head_dim,dtype", [(8, 8, torch.float32), (1, 8, torch.float32), (2, 8, torch.float32),
+                                                  (8, 16, torch.float32), (3, 8, torch.float32), (8, 8, torch.bfloat16)])
+@pytest.mark.parametrize("bias", ["none", "edge", "head"])
+def test_rows_over_one_to_many_tiles_match_the_oracle(heads, head_dim, dtype, bias):
+    from torchgt_b200 import SparseGraph, _cabi, sparse_graph_attention
+    _cabi.check(_cabi.load().tgt_debug_set_tile_edges(4))
+    group = 4 * 128 // 32     # edges of a tile of the widest lane group; narrower ones have up to 512
+    tile = {(8, 8): 64 if dtype == torch.bfloat16 else 32, (1, 8): 256, (2, 8): 128, (8, 16): group, (3, 8): 256}[heads, head_dim]
+    lengths = [m * tile + d for m in (1, 2, GROUP_TILES - 1, GROUP_TILES, GROUP_TILES + 1, 3 * GROUP_TILES) for d in (-1, 0, 1)]
+    lengths = [3, 0] + lengths[:12 if tile > 100 else 18] + [1, 0, 0, 2]
+    n = len(lengths) + 40
+    ei = _graph_with_rows_of(lengths, n, 5)
+    gen = torch.Generator().manual_seed(6)
+    q, k, v, dout = (torch.randn(n, heads, head_dim, generator=gen).to(dtype) for _ in range(4))
+    b = None if bias == "none" else torch.randn((ei.shape[1],) + ((heads,) if bias == "head" else ()), generator=gen) * 0.1
+    if bias == "edge" and heads == 3:
+        pytest.skip("a shared bias of three heads is expanded per head")
+    qc, kc, vc = (t.cuda().requires_grad_() for t in (q, k, v))
+    bc = None if b is None else b.cuda().requires_grad_()
+    out = sparse_graph_attention(qc, kc, vc, SparseGraph(ei.cuda(), n), bc)
+    out.backward(dout.cuda())
+    ref, _ = sao.forward_closed_form(q.float(), k.float(), v.float(), ei, b)
+    dq, dk, dv, dt = sao.backward_closed_form(q.float(), k.float(), v.float(), ei, dout.float(), b)
+    tol = TOL_F32 if dtype == torch.float32 else TOL_BF16
+    assert rel_err(out.detach().float(), ref) < tol
+    for got, want in ((qc.grad, dq), (kc.grad, dk), (vc.grad, dv)):
+        assert rel_err(got.float(), want) < tol
+    if b is not None:
+        assert rel_err(bc.grad, dt if bias == "head" else dt.sum(axis=1)) < tol
+
+
+@pytest.mark.parametrize("columns", [1, 8])
+def test_passes_one_by_one_and_in_one_call_agree(columns):
+    import ctypes
+    from torchgt_b200 import SparseGraph, _cabi
+    lib = _cabi.load()
+    n, heads, dim = 700, 8, 8
+    rng = np.random.default_rng(3)
+    ei = torch.from_numpy(np.concatenate([rng.integers(0, n, (2, 5000)), np.stack([np.zeros(900, int), rng.integers(0, n, 900)])],
+                                         axis=1)).cuda()
+    graph = SparseGraph(ei, n)
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    q, k, v, dout = (torch.randn(n, heads, dim, generator=gen, device="cuda") for _ in range(4))
+    bias = torch.randn(ei.shape[1] * columns, generator=gen, device="cuda") * 0.1
+    stream = torch.cuda.current_stream().cuda_stream
+    size = ctypes.c_size_t()
+    _cabi.check(lib.tgt_sparse_attn_scratch_bytes(graph.by_dst.byref(), graph.by_src.byref(), heads, dim, 0, 1, ctypes.byref(size)))
+    out, z = torch.empty_like(q), torch.empty(n, heads, device="cuda")
+    scratch = torch.empty(max(size.value, 1 << 20), dtype=torch.uint8, device="cuda")
+    _cabi.check(lib.tgt_sparse_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), columns, graph.by_dst.byref(),
+                                        out.data_ptr(), z.data_ptr(), heads, dim, 0, scratch.data_ptr(), scratch.numel(), stream))
+    results = []
+    for sequence in ((7,), (0,), (1, 2, 4), (3, 4), (1, 6)):
+        got = [torch.full_like(t, float("nan")) for t in (q, k, v, bias)]
+        scratch.fill_(255)
+        for passes in sequence:
+            entry = lib.tgt_sparse_attn_bwd_passes if passes else lib.tgt_sparse_attn_bwd
+            _cabi.check(entry(dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), bias.data_ptr(), columns, out.data_ptr(),
+                              z.data_ptr(), graph.by_dst.byref(), graph.by_src.byref(), *(t.data_ptr() for t in got), heads, dim,
+                              0, scratch.data_ptr(), scratch.numel(), stream, *([passes] if passes else [])))
+        torch.cuda.synchronize()
+        results.append(got)
+    for got in results[1:]:
+        for a, b in zip(got, results[0]):
+            assert torch.isfinite(a).all()
+            assert float((a - b).abs().max()) <= TOL_F32 * float(b.abs().max())

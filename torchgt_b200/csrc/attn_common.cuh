@@ -14,10 +14,9 @@
 // A row that crosses a range boundary leaves partial sums in shared memory ("head" = the range
 // starts inside the row, "tail" = the row starts here and runs past the range); after a barrier
 // the group that holds the tail adds the heads of the following groups in order.  If the row
-// also crosses the tile boundary the CTA writes its sum to a per-tile carry in global memory and
-// counts itself in on the row's arrival counter; the CTA that arrives last adds the carries in tile
-// order and finishes the row (nobody waits for anybody).  Every sum has a fixed order whichever CTA
-// does it: no floating-point atomics, bitwise reproducible results.
+// also crosses the tile boundary the CTA writes its sum to a per-tile carry in global memory, and a second
+// kernel adds the carries and finishes the row (finish_crossing_rows).  Every sum has a fixed order: no
+// floating-point atomics, bitwise reproducible results.
 //
 // Rows without edges are zero-filled.  The few between two rows of a range are filled by the group that walks over
 // them; aligned blocks of kGapRows rows that are empty as a whole are looked for by the first CTAs, 4,096 rows each, two
@@ -43,13 +42,6 @@ namespace tgt {
 #ifndef TGT_UNROLL
 #define TGT_UNROLL 4
 #endif
-// Lane groups up to this width finish the rows that cross tiles in a second kernel; wider ones do it
-// inside the walk kernel (the last tile to arrive).  Narrow groups have many small tiles (a thread
-// walks 32 edges at G = 2), where the fence and the arrival count of every CTA cost more than one
-// extra launch.
-#ifndef TGT_STITCH_KERNEL_MAX_G
-#define TGT_STITCH_KERNEL_MAX_G 4
-#endif
 // Which walks use 32-byte lanes when nobody forces a lane width (see lane_bytes()).  Measured on B200
 // (fp32, 8-float heads, 64K-node batches and their 2-, 4- and 8-rank head slices, 870K-node batch): the
 // forward gains on 128-byte rows (55 -> 50 us), the dQ pass on 64- and 128-byte rows (86 -> 80 us,
@@ -70,6 +62,9 @@ namespace tgt {
 #define TGT_WALK_BOUNDS __launch_bounds__(128)
 #endif
 
+#ifndef TGT_LEAST_GE
+#define TGT_LEAST_GE 8
+#endif
 constexpr int kBlockThreads = 128;
 constexpr int kUnroll = TGT_UNROLL;  // edges per lane group whose gathers are in flight together
 constexpr int kGeStep = 4;           // ge is a multiple of this (and of every batch size below)
@@ -78,11 +73,12 @@ constexpr int kGeStep = 4;           // ge is a multiple of this (and of every b
 // 256-byte rows; bf16 128-byte rows): batches of 4 edges are best everywhere except for fp32 rows of
 // 16 lanes (the 8 heads x 8 case, two lane groups per warp), where batches of 2 are 9-10 % faster
 // (64K benchmark step 176 -> 158 us, 870K step 5.11 -> 4.67 ms); narrower groups lose 20-70 % with 2.
-template <typename T, int W, int G>
-constexpr int walk_unroll() {
-  if (W == 32) return TGT_WIDE_UNROLL;
-  return (std::is_same<T, float>::value && G == 16 && TGT_UNROLL == 4) ? 2 : TGT_UNROLL;
+constexpr int walk_batch(bool fp32, int w, int g) {
+  if (w == 32) return TGT_WIDE_UNROLL;
+  return (fp32 && g == 16 && TGT_UNROLL == 4) ? 2 : TGT_UNROLL;
 }
+template <typename T, int W, int G>
+constexpr int walk_unroll() { return walk_batch(std::is_same<T, float>::value, W, G); }
 static_assert(kGeStep % TGT_WIDE_UNROLL == 0, "ge must stay a multiple of the batch size");
 static_assert(kGeStep % TGT_UNROLL == 0, "ge must stay a multiple of the batch size");
 
@@ -105,9 +101,6 @@ struct SegWalk {
   int n_tiles;
   int gap_ctas;    // CTAs that look for rows without edges (fill_gaps)
   float* gcarry;   // [n_tiles][2][gridDim.y * G * NACC] cross-tile partial sums
-  int* tile_done;  // [gridDim.y][n_tiles] arrivals per row that crosses tiles, indexed by the tile it
-                   // starts in; zero when the kernel starts.  Null: a second kernel finishes those rows
-  bool need_perm;  // stage perm[] (bias or dbias in original edge order)
 };
 
 inline int host_ge_max(int g) {
@@ -117,10 +110,10 @@ inline int host_ge_max(int g) {
 }
 
 // Edges per lane group: one balanced wave over the GPU when the graph is small enough, else the
-// largest tile.  `ctas_per_sm` is the occupancy the caller expects.
+// largest tile.  `ctas_per_sm` is the occupancy the caller expects, `step` the walk's batch.
 int forced_ge();  // 0 unless tgt_debug_set_tile_edges() overrides the choice
 
-inline int choose_ge(int64_t n_edges, int g, int ctas_per_sm) {
+inline int choose_ge(int64_t n_edges, int g, int step, int ctas_per_sm) {
   const int ng = kBlockThreads / g;
   const int ge_max = host_ge_max(g);
   if (forced_ge() > 0) {
@@ -133,7 +126,7 @@ inline int choose_ge(int64_t n_edges, int g, int ctas_per_sm) {
   const int64_t capacity = int64_t(sm_count()) * ctas_per_sm;
   int best = ge_max;
   double best_cost = 1e300;
-  for (int ge = (ge_max < 16 ? ge_max : 16); ge <= ge_max; ge += kGeStep) {
+  for (int ge = (ge_max < TGT_LEAST_GE ? ge_max : TGT_LEAST_GE); ge <= ge_max; ge += step) {
     const int64_t tiles = (n_edges + int64_t(ng) * ge - 1) / (int64_t(ng) * ge);
     const int64_t waves = (tiles + capacity - 1) / capacity;
     const double cost = double(waves) * (ge + 8);
@@ -145,12 +138,37 @@ inline int choose_ge(int64_t n_edges, int g, int ctas_per_sm) {
   return best;
 }
 
-template <int VEC>
+// Multiply-adds of a lane.  PAIRS takes two neighbouring values with one instruction (fma.rn.f32x2, sm_100; each value is
+// rounded as by fmaf) where that pays: everywhere in bf16 (16 heads x 8 at 64K nodes, forward 48.0 -> 45.5 us, backward
+// 144 -> 140) and in the fp32 forward (870K nodes 839 -> 781 us).  The fp32 gradient passes keep single ones: operands in
+// even register pairs cost them a resident CTA per SM (64K step with 8 heads x 8, backward 89.7 against 93.3 us).
+template <bool PAIRS, int VEC>
 __device__ __forceinline__ float dot(const float (&a)[VEC], const float (&b)[VEC]) {
+  if constexpr (PAIRS) {
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < VEC; j += 2) s = __ffma2_rn(make_float2(a[j], a[j + 1]), make_float2(b[j], b[j + 1]), s);
+    return s.x + s.y;
+  }
   float s = 0.f;
 #pragma unroll
   for (int j = 0; j < VEC; ++j) s = fmaf(a[j], b[j], s);
   return s;
+}
+
+// acc[AT + j] += w * x[j]
+template <bool PAIRS, int AT, int VEC, int NACC>
+__device__ __forceinline__ void add_scaled(float (&acc)[NACC], float w, const float (&x)[VEC]) {
+#pragma unroll
+  for (int j = 0; j < VEC; j += PAIRS ? 2 : 1) {
+    if constexpr (PAIRS) {
+      const float2 r = __ffma2_rn(make_float2(w, w), make_float2(x[j], x[j + 1]), make_float2(acc[AT + j], acc[AT + j + 1]));
+      acc[AT + j] = r.x;
+      acc[AT + j + 1] = r.y;
+    } else {
+      acc[AT + j] = fmaf(w, x[j], acc[AT + j]);
+    }
+  }
 }
 
 __device__ __forceinline__ float clamp_score(float raw) {
@@ -193,9 +211,6 @@ __device__ __forceinline__ float fast_exp(float x) {
   return e;
 }
 
-template <int G, class Policy>
-__device__ __forceinline__ void finish_row(const SegWalk& w, const Policy& pol, float* s_part, int tile);
-
 constexpr int kGapRows = 8;   // rows of an aligned block that fill_gaps fills when it is empty as a whole
 
 // Zero-fills the rows strictly between `before` and `after`, which have no edges, except the whole aligned blocks.
@@ -231,6 +246,7 @@ __device__ __forceinline__ void fill_gaps(const SegWalk& w, const Policy& pol) {
 
 // The walk.  Policy supplies:
 //   static constexpr int NACC;                     accumulators per lane
+//   static constexpr bool kPerm;                   whether it reads perm[] (bias in original edge order)
 //   static constexpr int kUnroll;                  edges per batch (walk_unroll<T, G>())
 //   struct Operands;                               what one edge loads
 //   void load(Operands&, int row, int other, int perm_e) const;      issue the gathers of one edge
@@ -242,7 +258,7 @@ __device__ __forceinline__ void fill_gaps(const SegWalk& w, const Policy& pol) {
 template <int G, class Policy>
 __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, int32_t* s_other,
                                           int32_t* s_seg, int32_t* s_perm, float* s_carry,
-                                          int32_t* s_carry_row, float* s_part, int32_t* s_finish) {
+                                          int32_t* s_carry_row) {
   constexpr int NG = TileGeom<G>::NG;
   constexpr int NACC = Policy::NACC;
   constexpr int kUnroll = Policy::kUnroll;   // edges per batch (shadows the default)
@@ -252,7 +268,6 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
   const int te = NG * w.ge;
   const int64_t t0 = int64_t(blockIdx.x) * te;
   const int n = int(min(int64_t(te), int64_t(w.n_edges) - t0));  // edges in this tile (>= 1)
-  release_dependents();   // the next kernel of the call may take this SM's slots as they free up
 
   // ---- stage the tile's indices.  Tile edge i lives at position i + i / ge: one pad word per
   // lane-group range, so the groups of a warp (which read ranges ge apart) hit different banks.
@@ -264,7 +279,7 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
     const int p = pos(i);
     s_seg[p] = __ldg(w.seg + t0 + i);
     s_other[p] = __ldg(w.other + t0 + i);
-    if (w.need_perm) s_perm[p] = __ldg(w.perm + t0 + i);
+    if (Policy::kPerm) s_perm[p] = __ldg(w.perm + t0 + i);
   }
   if (tid == 0) {
     s_halo[0] = t0 == 0 ? -1 : __ldg(w.seg + t0 - 1);
@@ -304,7 +319,7 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
       valid[u] = FULL || i < gend;
       const int ii = valid[u] ? gb_pos + (i - gb) : 0;
       row[u] = s_seg[ii];
-      pe[u] = w.need_perm ? s_perm[ii] : 0;
+      pe[u] = Policy::kPerm ? s_perm[ii] : 0;
       if (valid[u]) pol.load(ops[u], row[u], s_other[ii], pe[u]);
       else pol.clear(ops[u]);
     }
@@ -360,6 +375,7 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
     if (t0 + gend == w.n_edges) zero_gap(pol, cur, w.n_rows);  // this group owns the last edge
   }
   if (blockIdx.x < w.gap_ctas) fill_gaps<G, Policy>(w, pol);
+  release_dependents();   // the next kernel of the call may take this SM's slots as they free up
   __syncthreads();
 
   // ---- stitch rows that cross group boundaries, in group order
@@ -400,101 +416,93 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
       pol.finalize(r, acc);
     }
   }
-
-  // ---- rows that cross tile boundaries: every tile such a row touches has written one partial
-  // (the tile it starts in a tail carry, the others a head carry) and now counts itself in; the
-  // tile that arrives last finishes the row.  A tile touches at most two such rows.
-  if (w.n_tiles == 1 || w.tile_done == nullptr) return;
-  __threadfence();   // this thread's carries are visible device-wide before the arrival is counted
-  __syncthreads();
-  if (tid == 0) {
-    const int first_row = row_of(0);
-    auto arrive = [&](int row) {
-      const int start_tile = __ldg(w.ptr + row) / te;
-      const int end_tile = (__ldg(w.ptr + row + 1) - 1) / te;
-      const int before = atomicAdd(w.tile_done + int64_t(blockIdx.y) * w.n_tiles + start_tile, 1);
-      return before == end_tile - start_tile ? start_tile : -1;
-    };
-    __threadfence();
-    s_finish[0] = s_halo[0] == first_row ? arrive(first_row) : -1;              // a head carry was written
-    s_finish[1] = (tile_cont_out && s_halo[0] != last_row) ? arrive(last_row) : -1;  // a tail carry
-    __threadfence();   // the other tiles' carries are read after their arrivals were seen
-  }
-  __syncthreads();     // from here on the index arrays are dead: s_part may overlay them
-#pragma unroll 1
-  for (int f = 0; f < 2; ++f) {
-    const int start_tile = s_finish[f];
-    if (start_tile >= 0) {
-      finish_row<G, Policy>(w, pol, s_part, start_tile);
-      __syncthreads();
-    }
-  }
 }
 
-// Finishes the row that starts in `tile` and runs past its end, from the partials all its tiles have
-// delivered: that tile's tail carry and the head carries of the following tiles.  The partials are
-// dealt round-robin to 128 / G slots, each slot adds its share in tile order, then the slots are
-// combined in a fixed tree: the order depends neither on timing nor on which CTA runs this.
+// ---- rows that cross tiles ---------------------------------------------------------------------------------------
+// A second kernel, one lane group per tile: that of the tile in which a row that runs past the tile's end STARTS adds
+// up what the row's tiles have left (the tail carry of that tile, the head carries of the following ones) and finishes
+// it; rows of more than kGroupTiles further tiles are taken by the whole CTA.  Every sum has a fixed order.  Launched as
+// the dependent of the walk, and what does not depend on the walk is read before it has ended.
+constexpr int kGroupTiles = 8;
+constexpr int kCrossingThreads = 512;   // a row of every eighth edge has over a hundred carries at 64,000 nodes
 template <int G, class Policy>
-__device__ __forceinline__ void finish_row(const SegWalk& w, const Policy& pol, float* s_part, int tile) {
-  constexpr int NG = TileGeom<G>::NG;
-  constexpr int NACC = Policy::NACC;
-  const int te = NG * w.ge;
+__device__ __forceinline__ void finish_crossing_rows(const SegWalk& w, const Policy& pol) {
+  constexpr int NG = kCrossingThreads / G, NACC = Policy::NACC;
+  __shared__ float s_part[kCrossingThreads * NACC];
+  __shared__ int s_many[NG][3], s_n;   // rows of many tiles: first tile, further tiles, row
+  const int g = threadIdx.x / G, c = threadIdx.x % G;
+  const int te = TileGeom<G>::NG * w.ge;
+  const int tile = blockIdx.x * NG + g;
   const int64_t t1 = int64_t(tile + 1) * te;
-  const int r = __ldg(w.seg + t1 - 1);
-  const int last_tile = (__ldg(w.ptr + r + 1) - 1) / te;
-  const int slot = threadIdx.x / G, c = threadIdx.x % G;
-  const int lanes_all = gridDim.y * G;
-  const int64_t stride = int64_t(lanes_all) * NACC;
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  int row = -1, further = 0;
+  if (t1 < w.n_edges) {
+    const int r = __ldg(w.seg + t1 - 1), behind = __ldg(w.seg + t1);
+    const int begin = __ldg(w.ptr + r), end = __ldg(w.ptr + r + 1);
+    if (r == behind && begin >= t1 - te) {
+      row = r;
+      further = (end - 1) / te - tile;
+    }
+  }
+  if (row >= 0 && further > kGroupTiles && c == 0) {
+    const int at = atomicAdd(&s_n, 1);
+    s_many[at][0] = tile;
+    s_many[at][1] = further;
+    s_many[at][2] = row;
+  }
+  release_dependents();
+  dependent_wait();   // the walk's carries; every CTA waits, also those that have nothing to finish
+  const int64_t stride = int64_t(gridDim.y) * G * NACC;
   const float* base = w.gcarry + int64_t(blockIdx.y * G + c) * NACC;
   float acc[NACC];
+  auto carry = [&](int t, int which) { return base + (int64_t(t) * 2 + which) * stride; };   // 0 = head, 1 = tail
+  if (row >= 0 && further <= kGroupTiles) {
+    const float *tail = carry(tile, 1), *head = carry(tile + 1, 0);
 #pragma unroll
-  for (int a = 0; a < NACC; ++a) acc[a] = 0.f;
-  // partial 0 = tail carry of `tile`, partial i > 0 = head carry of tile + i
-  const int n_part = last_tile - tile + 1;
-#pragma unroll 4
-  for (int i = slot; i < n_part; i += NG) {
-    const float* p = base + (int64_t(tile + i) * 2 + (i == 0 ? 1 : 0)) * stride;
+    for (int a = 0; a < NACC; ++a) acc[a] = __ldcg(tail + a) + __ldcg(head + a);
+    for (int i = 2; i <= further; ++i) {
+      const float* p = carry(tile + i, 0);
 #pragma unroll
-    for (int a = 0; a < NACC; ++a) acc[a] += __ldcg(p + a);   // written by other CTAs of this launch: read at L2
+      for (int a = 0; a < NACC; ++a) acc[a] += __ldcg(p + a);
+    }
+    pol.finalize(row, acc);
   }
-  // combine the NG slots: halving tree through shared memory
-  float* mine = s_part + (slot * G + c) * NACC;
-#pragma unroll
-  for (int a = 0; a < NACC; ++a) mine[a] = acc[a];
   __syncthreads();
-  for (int half = NG / 2; half >= 1; half >>= 1) {
-    if (slot < half) {
-      const float* o = s_part + ((slot + half) * G + c) * NACC;
+  for (int j = 0; j < s_n; ++j) {
+    const int start = s_many[j][0], n = s_many[j][1];
 #pragma unroll
-      for (int a = 0; a < NACC; ++a) mine[a] += o[a];
+    for (int a = 0; a < NACC; ++a) acc[a] = 0.f;
+#pragma unroll 4
+    for (int i = g; i <= n; i += NG) {
+      const float* p = carry(start + i, i == 0 ? 1 : 0);
+#pragma unroll
+      for (int a = 0; a < NACC; ++a) acc[a] += __ldcg(p + a);
+    }
+#pragma unroll
+    for (int a = 0; a < NACC; ++a) s_part[a * kCrossingThreads + threadIdx.x] = acc[a];
+    __syncthreads();
+    for (int half = NG / 2; half >= 1; half >>= 1) {   // halving tree
+      if (g < half) {
+#pragma unroll
+        for (int a = 0; a < NACC; ++a)
+          s_part[a * kCrossingThreads + threadIdx.x] += s_part[a * kCrossingThreads + threadIdx.x + half * G];
+      }
+      __syncthreads();
+    }
+    if (g == 0) {
+#pragma unroll
+      for (int a = 0; a < NACC; ++a) acc[a] = s_part[a * kCrossingThreads + c];
+      pol.finalize(s_many[j][2], acc);
     }
     __syncthreads();
   }
-  if (slot == 0) {
-#pragma unroll
-    for (int a = 0; a < NACC; ++a) acc[a] = mine[a];
-    pol.finalize(r, acc);
-  }
 }
-
-// Second kernel for narrow lane groups: one CTA per tile; the CTA of the tile in which a row that runs
-// past the tile's end STARTS finishes that row.
-template <int G, class Policy>
-__device__ __forceinline__ void stitch_tiles(const SegWalk& w, const Policy& pol, float* s_part) {
-  const int tile = blockIdx.x;
-  const int te = TileGeom<G>::NG * w.ge;
-  const int64_t t1 = int64_t(tile + 1) * te;
-  release_dependents();
-  dependent_wait();                                  // the walk kernel's carries; every CTA waits, also those that return
-  if (t1 >= w.n_edges) return;                       // last tile: nothing runs past it
-  const int r = __ldg(w.seg + t1 - 1);
-  if (__ldg(w.seg + t1) != r) return;                // the tile ends on a row boundary
-  if (__ldg(w.ptr + r) < t1 - te) return;            // the row started in an earlier tile
-  finish_row<G, Policy>(w, pol, s_part, tile);
+// CTAs of that kernel in x for lane groups of g lanes.
+inline unsigned crossing_ctas(const SegWalk& w, int g) {
+  const int ng = kCrossingThreads / g;
+  return unsigned((w.n_tiles + ng - 1) / ng);
 }
-
-inline bool stitch_in_second_kernel(int g) { return g <= TGT_STITCH_KERNEL_MAX_G; }
 
 struct HeadSplit {
   int w;       // bytes one lane moves: 16 or 32
@@ -505,6 +513,8 @@ struct HeadSplit {
 };
 
 enum { kPassFwd = 0, kPassDq = 1, kPassDkv = 2 };
+// What a walk does with the edge bias; a kernel of its own for each, since the registers of the code that is not run count.
+enum BiasUse { kNoBias = 0, kReadBias = 1, kBiasGrad = 2 };
 
 // Lane width of the walk kernels: 0 = chosen by the library, 1 = 16-byte lanes, 2 = 32-byte lanes
 // wherever the head size allows.  Set by tgt_debug_set_lane_mode().
@@ -582,6 +592,16 @@ inline bool dispatch_shape(int dtype, int w, int lph, int g, F&& f) {
   return w == 16 ? dispatch_head<__nv_bfloat16, 16>(lph, g, f) : false;
 }
 
+// Calls f with the bias use as a compile-time constant; a walk whose MOST is kReadBias only reads.
+template <int MOST, class F>
+inline void dispatch_bias(int use, F&& f) {
+  if constexpr (MOST >= kBiasGrad) {
+    if (use == kBiasGrad) return f(std::integral_constant<int, kBiasGrad>{});
+  }
+  if (use != kNoBias) return f(std::integral_constant<int, kReadBias>{});
+  f(std::integral_constant<int, kNoBias>{});
+}
+
 int check_layout(const tgt_layout* L, const char* name);
 
 // Resident CTAs per SM of a walk kernel on the current device (asked from the runtime once per
@@ -599,16 +619,13 @@ inline int resident_ctas(Kernel kernel, int* cache) {
   return *cache;
 }
 
-// Tiling of one pass: edges per lane group, number of tiles, bytes of cross-tile carry followed by
-// the arrival counters (scratch_bytes = both).
+// Tiling of one pass: edges per lane group, number of tiles, bytes of cross-tile carry.
 struct TilePlan {
   int ge;
   int n_tiles;
   size_t carry_bytes;
-  size_t counter_bytes;
-  size_t scratch_bytes;
 };
-TilePlan plan_tiles(int64_t n_edges, const HeadSplit& hs, int nacc, int ctas_per_sm);
+TilePlan plan_tiles(int64_t n_edges, const HeadSplit& hs, int step, int nacc, int ctas_per_sm);
 
 // CTAs of a walk kernel in x: one per tile, and more where there are over kGapShare rows per tile.
 inline int gap_ctas(int64_t n_rows) { return int((n_rows + kGapShare - 1) / kGapShare); }
@@ -618,34 +635,30 @@ inline unsigned walk_ctas(const TilePlan& tp, int64_t n_rows) {
 }
 
 // Shared-memory bytes walk_tile needs (indices + carries), as the kernels declare them.
-template <int G, int NACC>
+template <int G, int NACC, bool PERM>
 struct TileSmem {
   static constexpr int TE = TileGeom<G>::TE_MAX;
   static constexpr int NG = TileGeom<G>::NG;
   struct Indices {
     int32_t other[TE + NG];
     int32_t seg[TE + NG + 2];   // padded rows + the two halo words
-    int32_t perm[TE + NG];
+    int32_t perm[PERM ? TE + NG : 1];
   };
-  union {
-    Indices idx;                          // while the tile is walked
-    float part[kBlockThreads * NACC];     // afterwards: slots of finish_row
-  };
+  Indices idx;
   float carry[NG * 2 * G * NACC];
   int32_t carry_row[NG * 2];
-  int32_t finish[2];
 };
 
 // The call every walk kernel makes.
 template <int G, class Policy>
-__device__ __forceinline__ void walk_tile_in(TileSmem<G, Policy::NACC>& sm, const SegWalk& w, const Policy& pol) {
+__device__ __forceinline__ void walk_tile_in(TileSmem<G, Policy::NACC, Policy::kPerm>& sm, const SegWalk& w, const Policy& pol) {
   if (blockIdx.x >= w.n_tiles) {     // launched for its share of the empty rows only
     release_dependents();
     dependent_wait();                // the rows may be what the previous kernel of the call works on
     fill_gaps<G, Policy>(w, pol);
     return;
   }
-  walk_tile<G, Policy>(w, pol, sm.idx.other, sm.idx.seg, sm.idx.perm, sm.carry, sm.carry_row, sm.part, sm.finish);
+  walk_tile<G, Policy>(w, pol, sm.idx.other, sm.idx.seg, sm.idx.perm, sm.carry, sm.carry_row);
 }
 
 }  // namespace tgt

@@ -15,7 +15,7 @@ std::atomic<int> g_forced_ge{0};
 std::atomic<int> g_lane_mode{0};
 // measured on B200: chaining the walk kernels gains 2-5 us per backward call; chaining the kernel that finishes
 // cross-tile rows to its walk kernel loses up to 10 us with lane groups of 4, so that link stays ordinary
-std::atomic<int> g_dependent_launch{kLinkWalk | kLinkAfterStitch};
+std::atomic<int> g_dependent_launch{kLinkWalk | kLinkStitch | kLinkAfterStitch};
 }  // namespace
 
 int lane_mode() { return g_lane_mode.load(std::memory_order_relaxed); }

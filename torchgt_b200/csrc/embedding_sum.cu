@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(kEmbThreads) embedding_pairs_kernel(const int6
 template <int G>
 struct SumPolicy {
   static constexpr int VEC = 4, NACC = 4;
+  static constexpr bool kPerm = true;
   static constexpr int kUnroll = 4;
   const float* __restrict__ grad;
   float* __restrict__ out;
@@ -91,9 +92,25 @@ struct SumParams {
 
 template <int G>
 __global__ void TGT_WALK_BOUNDS embedding_grad_kernel(const SumParams p) {
-  __shared__ TileSmem<G, SumPolicy<G>::NACC> sm;
+  __shared__ TileSmem<G, SumPolicy<G>::NACC, true> sm;
   const SumPolicy<G> pol{p.grad, p.out, p.skip, p.features, p.share, threadIdx.x % G};
   walk_tile_in<G, SumPolicy<G>>(sm, p.walk, pol);
+}
+
+template <int G>
+__global__ void __launch_bounds__(kCrossingThreads) embedding_grad_crossing_kernel(const SumParams p) {
+  const SumPolicy<G> pol{p.grad, p.out, p.skip, p.features, p.share, threadIdx.x % G};
+  finish_crossing_rows<G, SumPolicy<G>>(p.walk, pol);
+}
+
+template <int G>
+int launch_grad(const SumParams& p, unsigned ctas, cudaStream_t stream) {
+  embedding_grad_kernel<G><<<ctas, kBlockThreads, 0, stream>>>(p);
+  if (p.walk.n_tiles > 1)
+    TGT_CHECK_CUDA(launch_chained(embedding_grad_crossing_kernel<G>, dim3(crossing_ctas(p.walk, G)), kCrossingThreads, stream,
+                                  kLinkStitch, p));
+  TGT_CHECK_CUDA(cudaGetLastError());
+  return TGT_OK;
 }
 
 bool table_supported(int hidden) { return hidden == 32 || hidden == 64 || hidden == 128; }
@@ -114,7 +131,7 @@ int grad_ctas() {
 int plan_grad(int64_t pairs, int64_t n_table, int hidden, GradPlan* g) {
   if (!split_heads(1, hidden, TGT_F32, 16, &g->hs)) return set_error(TGT_ERR_UNSUPPORTED, "hidden=%d", hidden);
   const int ctas = hidden == 32 ? grad_ctas<8>() : hidden == 64 ? grad_ctas<16>() : grad_ctas<32>();
-  g->tiles = plan_tiles(pairs, g->hs, 4, ctas);
+  g->tiles = plan_tiles(pairs, g->hs, SumPolicy<16>::kUnroll, 4, ctas);
   const int rc = tgt_edge_layout_sizes_i32(n_table, pairs, &g->layout_bytes);
   if (rc != TGT_OK) return rc;
   size_t off = 0;
@@ -130,7 +147,7 @@ int plan_grad(int64_t pairs, int64_t n_table, int hidden, GradPlan* g) {
   g->seg = take(size_t(pairs) * 4);
   g->status = take(4);
   g->layout = take(g->layout_bytes);
-  g->walk = take(g->tiles.scratch_bytes);
+  g->walk = take(g->tiles.carry_bytes);
   g->total = off;
   return TGT_OK;
 }
@@ -212,13 +229,6 @@ extern "C" int tgt_embedding_sum_grad(const float* dout, const int64_t* ids, int
   p.walk.n_rows = int(n_table); p.walk.n_edges = int(pairs);
   p.walk.ge = g.tiles.ge; p.walk.n_tiles = g.tiles.n_tiles; p.walk.gap_ctas = gap_ctas(n_table);
   p.walk.gcarry = reinterpret_cast<float*>(base + g.walk);
-  p.walk.tile_done = reinterpret_cast<int*>(base + g.walk + g.tiles.carry_bytes);
-  p.walk.need_perm = true;
-  if (g.tiles.n_tiles > 1) TGT_CHECK_CUDA(cudaMemsetAsync(p.walk.tile_done, 0, g.tiles.counter_bytes, stream));
   const unsigned ctas = walk_ctas(g.tiles, n_table);
-  if (hidden == 32) embedding_grad_kernel<8><<<ctas, kBlockThreads, 0, stream>>>(p);
-  else if (hidden == 64) embedding_grad_kernel<16><<<ctas, kBlockThreads, 0, stream>>>(p);
-  else embedding_grad_kernel<32><<<ctas, kBlockThreads, 0, stream>>>(p);
-  TGT_CHECK_CUDA(cudaGetLastError());
-  return TGT_OK;
+  return hidden == 32 ? launch_grad<8>(p, ctas, stream) : hidden == 64 ? launch_grad<16>(p, ctas, stream) : launch_grad<32>(p, ctas, stream);
 }

@@ -17,10 +17,6 @@ __global__ void __launch_bounds__(256) bwd_stats_kernel(const BwdParams p) {
   const int64_t total = p.n_rows * chunks;
   const bool live = idx < total;
   release_dependents();   // pass A stages its edge indices while this kernel drains
-  // the arrival counters of both walks, which start only after this kernel has completed: saves the memset
-  // node in front of the call
-  if (blockIdx.x == 0 && p.clear_words != nullptr)
-    for (int i = threadIdx.x; i < p.n_clear_words; i += blockDim.x) p.clear_words[i] = 0;
   float g[VEC], o[VEC];
 #pragma unroll
   for (int j = 0; j < VEC; ++j) g[j] = o[j] = 0.f;
@@ -29,7 +25,7 @@ __global__ void __launch_bounds__(256) bwd_stats_kernel(const BwdParams p) {
     Vec16<T>::load(reinterpret_cast<const T*>(static_cast<const char*>(p.dout) + row * p.g_row_bytes) + col * VEC, g);
     Vec16<T>::load(static_cast<const T*>(p.out) + idx * VEC, o);
   }
-  const float delta = group_sum<LPH>(dot<VEC>(g, o));
+  const float delta = group_sum<LPH>(dot<false>(g, o));
   if (live && (idx % LPH) == 0) {
     const int64_t row = idx / chunks;
     const int head = int(idx % chunks) / LPH;
@@ -40,53 +36,44 @@ __global__ void __launch_bounds__(256) bwd_stats_kernel(const BwdParams p) {
 
 enum { kWalkDq = 0, kWalkDkv = 1, kWalkDqFused = 2 };
 
-int bwd_resident_ctas(int dtype, const HeadSplit& hs, int which) {
-  static int cache[kMaxDevices][2][3][2][6][6] = {};   // occupancy is a property of the device
+int bwd_resident_ctas(int dtype, const HeadSplit& hs, int which, int use) {
+  static int cache[kMaxDevices][2][3][3][2][6][6] = {};   // occupancy is a property of the device
   auto log2i = [](int x) { int l = 0; while ((1 << l) < x) ++l; return l; };
   const int dev = current_device();
-  int* slot = &cache[dev < 0 ? 0 : dev][hs.w == 32 ? 1 : 0][which][dtype == TGT_F32 ? 0 : 1][log2i(hs.lph)][log2i(hs.g)];
-  if (which == kWalkDkv) return bwd::occupancy_dkv(dtype, hs, slot);
-  if (which == kWalkDqFused) return bwd::occupancy_dq_fused(dtype, hs, slot);
+  int* slot = &cache[dev < 0 ? 0 : dev][hs.w == 32 ? 1 : 0][which][use][dtype == TGT_F32 ? 0 : 1][log2i(hs.lph)][log2i(hs.g)];
+  if (which == kWalkDkv) return bwd::occupancy_dkv(dtype, hs, use, slot);
+  if (which == kWalkDqFused) return bwd::occupancy_dq_fused(dtype, hs, use, slot);
   return bwd::occupancy_dq(dtype, hs, slot);
 }
 
 struct BwdScratch {
-  size_t stats, carry_a, carry_b, counters, counter_bytes, total;
+  size_t stats, carry_a, carry_b, total;
   TilePlan plan_a, plan_a_fused, plan_b;
 };
 
 // hs: lane layout of pass A (by destination), hsb: of pass B (by source); they may use different lane widths
 BwdScratch plan_bwd_scratch(const tgt_layout* by_dst, const HeadSplit& hs, const HeadSplit& hsb, int heads,
-                            int dtype) {
+                            int dtype, int use) {
   BwdScratch s;
   const int vec = hs.w / (dtype == TGT_F32 ? 4 : 2);
   const int vecb = hsb.w / (dtype == TGT_F32 ? 4 : 2);
-  s.plan_a = plan_tiles(by_dst->n_edges, hs, vec, bwd_resident_ctas(dtype, hs, kWalkDq));
-  s.plan_a_fused = plan_tiles(by_dst->n_edges, hs, 2 * vec + 1, bwd_resident_ctas(dtype, hs, kWalkDqFused));
-  s.plan_b = plan_tiles(by_dst->n_edges, hsb, 2 * vecb, bwd_resident_ctas(dtype, hsb, kWalkDkv));
+  s.plan_a = plan_tiles(by_dst->n_edges, hs, walk_batch(dtype == TGT_F32, hs.w, hs.g), vec, bwd_resident_ctas(dtype, hs, kWalkDq, use));
+  s.plan_a_fused = plan_tiles(by_dst->n_edges, hs, walk_batch(dtype == TGT_F32, hs.w, hs.g), 2 * vec + 1, bwd_resident_ctas(dtype, hs, kWalkDqFused, use < kReadBias ? use : kReadBias));
+  s.plan_b = plan_tiles(by_dst->n_edges, hsb, walk_batch(dtype == TGT_F32, hsb.w, hsb.g), 2 * vecb, bwd_resident_ctas(dtype, hsb, kWalkDkv, use));
   size_t off = 0;
   s.stats = off; off += round_up(size_t(by_dst->n_rows) * heads * 8, 256);
   s.carry_a = off;
   off += s.plan_a.carry_bytes > s.plan_a_fused.carry_bytes ? s.plan_a.carry_bytes : s.plan_a_fused.carry_bytes;
   s.carry_b = off; off += s.plan_b.carry_bytes;
-  // arrival counters of both passes side by side (one memset clears them): pass A first
-  s.counters = off;
-  const size_t ca = s.plan_a.counter_bytes > s.plan_a_fused.counter_bytes ? s.plan_a.counter_bytes
-                                                                           : s.plan_a_fused.counter_bytes;
-  s.counter_bytes = ca + s.plan_b.counter_bytes;
-  off += s.counter_bytes;
   s.total = off;
   return s;
 }
 
-void fill_walk(SegWalk* w, const tgt_layout& L, const TilePlan& tp, float* carry, int* counters,
-               bool need_perm) {
+void fill_walk(SegWalk* w, const tgt_layout& L, const TilePlan& tp, float* carry) {
   w->ptr = L.ptr; w->other = L.other; w->perm = L.perm; w->seg = L.seg;
   w->n_rows = int(L.n_rows); w->n_edges = int(L.n_edges);
   w->ge = tp.ge; w->n_tiles = tp.n_tiles; w->gap_ctas = gap_ctas(L.n_rows);
   w->gcarry = carry;
-  w->tile_done = counters;
-  w->need_perm = need_perm;
 }
 
 }  // namespace
@@ -123,8 +110,10 @@ extern "C" int tgt_sparse_attn_scratch_bytes(const tgt_layout* by_dst, const tgt
           (wb == 32 && lane_bytes(heads, head_dim, dtype, true, kPassDkv) != 32))
         continue;
       if (!split_heads(heads, head_dim, dtype, wa, &a) || !split_heads(heads, head_dim, dtype, wb, &b)) continue;
-      const size_t t = plan_bwd_scratch(by_dst, a, b, heads, dtype).total;
-      if (t > need) need = t;
+      for (const int use : {kNoBias, kReadBias, kBiasGrad}) {
+        const size_t t = plan_bwd_scratch(by_dst, a, b, heads, dtype, use).total;
+        if (t > need) need = t;
+      }
     }
   *bytes = need;
   return TGT_OK;
@@ -221,7 +210,12 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
     }
     return TGT_OK;
   }
-  const BwdScratch sc = plan_bwd_scratch(by_dst, hs, hsb, heads, dtype);
+  // With both passes in one call pass A derives the statistics itself, and pass B, which has the gradient of every
+  // edge's score at hand, writes dbias.
+  const bool dbias_in_dkv = dbias != nullptr && (passes & 6) == 6;
+  if (dbias_in_dkv) passes &= ~1;
+  const BwdScratch sc = plan_bwd_scratch(by_dst, hs, hsb, heads, dtype,
+                                         bias == nullptr ? kNoBias : dbias_in_dkv ? kBiasGrad : kReadBias);
   if (scratch == nullptr || scratch_bytes < sc.total)
     return set_error(TGT_ERR_WORKSPACE, "scratch holds %zu bytes, %zu needed", scratch_bytes,
                      sc.total);
@@ -231,6 +225,7 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
   p.dout = dout; p.q = q; p.k = k; p.v = v; p.out = out; p.z = z;
   p.bias = bias; p.bias_heads = bias_heads;
   p.dq = dq; p.dk = dk; p.dv = dv; p.dbias = dbias;
+  p.dbias_in_dkv = dbias_in_dkv;
   p.stats = reinterpret_cast<float2*>(base + sc.stats);
   p.heads = heads;
   p.row_elems = heads * head_dim;
@@ -240,22 +235,6 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
   p.n_rows = n_rows;
   p.inv_scale = 1.0f / sqrtf(float(head_dim));
 
-  const bool second_kernel = stitch_in_second_kernel(hs.g);      // pass A
-  const bool second_kernel_b = stitch_in_second_kernel(hsb.g);   // pass B
-  int* counters_a = second_kernel ? nullptr : reinterpret_cast<int*>(base + sc.counters);
-  int* counters_b = second_kernel_b ? nullptr
-                                    : reinterpret_cast<int*>(base + sc.counters + sc.counter_bytes -
-                                                             sc.plan_b.counter_bytes);
-  p.clear_words = nullptr;
-  p.n_clear_words = 0;
-  if ((passes & 6) && !(second_kernel && second_kernel_b)) {
-    if (passes & 1) {   // the statistics kernel clears them on its way
-      p.clear_words = reinterpret_cast<int*>(base + sc.counters);
-      p.n_clear_words = int(sc.counter_bytes / sizeof(int));
-    } else {
-      TGT_CHECK_CUDA(cudaMemsetAsync(base + sc.counters, 0, sc.counter_bytes, stream));
-    }
-  }
   // from here on the kernels of this call follow one another on the stream without anything in between, and
   // each is launched as the dependent of the one before
   int link = 0;
@@ -270,27 +249,25 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
     });
     link = kLinkWalk;
   }
-  // one walk kernel per pass, plus the kernel that finishes cross-tile rows when the lane group is narrow
+  // one walk kernel per pass, and the kernel that finishes the rows that cross tiles
   bool built = true;
-  if ((passes & 2) && dbias == nullptr) {
+  if ((passes & 2) && (dbias == nullptr || p.dbias_in_dkv)) {
     // pass A that derives the row statistics itself (and leaves them in scratch for pass B)
-    fill_walk(&p.walk, *by_dst, sc.plan_a_fused, reinterpret_cast<float*>(base + sc.carry_a), counters_a,
-              bias != nullptr);
+    fill_walk(&p.walk, *by_dst, sc.plan_a_fused, reinterpret_cast<float*>(base + sc.carry_a));
     const dim3 grid(walk_ctas(sc.plan_a_fused, n_rows), hs.groups);
-    built = bwd::launch_dq_fused(p, dtype, hs, grid, second_kernel, link, stream);
-    link = second_kernel && p.walk.n_tiles > 1 ? kLinkAfterStitch : kLinkWalk;
+    built = bwd::launch_dq_fused(p, dtype, hs, grid, link, stream);
+    link = p.walk.n_tiles > 1 ? kLinkAfterStitch : kLinkWalk;
   } else if (passes & 2) {
     // pass A with per-edge dbias: uses the statistics of the pre-pass (stage 1)
-    fill_walk(&p.walk, *by_dst, sc.plan_a, reinterpret_cast<float*>(base + sc.carry_a), counters_a, true);
+    fill_walk(&p.walk, *by_dst, sc.plan_a, reinterpret_cast<float*>(base + sc.carry_a));
     const dim3 grid(walk_ctas(sc.plan_a, n_rows), hs.groups);
-    built = bwd::launch_dq(p, dtype, hs, grid, second_kernel, link, stream);
-    link = second_kernel && p.walk.n_tiles > 1 ? kLinkAfterStitch : kLinkWalk;
+    built = bwd::launch_dq(p, dtype, hs, grid, link, stream);
+    link = p.walk.n_tiles > 1 ? kLinkAfterStitch : kLinkWalk;
   }
   if (built && (passes & 4)) {
-    fill_walk(&p.walk, *by_src, sc.plan_b, reinterpret_cast<float*>(base + sc.carry_b), counters_b,
-              bias != nullptr);
+    fill_walk(&p.walk, *by_src, sc.plan_b, reinterpret_cast<float*>(base + sc.carry_b));
     const dim3 grid(walk_ctas(sc.plan_b, n_rows), hsb.groups);
-    built = bwd::launch_dkv(p, dtype, hsb, grid, second_kernel_b, link, stream);
+    built = bwd::launch_dkv(p, dtype, hsb, grid, link, stream);
   }
   if (!built) return set_error(TGT_ERR_UNSUPPORTED, "no kernel is built for this head layout");
   TGT_CHECK_CUDA(cudaGetLastError());

@@ -35,29 +35,32 @@ struct BwdParams {
   void* dk;
   void* dv;
   float* dbias;
+  bool dbias_in_dkv;  // pass B writes dbias, not pass A
   float2* stats;  // [n_rows, heads]
   int heads, row_elems;
   int64_t q_row_bytes, kv_row_bytes, g_row_bytes;   // distance between rows of q, of k / v and of dout
   int64_t n_rows;
   float inv_scale;
-  int* clear_words;      // arrival counters the statistics pre-pass zeroes for the two walks (or null)
-  int n_clear_words;
   SegWalk walk;
 };
 
-// What sparse_attn_bwd.cu asks of each pass: launch it (plus the kernel that finishes cross-tile rows when
-// `second_kernel`; `link` != 0 = the kernel enqueued just before on the stream belongs to the same call, so
+// Bias use of a walk that writes dbias if it is pass B's.
+inline int bias_use(const BwdParams& p) {
+  return p.bias == nullptr ? kNoBias : (p.dbias_in_dkv ? kBiasGrad : kReadBias);
+}
+
+// What sparse_attn_bwd.cu asks of each pass: launch it and the kernel that finishes the rows that cross tiles (`link` != 0 = the kernel enqueued just before on the stream belongs to the same call, so
 // the walk kernel is launched as its dependent, see launch_chained), and the resident CTAs per SM of its walk kernel.  Both return false / 0 when no kernel
 // is built for the lane layout.
-bool launch_dq(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, bool second_kernel, int link,
+bool launch_dq(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, int link,
                cudaStream_t stream);
-bool launch_dq_fused(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, bool second_kernel, int link,
+bool launch_dq_fused(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, int link,
                      cudaStream_t stream);
-bool launch_dkv(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, bool second_kernel, int link,
+bool launch_dkv(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, int link,
                 cudaStream_t stream);
 int occupancy_dq(int dtype, const HeadSplit& hs, int* cache_slot);
-int occupancy_dq_fused(int dtype, const HeadSplit& hs, int* cache_slot);
-int occupancy_dkv(int dtype, const HeadSplit& hs, int* cache_slot);
+int occupancy_dq_fused(int dtype, const HeadSplit& hs, int use, int* cache_slot);
+int occupancy_dkv(int dtype, const HeadSplit& hs, int use, int* cache_slot);
 
 }  // namespace bwd
 }  // namespace tgt

@@ -10,6 +10,8 @@ template <typename T, int W, int LPH, int G>
 struct DqPolicy {
   static constexpr int VEC = Lane<T, W>::kElems;
   static constexpr int NACC = VEC;
+  static constexpr bool kPairs = sizeof(T) == 2;
+  static constexpr bool kPerm = true;
   static constexpr int kUnroll = walk_unroll<T, W, G>();
 
   const T* __restrict__ q;
@@ -54,10 +56,10 @@ struct DqPolicy {
     float a[VEC], b[VEC];
     Lane<T, W>::unpack(o.q, a);
     Lane<T, W>::unpack(o.k, b);
-    const float raw = group_sum<LPH>(dot<VEC>(a, b)) * inv_scale;
+    const float raw = group_sum<LPH>(dot<kPairs>(a, b)) * inv_scale;
     Lane<T, W>::unpack(o.g, a);
     Lane<T, W>::unpack(o.v, b);
-    const float gv = group_sum<LPH>(dot<VEC>(a, b));
+    const float gv = group_sum<LPH>(dot<kPairs>(a, b));
     const float wgt = fast_exp(clamp_score(raw) + o.b);
     const float dt = valid ? (gv - o.st.y) * o.st.x * wgt : 0.f;
     if (dbias != nullptr) {
@@ -76,8 +78,7 @@ struct DqPolicy {
                                              const Scalars& s) const {
     float kf[VEC];
     Lane<T, W>::unpack(o.k, kf);
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) acc[j] = fmaf(s.da, kf[j], acc[j]);
+    add_scaled<kPairs, 0>(acc, s.da, kf);
   }
   __device__ __forceinline__ void finalize(int row, const float (&acc)[NACC]) const {
     float o[VEC];
@@ -124,29 +125,28 @@ __device__ __forceinline__ DqPolicy<T, W, LPH, G> make_dq_policy(const BwdParams
 template <typename T, int W, int LPH, int G>
 __global__ void TGT_WALK_BOUNDS bwd_dq_kernel(const BwdParams p) {
   using Policy = DqPolicy<T, W, LPH, G>;
-  __shared__ TileSmem<G, Policy::NACC> sm;
+  __shared__ TileSmem<G, Policy::NACC, true> sm;
   const Policy pol = make_dq_policy<T, W, LPH, G>(p);
   walk_tile_in<G, Policy>(sm, p.walk, pol);
 }
 
 template <typename T, int W, int LPH, int G>
-__global__ void __launch_bounds__(kBlockThreads) bwd_dq_stitch_kernel(const BwdParams p) {
+__global__ void __launch_bounds__(kCrossingThreads) bwd_dq_stitch_kernel(const BwdParams p) {
   using Policy = DqPolicy<T, W, LPH, G>;
   const Policy pol = make_dq_policy<T, W, LPH, G>(p);
-  __shared__ float s_part[kBlockThreads * Policy::NACC];
-  stitch_tiles<G, Policy>(p.walk, pol, s_part);
+  finish_crossing_rows<G, Policy>(p.walk, pol);
 }
 
 
 }  // namespace
 
-bool launch_dq(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, bool second_kernel, int link,
+bool launch_dq(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, int link,
                cudaStream_t stream) {
   return dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
     launch_chained(bwd_dq_kernel<typename S::T, S::W, S::LPH, S::G>, grid, kBlockThreads, stream, link, p);
-    if (second_kernel && p.walk.n_tiles > 1)
-      launch_chained(bwd_dq_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(p.walk.n_tiles, grid.y), kBlockThreads, stream, kLinkStitch, p);
+    if (p.walk.n_tiles > 1)
+      launch_chained(bwd_dq_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(crossing_ctas(p.walk, S::G), grid.y), kCrossingThreads, stream, kLinkStitch, p);
   });
 }
 

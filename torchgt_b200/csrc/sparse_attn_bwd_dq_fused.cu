@@ -6,10 +6,12 @@ namespace bwd {
 namespace {
 
 // ---- pass A without a statistics pre-pass (no dbias) ---------------------------------------------
-template <typename T, int W, int LPH, int G>
+template <typename T, int W, int LPH, int G, int BIAS>
 struct DqFusedPolicy {
   static constexpr int VEC = Lane<T, W>::kElems;
   static constexpr int NACC = 2 * VEC + 1;  // A1, A2, S
+  static constexpr bool kPairs = sizeof(T) == 2;
+  static constexpr bool kPerm = BIAS != kNoBias;
   static constexpr int kUnroll = walk_unroll<T, W, G>();
 
   const T* __restrict__ q;
@@ -41,7 +43,7 @@ struct DqFusedPolicy {
     o.v = Lane<T, W>::raw_at(v, so);
     o.q = Lane<T, W>::raw_at(q, unsigned(row) * q_vecs + cvec);
     o.g = Lane<T, W>::raw_at(dout, unsigned(row) * g_vecs + cvec);
-    o.b = bias != nullptr ? __ldg(bias + int64_t(pe) * bias_stride + bias_off) : 0.f;
+    o.b = BIAS != kNoBias ? __ldg(bias + int64_t(pe) * bias_stride + bias_off) : 0.f;
   }
   __device__ __forceinline__ void clear(Operands& o) const {
     o.k = o.v = o.q = o.g = Lane<T, W>::raw_zero();
@@ -51,10 +53,10 @@ struct DqFusedPolicy {
     float a[VEC], b[VEC];
     Lane<T, W>::unpack(o.q, a);
     Lane<T, W>::unpack(o.k, b);
-    const float raw = group_sum<LPH>(dot<VEC>(a, b)) * inv_scale;
+    const float raw = group_sum<LPH>(dot<kPairs>(a, b)) * inv_scale;
     Lane<T, W>::unpack(o.g, a);
     Lane<T, W>::unpack(o.v, b);
-    const float gv = group_sum<LPH>(dot<VEC>(a, b));
+    const float gv = group_sum<LPH>(dot<kPairs>(a, b));
     const float wgt = valid ? fast_exp(clamp_score(raw) + o.b) : 0.f;
     Scalars s;
     s.wgv = wgt * gv;
@@ -66,11 +68,8 @@ struct DqFusedPolicy {
                                              const Scalars& s) const {
     float kf[VEC];
     Lane<T, W>::unpack(o.k, kf);
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) {
-      acc[j] = fmaf(s.wgv_m, kf[j], acc[j]);
-      acc[VEC + j] = fmaf(s.wm, kf[j], acc[VEC + j]);
-    }
+    add_scaled<kPairs, 0>(acc, s.wgv_m, kf);
+    add_scaled<kPairs, VEC>(acc, s.wm, kf);
     acc[2 * VEC] += s.wgv;
   }
   __device__ __forceinline__ void finalize(int row, const float (&acc)[NACC]) const {
@@ -90,11 +89,11 @@ struct DqFusedPolicy {
   }
 };
 
-template <typename T, int W, int LPH, int G>
-__device__ __forceinline__ DqFusedPolicy<T, W, LPH, G> make_dq_fused_policy(const BwdParams& p) {
+template <typename T, int W, int LPH, int G, int BIAS>
+__device__ __forceinline__ DqFusedPolicy<T, W, LPH, G, BIAS> make_dq_fused_policy(const BwdParams& p) {
   constexpr int VEC = Lane<T, W>::kElems;
   const int c = threadIdx.x % G;
-  DqFusedPolicy<T, W, LPH, G> pol;
+  DqFusedPolicy<T, W, LPH, G, BIAS> pol;
   pol.q = static_cast<const T*>(p.q);
   pol.k = static_cast<const T*>(p.k);
   pol.v = static_cast<const T*>(p.v);
@@ -117,40 +116,43 @@ __device__ __forceinline__ DqFusedPolicy<T, W, LPH, G> make_dq_fused_policy(cons
   return pol;
 }
 
-template <typename T, int W, int LPH, int G>
+template <typename T, int W, int LPH, int G, int BIAS>
 __global__ void TGT_WALK_BOUNDS bwd_dq_fused_kernel(const BwdParams p) {
-  using Policy = DqFusedPolicy<T, W, LPH, G>;
-  __shared__ TileSmem<G, Policy::NACC> sm;
-  const Policy pol = make_dq_fused_policy<T, W, LPH, G>(p);
+  using Policy = DqFusedPolicy<T, W, LPH, G, BIAS>;
+  __shared__ TileSmem<G, Policy::NACC, Policy::kPerm> sm;
+  const Policy pol = make_dq_fused_policy<T, W, LPH, G, BIAS>(p);
   walk_tile_in<G, Policy>(sm, p.walk, pol);
 }
 
-template <typename T, int W, int LPH, int G>
-__global__ void __launch_bounds__(kBlockThreads) bwd_dq_fused_stitch_kernel(const BwdParams p) {
-  using Policy = DqFusedPolicy<T, W, LPH, G>;
-  const Policy pol = make_dq_fused_policy<T, W, LPH, G>(p);
-  __shared__ float s_part[kBlockThreads * Policy::NACC];
-  stitch_tiles<G, Policy>(p.walk, pol, s_part);
+template <typename T, int W, int LPH, int G, int BIAS>
+__global__ void __launch_bounds__(kCrossingThreads) bwd_dq_fused_stitch_kernel(const BwdParams p) {
+  using Policy = DqFusedPolicy<T, W, LPH, G, BIAS>;
+  const Policy pol = make_dq_fused_policy<T, W, LPH, G, BIAS>(p);
+  finish_crossing_rows<G, Policy>(p.walk, pol);
 }
 
 
 }  // namespace
 
-bool launch_dq_fused(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, bool second_kernel, int link,
+bool launch_dq_fused(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, int link,
                      cudaStream_t stream) {
   return dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
-    launch_chained(bwd_dq_fused_kernel<typename S::T, S::W, S::LPH, S::G>, grid, kBlockThreads, stream, link, p);
-    if (second_kernel && p.walk.n_tiles > 1)
-      launch_chained(bwd_dq_fused_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(p.walk.n_tiles, grid.y), kBlockThreads, stream, kLinkStitch, p);
+    dispatch_bias<kReadBias>(bias_use(p), [&](auto use) {
+      launch_chained(bwd_dq_fused_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value>, grid, kBlockThreads, stream, link, p);
+    });
+    if (p.walk.n_tiles > 1)
+      launch_chained(bwd_dq_fused_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), kCrossingThreads, stream, kLinkStitch, p);
   });
 }
 
-int occupancy_dq_fused(int dtype, const HeadSplit& hs, int* cache_slot) {
+int occupancy_dq_fused(int dtype, const HeadSplit& hs, int use, int* cache_slot) {
   int result = 4;
   dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
-    result = resident_ctas(bwd_dq_fused_kernel<typename S::T, S::W, S::LPH, S::G>, cache_slot);
+    dispatch_bias<kReadBias>(use, [&](auto u) {
+      result = resident_ctas(bwd_dq_fused_kernel<typename S::T, S::W, S::LPH, S::G, decltype(u)::value>, cache_slot);
+    });
   });
   return result;
 }

@@ -6,10 +6,12 @@
 namespace tgt {
 namespace {
 
-template <typename T, int W, int LPH, int G>
+template <typename T, int W, int LPH, int G, int BIAS>
 struct FwdPolicy {
   static constexpr int VEC = Lane<T, W>::kElems;
   static constexpr int NACC = VEC + 1;  // w*V and, last, the sum of w
+  static constexpr bool kPairs = true;
+  static constexpr bool kPerm = BIAS != kNoBias;
   static constexpr int kUnroll = walk_unroll<T, W, G>();
 
   const T* __restrict__ q;
@@ -39,7 +41,7 @@ struct FwdPolicy {
     o.k = Lane<T, W>::raw_at(k, so);
     o.v = Lane<T, W>::raw_at(v, so);
     o.q = Lane<T, W>::raw_at(q, unsigned(row) * q_vecs + cvec);
-    o.b = bias != nullptr ? __ldg(bias + int64_t(pe) * bias_stride + bias_off) : 0.f;
+    o.b = BIAS != kNoBias ? __ldg(bias + int64_t(pe) * bias_stride + bias_off) : 0.f;
   }
   __device__ __forceinline__ void clear(Operands& o) const {
     o.k = o.v = o.q = Lane<T, W>::raw_zero();
@@ -49,7 +51,7 @@ struct FwdPolicy {
     float qf[VEC], kf[VEC];
     Lane<T, W>::unpack(o.q, qf);
     Lane<T, W>::unpack(o.k, kf);
-    const float raw = group_sum<LPH>(dot<VEC>(qf, kf)) * inv_scale;
+    const float raw = group_sum<LPH>(dot<kPairs>(qf, kf)) * inv_scale;
     Scalars s;
     s.w = valid ? fast_exp(clamp_score(raw) + o.b) : 0.f;
     return s;
@@ -58,8 +60,7 @@ struct FwdPolicy {
                                              const Scalars& s) const {
     float vf[VEC];
     Lane<T, W>::unpack(o.v, vf);
-#pragma unroll
-    for (int j = 0; j < VEC; ++j) acc[j] = fmaf(s.w, vf[j], acc[j]);
+    add_scaled<kPairs, 0>(acc, s.w, vf);
     acc[VEC] += s.w;
   }
   __device__ __forceinline__ void finalize(int row, const float (&acc)[NACC]) const {
@@ -93,11 +94,11 @@ struct FwdParams {
   SegWalk walk;
 };
 
-template <typename T, int W, int LPH, int G>
-__device__ __forceinline__ FwdPolicy<T, W, LPH, G> make_policy(const FwdParams& p) {
+template <typename T, int W, int LPH, int G, int BIAS>
+__device__ __forceinline__ FwdPolicy<T, W, LPH, G, BIAS> make_policy(const FwdParams& p) {
   constexpr int VEC = Lane<T, W>::kElems;
   const int c = threadIdx.x % G;
-  FwdPolicy<T, W, LPH, G> pol;
+  FwdPolicy<T, W, LPH, G, BIAS> pol;
   pol.q = static_cast<const T*>(p.q);
   pol.k = static_cast<const T*>(p.k);
   pol.v = static_cast<const T*>(p.v);
@@ -117,46 +118,45 @@ __device__ __forceinline__ FwdPolicy<T, W, LPH, G> make_policy(const FwdParams& 
   return pol;
 }
 
-template <typename T, int W, int LPH, int G>
+template <typename T, int W, int LPH, int G, int BIAS>
 __global__ void TGT_WALK_BOUNDS fwd_kernel(const FwdParams p) {
-  using Policy = FwdPolicy<T, W, LPH, G>;
-  __shared__ TileSmem<G, Policy::NACC> sm;
-  const Policy pol = make_policy<T, W, LPH, G>(p);
+  using Policy = FwdPolicy<T, W, LPH, G, BIAS>;
+  __shared__ TileSmem<G, Policy::NACC, Policy::kPerm> sm;
+  const Policy pol = make_policy<T, W, LPH, G, BIAS>(p);
   walk_tile_in<G, Policy>(sm, p.walk, pol);
 }
 
-template <typename T, int W, int LPH, int G>
-__global__ void __launch_bounds__(kBlockThreads) fwd_stitch_kernel(const FwdParams p) {
-  using Policy = FwdPolicy<T, W, LPH, G>;
-  const Policy pol = make_policy<T, W, LPH, G>(p);
-  __shared__ float s_part[kBlockThreads * Policy::NACC];
-  stitch_tiles<G, Policy>(p.walk, pol, s_part);
+template <typename T, int W, int LPH, int G, int BIAS>
+__global__ void __launch_bounds__(kCrossingThreads) fwd_stitch_kernel(const FwdParams p) {
+  using Policy = FwdPolicy<T, W, LPH, G, BIAS>;
+  const Policy pol = make_policy<T, W, LPH, G, BIAS>(p);
+  finish_crossing_rows<G, Policy>(p.walk, pol);
 }
 
-// Resident CTAs per SM of fwd_kernel<T, W, LPH, G> for the run-time triple.
-int fwd_resident_ctas(int dtype, const HeadSplit& hs) {
-  static int cache[kMaxDevices][2][2][6][6] = {};   // occupancy is a property of the device
+// Resident CTAs per SM of fwd_kernel for the run-time lane shape and bias use.
+int fwd_resident_ctas(int dtype, const HeadSplit& hs, int bias_use) {
+  static int cache[kMaxDevices][2][2][2][6][6] = {};   // occupancy is a property of the device
   auto log2i = [](int x) { int l = 0; while ((1 << l) < x) ++l; return l; };
   const int dev = current_device();
-  int* slot = &cache[dev < 0 ? 0 : dev][hs.w == 32 ? 1 : 0][dtype == TGT_F32 ? 0 : 1][log2i(hs.lph)][log2i(hs.g)];
+  int* slot = &cache[dev < 0 ? 0 : dev][bias_use][hs.w == 32 ? 1 : 0][dtype == TGT_F32 ? 0 : 1][log2i(hs.lph)][log2i(hs.g)];
   int result = 4;
   dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
-    result = resident_ctas(fwd_kernel<typename S::T, S::W, S::LPH, S::G>, slot);
+    dispatch_bias<kReadBias>(bias_use, [&](auto use) {
+      result = resident_ctas(fwd_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value>, slot);
+    });
   });
   return result;
 }
 
 }  // namespace
 
-TilePlan plan_tiles(int64_t n_edges, const HeadSplit& hs, int nacc, int ctas_per_sm) {
+TilePlan plan_tiles(int64_t n_edges, const HeadSplit& hs, int step, int nacc, int ctas_per_sm) {
   TilePlan t;
-  t.ge = choose_ge(n_edges, hs.g, ctas_per_sm);
+  t.ge = choose_ge(n_edges, hs.g, step, ctas_per_sm);
   const int64_t te = int64_t(kBlockThreads / hs.g) * t.ge;
   t.n_tiles = int((n_edges + te - 1) / te);
   t.carry_bytes = round_up(size_t(t.n_tiles) * 2 * size_t(hs.groups) * hs.g * nacc * 4, 256);
-  t.counter_bytes = round_up(size_t(t.n_tiles) * hs.groups * 4, 256);
-  t.scratch_bytes = t.carry_bytes + t.counter_bytes;
   return t;
 }
 
@@ -165,7 +165,12 @@ size_t fwd_scratch_bytes_w(const tgt_layout* L, int heads, int head_dim, int dty
   HeadSplit hs;
   if (!split_heads(heads, head_dim, dtype, w, &hs) || L->n_edges == 0) return 0;
   const int nacc = w / (dtype == TGT_F32 ? 4 : 2) + 1;
-  return plan_tiles(L->n_edges, hs, nacc, fwd_resident_ctas(dtype, hs)).scratch_bytes;
+  size_t need = 0;
+  for (const int use : {kNoBias, kReadBias}) {
+    const size_t bytes = plan_tiles(L->n_edges, hs, walk_batch(dtype == TGT_F32, hs.w, hs.g), nacc, fwd_resident_ctas(dtype, hs, use)).carry_bytes;
+    if (bytes > need) need = bytes;
+  }
+  return need;
 }
 
 // What a caller must provide: enough for whichever lane width the call ends up using (the width depends
@@ -231,10 +236,11 @@ extern "C" int tgt_sparse_attn_fwd_strided(const void* q, int64_t q_row_bytes, c
     return TGT_OK;
   }
   const int nacc = hs.w / int(elem) + 1;
-  const TilePlan tp = plan_tiles(L.n_edges, hs, nacc, fwd_resident_ctas(dtype, hs));
-  if (scratch == nullptr || scratch_bytes < tp.scratch_bytes)
+  const int bias_use = bias != nullptr ? kReadBias : kNoBias;
+  const TilePlan tp = plan_tiles(L.n_edges, hs, walk_batch(dtype == TGT_F32, hs.w, hs.g), nacc, fwd_resident_ctas(dtype, hs, bias_use));
+  if (scratch == nullptr || scratch_bytes < tp.carry_bytes)
     return set_error(TGT_ERR_WORKSPACE, "scratch holds %zu bytes, %zu needed", scratch_bytes,
-                     tp.scratch_bytes);
+                     tp.carry_bytes);
 
   FwdParams p;
   p.q = q; p.k = k; p.v = v; p.bias = bias; p.bias_heads = bias_heads;
@@ -248,18 +254,15 @@ extern "C" int tgt_sparse_attn_fwd_strided(const void* q, int64_t q_row_bytes, c
   p.walk.n_rows = int(L.n_rows); p.walk.n_edges = int(L.n_edges);
   p.walk.ge = tp.ge; p.walk.n_tiles = tp.n_tiles; p.walk.gap_ctas = gap_ctas(L.n_rows);
   p.walk.gcarry = static_cast<float*>(scratch);
-  const bool second_kernel = stitch_in_second_kernel(hs.g);
-  p.walk.tile_done = second_kernel ? nullptr : reinterpret_cast<int*>(static_cast<char*>(scratch) + tp.carry_bytes);
-  p.walk.need_perm = bias != nullptr;
-  if (tp.n_tiles > 1 && !second_kernel)
-    TGT_CHECK_CUDA(cudaMemsetAsync(p.walk.tile_done, 0, tp.counter_bytes, stream));
 
   const dim3 grid(walk_ctas(tp, L.n_rows), hs.groups);
   const bool built = dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
-    fwd_kernel<typename S::T, S::W, S::LPH, S::G><<<grid, kBlockThreads, 0, stream>>>(p);
-    if (second_kernel && tp.n_tiles > 1)
-      launch_chained(fwd_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(p.walk.n_tiles, grid.y), kBlockThreads, stream, kLinkStitch, p);
+    dispatch_bias<kReadBias>(bias_use, [&](auto use) {
+      fwd_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value><<<grid, kBlockThreads, 0, stream>>>(p);
+    });
+    if (tp.n_tiles > 1)
+      launch_chained(fwd_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), kCrossingThreads, stream, kLinkStitch, p);
   });
   if (!built) return set_error(TGT_ERR_UNSUPPORTED, "no kernel is built for this head layout");
   TGT_CHECK_CUDA(cudaGetLastError());
