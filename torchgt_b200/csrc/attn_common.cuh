@@ -62,12 +62,12 @@ namespace tgt {
 #define TGT_WALK_BOUNDS __launch_bounds__(128)
 #endif
 
-#ifndef TGT_LEAST_GE
-#define TGT_LEAST_GE 8
-#endif
 constexpr int kBlockThreads = 128;
 constexpr int kUnroll = TGT_UNROLL;  // edges per lane group whose gathers are in flight together
-constexpr int kGeStep = 4;           // ge is a multiple of this (and of every batch size below)
+constexpr int kGeStep = 4;           // a forced ge is a multiple of this (and of every batch size below)
+// Fewest edges per lane group: with 16, 1,000 nodes take 10.0 + 23.7 us forward and backward, with 8 7.5 + 16.2, with 4
+// 6.9 + 16.2; 4,096 nodes take 9.3 + 22.6, 9.4 + 25.4, 9.4 + 25.4.
+constexpr int kLeastEdges = 8;
 
 // Batch size of the walk for element type T and lane-group width G.  Measured on B200 (fp32, 8-byte to
 // 256-byte rows; bf16 128-byte rows): batches of 4 edges are best everywhere except for fp32 rows of
@@ -122,18 +122,24 @@ inline int choose_ge(int64_t n_edges, int g, int step, int ctas_per_sm) {
   }
   // Time is roughly (number of CTA waves) x (work of one tile); a tile costs its ge edges per lane
   // group plus a fixed part (index staging, barriers, stitching) worth about 8 edges.  Few, full
-  // waves win; with many waves the tail does not matter and larger tiles amortise the fixed part.
+  // waves win; with many waves the tail does not matter and larger tiles amortise the fixed part.  Of the tiles that
+  // need the same number of waves the smallest is best.
   const int64_t capacity = int64_t(sm_count()) * ctas_per_sm;
+  const int least = ge_max < kLeastEdges ? ge_max : kLeastEdges;
   int best = ge_max;
   double best_cost = 1e300;
-  for (int ge = (ge_max < TGT_LEAST_GE ? ge_max : TGT_LEAST_GE); ge <= ge_max; ge += step) {
-    const int64_t tiles = (n_edges + int64_t(ng) * ge - 1) / (int64_t(ng) * ge);
-    const int64_t waves = (tiles + capacity - 1) / capacity;
+  const int64_t fewest = (n_edges + capacity * ng * ge_max - 1) / (capacity * ng * ge_max);
+  for (int64_t waves = fewest < 1 ? 1 : fewest; waves <= fewest + 15; ++waves) {
+    const int64_t lanes = capacity * ng * waves;
+    int ge = int((n_edges + lanes - 1) / lanes + step - 1) / step * step;   // the smallest tile that needs no more waves
+    if (ge < least) ge = least;
+    if (ge > ge_max) continue;
     const double cost = double(waves) * (ge + 8);
-    if (cost < best_cost - 1e-9) {
+    if (cost < best_cost) {
       best_cost = cost;
       best = ge;
     }
+    if (ge == least) break;
   }
   return best;
 }

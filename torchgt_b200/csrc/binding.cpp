@@ -285,7 +285,7 @@ using torch::autograd::variable_list;
 struct SparseGraphAttentionBackward : public torch::autograd::Node {
   std::shared_ptr<Graph> graph;
   SavedVariable q, k, v, bias, out, z;
-  int dtype = 0;
+  int heads = 0, head_dim = 0, dtype = 0;
   bool with_dbias = false;   // the statistics of the forward's output are read only then, so only then is it kept
 
   variable_list apply(variable_list&& grads) override {
@@ -301,8 +301,7 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
     const at::Tensor dout = grads[0].contiguous();
     at::Tensor dq = at::empty_like(q_), dk = at::empty_like(k_), dv = at::empty_like(v_), dbias;
     if (want_dbias) dbias = at::empty_like(bias_);
-    attention_backward(*graph, dout, q_, k_, v_, bias_, out_, z_, dq, dk, dv, dbias, int(q_.size(1)), int(q_.size(2)),
-                       dtype);
+    attention_backward(*graph, dout, q_, k_, v_, bias_, out_, z_, dq, dk, dv, dbias, heads, head_dim, dtype);
     return {dq, dk, dv, dbias};
   }
   std::string name() const override { return "SparseGraphAttentionBackward"; }
@@ -312,22 +311,22 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
   }
 };
 
-at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in,
-                     const std::optional<at::Tensor>& bias_in, const std::shared_ptr<Graph>& graph) {
-  const at::Tensor bias = bias_in.has_value() ? *bias_in : at::Tensor();
+}  // namespace
+
+at::Tensor attention_over_rows(const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in, const at::Tensor& bias,
+                               const std::shared_ptr<Graph>& graph, int heads, int head_dim) {
   // the node has no forward-mode formula: refuse a dual tensor rather than drop its tangent
   for (const at::Tensor* t : {&q_in, &k_in, &v_in, &bias})
     TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(*t),
                                 "sparse_graph_attention does not support forward-mode AD");
   const at::Tensor q = q_in.contiguous(), k = k_in.contiguous(), v = v_in.contiguous();
-  const int heads = int(q.size(1)), head_dim = int(q.size(2));
   const int dtype = dtype_of(q);
   const c10::cuda::CUDAGuard guard(q.device());
   at::Tensor out, z;
   {
     const at::AutoDispatchBelowADInplaceOrView below;
     out = at::empty_like(q);
-    z = at::empty({q.size(0), heads}, q.options().dtype(at::kFloat));
+    z = at::empty({graph->n_rows, heads}, q.options().dtype(at::kFloat));
     attention_forward(*graph, q, k, v, bias, out, z, heads, head_dim, dtype);
   }
   if (torch::autograd::compute_requires_grad(q, k, v, bias)) {
@@ -335,6 +334,8 @@ at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::T
                                                              torch::autograd::deleteNode);
     node->set_next_edges(torch::autograd::collect_next_edges(q, k, v, bias));
     node->graph = graph;
+    node->heads = heads;
+    node->head_dim = head_dim;
     node->dtype = dtype;
     node->with_dbias = bias.defined() && bias.requires_grad();
     node->q = SavedVariable(q, false);
@@ -346,6 +347,13 @@ at::Tensor attention(const at::Tensor& q_in, const at::Tensor& k_in, const at::T
     if (node->with_dbias) node->out = SavedVariable(out, true);
   }
   return out;
+}
+
+namespace {
+
+at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const std::optional<at::Tensor>& bias,
+                     const std::shared_ptr<Graph>& graph) {
+  return attention_over_rows(q, k, v, bias.value_or(at::Tensor()), graph, int(q.size(1)), int(q.size(2)));
 }
 
 // The two passes without an autograd node, for callers that keep one of their own (torchgt_b200/sparse_attn.py).

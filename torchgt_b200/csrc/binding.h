@@ -113,6 +113,10 @@ void attention_backward(Graph& g, const at::Tensor& dout, const at::Tensor& q, c
                         const at::Tensor& dk, const at::Tensor& dv, const at::Tensor& dbias, int heads, int head_dim,
                         int dtype);
 
+// The attention as one autograd node: q, k and v of any one shape that is graph->n_rows rows of heads * head_dim values
+at::Tensor attention_over_rows(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
+                               const std::shared_ptr<Graph>& graph, int heads, int head_dim);
+
 void bind_batching(pybind11::module_& m);   // binding_batch.cpp
 void bind_dense(pybind11::module_& m);      // binding_dense.cpp
 

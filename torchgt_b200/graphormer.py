@@ -16,10 +16,12 @@ import torch
 from torch import nn
 from torch.nn import functional as F
 
+from . import _cabi
 from .attn_module import CoreAttention
 from .gt_sp.initialize import get_sequence_parallel_group, sequence_parallel_is_initialized
 from .layer_norm import LayerNorm, add_layer_norm
-from .linear import Linear, embedding_sum, feed_forward, linear3, passes_through, unobserved
+from .graph import graph_for
+from .linear import Linear, embedding_sum, feed_forward, linear3, passes_through, plain_call, plain_modules, unobserved
 from .gt_sp.layer import DistributedAttentionNoMerge
 
 
@@ -118,7 +120,40 @@ class EncoderLayer(nn.Module):
         rows = get_global_token_rows_on(x.device, get_last_batch_flag())
         return fused.attention_block(px, x, self.self_attention_norm, mha, edge_index, rows)
 
+    def _native_layer(self, x, attn_bias, edge_index, attn_type):
+        """The whole layer as one call into the host module: the operations below, without a return to Python between
+        them.  None where somebody could notice: sequence parallelism, a dropout that drops, subclassed, replaced or hooked
+        modules, missing biases, tracing, compiling, autocast, tensor subclasses, other dtypes and devices."""
+        if attn_type != "sparse" or attn_bias is not None or edge_index is None:
+            return None
+        if not (x.is_cuda and x.dtype == torch.float32 and x.dim() == 3):
+            return None
+        mha, ffn = self.self_attention, self.ffn
+        if sequence_parallel_is_initialized() if mha.sequence_parallel is None else mha.sequence_parallel:
+            return None
+        core = mha.dist_attn.local_attn
+        if not (plain_modules((mha, MultiHeadAttention), (core, CoreAttention), (ffn, FeedForwardNetwork),
+                              (ffn.gelu, nn.GELU), (self.self_attention_dropout, nn.Dropout), (self.ffn_dropout, nn.Dropout)) and
+                core.hidden_size_per_attention_head == mha.att_size and ffn.gelu.approximate == "none" and
+                not any(d.training and d.p != 0.0 for d in (self.self_attention_dropout, self.ffn_dropout))):
+            return None
+        norm, ffn_norm = self.self_attention_norm, self.ffn_norm
+        projections = (mha.linear_q, mha.linear_k, mha.linear_v, mha.output_layer)
+        layers = (norm, *projections, ffn_norm, ffn.layer1, ffn.layer2)
+        if not (plain_modules((norm, LayerNorm), (ffn_norm, LayerNorm), *((m, Linear) for m in layers[1:5] + layers[6:])) and
+                len(norm.normalized_shape) == 1 and len(ffn_norm.normalized_shape) == 1):
+            return None
+        tensors = [m._parameters.get(name) for m in layers for name in ("weight", "bias")]
+        if any(t is None for t in tensors) or not plain_call(x, *tensors):
+            return None
+        graph = graph_for(edge_index, x.size(0) * x.size(1))
+        graph.native.poll()
+        return _cabi.native().encoder_layer(x, graph.native, mha.num_heads, mha.att_size, tensors, norm.eps, ffn_norm.eps)
+
     def forward(self, x, attn_bias=None, edge_index=None, attn_type=None, mask=None):
+        y = self._native_layer(x, attn_bias, edge_index, attn_type)
+        if y is not None:
+            return y
         y = self._fused_attention_half(x, attn_bias, edge_index, attn_type)
         if y is None:
             y = self.self_attention(self.self_attention_norm(x), attn_bias, edge_index, attn_type=attn_type)

@@ -47,15 +47,15 @@ def wgrad(dy: torch.Tensor, x: torch.Tensor, with_bias: bool = True):
     return dw, db
 
 
-def _plain_call(x, weight, bias) -> bool:
-    """No tracer, compiler, autocast or tensor subclass wants to see ``F.linear`` itself."""
+def plain_call(*tensors) -> bool:
+    """No tracer, compiler, autocast or tensor subclass wants to see PyTorch's own operation."""
     return not (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch.is_autocast_enabled("cuda") or
-                has_torch_function_variadic(x, weight, bias))
+                has_torch_function_variadic(*tensors))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias) -> torch.Tensor:
     """``F.linear(x, weight, bias)``."""
-    if x.is_cuda and _plain_call(x, weight, bias):
+    if x.is_cuda and plain_call(x, weight, bias):
         return _cabi.native().linear(x, weight, bias)
     return F.linear(x, weight, bias)
 
@@ -76,10 +76,23 @@ def unobserved(module: torch.nn.Module, kind: type) -> bool:
                     _module._global_backward_pre_hooks))
 
 
+def plain_modules(*pairs) -> bool:
+    """Every (module, kind) is :func:`unobserved`."""
+    if any((_module._global_forward_hooks, _module._global_forward_pre_hooks, _module._global_backward_hooks,
+            _module._global_backward_pre_hooks)):
+        return False
+    for module, kind in pairs:
+        own = module.__dict__
+        if type(module) is not kind or "forward" in own or own["_forward_hooks"] or own["_forward_pre_hooks"] or \
+                own["_backward_hooks"] or own["_backward_pre_hooks"]:
+            return False
+    return True
+
+
 def linear3(x: torch.Tensor, a: torch.nn.Module, b: torch.nn.Module, c: torch.nn.Module):
     """``a(x), b(x), c(x)``: one node that reads ``x`` once each way where the three are plain layers of equal shape."""
     layers = (a, b, c)
-    if x.is_cuda and all(unobserved(m, Linear) and _plain_call(x, m.weight, m.bias) for m in layers):
+    if x.is_cuda and all(unobserved(m, Linear) and plain_call(x, m.weight, m.bias) for m in layers):
         return _cabi.native().linear3(x, [m.weight for m in layers], [m.bias for m in layers])
     return a(x), b(x), c(x)
 
@@ -88,7 +101,7 @@ def feed_forward(x: torch.Tensor, first: torch.nn.Module, second: torch.nn.Modul
     """``(residual +) second(act(first(x)))`` with ``activation`` "relu" or "gelu" (exact), one node whose activation is
     part of the products' kernels, or None where the caller has to go through the modules."""
     if not (x.is_cuda and unobserved(first, Linear) and unobserved(second, Linear) and first.bias is not None and
-            second.bias is not None and _plain_call(x, first.weight, first.bias) and
+            second.bias is not None and plain_call(x, first.weight, first.bias) and
             not has_torch_function_variadic(second.weight, second.bias, residual)):
         return None
     return _cabi.native().feed_forward(x, first.weight, first.bias, second.weight, second.bias, activation, residual)
@@ -102,7 +115,7 @@ def passes_through(dropout: torch.nn.Module) -> bool:
 def embedding_sum(embedding: torch.nn.Module, ids: torch.Tensor) -> torch.Tensor:
     """``embedding(ids).sum(dim=-2)``; the gathered vectors are never stored (csrc/embedding_sum.cu)."""
     if (ids.is_cuda and unobserved(embedding, torch.nn.Embedding) and embedding.max_norm is None and not embedding.sparse and
-            not embedding.scale_grad_by_freq and _plain_call(ids, embedding.weight, None)):
+            not embedding.scale_grad_by_freq and plain_call(ids, embedding.weight, None)):
         padding = -1 if embedding.padding_idx is None else embedding.padding_idx
         return _cabi.native().embedding_sum(embedding.weight, ids, padding)
     return embedding(ids).sum(dim=-2)
