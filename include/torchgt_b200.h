@@ -135,6 +135,20 @@ TGT_API int tgt_edge_layout_build_i32(const int32_t* edge_index, int64_t n_edges
                                       int32_t* deferred_status, void* stream);
 
 /*
+ * Both orientations of one int64 list: the first build also writes the checked endpoints as int32 to `kept`
+ * (tgt_edge_layout_kept_words(n_edges) words on the device, 16-byte aligned), from which the second one (n_edges > 0,
+ * workspace of tgt_edge_layout_sizes_i32) sorts without reading the list again.  An endpoint out of range is kept as 0.
+ */
+TGT_API int tgt_edge_layout_kept_words(int64_t n_edges, size_t* words);
+TGT_API int tgt_edge_layout_build_keep(const int64_t* edge_index, int64_t n_edges, int64_t n_rows,
+                                       int group_by, int32_t* ptr, int32_t* other, int32_t* perm,
+                                       int32_t* seg, void* workspace, size_t workspace_bytes,
+                                       int32_t* deferred_status, int32_t* kept, void* stream);
+TGT_API int tgt_edge_layout_build_kept(const int32_t* kept, int64_t n_edges, int64_t n_rows, int group_by,
+                                       int32_t* ptr, int32_t* other, int32_t* perm, int32_t* seg,
+                                       void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * Batch edge construction on the device: the reference's host-side helpers applied in one pass to the
  * RAW edges of a batch of `graphs` graphs (node ids 0..n_g-1 inside each graph), writing an int32
  * [2, out_total] edge list for tgt_edge_layout_build_i32.

@@ -286,3 +286,31 @@ def test_a_graph_from_an_int32_list_allocates_no_narrow_copy():
     graph.check()
     # other, perm, seg and the workspace; a megabyte of rounding per allocation is below the 16 MB of a copy
     assert torch.cuda.max_memory_allocated() - before < 3 * 4 * n_edges + need.value + (6 << 20)
+
+
+@pytest.mark.parametrize("n_rows,n_edges", [(1, 1), (3, 2), (40, 63), (40, 64), (40, 65), (70000, 200003)])
+def test_second_orientation_from_what_the_first_kept(n_rows, n_edges):
+    """The sources' layout from the endpoints the first build kept (same stream), from the list itself (another stream, as
+    before), and the CPU's stable sort; rows without edges in runs of every length up to thousands."""
+    from torchgt_b200 import SparseGraph
+    gen = torch.Generator().manual_seed(n_edges)
+    used = torch.randperm(n_rows, generator=gen)[:max(1, n_rows // 50)]
+    ei = used[torch.randint(0, used.numel(), (2, n_edges), generator=gen)]
+    here, there = SparseGraph(ei.cuda(), n_rows), SparseGraph(ei.cuda(), n_rows)
+    kept = here.by_src
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        other = there.by_src
+        torch.cuda.synchronize()
+    perm = torch.sort(ei[0], stable=True).indices
+    ptr = torch.cat([torch.zeros(1, dtype=torch.long), torch.bincount(ei[0], minlength=n_rows).cumsum(0)])
+    for layout in (kept, other):
+        assert torch.equal(layout.perm.cpu().long(), perm)
+        assert torch.equal(layout.seg.cpu().long(), ei[0][perm])
+        assert torch.equal(layout.other.cpu().long(), ei[1][perm])
+        assert torch.equal(layout.ptr.cpu().long(), ptr)
+    here.check()
+    bad = ei.clone()
+    bad[0, 0] = n_rows
+    with pytest.raises(Exception, match="outside"):
+        SparseGraph(bad.cuda(), n_rows).by_src.verify()

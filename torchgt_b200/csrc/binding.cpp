@@ -114,28 +114,42 @@ CheckWords& check_words() {
 }  // namespace
 
 // ---- layouts ------------------------------------------------------------------------------------------------
-Layout::Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by_) : group_by(group_by_) {
+Layout::Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by_, Kept* kept) : group_by(group_by_) {
   const int64_t n_edges = edge_index.size(1);
+  const bool wide = edge_index.scalar_type() == at::kLong, from_kept = kept != nullptr && kept->endpoints.defined();
   size_t ws = 0;
-  check((edge_index.scalar_type() == at::kLong ? tgt_edge_layout_sizes : tgt_edge_layout_sizes_i32)(n_rows, n_edges, &ws));
+  check((wide && !from_kept ? tgt_edge_layout_sizes : tgt_edge_layout_sizes_i32)(n_rows, n_edges, &ws));
   const c10::cuda::CUDAGuard guard(edge_index.device());
   const auto i32 = edge_index.options().dtype(at::kInt);
   ptr = at::empty({n_rows + 1}, i32);
   other = at::empty({n_edges}, i32);
   perm = at::empty({n_edges}, i32);
   seg = at::empty({n_edges}, i32);
-  bad_index = at::empty({1}, i32);
+  bad_index = from_kept ? kept->bad_index : at::empty({1}, i32);
   at::Tensor workspace = at::empty({int64_t(ws < 16 ? 16 : ws)}, edge_index.options().dtype(at::kByte));
   auto words = [](const at::Tensor& t) { return static_cast<int32_t*>(tgt_host::ptr(t)); };
   const void* edges = tgt_host::ptr(edge_index);
   void* stream = stream_of(edge_index);
-  check(edge_index.scalar_type() == at::kLong
-            ? tgt_edge_layout_build(static_cast<const int64_t*>(edges), n_edges, n_rows, group_by, words(ptr),
-                                    words(other), words(perm), words(seg), workspace.data_ptr(), workspace.numel(),
-                                    words(bad_index), stream)
-            : tgt_edge_layout_build_i32(static_cast<const int32_t*>(edges), n_edges, n_rows, group_by, words(ptr),
-                                        words(other), words(perm), words(seg), workspace.data_ptr(),
-                                        workspace.numel(), words(bad_index), stream));
+  if (from_kept) {
+    check(tgt_edge_layout_build_kept(words(kept->endpoints), n_edges, n_rows, group_by, words(ptr), words(other), words(perm),
+                                     words(seg), workspace.data_ptr(), workspace.numel(), stream));
+  } else if (wide && kept != nullptr && n_edges > 0 && !capturing(edge_index)) {
+    size_t kept_words = 0;
+    check(tgt_edge_layout_kept_words(n_edges, &kept_words));
+    at::Tensor endpoints = at::empty({int64_t(kept_words)}, i32);
+    check(tgt_edge_layout_build_keep(static_cast<const int64_t*>(edges), n_edges, n_rows, group_by, words(ptr), words(other),
+                                     words(perm), words(seg), workspace.data_ptr(), workspace.numel(), words(bad_index),
+                                     words(endpoints), stream));
+    kept->endpoints = std::move(endpoints);
+    kept->bad_index = bad_index;
+    kept->stream = stream;
+  } else {
+    check(wide ? tgt_edge_layout_build(static_cast<const int64_t*>(edges), n_edges, n_rows, group_by, words(ptr), words(other),
+                                       words(perm), words(seg), workspace.data_ptr(), workspace.numel(), words(bad_index), stream)
+               : tgt_edge_layout_build_i32(static_cast<const int32_t*>(edges), n_edges, n_rows, group_by, words(ptr),
+                                           words(other), words(perm), words(seg), workspace.data_ptr(), workspace.numel(),
+                                           words(bad_index), stream));
+  }
   c.n_rows = n_rows;
   c.n_edges = n_edges;
   c.ptr = words(ptr);
@@ -212,14 +226,18 @@ void Layout::verify() {
 
 Graph::Graph(const at::Tensor& edge_index, int64_t rows)
     : n_rows(rows), n_edges(edge_index.size(1)), edge_index_(edge_index),
-      by_dst_(std::make_shared<Layout>(edge_index, rows, 1)) {}
+      by_dst_(std::make_shared<Layout>(edge_index, rows, 1, &kept_)) {}
 
 std::shared_ptr<Layout> Graph::by_src() {
   at::Tensor done;   // outlives the lock: a tensor that Python has seen takes the interpreter lock on its way out
   std::lock_guard<std::mutex> lock(mutex_);
   if (!by_src_) {
-    by_src_ = std::make_shared<Layout>(edge_index_, n_rows, 0);
+    // what the first build kept is complete, and its memory safe, on the stream of that build only; in a capture it would
+    // tie the graph's replays to an array that is given back here
+    const bool usable = kept_.endpoints.defined() && kept_.stream == stream_of(edge_index_) && !capturing(edge_index_);
+    by_src_ = std::make_shared<Layout>(edge_index_, n_rows, 0, usable ? &kept_ : nullptr);
     built_.store(by_src_.get(), std::memory_order_release);
+    kept_ = {};
     done = std::move(edge_index_);
   }
   return by_src_;
@@ -403,7 +421,9 @@ PYBIND11_MODULE(_native, m) {
     }
   });
   py::class_<Layout, std::shared_ptr<Layout>>(m, "Layout")
-      .def(py::init<const at::Tensor&, int64_t, int>(), Unlocked())
+      .def(py::init([](const at::Tensor& edges, int64_t rows, int group_by) {
+             return std::make_shared<Layout>(edges, rows, group_by);
+           }), Unlocked())
       .def("poll", &Layout::poll)   // waits for nothing, and nobody waits for the interpreter under its mutex
       .def("verify", &Layout::verify, Unlocked())
       .def_property_readonly("verified", &Layout::verified)

@@ -62,7 +62,13 @@ inline float* fptr(const at::Tensor& t) { return static_cast<float*>(ptr(t)); }
 // the result of its range check arrives in a pinned word behind an event.
 class Layout {
  public:
-  Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by);
+  // What the build of one orientation of an int64 list keeps for the other's: both endpoints in 32 bits, checked
+  // (tgt_edge_layout_build_keep), until that one is built or its graph goes.
+  struct Kept {
+    at::Tensor endpoints, bad_index;
+    void* stream = nullptr;
+  };
+  Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by, Kept* kept = nullptr);
   ~Layout();
   Layout(const Layout&) = delete;
   Layout& operator=(const Layout&) = delete;
@@ -98,7 +104,8 @@ class Graph {
 
  private:
   std::mutex mutex_;
-  at::Tensor edge_index_;   // kept until by_src is built
+  at::Tensor edge_index_;   // until by_src is built, as is what its build can use
+  Layout::Kept kept_;
   std::shared_ptr<Layout> by_dst_, by_src_;
   std::atomic<Layout*> built_{nullptr};   // by_src_ once it is there, for whoever must not wait for its construction
   struct Need { int heads, head_dim, dtype, phase; size_t bytes; };

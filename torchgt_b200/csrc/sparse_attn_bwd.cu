@@ -51,15 +51,20 @@ struct BwdScratch {
   TilePlan plan_a, plan_a_fused, plan_b;
 };
 
-// hs: lane layout of pass A (by destination), hsb: of pass B (by source); they may use different lane widths
+// hs: lane layout of pass A (by destination), hsb: of pass B (by source); they may use different lane widths.  Only the
+// plans of the `walks` that run are made (bit 1 << kWalk...): the statistics, which outlive a call, come first.
 BwdScratch plan_bwd_scratch(const tgt_layout* by_dst, const HeadSplit& hs, const HeadSplit& hsb, int heads,
-                            int dtype, int use) {
-  BwdScratch s;
-  const int vec = hs.w / (dtype == TGT_F32 ? 4 : 2);
-  const int vecb = hsb.w / (dtype == TGT_F32 ? 4 : 2);
-  s.plan_a = plan_tiles(by_dst->n_edges, hs, walk_batch(dtype == TGT_F32, hs.w, hs.g), vec, bwd_resident_ctas(dtype, hs, kWalkDq, use));
-  s.plan_a_fused = plan_tiles(by_dst->n_edges, hs, walk_batch(dtype == TGT_F32, hs.w, hs.g), 2 * vec + 1, bwd_resident_ctas(dtype, hs, kWalkDqFused, use < kReadBias ? use : kReadBias));
-  s.plan_b = plan_tiles(by_dst->n_edges, hsb, walk_batch(dtype == TGT_F32, hsb.w, hsb.g), 2 * vecb, bwd_resident_ctas(dtype, hsb, kWalkDkv, use));
+                            int dtype, int use, int walks) {
+  BwdScratch s = {};
+  const bool fp32 = dtype == TGT_F32;
+  const int vec = hs.w / (fp32 ? 4 : 2), vecb = hsb.w / (fp32 ? 4 : 2);
+  const int64_t n = by_dst->n_edges;
+  const int step = walk_batch(fp32, hs.w, hs.g);
+  if (walks >> kWalkDq & 1) s.plan_a = plan_tiles(n, hs, step, vec, bwd_resident_ctas(dtype, hs, kWalkDq, use));
+  if (walks >> kWalkDqFused & 1)
+    s.plan_a_fused = plan_tiles(n, hs, step, 2 * vec + 1, bwd_resident_ctas(dtype, hs, kWalkDqFused, use < kReadBias ? use : kReadBias));
+  if (walks >> kWalkDkv & 1)
+    s.plan_b = plan_tiles(n, hsb, walk_batch(fp32, hsb.w, hsb.g), 2 * vecb, bwd_resident_ctas(dtype, hsb, kWalkDkv, use));
   size_t off = 0;
   s.stats = off; off += round_up(size_t(by_dst->n_rows) * heads * 8, 256);
   s.carry_a = off;
@@ -111,7 +116,7 @@ extern "C" int tgt_sparse_attn_scratch_bytes(const tgt_layout* by_dst, const tgt
         continue;
       if (!split_heads(heads, head_dim, dtype, wa, &a) || !split_heads(heads, head_dim, dtype, wb, &b)) continue;
       for (const int use : {kNoBias, kReadBias, kBiasGrad}) {
-        const size_t t = plan_bwd_scratch(by_dst, a, b, heads, dtype, use).total;
+        const size_t t = plan_bwd_scratch(by_dst, a, b, heads, dtype, use, 7).total;
         if (t > need) need = t;
       }
     }
@@ -215,7 +220,9 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
   const bool dbias_in_dkv = dbias != nullptr && (passes & 6) == 6;
   if (dbias_in_dkv) passes &= ~1;
   const BwdScratch sc = plan_bwd_scratch(by_dst, hs, hsb, heads, dtype,
-                                         bias == nullptr ? kNoBias : dbias_in_dkv ? kBiasGrad : kReadBias);
+                                         bias == nullptr ? kNoBias : dbias_in_dkv ? kBiasGrad : kReadBias,
+                                         (passes & 2 ? 1 << (dbias == nullptr || dbias_in_dkv ? kWalkDqFused : kWalkDq) : 0) |
+                                             (passes & 4 ? 1 << kWalkDkv : 0));
   if (scratch == nullptr || scratch_bytes < sc.total)
     return set_error(TGT_ERR_WORKSPACE, "scratch holds %zu bytes, %zu needed", scratch_bytes,
                      sc.total);
