@@ -8,6 +8,7 @@
 #include <pybind11/stl.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
 namespace py = pybind11;
@@ -374,6 +375,18 @@ at::Tensor attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor&
   return attention_over_rows(q, k, v, bias.value_or(at::Tensor()), graph, int(q.size(1)), int(q.size(2)));
 }
 
+// The plain call of sparse_graph_attention: no bias, a prebuilt graph, nobody tracing.  Nothing where any of its checks is
+// not clearly met: the caller goes through them one by one and words the errors.
+std::optional<at::Tensor> plain_attention(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                                          const std::shared_ptr<Graph>& graph) {
+  const bool plain = q.is_cuda() && k.is_cuda() && v.is_cuda() && q.dim() == 3 && q.sizes() == k.sizes() && q.sizes() == v.sizes() &&
+                     (q.scalar_type() == at::kFloat || q.scalar_type() == at::kBFloat16) && k.scalar_type() == q.scalar_type() &&
+                     v.scalar_type() == q.scalar_type() && q.size(0) == graph->n_rows && !torch::jit::tracer::isTracing();
+  if (!plain) return std::nullopt;
+  graph->poll();
+  return attention_over_rows(q, k, v, at::Tensor(), graph, int(q.size(1)), int(q.size(2)));
+}
+
 // The two passes without an autograd node, for callers that keep one of their own (torchgt_b200/sparse_attn.py).
 std::pair<at::Tensor, at::Tensor> forward_pass(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
                                                const std::optional<at::Tensor>& bias, const std::shared_ptr<Graph>& graph) {
@@ -441,6 +454,7 @@ PYBIND11_MODULE(_native, m) {
       .def("poll", &Graph::poll);
   m.def("take_gradients", &take_gradients, Unlocked());
   m.def("attention", &attention, Unlocked());
+  m.def("plain_attention", &plain_attention, Unlocked());
   m.def("attention_forward", &forward_pass, Unlocked());
   m.def("attention_backward", &backward_pass, Unlocked());
   bind_batching(m);

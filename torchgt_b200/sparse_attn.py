@@ -71,6 +71,10 @@ def sparse_graph_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     ``edge_index`` columns, shape [E] (shared by all heads) or [E, H]; it is added after the clamp.
     Returns [N, H, D].  Raises if the tensors are not on a CUDA device: there is no CPU path.
     """
+    if bias is None and type(edge_index) is SparseGraph:
+        out = _cabi.native().plain_attention(q, k, v, edge_index.native)
+        if out is not None:
+            return out
     if not (q.is_cuda and k.is_cuda and v.is_cuda):
         raise RuntimeError("torchgt_b200.sparse_graph_attention needs CUDA tensors (no CPU fallback)")
     if q.dim() != 3 or q.shape != k.shape or q.shape != v.shape:
