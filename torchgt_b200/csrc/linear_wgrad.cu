@@ -156,6 +156,12 @@ __global__ void __launch_bounds__(kWgThreads, 2) linear_wgrad_kernel(const __gri
       tc::commit(s_done + n % 2);
     }
     if (chunk + gridDim.x < chunks) load(chunk + gridDim.x);
+    // 64 x 64 at 320,000 rows 48.5 -> 44.1 us, with the sums; of the CTAs that read the same rows one each
+    if (tid == 0 && p.rows * (p.in + int64_t(p.count) * p.out) * 4 >= tc::kPrefetchFrom) {
+      const int64_t ahead = (chunk + 2 * int64_t(gridDim.x)) * kWgChunk;
+      if (tile == 0) tc::prefetch_rows(from, ahead, kWgChunk, p.rows, p.out);
+      if (blockIdx.y == 0) tc::prefetch_rows(p.x, ahead, kWgChunk, p.rows, p.in);
+    }
     if (n > 0) drain(n - 1);
   }
   if (n > 0) drain(n - 1);

@@ -69,6 +69,19 @@ __device__ __forceinline__ void multiply(uint32_t d, uint64_t a, uint64_t b, uin
       ::"r"(d), "l"(a), "l"(b), "r"(instr), "r"(uint32_t(add)) : "memory");
 }
 
+// Brings n of `rows` rows from `row` on into the L2 (rows of `width` values, a multiple of 4, from a 16-byte boundary on): the
+// kernels hold one step's rows in registers, which is not far enough ahead of memory.
+__device__ __forceinline__ void prefetch_rows(const float* from, int64_t row, int64_t n, int64_t rows, int width) {
+  const int64_t left = rows - row;
+  if (left <= 0) return;
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(from + row * width),
+               "r"(uint32_t((left < n ? left : n) * width * 4)) : "memory");
+}
+
+// Bytes of rows from which on they are taken not to be in the L2 (126 MB, shared with what was written meanwhile).  Shorter lists
+// lose by the prefetch: 64,001 rows of 64 x 64 12.0 -> 12.3 us.
+constexpr int64_t kPrefetchFrom = int64_t(64) << 20;
+
 // ---- completion ------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void barrier_init(uint64_t* bar) {   // by one thread
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_address(bar)) : "memory");
