@@ -42,15 +42,15 @@ namespace tgt {
 #ifndef TGT_UNROLL
 #define TGT_UNROLL 4
 #endif
-// Which walks use 32-byte lanes when nobody forces a lane width (see lane_bytes()).  Measured on B200
-// (fp32, 8-float heads, 64K-node batches and their 2-, 4- and 8-rank head slices, 870K-node batch): the
-// forward gains on 128-byte rows (55 -> 50 us), the dQ pass on 64- and 128-byte rows (86 -> 80 us,
-// 72 -> 62 us).  On 256-byte rows they tie at 64K nodes and lose 4-5 % at 870K nodes, where K and V no
-// longer fit the L2 and the higher occupancy of the 16-byte-lane kernels (64-72 registers) counts; both
-// lose on 32-byte rows, and the dK/dV pass, with twice the accumulators per lane, loses 10-40 % everywhere.
+// Which walks use 32-byte lanes when nobody forces a lane width (see lane_bytes()).  Measured on B200, 64,000 nodes, us with
+// 16- | 32-byte lanes: rows of 512 bytes (8 heads x 16) forward 68.0 | 59.8, backward 187 | 166, 16 heads x 8 with a bias per head
+// 78.6 | 64.5 and 217 | 205, of 384 (12 x 8) 59.1 | 56.3 and 178 | 165: half the lane groups and no exchange between the lanes of a
+// head.  Rows of 128 bytes 21.9 | 21.7 forward, dQ 3 us less, but not the dK/dV pass, which has twice the accumulators per lane.
+// Rows of 256 bytes 31.7 | 33.5 and 89.6 | 96.2 (870,000 nodes 797 | 849 and 2440 | 2556), where two lane groups per warp at 56 to
+// 72 registers count for more; 64 bytes 15.7 | 19.8 and 39.7 | 56.5; 32 bytes 73 | 137 and 194 | 239.
 #ifndef TGT_WIDE_DEFAULT
-#define TGT_WIDE_DEFAULT(pass, row_bytes) \
-  ((pass) != kPassDkv && (row_bytes) <= 128 && (row_bytes) >= ((pass) == kPassDq ? 64 : 128))
+#define TGT_WIDE_DEFAULT(pass, row_bytes, lanes, n_edges) \
+  ((row_bytes) > 256 ? (lanes) >= 4 && (n_edges) >= kWideFrom : ((pass) != kPassDkv && (row_bytes) == 128))
 #endif
 // Edges per batch of the walk with 32-byte lanes (their operands take twice the registers).
 #ifndef TGT_WIDE_UNROLL
@@ -528,13 +528,15 @@ int lane_mode();
 
 // Bytes per lane for heads of head_dim elements.  32-byte lanes need heads that are whole multiples of
 // 32 bytes and 32-byte aligned tensors and strides (`can32`).
-inline int lane_bytes(int heads, int head_dim, int dtype, bool can32, int pass) {
+inline int lane_bytes(int heads, int head_dim, int dtype, bool can32, int pass, int64_t n_edges) {
   const int head_bytes = head_dim * (dtype == TGT_F32 ? 4 : 2);
   if (!can32 || dtype != TGT_F32 || head_bytes % 32 != 0 || head_bytes > 128) return 16;
   const int mode = lane_mode();
   if (mode == 1) return 16;
   if (mode == 2) return 32;
-  return TGT_WIDE_DEFAULT(pass, heads * head_bytes) ? 32 : 16;
+  int group = head_bytes / 32;   // lanes of a group of 32-byte lanes, as split_heads makes them
+  for (int hpg = 1; hpg * 2 * (head_bytes / 32) <= 32 && heads % (hpg * 2) == 0; hpg *= 2) group *= 2;
+  return TGT_WIDE_DEFAULT(pass, heads * head_bytes, group, n_edges) ? 32 : 16;
 }
 
 // Returns false when (heads, head_dim, dtype) cannot be mapped onto lanes of w bytes.
