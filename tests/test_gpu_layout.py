@@ -288,7 +288,8 @@ def test_a_graph_from_an_int32_list_allocates_no_narrow_copy():
     assert torch.cuda.max_memory_allocated() - before < 3 * 4 * n_edges + need.value + (6 << 20)
 
 
-@pytest.mark.parametrize("n_rows,n_edges", [(1, 1), (3, 2), (40, 63), (40, 64), (40, 65), (70000, 200003)])
+@pytest.mark.parametrize("n_rows,n_edges", [(1, 1), (3, 2), (40, 65), (70000, 200003), (5000, (1 << 20) - 1), (5000, 1 << 20),
+                                            (70000, (1 << 20) + 63), (900, (1 << 20) + 64), (70000, (1 << 20) + 65)])
 def test_second_orientation_from_what_the_first_kept(n_rows, n_edges):
     """The sources' layout from the endpoints the first build kept (same stream), from the list itself (another stream, as
     before), and the CPU's stable sort; rows without edges in runs of every length up to thousands."""

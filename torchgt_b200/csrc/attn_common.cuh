@@ -48,6 +48,9 @@ namespace tgt {
 // head.  Rows of 128 bytes 21.9 | 21.7 forward, dQ 3 us less, but not the dK/dV pass, which has twice the accumulators per lane.
 // Rows of 256 bytes 31.7 | 33.5 and 89.6 | 96.2 (870,000 nodes 797 | 849 and 2440 | 2556), where two lane groups per warp at 56 to
 // 72 registers count for more; 64 bytes 15.7 | 19.8 and 39.7 | 56.5; 32 bytes 73 | 137 and 194 | 239.
+// Wide rows in groups of two lanes (10 heads x 8) 61.1 | 70.5 and 184 | 214.  Short lists wait for the lanes' longer chains
+// (8 x 16: 45,000 edges 9.8 | 10.6 and 26.4 | 35.1, 197,000 26.3 | 24.3 and 75.7 | 75.5, 263,000 35.3 | 31.9 and 92.3 | 91.1).
+constexpr int64_t kWideFrom = 250000;   // edges
 #ifndef TGT_WIDE_DEFAULT
 #define TGT_WIDE_DEFAULT(pass, row_bytes, lanes, n_edges) \
   ((row_bytes) > 256 ? (lanes) >= 4 && (n_edges) >= kWideFrom : ((pass) != kPassDkv && (row_bytes) == 128))
