@@ -50,10 +50,11 @@ namespace tgt {
 // 72 registers count for more; 64 bytes 15.7 | 19.8 and 39.7 | 56.5; 32 bytes 73 | 137 and 194 | 239.
 // Wide rows in groups of two lanes (10 heads x 8) 61.1 | 70.5 and 184 | 214.  Short lists wait for the lanes' longer chains
 // (8 x 16: 45,000 edges 9.8 | 10.6 and 26.4 | 35.1, 197,000 26.3 | 24.3 and 75.7 | 75.5, 263,000 35.3 | 31.9 and 92.3 | 91.1).
+// Groups of four lanes pay without a bias only (12 x 8 with a bias per head 69.8 | 115 and 214 | 229).
 constexpr int64_t kWideFrom = 250000;   // edges
 #ifndef TGT_WIDE_DEFAULT
-#define TGT_WIDE_DEFAULT(pass, row_bytes, lanes, n_edges) \
-  ((row_bytes) > 256 ? (lanes) >= 4 && (n_edges) >= kWideFrom : ((pass) != kPassDkv && (row_bytes) == 128))
+#define TGT_WIDE_DEFAULT(pass, row_bytes, lanes, n_edges, biased) \
+  ((row_bytes) > 256 ? (lanes) >= ((biased) ? 8 : 4) && (n_edges) >= kWideFrom : ((pass) != kPassDkv && (row_bytes) == 128))
 #endif
 // Edges per batch of the walk with 32-byte lanes (their operands take twice the registers).
 #ifndef TGT_WIDE_UNROLL
@@ -491,7 +492,9 @@ __device__ __forceinline__ void finish_crossing_rows(const SegWalk& w, const Pol
 #pragma unroll
     for (int a = 0; a < NACC; ++a) s_part[a * kCrossingThreads + threadIdx.x] = acc[a];
     __syncthreads();
-    for (int half = NG / 2; half >= 1; half >>= 1) {   // halving tree
+    int half = NG / 2;
+    while (half > n) half >>= 1;     // the groups behind the row's n + 1 carries have nothing
+    for (; half >= 1; half >>= 1) {  // halving tree
       if (g < half) {
 #pragma unroll
         for (int a = 0; a < NACC; ++a)
@@ -531,7 +534,7 @@ int lane_mode();
 
 // Bytes per lane for heads of head_dim elements.  32-byte lanes need heads that are whole multiples of
 // 32 bytes and 32-byte aligned tensors and strides (`can32`).
-inline int lane_bytes(int heads, int head_dim, int dtype, bool can32, int pass, int64_t n_edges) {
+inline int lane_bytes(int heads, int head_dim, int dtype, bool can32, int pass, int64_t n_edges, bool biased) {
   const int head_bytes = head_dim * (dtype == TGT_F32 ? 4 : 2);
   if (!can32 || dtype != TGT_F32 || head_bytes % 32 != 0 || head_bytes > 128) return 16;
   const int mode = lane_mode();
@@ -539,7 +542,7 @@ inline int lane_bytes(int heads, int head_dim, int dtype, bool can32, int pass, 
   if (mode == 2) return 32;
   int group = head_bytes / 32;   // lanes of a group of 32-byte lanes, as split_heads makes them
   for (int hpg = 1; hpg * 2 * (head_bytes / 32) <= 32 && heads % (hpg * 2) == 0; hpg *= 2) group *= 2;
-  return TGT_WIDE_DEFAULT(pass, heads * head_bytes, group, n_edges) ? 32 : 16;
+  return TGT_WIDE_DEFAULT(pass, heads * head_bytes, group, n_edges, biased) ? 32 : 16;
 }
 
 // Returns false when (heads, head_dim, dtype) cannot be mapped onto lanes of w bytes.

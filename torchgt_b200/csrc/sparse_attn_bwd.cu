@@ -111,8 +111,8 @@ extern "C" int tgt_sparse_attn_scratch_bytes(const tgt_layout* by_dst, const tgt
   for (int wa = 16; wa <= 32; wa += 16)
     for (int wb = 16; wb <= 32; wb += 16) {
       HeadSplit a, b;
-      if ((wa == 32 && lane_bytes(heads, head_dim, dtype, true, kPassDq, by_dst->n_edges) != 32) ||
-          (wb == 32 && lane_bytes(heads, head_dim, dtype, true, kPassDkv, by_dst->n_edges) != 32))
+      if ((wa == 32 && lane_bytes(heads, head_dim, dtype, true, kPassDq, by_dst->n_edges, false) != 32) ||
+          (wb == 32 && lane_bytes(heads, head_dim, dtype, true, kPassDkv, by_dst->n_edges, false) != 32))
         continue;
       if (!split_heads(heads, head_dim, dtype, wa, &a) || !split_heads(heads, head_dim, dtype, wb, &b)) continue;
       for (const int use : {kNoBias, kReadBias, kBiasGrad}) {
@@ -175,8 +175,8 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
                      aligned32(dk) && aligned32(dv) && dout_row_bytes % 32 == 0 && q_row_bytes % 32 == 0 &&
                      kv_row_bytes % 32 == 0;
   HeadSplit hs, hsb;   // lane layouts of pass A (dQ) and pass B (dK/dV)
-  if (!split_heads(heads, head_dim, dtype, lane_bytes(heads, head_dim, dtype, can32, kPassDq, by_dst->n_edges), &hs) ||
-      !split_heads(heads, head_dim, dtype, lane_bytes(heads, head_dim, dtype, can32, kPassDkv, by_dst->n_edges), &hsb))
+  if (!split_heads(heads, head_dim, dtype, lane_bytes(heads, head_dim, dtype, can32, kPassDq, by_dst->n_edges, bias != nullptr), &hs) ||
+      !split_heads(heads, head_dim, dtype, lane_bytes(heads, head_dim, dtype, can32, kPassDkv, by_dst->n_edges, bias != nullptr), &hsb))
     return set_error(TGT_ERR_UNSUPPORTED,
                      "heads=%d head_dim=%d dtype=%d: head_dim must be a power of two multiple of "
                      "16 bytes, at most 512 bytes per head",

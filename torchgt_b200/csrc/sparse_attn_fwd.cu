@@ -177,7 +177,7 @@ size_t fwd_scratch_bytes_w(const tgt_layout* L, int heads, int head_dim, int dty
 // on pointer alignment, which the size query does not see).
 size_t fwd_scratch_bytes(const tgt_layout* L, int heads, int head_dim, int dtype) {
   size_t need = fwd_scratch_bytes_w(L, heads, head_dim, dtype, 16);
-  if (lane_bytes(heads, head_dim, dtype, true, kPassFwd, L->n_edges) == 32) {
+  if (lane_bytes(heads, head_dim, dtype, true, kPassFwd, L->n_edges, false) == 32) {
     const size_t wide = fwd_scratch_bytes_w(L, heads, head_dim, dtype, 32);
     if (wide > need) need = wide;
   }
@@ -208,7 +208,7 @@ extern "C" int tgt_sparse_attn_fwd_strided(const void* q, int64_t q_row_bytes, c
   const bool can32 = aligned32(q) && aligned32(k) && aligned32(v) && aligned32(out) && q_row_bytes % 32 == 0 &&
                      kv_row_bytes % 32 == 0;
   HeadSplit hs;
-  if (!split_heads(heads, head_dim, dtype, lane_bytes(heads, head_dim, dtype, can32, kPassFwd, by_dst->n_edges), &hs))
+  if (!split_heads(heads, head_dim, dtype, lane_bytes(heads, head_dim, dtype, can32, kPassFwd, by_dst->n_edges, bias != nullptr), &hs))
     return set_error(TGT_ERR_UNSUPPORTED,
                      "heads=%d head_dim=%d dtype=%d: head_dim must be a power of two multiple of "
                      "16 bytes, at most 512 bytes per head",
