@@ -50,8 +50,8 @@ ROTATING_SETS = 4
 
 def ncu_traffic(workload, dtype_name):
     """dram__bytes_read.sum + dram__bytes_write.sum per launch of each phase, as recorded next to the ncu
-    summary of that workload under profiles/ (the dQ phase includes the row-statistics kernel); None when
-    no capture of this workload is on file."""
+    summary of that workload under profiles/ (taken before the dQ phase was one kernel); None when no capture of this
+    workload, or of a phase, is on file."""
     path = ROOT / "profiles" / f"sparse_attn_{workload}_{dtype_name}_traffic.json"
     try:
         return {k: float(v) for k, v in json.loads(path.read_text())["dram_bytes_per_launch"].items()}
@@ -76,7 +76,7 @@ def algorithmic_bytes(n_rows, n_edges, heads, head_dim, elem, bias_bytes):
     fwd = 2 * n_rows * r + n_edges * (2 * r + bias_bytes)
     dq = 4 * n_rows * r + n_edges * (2 * r + bias_bytes)
     dkv = 4 * n_rows * r + n_edges * (2 * r + bias_bytes)
-    return {"fwd_kernel": fwd, "bwd_dq_kernel": dq, "bwd_dkv_kernel": dkv}
+    return {"fwd_kernel": fwd, "bwd_dq_fused_kernel": dq, "bwd_dkv_kernel": dkv}
 
 
 class ClockSampler:
@@ -499,15 +499,15 @@ class OpBuffers:
             1 if self.bias is not None else 0, self.graph.by_dst.byref(), p(self.out), p(self.z), HEADS, HEAD_DIM,
             self.code, p(self.scratch_f), self.scratch_f.numel(), stream))
 
-    def bwd(self, stream, passes):
+    def bwd(self, stream, passes, with_dbias=True):
         from torchgt_b200 import _cabi
         lib = _cabi.load()
         p = lambda t: None if t is None else t.data_ptr()
         _cabi.check(lib.tgt_sparse_attn_bwd_strided(
             p(self.dout), self.row_bytes, p(self.q), self.row_bytes, p(self.k), p(self.v), self.kv_row_bytes,
             p(self.bias), 1 if self.bias is not None else 0, p(self.out), p(self.z), self.graph.by_dst.byref(),
-            self.graph.by_src.byref(), p(self.dq), p(self.dk), p(self.dv), p(self.dbias), HEADS, HEAD_DIM, self.code,
-            p(self.scratch_b), self.scratch_b.numel(), stream, passes))
+            self.graph.by_src.byref(), p(self.dq), p(self.dk), p(self.dv), p(self.dbias) if with_dbias else None, HEADS, HEAD_DIM,
+            self.code, p(self.scratch_b), self.scratch_b.numel(), stream, passes))
 
 
 def capture(fn):
@@ -523,12 +523,10 @@ def capture(fn):
     return g
 
 
-def kernels_per_step(graph, with_dbias=True, ranks=1, elem=4):
-    # forward, dQ pass, dK/dV pass: one kernel each, plus a second small kernel each where rows are at most
-    # 64 bytes wide (there the rows that cross tiles are finished separately); the row-statistics pre-pass
-    # runs only when dbias is computed
-    row_bytes = HEADS // max(1, ranks) * HEAD_DIM * elem
-    return 3 * (2 if row_bytes <= 64 else 1) + (1 if with_dbias else 0)
+def kernels_per_step():
+    """Forward, dQ pass, dK/dV pass: a walk each, and the kernel that finishes the rows that cross its tiles (dbias is written
+    by the dK/dV pass)."""
+    return 6
 
 
 def measure_device_resident(sets, steps, warmup):
@@ -537,7 +535,7 @@ def measure_device_resident(sets, steps, warmup):
     import copy
     n_sets = len(sets)
     step_graphs = [capture(lambda s, b=b: (b.fwd(s), b.bwd(s, 7 if b.dbias is not None else 6))) for b in sets]
-    phase_graphs = [[capture(lambda s, b=b: b.fwd(s)), capture(lambda s, b=b: b.bwd(s, 3 if b.dbias is not None else 2)),
+    phase_graphs = [[capture(lambda s, b=b: b.fwd(s)), capture(lambda s, b=b: b.bwd(s, 2, with_dbias=False)),
                      capture(lambda s, b=b: b.bwd(s, 4))] for b in sets]
     torch.cuda.synchronize()
     start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -555,7 +553,7 @@ def measure_device_resident(sets, steps, warmup):
 
     # ---- device-resident throughput: K back-to-back steps over rotating input sets -------------------
     ms_per_step = timed(step_graphs)
-    # ---- the same step with the bias as a plain input (no dbias: no statistics pre-pass) ---------------
+    # ---- the same step with the bias as a plain input (no dbias) ---------------
     plain_sets = []
     for b in sets:
         b2 = copy.copy(b)
@@ -565,7 +563,7 @@ def measure_device_resident(sets, steps, warmup):
     ms_no_dbias = timed(plain_graphs)
     plain_graphs.clear()
     # ---- per-phase durations (each phase its own graph, events around every replay) ------------------
-    names = ["fwd_kernel", "bwd_dq_kernel", "bwd_dkv_kernel"]
+    names = ["fwd_kernel", "bwd_dq_fused_kernel", "bwd_dkv_kernel"]
     phase_steps = min(steps, 200)
     evs = [[torch.cuda.Event(enable_timing=True) for _ in range(4)] for _ in range(phase_steps)]
     for i in range(phase_steps):
@@ -757,7 +755,7 @@ def run_single_gpu(args, dtype):
                 "one_step_at_a_time_ms": results["full"] * 1e3,
                 "graph_resident_value": n_edges / results["graph_resident"],
                 "graph_resident_ms_per_step": results["graph_resident"] * 1e3},
-        "gpu_launches": kernels_per_step(graph, elem=elem) * args.steps,
+        "gpu_launches": kernels_per_step() * args.steps,
         "roofline": {"bound": "hbm", "kernel": dominant, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": f"of {peak_kind}",
                      "traffic": (ncu_traffic(args.workload, args.dtype) or {}).get(dominant),
@@ -1087,7 +1085,7 @@ def run_multi_gpu(args, dtype, rank, world):
         step_bytes = sum(bytes_.values())
         per_rank_io = 4 * (L + 1) * HEADS * HEAD_DIM * elem
         # kernels: the attention phases; per step two pushes, two pulls, four barriers, one global-row kernel
-        launches = kernels_per_step(graph, with_dbias=False, ranks=world, elem=elem) + (9 if px is not None else 12)
+        launches = kernels_per_step() + (9 if px is not None else 12)
         line = {
             "metric": "sparse_graph_attention_fwd_bwd_edges_per_s", "value": n_edges / (ms_per_step * 1e-3),
             "unit": "edges/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
