@@ -434,9 +434,13 @@ __device__ __forceinline__ void walk_tile(const SegWalk& w, const Policy& pol, i
 // it; rows of more than kGroupTiles further tiles are taken by the whole CTA.  Every sum has a fixed order.  Launched as
 // the dependent of the walk, and what does not depend on the walk is read before it has ended.
 constexpr int kGroupTiles = 8;
-constexpr int kCrossingThreads = 512;   // a row of every eighth edge has over a hundred carries at 64,000 nodes
+// Threads of its CTAs.  A row of every eighth edge has over a hundred carries at 64,000 nodes, which wide groups need many
+// slots for; narrow ones have enough of them, and CTAs of 512 threads would hold hundreds of tiles each (64,000 nodes backward, 512 |
+// 128 threads: one bf16 head of 8 58.1 | 46.1 us, two with a bias gradient 52.1 | 44.1, four fp32 heads 63.7 | 61.3).
+constexpr int crossing_threads(int g) { return g <= 4 ? 128 : 512; }
 template <int G, class Policy>
 __device__ __forceinline__ void finish_crossing_rows(const SegWalk& w, const Policy& pol) {
+  constexpr int kCrossingThreads = crossing_threads(G);
   constexpr int NG = kCrossingThreads / G, NACC = Policy::NACC;
   __shared__ float s_part[kCrossingThreads * NACC];
   __shared__ int s_many[NG][3], s_n;   // rows of many tiles: first tile, further tiles, row
@@ -512,7 +516,7 @@ __device__ __forceinline__ void finish_crossing_rows(const SegWalk& w, const Pol
 }
 // CTAs of that kernel in x for lane groups of g lanes.
 inline unsigned crossing_ctas(const SegWalk& w, int g) {
-  const int ng = kCrossingThreads / g;
+  const int ng = crossing_threads(g) / g;
   return unsigned((w.n_tiles + ng - 1) / ng);
 }
 

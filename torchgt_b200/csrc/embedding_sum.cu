@@ -98,7 +98,7 @@ __global__ void TGT_WALK_BOUNDS embedding_grad_kernel(const SumParams p) {
 }
 
 template <int G>
-__global__ void __launch_bounds__(kCrossingThreads) embedding_grad_crossing_kernel(const SumParams p) {
+__global__ void __launch_bounds__(crossing_threads(G)) embedding_grad_crossing_kernel(const SumParams p) {
   const SumPolicy<G> pol{p.grad, p.out, p.skip, p.features, p.share, threadIdx.x % G};
   finish_crossing_rows<G, SumPolicy<G>>(p.walk, pol);
 }
@@ -107,7 +107,7 @@ template <int G>
 int launch_grad(const SumParams& p, unsigned ctas, cudaStream_t stream) {
   embedding_grad_kernel<G><<<ctas, kBlockThreads, 0, stream>>>(p);
   if (p.walk.n_tiles > 1)
-    TGT_CHECK_CUDA(launch_chained(embedding_grad_crossing_kernel<G>, dim3(crossing_ctas(p.walk, G)), kCrossingThreads, stream,
+    TGT_CHECK_CUDA(launch_chained(embedding_grad_crossing_kernel<G>, dim3(crossing_ctas(p.walk, G)), crossing_threads(G), stream,
                                   kLinkStitch, p));
   TGT_CHECK_CUDA(cudaGetLastError());
   return TGT_OK;

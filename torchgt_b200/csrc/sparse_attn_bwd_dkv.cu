@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(kBlockThreads, sizeof(T) == 2 && BIAS == kBias
 }
 
 template <typename T, int W, int LPH, int G, int BIAS>
-__global__ void __launch_bounds__(kCrossingThreads) bwd_dkv_stitch_kernel(const BwdParams p) {
+__global__ void __launch_bounds__(crossing_threads(G)) bwd_dkv_stitch_kernel(const BwdParams p) {
   using Policy = DkvPolicy<T, W, LPH, G, BIAS>;
   const Policy pol = make_dkv_policy<T, W, LPH, G, BIAS>(p);
   finish_crossing_rows<G, Policy>(p.walk, pol);
@@ -163,7 +163,7 @@ bool launch_dkv(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, i
       launch_chained(bwd_dkv_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value>, grid, kBlockThreads, stream, link, p);
     });
     if (p.walk.n_tiles > 1)
-      launch_chained(bwd_dkv_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), kCrossingThreads, stream, kLinkStitch, p);
+      launch_chained(bwd_dkv_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), crossing_threads(S::G), stream, kLinkStitch, p);
   });
 }
 

@@ -131,7 +131,7 @@ __global__ void TGT_WALK_BOUNDS bwd_dq_kernel(const BwdParams p) {
 }
 
 template <typename T, int W, int LPH, int G>
-__global__ void __launch_bounds__(kCrossingThreads) bwd_dq_stitch_kernel(const BwdParams p) {
+__global__ void __launch_bounds__(crossing_threads(G)) bwd_dq_stitch_kernel(const BwdParams p) {
   using Policy = DqPolicy<T, W, LPH, G>;
   const Policy pol = make_dq_policy<T, W, LPH, G>(p);
   finish_crossing_rows<G, Policy>(p.walk, pol);
@@ -146,7 +146,7 @@ bool launch_dq(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, in
     using S = decltype(sh);
     launch_chained(bwd_dq_kernel<typename S::T, S::W, S::LPH, S::G>, grid, kBlockThreads, stream, link, p);
     if (p.walk.n_tiles > 1)
-      launch_chained(bwd_dq_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(crossing_ctas(p.walk, S::G), grid.y), kCrossingThreads, stream, kLinkStitch, p);
+      launch_chained(bwd_dq_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(crossing_ctas(p.walk, S::G), grid.y), crossing_threads(S::G), stream, kLinkStitch, p);
   });
 }
 

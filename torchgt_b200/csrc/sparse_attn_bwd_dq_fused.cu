@@ -125,7 +125,7 @@ __global__ void TGT_WALK_BOUNDS bwd_dq_fused_kernel(const BwdParams p) {
 }
 
 template <typename T, int W, int LPH, int G, int BIAS>
-__global__ void __launch_bounds__(kCrossingThreads) bwd_dq_fused_stitch_kernel(const BwdParams p) {
+__global__ void __launch_bounds__(crossing_threads(G)) bwd_dq_fused_stitch_kernel(const BwdParams p) {
   using Policy = DqFusedPolicy<T, W, LPH, G, BIAS>;
   const Policy pol = make_dq_fused_policy<T, W, LPH, G, BIAS>(p);
   finish_crossing_rows<G, Policy>(p.walk, pol);
@@ -142,7 +142,7 @@ bool launch_dq_fused(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 gr
       launch_chained(bwd_dq_fused_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value>, grid, kBlockThreads, stream, link, p);
     });
     if (p.walk.n_tiles > 1)
-      launch_chained(bwd_dq_fused_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), kCrossingThreads, stream, kLinkStitch, p);
+      launch_chained(bwd_dq_fused_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), crossing_threads(S::G), stream, kLinkStitch, p);
   });
 }
 

@@ -127,7 +127,7 @@ __global__ void TGT_WALK_BOUNDS fwd_kernel(const FwdParams p) {
 }
 
 template <typename T, int W, int LPH, int G, int BIAS>
-__global__ void __launch_bounds__(kCrossingThreads) fwd_stitch_kernel(const FwdParams p) {
+__global__ void __launch_bounds__(crossing_threads(G)) fwd_stitch_kernel(const FwdParams p) {
   using Policy = FwdPolicy<T, W, LPH, G, BIAS>;
   const Policy pol = make_policy<T, W, LPH, G, BIAS>(p);
   finish_crossing_rows<G, Policy>(p.walk, pol);
@@ -262,7 +262,7 @@ extern "C" int tgt_sparse_attn_fwd_strided(const void* q, int64_t q_row_bytes, c
       fwd_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value><<<grid, kBlockThreads, 0, stream>>>(p);
     });
     if (tp.n_tiles > 1)
-      launch_chained(fwd_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), kCrossingThreads, stream, kLinkStitch, p);
+      launch_chained(fwd_stitch_kernel<typename S::T, S::W, S::LPH, S::G, kNoBias>, dim3(crossing_ctas(p.walk, S::G), grid.y), crossing_threads(S::G), stream, kLinkStitch, p);
   });
   if (!built) return set_error(TGT_ERR_UNSUPPORTED, "no kernel is built for this head layout");
   TGT_CHECK_CUDA(cudaGetLastError());
