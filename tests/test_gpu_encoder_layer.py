@@ -69,3 +69,39 @@ def test_what_can_be_noticed_goes_through_the_modules():
         assert call() is None
     with pytest.raises(ValueError, match="rows"):
         layer._native_layer(x[:, 1:], None, graph, "sparse")
+
+
+@pytest.mark.parametrize("nodes", [300, 1500])
+@pytest.mark.parametrize("name", ["linear_q", "linear_k", "linear_v"])
+@pytest.mark.parametrize("width", [32, 128])
+def test_projections_of_unequal_widths_are_refused(name, width, nodes):
+    """The kernels read and write rows of heads * head_dim values: a pruned or replaced projection is refused by the modules,
+    and by the host module, whoever calls it, before the attention is launched."""
+    from torchgt_b200 import _cabi
+    from torchgt_b200.linear import Linear
+    layer, graph, x, _ = _layer(64, 8, 64, nodes)
+    mha = layer.self_attention
+    setattr(mha, name, Linear(64, width).cuda())
+    assert layer._native_layer(x, None, graph, "sparse") is None
+    with pytest.raises(ValueError):
+        layer(x, None, graph, "sparse")
+    native = _cabi.native()
+    modules = (layer.self_attention_norm, mha.linear_q, mha.linear_k, mha.linear_v, mha.output_layer, layer.ffn_norm,
+               layer.ffn.layer1, layer.ffn.layer2)
+    tensors = [t for m in modules for t in (m.weight, m.bias)]
+    with pytest.raises(ValueError, match="share the shape"):
+        native.encoder_layer(x, graph.native, 8, 8, tensors, 1e-5, 1e-5)
+
+
+@pytest.mark.parametrize("wrong", ["rows", "heads", "dtype"])
+def test_the_attention_itself_refuses_rows_that_are_not_the_graphs(wrong):
+    from torchgt_b200 import _cabi
+    _, graph, _, _ = _layer(64, 8, 64, 300)
+    native = _cabi.native()
+    good = torch.randn(300, 8, 8, device="cuda")
+    other = {"rows": good[:299], "heads": good[:, :4], "dtype": good.bfloat16()}[wrong]
+    calls = [(other, good, good), (good, other, good), (good, good, other)] + ([(other,) * 3] if wrong == "rows" else [])
+    for q, k, v in calls:
+        for run in (lambda: native.attention(q, k, v, None, graph.native), lambda: native.attention_forward(q, k, v, None, graph.native)):
+            with pytest.raises(TypeError if wrong == "dtype" else ValueError):
+                run()

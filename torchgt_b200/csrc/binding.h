@@ -120,7 +120,8 @@ void attention_backward(Graph& g, const at::Tensor& dout, const at::Tensor& q, c
                         const at::Tensor& dk, const at::Tensor& dv, const at::Tensor& dbias, int heads, int head_dim,
                         int dtype);
 
-// The attention as one autograd node: q, k and v of any one shape that is graph->n_rows rows of heads * head_dim values
+// The attention as one autograd node: q, k and v of any one shape that is graph->n_rows rows of heads * head_dim values (a
+// ValueError otherwise)
 at::Tensor attention_over_rows(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias,
                                const std::shared_ptr<Graph>& graph, int heads, int head_dim);
 

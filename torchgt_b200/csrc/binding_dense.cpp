@@ -669,7 +669,6 @@ at::Tensor encoder_layer(const at::Tensor& x, const std::shared_ptr<Graph>& grap
   auto weight = [&p](int i) -> const at::Tensor& { return *p[2 * i]; };
   const at::Tensor y = layer_norm(x, weight(0), *p[1], eps);
   const std::vector<at::Tensor> qkv = linear3(y, {weight(1), weight(2), weight(3)}, {p[3], p[5], p[7]});
-  TORCH_CHECK(qkv[0].size(-1) == int64_t(heads) * head_dim, "the projections are not heads * head_dim wide");
   const at::Tensor attended = attention_over_rows(qkv[0], qkv[1], qkv[2], at::Tensor(), graph, heads, head_dim);
   const auto [normed, sum] = add_layer_norm(x, tgt_host::linear(attended, weight(4), p[9]), weight(5), *p[11], ffn_eps, true);
   return feed_forward(normed, weight(6), *p[13], weight(7), *p[15], "gelu", sum);

@@ -123,7 +123,8 @@ class EncoderLayer(nn.Module):
     def _native_layer(self, x, attn_bias, edge_index, attn_type):
         """The whole layer as one call into the host module: the operations below, without a return to Python between
         them.  None where somebody could notice: sequence parallelism, a dropout that drops, subclassed, replaced or hooked
-        modules, missing biases, tracing, compiling, autocast, tensor subclasses, other dtypes and devices."""
+        modules, missing biases, projections of another width, tracing, compiling, autocast, tensor subclasses, other dtypes
+        and devices."""
         if attn_type != "sparse" or attn_bias is not None or edge_index is None:
             return None
         if not (x.is_cuda and x.dtype == torch.float32 and x.dim() == 3):
@@ -145,6 +146,9 @@ class EncoderLayer(nn.Module):
             return None
         tensors = [m._parameters.get(name) for m in layers for name in ("weight", "bias")]
         if any(t is None for t in tensors) or not plain_call(x, *tensors):
+            return None
+        width = mha.num_heads * mha.att_size     # other projections: the modules say what is wrong
+        if not tensors[2].shape[0] == tensors[4].shape[0] == tensors[6].shape[0] == width:
             return None
         graph = graph_for(edge_index, x.size(0) * x.size(1))
         graph.native.poll()
