@@ -449,6 +449,26 @@ def test_dependent_launches_change_no_bit(heads, head_dim, dtype, with_bias):
                                TOL_F32 if dtype == torch.float32 else TOL_BF16)
 
 
+@pytest.mark.parametrize("heads,head_dim", [(8, 8), (4, 16), (8, 16), (16, 8), (4, 8), (2, 8), (1, 8), (12, 8), (2, 32)])
+def test_a_score_has_the_same_bits_in_every_pass(heads, head_dim):
+    """Rows of one edge in and one out: dV = w / (w + 1e-6) dO, whose relative error is that of an addition, a division and
+    two products, 4 * 2^-24 of each value, where the weight has the forward's bits.  A score that is off by an ulp of its
+    own (4.8e-7 for scores over 4, clamped at 5) moves the weight by as much."""
+    n = 4000
+    gen = torch.Generator().manual_seed(heads * head_dim)
+    ei = torch.stack([torch.randperm(n, generator=gen), torch.arange(n)])
+    q, k, v, dout = (1.5 * torch.randn(n, heads, head_dim, generator=gen) for _ in range(4))
+    res = _run_cuda(q, k, v, ei, dout)
+    s, d = ei
+    raw = (k[s].double() * q[d].double()).sum(-1) / head_dim ** 0.5
+    w = raw.clamp(-5, 5).exp()
+    want = torch.empty(n, heads, head_dim, dtype=torch.float64)
+    want[s] = (w / (w + 1e-6))[..., None] * dout[d].double()
+    off = (res["dv"].cpu().double() - want).abs() / want.abs()
+    # w / (w + 1e-6) moves by at most 1e-6 / w, 1.5e-4, of what moves w
+    assert float(off.max()) <= 4.01 * 2.0 ** -24, float(off.max())
+
+
 @pytest.mark.parametrize("heads,dtype", [(8, torch.float32), (1, torch.float32), (8, torch.bfloat16)])
 @pytest.mark.parametrize("rows,edges", [(200_003, 37), (200_003, 3000), (513, 1)])
 def test_rows_far_beyond_the_edges_are_zero_filled(heads, dtype, rows, edges):

@@ -152,6 +152,9 @@ inline int choose_ge(int64_t n_edges, int g, int step, int ctas_per_sm) {
 // rounded as by fmaf) where that pays: everywhere in bf16 (16 heads x 8 at 64K nodes, forward 48.0 -> 45.5 us, backward
 // 144 -> 140) and in the fp32 forward (870K nodes 839 -> 781 us).  The fp32 gradient passes keep single ones: operands in
 // even register pairs cost them a resident CTA per SM (64K step with 8 heads x 8, backward 89.7 against 93.3 us).
+// Either way the even and the odd positions are summed apart: a score has the same bits in every pass, and what rounds it
+// cancels between an edge's weight and the sum of its row's weights.  With one running sum in the gradient passes and two in the
+// forward rows of one edge had dQ off by 3.5e-7 (2-norm, relative) and dV by 8.9e-8, not 2.3e-7 and 5.6e-8.
 template <bool PAIRS, int VEC>
 __device__ __forceinline__ float dot(const float (&a)[VEC], const float (&b)[VEC]) {
   if constexpr (PAIRS) {
@@ -160,10 +163,13 @@ __device__ __forceinline__ float dot(const float (&a)[VEC], const float (&b)[VEC
     for (int j = 0; j < VEC; j += 2) s = __ffma2_rn(make_float2(a[j], a[j + 1]), make_float2(b[j], b[j + 1]), s);
     return s.x + s.y;
   }
-  float s = 0.f;
+  float even = 0.f, odd = 0.f;
 #pragma unroll
-  for (int j = 0; j < VEC; ++j) s = fmaf(a[j], b[j], s);
-  return s;
+  for (int j = 0; j < VEC; j += 2) {
+    even = fmaf(a[j], b[j], even);
+    odd = fmaf(a[j + 1], b[j + 1], odd);
+  }
+  return even + odd;
 }
 
 // acc[AT + j] += w * x[j]
