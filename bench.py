@@ -523,10 +523,10 @@ def capture(fn):
     return g
 
 
-def kernels_per_step():
+def kernels_per_step(dbias, dtype):
     """Forward, dQ pass, dK/dV pass: a walk each, and the kernel that finishes the rows that cross its tiles (dbias is written
-    by the dK/dV pass)."""
-    return 6
+    by the dK/dV pass); in fp32 the row statistics are a kernel of their own when dbias is wanted."""
+    return 7 if dbias and dtype == torch.float32 else 6
 
 
 def measure_device_resident(sets, steps, warmup):
@@ -755,7 +755,7 @@ def run_single_gpu(args, dtype):
                 "one_step_at_a_time_ms": results["full"] * 1e3,
                 "graph_resident_value": n_edges / results["graph_resident"],
                 "graph_resident_ms_per_step": results["graph_resident"] * 1e3},
-        "gpu_launches": kernels_per_step() * args.steps,
+        "gpu_launches": kernels_per_step(True, dtype) * args.steps,
         "roofline": {"bound": "hbm", "kernel": dominant, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": f"of {peak_kind}",
                      "traffic": (ncu_traffic(args.workload, args.dtype) or {}).get(dominant),
@@ -1085,7 +1085,7 @@ def run_multi_gpu(args, dtype, rank, world):
         step_bytes = sum(bytes_.values())
         per_rank_io = 4 * (L + 1) * HEADS * HEAD_DIM * elem
         # kernels: the attention phases; per step two pushes, two pulls, four barriers, one global-row kernel
-        launches = kernels_per_step() + (9 if px is not None else 12)
+        launches = kernels_per_step(False, dtype) + (9 if px is not None else 12)
         line = {
             "metric": "sparse_graph_attention_fwd_bwd_edges_per_s", "value": n_edges / (ms_per_step * 1e-3),
             "unit": "edges/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,

@@ -295,10 +295,11 @@ TGT_API int tgt_sparse_attn_bwd(const void* dout, const void* q, const void* k, 
  * The same backward with its stages selectable by bit mask: 2 = pass A (dQ and, into `scratch`, the
  * per-row statistics 1/(Z+1e-6) and dO.O that pass B reads), 4 = pass B (dK, dV; needs the statistics
  * a pass A left in the same scratch for the same inputs), 1 = streaming pre-pass that computes the
- * statistics from dO and O — required (in the same or an earlier call) only when dbias is wanted,
- * because dbias needs them per edge before a row is complete.  tgt_sparse_attn_bwd runs 6, or 7 with
- * dbias; where one call runs 2 and 4, dbias is written by pass B, pass A derives the statistics and stage 1
- * is left out.  Lets a caller time or overlap the stages; replaces the same reference code.
+ * statistics from dO and O — required (in the same or an earlier call) where pass A runs alone with dbias, which
+ * it writes then.  tgt_sparse_attn_bwd runs 6, or 7 with dbias.  Where one call runs 2 and 4 with dbias, pass B writes
+ * it, and stage 1 is run in fp32 if `out` is given and left out otherwise: in bf16 pass A derives the statistics more
+ * exactly than the rounded output holds them.  Lets a caller time or overlap the stages; replaces the same
+ * reference code.
  */
 TGT_API int tgt_sparse_attn_bwd_passes(const void* dout, const void* q, const void* k, const void* v,
                                        const float* bias, int bias_heads, const void* out,

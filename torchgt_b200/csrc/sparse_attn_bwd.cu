@@ -43,7 +43,7 @@ int bwd_resident_ctas(int dtype, const HeadSplit& hs, int which, int use) {
   int* slot = &cache[dev < 0 ? 0 : dev][hs.w == 32 ? 1 : 0][which][use][dtype == TGT_F32 ? 0 : 1][log2i(hs.lph)][log2i(hs.g)];
   if (which == kWalkDkv) return bwd::occupancy_dkv(dtype, hs, use, slot);
   if (which == kWalkDqFused) return bwd::occupancy_dq_fused(dtype, hs, use, slot);
-  return bwd::occupancy_dq(dtype, hs, slot);
+  return bwd::occupancy_dq(dtype, hs, use == kBiasGrad, slot);
 }
 
 struct BwdScratch {
@@ -195,6 +195,11 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
   const size_t elem = dtype == TGT_F32 ? 4 : 2;
   const int64_t row_bytes = int64_t(heads) * head_dim * int64_t(elem);
   TGT_CHECK_ARG(dout && q && k && v && z && dq && dk && dv, "tensor pointers must not be null");
+  // With both passes in one call pass B, which has the gradient of every edge's score at hand, writes dbias.  Pass A then takes
+  // the form without statistics in bf16, but in fp32 the one that subtracts delta edge by edge (sparse_attn_bwd.cuh says why).
+  const bool dbias_in_dkv = dbias != nullptr && (passes & 6) == 6;
+  const bool fused = dbias == nullptr || (dbias_in_dkv && (dtype == TGT_BF16 || (out == nullptr && !(passes & 1))));
+  if (dbias_in_dkv) passes = fused ? passes & ~1 : passes | 1;
   TGT_CHECK_ARG(out != nullptr || !(passes & 1), "out is needed by the row-statistics pre-pass (dbias)");
   TGT_CHECK_ARG(dout_row_bytes >= row_bytes && q_row_bytes >= row_bytes && kv_row_bytes >= row_bytes &&
                     dout_row_bytes % 16 == 0 && q_row_bytes % 16 == 0 && kv_row_bytes % 16 == 0,
@@ -216,13 +221,9 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
     }
     return TGT_OK;
   }
-  // With both passes in one call pass A derives the statistics itself, and pass B, which has the gradient of every
-  // edge's score at hand, writes dbias.
-  const bool dbias_in_dkv = dbias != nullptr && (passes & 6) == 6;
-  if (dbias_in_dkv) passes &= ~1;
   const BwdScratch sc = plan_bwd_scratch(by_dst, hs, hsb, heads, dtype,
                                          bias == nullptr ? kNoBias : dbias_in_dkv ? kBiasGrad : kReadBias,
-                                         (passes & 2 ? 1 << (dbias == nullptr || dbias_in_dkv ? kWalkDqFused : kWalkDq) : 0) |
+                                         (passes & 2 ? 1 << (fused ? kWalkDqFused : kWalkDq) : 0) |
                                              (passes & 4 ? 1 << kWalkDkv : 0));
   if (scratch == nullptr || scratch_bytes < sc.total)
     return set_error(TGT_ERR_WORKSPACE, "scratch holds %zu bytes, %zu needed", scratch_bytes,
@@ -259,14 +260,14 @@ extern "C" int tgt_sparse_attn_bwd_strided(const void* dout, int64_t dout_row_by
   }
   // one walk kernel per pass, and the kernel that finishes the rows that cross tiles
   bool built = true;
-  if ((passes & 2) && (dbias == nullptr || p.dbias_in_dkv)) {
+  if ((passes & 2) && fused) {
     // pass A that derives the row statistics itself (and leaves them in scratch for pass B)
     fill_walk(&p.walk, *by_dst, sc.plan_a_fused, reinterpret_cast<float*>(base + sc.carry_a));
     const dim3 grid(walk_ctas(sc.plan_a_fused, n_rows), hs.groups);
     built = bwd::launch_dq_fused(p, dtype, hs, grid, link, stream);
     link = p.walk.n_tiles > 1 ? kLinkAfterStitch : kLinkWalk;
   } else if (passes & 2) {
-    // pass A with per-edge dbias: uses the statistics of the pre-pass (stage 1)
+    // pass A of the statistics of the pre-pass (stage 1); writes dbias unless pass B does
     fill_walk(&p.walk, *by_dst, sc.plan_a, reinterpret_cast<float*>(base + sc.carry_a));
     const dim3 grid(walk_ctas(sc.plan_a, n_rows), hs.groups);
     built = bwd::launch_dq(p, dtype, hs, grid, link, stream);

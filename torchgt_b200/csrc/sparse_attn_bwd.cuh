@@ -6,8 +6,11 @@
 // delta_d = inv_d * sum_e w_e (dO_d . V_s) is a sum over the same edges, so the pass accumulates
 //   A1 = sum mask w (dO.V) K,  A2 = sum mask w K,  S = sum w (dO.V)
 // and finishes the row with delta = inv S, dQ = inv (A1 - delta A2) / sqrt(D): no separate statistics
-// pass and no read of O.  Only when dbias is wanted (it needs delta per edge) a streaming pre-pass
-// computes the statistics from dO and O first and pass A uses them per edge.
+// pass and no read of O.  Where dbias is wanted in fp32 a streaming pre-pass computes the statistics from dO and O
+// first and pass A subtracts delta edge by edge: the difference of the two rounded sums is less exact where V has a
+// mean (mean 1 and 3 of its standard deviation, 30 to 1,000 edges per row: dQ 1.2 to 1.4 times as far from 64 bits).
+// In bf16 delta from the rounded O costs far more than that (dbias 1e-3 off, not 1e-7), and the sums are as above.
+// Without dbias there may be no O, and it is the sums in both.
 // With G = dO, inv = 1/(Z+1e-6), w = exp(clamp(raw)+bias):
 //   dw = (G_d.V_s - G_d.O_d) * inv_d      dV_s += w * inv_d * G_d      dt = dw * w  (= dbias)
 //   da = dt * [-5 <= raw <= 5]            dQ_d += da * K_s / sqrt(D)   dK_s += da * Q_d / sqrt(D)
@@ -58,7 +61,7 @@ bool launch_dq_fused(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 gr
                      cudaStream_t stream);
 bool launch_dkv(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, int link,
                 cudaStream_t stream);
-int occupancy_dq(int dtype, const HeadSplit& hs, int* cache_slot);
+int occupancy_dq(int dtype, const HeadSplit& hs, bool dbias_in_dkv, int* cache_slot);
 int occupancy_dq_fused(int dtype, const HeadSplit& hs, int use, int* cache_slot);
 int occupancy_dkv(int dtype, const HeadSplit& hs, int use, int* cache_slot);
 

@@ -1,12 +1,13 @@
-// Backward of the sparse graph attention, pass A with per-edge dbias (see sparse_attn_bwd.cuh).
+// Backward of the sparse graph attention, pass A from the row statistics of the pre-pass (see sparse_attn_bwd.cuh).
 #include "sparse_attn_bwd.cuh"
 
 namespace tgt {
 namespace bwd {
 namespace {
 
-// ---- pass A: dQ and dbias -----------------------------------------------------------------------
-template <typename T, int W, int LPH, int G>
+// ---- pass A with a statistics pre-pass -----------------------------------------------------------
+// BIAS is kBiasGrad where the pass runs alone and writes dbias, kReadBias where pass B does.
+template <typename T, int W, int LPH, int G, int BIAS>
 struct DqPolicy {
   static constexpr int VEC = Lane<T, W>::kElems;
   static constexpr int NACC = VEC;
@@ -20,7 +21,7 @@ struct DqPolicy {
   const T* __restrict__ dout;
   const float2* __restrict__ stats;
   const float* __restrict__ bias;
-  float* __restrict__ dbias;
+  float* __restrict__ dbias;   // original edge order
   T* __restrict__ dq;
   int bias_stride, bias_off;
   unsigned row_vecs, cvec, q_vecs, kv_vecs, g_vecs;
@@ -45,7 +46,7 @@ struct DqPolicy {
     o.q = Lane<T, W>::raw_at(q, unsigned(row) * q_vecs + cvec);
     o.g = Lane<T, W>::raw_at(dout, unsigned(row) * g_vecs + cvec);
     o.st = __ldg(stats + int64_t(row) * heads + head);
-    o.b = bias != nullptr ? __ldg(bias + int64_t(pe) * bias_stride + bias_off) : 0.f;
+    o.b = __ldg(bias + int64_t(pe) * bias_stride + bias_off);
   }
   __device__ __forceinline__ void clear(Operands& o) const {
     o.k = o.v = o.q = o.g = Lane<T, W>::raw_zero();
@@ -62,7 +63,7 @@ struct DqPolicy {
     const float gv = group_sum<LPH>(dot<kPairs>(a, b));
     const float wgt = fast_exp(clamp_score(raw) + o.b);
     const float dt = valid ? (gv - o.st.y) * o.st.x * wgt : 0.f;
-    if (dbias != nullptr) {
+    if (BIAS == kBiasGrad) {
       if (bias_stride == 1) {
         const float s = sum_over_heads<LPH, G>(dt);   // every head's dt sits on all LPH lanes of the head
         if (valid && group_leader) dbias[pe] = s;
@@ -94,11 +95,11 @@ struct DqPolicy {
   }
 };
 
-template <typename T, int W, int LPH, int G>
-__device__ __forceinline__ DqPolicy<T, W, LPH, G> make_dq_policy(const BwdParams& p) {
+template <typename T, int W, int LPH, int G, int BIAS>
+__device__ __forceinline__ DqPolicy<T, W, LPH, G, BIAS> make_dq_policy(const BwdParams& p) {
   constexpr int VEC = Lane<T, W>::kElems;
   const int c = threadIdx.x % G;
-  DqPolicy<T, W, LPH, G> pol;
+  DqPolicy<T, W, LPH, G, BIAS> pol;
   pol.q = static_cast<const T*>(p.q);
   pol.k = static_cast<const T*>(p.k);
   pol.v = static_cast<const T*>(p.v);
@@ -122,21 +123,29 @@ __device__ __forceinline__ DqPolicy<T, W, LPH, G> make_dq_policy(const BwdParams
   return pol;
 }
 
-template <typename T, int W, int LPH, int G>
+template <typename T, int W, int LPH, int G, int BIAS>
 __global__ void TGT_WALK_BOUNDS bwd_dq_kernel(const BwdParams p) {
-  using Policy = DqPolicy<T, W, LPH, G>;
+  using Policy = DqPolicy<T, W, LPH, G, BIAS>;
   __shared__ TileSmem<G, Policy::NACC, true> sm;
-  const Policy pol = make_dq_policy<T, W, LPH, G>(p);
+  const Policy pol = make_dq_policy<T, W, LPH, G, BIAS>(p);
   walk_tile_in<G, Policy>(sm, p.walk, pol);
 }
 
-template <typename T, int W, int LPH, int G>
+template <typename T, int W, int LPH, int G, int BIAS>
 __global__ void __launch_bounds__(crossing_threads(G)) bwd_dq_stitch_kernel(const BwdParams p) {
-  using Policy = DqPolicy<T, W, LPH, G>;
-  const Policy pol = make_dq_policy<T, W, LPH, G>(p);
+  using Policy = DqPolicy<T, W, LPH, G, BIAS>;
+  const Policy pol = make_dq_policy<T, W, LPH, G, BIAS>(p);
   finish_crossing_rows<G, Policy>(p.walk, pol);
 }
 
+// Calls f with the bias use of pass A as a compile-time constant; in bf16 a call whose pass B writes dbias takes the other pass A.
+template <typename T, class F>
+void dispatch_use(bool dbias_in_dkv, F&& f) {
+  if constexpr (sizeof(T) == 4) {
+    if (dbias_in_dkv) return f(std::integral_constant<int, kReadBias>{});
+  }
+  f(std::integral_constant<int, kBiasGrad>{});
+}
 
 }  // namespace
 
@@ -144,17 +153,21 @@ bool launch_dq(const BwdParams& p, int dtype, const HeadSplit& hs, dim3 grid, in
                cudaStream_t stream) {
   return dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
-    launch_chained(bwd_dq_kernel<typename S::T, S::W, S::LPH, S::G>, grid, kBlockThreads, stream, link, p);
-    if (p.walk.n_tiles > 1)
-      launch_chained(bwd_dq_stitch_kernel<typename S::T, S::W, S::LPH, S::G>, dim3(crossing_ctas(p.walk, S::G), grid.y), crossing_threads(S::G), stream, kLinkStitch, p);
+    dispatch_use<typename S::T>(p.dbias_in_dkv, [&](auto use) {
+      launch_chained(bwd_dq_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value>, grid, kBlockThreads, stream, link, p);
+      if (p.walk.n_tiles > 1)
+        launch_chained(bwd_dq_stitch_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value>, dim3(crossing_ctas(p.walk, S::G), grid.y), crossing_threads(S::G), stream, kLinkStitch, p);
+    });
   });
 }
 
-int occupancy_dq(int dtype, const HeadSplit& hs, int* cache_slot) {
+int occupancy_dq(int dtype, const HeadSplit& hs, bool dbias_in_dkv, int* cache_slot) {
   int result = 4;
   dispatch_shape(dtype, hs.w, hs.lph, hs.g, [&](auto sh) {
     using S = decltype(sh);
-    result = resident_ctas(bwd_dq_kernel<typename S::T, S::W, S::LPH, S::G>, cache_slot);
+    dispatch_use<typename S::T>(dbias_in_dkv, [&](auto use) {
+      result = resident_ctas(bwd_dq_kernel<typename S::T, S::W, S::LPH, S::G, decltype(use)::value>, cache_slot);
+    });
   });
   return result;
 }

@@ -5,7 +5,7 @@ namespace tgt {
 namespace bwd {
 namespace {
 
-// ---- pass A without a statistics pre-pass (no dbias) ---------------------------------------------
+// ---- pass A without a statistics pre-pass (no dbias, or bf16) ---------------------------------------------
 template <typename T, int W, int LPH, int G, int BIAS>
 struct DqFusedPolicy {
   static constexpr int VEC = Lane<T, W>::kElems;
