@@ -136,9 +136,11 @@ TGT_API int tgt_edge_layout_build_i32(const int32_t* edge_index, int64_t n_edges
 
 /*
  * Both orientations of one int64 list: the first build also writes the checked endpoints as int32 to `kept`
- * (tgt_edge_layout_kept_words(n_edges) words on the device, 16-byte aligned), from which the second one (n_edges > 0,
- * workspace of tgt_edge_layout_sizes_i32) sorts without reading the list again.  An endpoint out of range is kept as 0.
+ * (tgt_edge_layout_kept_words(n_edges) words on the device, 16-byte aligned), from which the second one (n_edges > 0)
+ * sorts without reading the list again.  An endpoint out of range is kept as 0.  Both are content with the workspace of
+ * tgt_edge_layout_sizes_kept, 8 bytes per edge less than that of tgt_edge_layout_sizes: `kept` takes the place.
  */
+TGT_API int tgt_edge_layout_sizes_kept(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes);
 TGT_API int tgt_edge_layout_kept_words(int64_t n_edges, size_t* words);
 TGT_API int tgt_edge_layout_build_keep(const int64_t* edge_index, int64_t n_edges, int64_t n_rows,
                                        int group_by, int32_t* ptr, int32_t* other, int32_t* perm,

@@ -315,3 +315,41 @@ def test_second_orientation_from_what_the_first_kept(n_rows, n_edges):
     bad[0, 0] = n_rows
     with pytest.raises(Exception, match="outside"):
         SparseGraph(bad.cuda(), n_rows).by_src.verify()
+
+
+def test_what_is_kept_for_the_second_orientation_is_bounded():
+    """A graph built where no gradients are recorded holds its one orientation and nothing else; elsewhere 8 bytes per edge
+    more until the second is built, in the place of two of the workspace's arrays and not on top of them."""
+    import ctypes
+    from torchgt_b200 import SparseGraph, _cabi
+    n_rows, n_edges = 4000, 1 << 21
+    layout, slack = 4 * (3 * n_edges + n_rows), 6 << 20
+    edges = torch.randint(0, n_rows, (2, n_edges), device="cuda")
+    need, second = ctypes.c_size_t(), ctypes.c_size_t()
+    _cabi.check(_cabi.load().tgt_edge_layout_sizes(n_rows, n_edges, ctypes.byref(need)))
+    _cabi.check(_cabi.load().tgt_edge_layout_sizes_kept(n_rows, n_edges, ctypes.byref(second)))
+    assert need.value - second.value == 8 * n_edges
+
+    def build():
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        graph = SparseGraph(edges, n_rows)
+        graph.check()
+        return graph, before, torch.cuda.max_memory_allocated() - before, torch.cuda.memory_allocated() - before
+
+    with torch.no_grad():
+        graph, before, peak, held = build()
+    assert peak < layout + need.value + slack
+    assert held < layout + slack
+    with torch.no_grad():
+        by_src = graph.by_src                       # from the list itself
+    assert torch.equal(by_src.seg.long(), edges[0].sort().values)
+    del graph, by_src
+    graph, before, peak, held = build()
+    assert peak < layout + need.value + slack
+    assert held < layout + 8 * n_edges + slack
+    torch.cuda.reset_peak_memory_stats()
+    graph.by_src.verify()
+    assert torch.cuda.max_memory_allocated() - before < 2 * layout + 8 * n_edges + second.value + slack
+    assert torch.cuda.memory_allocated() - before < 2 * layout + slack

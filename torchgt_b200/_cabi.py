@@ -62,6 +62,7 @@ SIGNATURES = {
                                       c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
     "tgt_edge_layout_build_i32": (c_int, [c_void_p, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p,
                                           c_void_p, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "tgt_edge_layout_sizes_kept": (c_int, [c_int64, c_int64, POINTER(c_size_t)]),
     "tgt_edge_layout_kept_words": (c_int, [c_int64, POINTER(c_size_t)]),
     "tgt_edge_layout_build_keep": (c_int, [c_void_p, c_int64, c_int64, c_int, c_void_p, c_void_p, c_void_p,
                                            c_void_p, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p]),

@@ -117,16 +117,19 @@ CheckWords& check_words() {
 }  // namespace
 
 // Edges from which on the first build of an int64 list keeps its endpoints for the second.  Shorter lists are bound by the host,
-// which pays 3 us for the array (a list of 30,000 edges 104.9 -> 108.1 us), and save one or two.
+// which pays 3 us for the array (a list of 30,000 edges 104.9 -> 108.1 us), and save one or two.  They take the place of arrays of
+// the build's workspace, but stay, 8 bytes per edge, until the second build or the graph's end: kept only where gradients are
+// recorded, since nothing else asks for the second orientation.
 constexpr int64_t kKeepFrom = int64_t(1) << 20;
 
 // ---- layouts ------------------------------------------------------------------------------------------------
 Layout::Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by_, Kept* kept) : group_by(group_by_) {
+  const c10::cuda::CUDAGuard guard(edge_index.device());
   const int64_t n_edges = edge_index.size(1);
   const bool wide = edge_index.scalar_type() == at::kLong, from_kept = kept != nullptr && kept->endpoints.defined();
+  const bool keep = wide && kept != nullptr && !from_kept && n_edges >= kKeepFrom && at::GradMode::is_enabled() && !capturing(edge_index);
   size_t ws = 0;
-  check((wide && !from_kept ? tgt_edge_layout_sizes : tgt_edge_layout_sizes_i32)(n_rows, n_edges, &ws));
-  const c10::cuda::CUDAGuard guard(edge_index.device());
+  check((keep || from_kept ? tgt_edge_layout_sizes_kept : wide ? tgt_edge_layout_sizes : tgt_edge_layout_sizes_i32)(n_rows, n_edges, &ws));
   const auto i32 = edge_index.options().dtype(at::kInt);
   ptr = at::empty({n_rows + 1}, i32);
   other = at::empty({n_edges}, i32);
@@ -140,7 +143,7 @@ Layout::Layout(const at::Tensor& edge_index, int64_t n_rows, int group_by_, Kept
   if (from_kept) {
     check(tgt_edge_layout_build_kept(words(kept->endpoints), n_edges, n_rows, group_by, words(ptr), words(other), words(perm),
                                      words(seg), workspace.data_ptr(), workspace.numel(), stream));
-  } else if (wide && kept != nullptr && n_edges >= kKeepFrom && !capturing(edge_index)) {
+  } else if (keep) {
     size_t kept_words = 0;
     check(tgt_edge_layout_kept_words(n_edges, &kept_words));
     at::Tensor endpoints = at::empty({int64_t(kept_words)}, i32);

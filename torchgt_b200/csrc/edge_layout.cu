@@ -134,8 +134,9 @@ struct Workspace {
   size_t keys, iota, narrow, flag, cub, total, cub_bytes;
 };
 
-// `wide`: the list is int64, and a narrow copy of it is made (extract_keys_kernel).
-int plan_workspace(int64_t n_rows, int64_t n_edges, bool wide, Workspace* w) {
+// The list a build reads: int64 (a narrow copy is made, extract_keys_kernel), int32, or endpoints kept outside the workspace.
+enum Source { kWide, kNarrow, kKept };
+int plan_workspace(int64_t n_rows, int64_t n_edges, Source from, Workspace* w) {
   size_t sort_bytes = 0;
   if (n_edges > 0) {
     cudaError_t e = cub::DeviceRadixSort::SortPairs(
@@ -147,9 +148,9 @@ int plan_workspace(int64_t n_rows, int64_t n_edges, bool wide, Workspace* w) {
   }
   const size_t e4 = round_up(size_t(n_edges) * 4, 256);
   size_t off = 0;
-  w->keys = off; off += e4;
+  w->keys = off; off += from == kKept ? 0 : e4;
   w->iota = off; off += e4;
-  w->narrow = off; off += wide ? e4 : 0;
+  w->narrow = off; off += from == kWide ? e4 : 0;
   w->flag = off; off += 256;
   w->cub = off;
   w->cub_bytes = round_up(sort_bytes, 256) + 256;
@@ -158,13 +159,13 @@ int plan_workspace(int64_t n_rows, int64_t n_edges, bool wide, Workspace* w) {
   return TGT_OK;
 }
 
-int workspace_size(int64_t n_rows, int64_t n_edges, bool wide, size_t* workspace_bytes) {
+int workspace_size(int64_t n_rows, int64_t n_edges, Source from, size_t* workspace_bytes) {
   TGT_CHECK_ARG(n_rows >= 0 && n_edges >= 0, "n_rows and n_edges must be >= 0");
   TGT_CHECK_ARG(n_rows < (int64_t(1) << 31) - 1 && n_edges < (int64_t(1) << 31) - 1,
                 "n_rows and n_edges must fit in int32");
   TGT_CHECK_ARG(workspace_bytes, "null output pointer");
   Workspace w;
-  const int rc = plan_workspace(n_rows, n_edges, wide, &w);
+  const int rc = plan_workspace(n_rows, n_edges, from, &w);
   if (rc != TGT_OK) return rc;
   *workspace_bytes = w.total;
   return TGT_OK;
@@ -190,7 +191,7 @@ int build_layout(const I* edge_index, int64_t n_edges, int64_t n_rows, int group
   TGT_CHECK_ARG(aligned16(edge_index) && aligned16(workspace), "pointers must be 16-byte aligned");
 
   Workspace w;
-  int rc = plan_workspace(n_rows, n_edges, sizeof(I) == 8, &w);
+  int rc = plan_workspace(n_rows, n_edges, kept != nullptr ? kKept : sizeof(I) == 8 ? kWide : kNarrow, &w);
   if (rc != TGT_OK) return rc;
   if (workspace_bytes < w.total)
     return set_error(TGT_ERR_WORKSPACE, "workspace holds %zu bytes, %zu needed", workspace_bytes,
@@ -242,7 +243,7 @@ int build_from_kept(const int32_t* kept, int64_t n_edges, int64_t n_rows, int gr
   TGT_CHECK_ARG(group_by == 0 || group_by == 1, "group_by must be 0 (source) or 1 (destination)");
   TGT_CHECK_ARG(aligned16(kept) && aligned16(workspace), "pointers must be 16-byte aligned");
   Workspace w;
-  const int rc = plan_workspace(n_rows, n_edges, false, &w);
+  const int rc = plan_workspace(n_rows, n_edges, kKept, &w);
   if (rc != TGT_OK) return rc;
   if (workspace_bytes < w.total)
     return set_error(TGT_ERR_WORKSPACE, "workspace holds %zu bytes, %zu needed", workspace_bytes, w.total);
@@ -332,11 +333,15 @@ __global__ void edge_prepare_kernel(const PrepareParams p) {
 }  // namespace tgt
 
 extern "C" int tgt_edge_layout_sizes(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes) {
-  return tgt::workspace_size(n_rows, n_edges, true, workspace_bytes);
+  return tgt::workspace_size(n_rows, n_edges, tgt::kWide, workspace_bytes);
 }
 
 extern "C" int tgt_edge_layout_sizes_i32(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes) {
-  return tgt::workspace_size(n_rows, n_edges, false, workspace_bytes);
+  return tgt::workspace_size(n_rows, n_edges, tgt::kNarrow, workspace_bytes);
+}
+
+extern "C" int tgt_edge_layout_sizes_kept(int64_t n_rows, int64_t n_edges, size_t* workspace_bytes) {
+  return tgt::workspace_size(n_rows, n_edges, tgt::kKept, workspace_bytes);
 }
 
 extern "C" int tgt_edge_layout_build(const int64_t* edge_index, int64_t n_edges, int64_t n_rows,
