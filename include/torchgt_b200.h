@@ -285,7 +285,7 @@ TGT_API int tgt_sparse_attn_fwd_noalloc(const void* q, const void* k, const void
  * Pass A walks by_dst (dQ, dbias, per-row statistics), pass B walks by_src (dK, dV); scores are
  * recomputed, nothing per-edge is read from forward.  dbias is device fp32 in ORIGINAL edge order
  * with the shape bias has, or NULL when not wanted.  `out` (the forward result) is read only when
- * dbias is wanted and may be NULL otherwise.  Deterministic (every floating-point sum has a fixed order).
+ * dbias is wanted in fp32 and may be NULL otherwise.  Deterministic (every floating-point sum has a fixed order).
  */
 TGT_API int tgt_sparse_attn_bwd(const void* dout, const void* q, const void* k, const void* v,
                         const float* bias, int bias_heads, const void* out, const float* z,

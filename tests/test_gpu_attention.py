@@ -569,3 +569,51 @@ def test_saved_tensor_hooks_see_everything_the_backward_keeps():
     assert sorted(shapes) == sorted([(50, 8, 8)] * 4 + [(50, 8), (ei.shape[1],)])   # q, k, v, out; sums of weights; bias
     for a, b in zip(torch.autograd.grad(out.square().sum(), (q, k, v, bias)), want):
         assert torch.equal(a, b)
+
+
+def test_bf16_keeps_no_output_for_the_gradient_of_the_bias():
+    """Nothing of a bf16 call's backward reads the output: it is not saved, the caller may change it in place, and the C entry
+    takes a null pointer (in fp32 too, where the stages do not ask for the statistics of the output)."""
+    import ctypes
+    from torchgt_b200 import SparseGraph, _cabi, sparse_graph_attention
+    ei = random_graph(3, 50, 4.0).cuda()
+    graph = SparseGraph(ei, 50)
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    rows = [torch.randn(50, 8, 8, device="cuda", generator=gen) for _ in range(4)]
+    bias = torch.randn(ei.shape[1], device="cuda", generator=gen).requires_grad_()
+    q, k, v, dout = (t.bfloat16() for t in rows)
+    q, k, v = (t.requires_grad_() for t in (q, k, v))
+    want = torch.autograd.grad(sparse_graph_attention(q, k, v, graph, bias), (q, k, v, bias), dout)
+    shapes = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: shapes.append(tuple(t.shape)) or t, lambda t: t):
+        out = sparse_graph_attention(q, k, v, graph, bias)
+    assert sorted(shapes) == sorted([(50, 8, 8)] * 3 + [(50, 8), (ei.shape[1],)])   # q, k, v; sums of weights; bias
+    out.mul_(2.0)
+    for a, b in zip(torch.autograd.grad(out, (q, k, v, bias), dout / 2), want):
+        assert torch.equal(a, b)
+    traced = torch.jit.trace(lambda *t: sparse_graph_attention(*t[:3], graph, t[3]), (q, k, v, bias), check_trace=False)
+    for a, b in zip(torch.autograd.grad(traced(q, k, v, bias), (q, k, v, bias), dout), want):
+        assert torch.equal(a, b)
+    lib, stream = _cabi.load(), torch.cuda.current_stream().cuda_stream
+    for dtype, passes in ((torch.bfloat16, 7), (torch.bfloat16, 0), (torch.float32, 6)):
+        code, size = (0 if dtype == torch.float32 else 1), ctypes.c_size_t()
+        q, k, v, dout = (t.to(dtype).requires_grad_() for t in rows)
+        out = sparse_graph_attention(q, k, v, graph, bias)
+        want = torch.autograd.grad(out, (q, k, v, bias), dout)
+        z = _cabi.native().attention_forward(q, k, v, bias, graph.native)[1]
+        _cabi.check(lib.tgt_sparse_attn_scratch_bytes(graph.by_dst.byref(), graph.by_src.byref(), 8, 8, code, 1, ctypes.byref(size)))
+        scratch = torch.full((max(size.value, 16),), 255, dtype=torch.uint8, device="cuda")
+        got = [torch.full_like(t, float("nan")) for t in want]
+        _cabi.check(lib.tgt_sparse_attn_bwd_strided(
+            dout.data_ptr(), 64 * dout.element_size(), q.data_ptr(), 64 * q.element_size(), k.data_ptr(), v.data_ptr(),
+            64 * q.element_size(), bias.data_ptr(), 1, None, z.data_ptr(), graph.by_dst.byref(), graph.by_src.byref(),
+            *(t.data_ptr() for t in got), 8, 8, code, scratch.data_ptr(), scratch.numel(), stream, passes))
+        for a, b in zip(got, want):
+            if dtype == torch.bfloat16:
+                assert torch.equal(a, b)
+            else:                                           # the other of the two routes to dQ
+                assert float((a - b).abs().max()) <= TOL_F32 * float(b.abs().max()) + 1e-6
+    assert lib.tgt_sparse_attn_bwd_strided(                 # fp32, statistics of the output asked for
+        dout.data_ptr(), 256, q.data_ptr(), 256, k.data_ptr(), v.data_ptr(), 256, bias.data_ptr(), 1, None, z.data_ptr(),
+        graph.by_dst.byref(), graph.by_src.byref(), *(t.data_ptr() for t in got), 8, 8, 0, scratch.data_ptr(), scratch.numel(),
+        stream, 7) == 1

@@ -328,7 +328,8 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
   std::shared_ptr<Graph> graph;
   SavedVariable q, k, v, bias, out, z;
   int heads = 0, head_dim = 0, dtype = 0;
-  bool with_dbias = false;   // the statistics of the forward's output are read only then, so only then is it kept
+  bool with_dbias = false;
+  bool reads_out() const { return with_dbias && dtype == TGT_F32; }   // tgt_sparse_attn_bwd: the output is kept only then
 
   variable_list apply(variable_list&& grads) override {
     return reporting([&] { return backward(grads); });
@@ -337,7 +338,7 @@ struct SparseGraphAttentionBackward : public torch::autograd::Node {
     if (!grads[0].defined()) return variable_list(4);
     const at::Tensor q_ = q.unpack(), k_ = k.unpack(), v_ = v.unpack(), bias_ = bias.unpack(), z_ = z.unpack();
     const bool want_dbias = with_dbias && task_should_compute_output(3);
-    const at::Tensor out_ = want_dbias ? out.unpack(shared_from_this()) : at::Tensor();
+    const at::Tensor out_ = want_dbias && reads_out() ? out.unpack(shared_from_this()) : at::Tensor();
     const at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard guard(q_.device());
     const at::Tensor dout = grads[0].contiguous();
@@ -387,7 +388,7 @@ at::Tensor attention_over_rows(const at::Tensor& q_in, const at::Tensor& k_in, c
     node->bias = SavedVariable(bias, false);
     node->z = SavedVariable(z, false);
     torch::autograd::set_history(out, node);
-    if (node->with_dbias) node->out = SavedVariable(out, true);
+    if (node->reads_out()) node->out = SavedVariable(out, true);
   }
   return out;
 }
@@ -424,13 +425,13 @@ std::pair<at::Tensor, at::Tensor> forward_pass(const at::Tensor& q, const at::Te
 
 std::vector<std::optional<at::Tensor>> backward_pass(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k,
                                                      const at::Tensor& v, const std::optional<at::Tensor>& bias,
-                                                     const at::Tensor& out, const at::Tensor& z,
+                                                     const std::optional<at::Tensor>& out, const at::Tensor& z,
                                                      const std::shared_ptr<Graph>& graph, bool want_dbias) {
   const c10::cuda::CUDAGuard guard(q.device());
   const at::Tensor bias_ = bias.value_or(at::Tensor());
   at::Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dbias;
   if (want_dbias) dbias = at::empty_like(bias_);
-  attention_backward(*graph, dout.contiguous(), q, k, v, bias_, out, z, dq, dk, dv, dbias, int(q.size(1)),
+  attention_backward(*graph, dout.contiguous(), q, k, v, bias_, out.value_or(at::Tensor()), z, dq, dk, dv, dbias, int(q.size(1)),
                      int(q.size(2)), dtype_of(q));
   return {dq, dk, dv, want_dbias ? std::optional<at::Tensor>(dbias) : std::nullopt};
 }

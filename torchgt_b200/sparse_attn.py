@@ -46,7 +46,8 @@ class _TracedAttention(torch.autograd.Function):
     def forward(ctx, q, k, v, bias, graph: SparseGraph):
         out, z = _cabi.native().attention_forward(q, k, v, bias, graph.native)
         ctx.graph = graph
-        ctx.save_for_backward(q, k, v, bias, out, z)
+        reads_out = bias is not None and ctx.needs_input_grad[3] and q.dtype == torch.float32
+        ctx.save_for_backward(q, k, v, bias, out if reads_out else None, z)
         return out
 
     @staticmethod
