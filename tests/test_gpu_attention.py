@@ -436,9 +436,8 @@ def test_dependent_launches_change_no_bit(heads, head_dim, dtype, with_bias):
             for _ in range(2):
                 results.setdefault(links, []).append(_run_cuda(q, k, v, ei, dout, bias, dtype=dtype, tile_edges=8))
     finally:
-        _cabi.check(lib.tgt_debug_set_dependent_launch(5))
-    assert lib.tgt_debug_set_dependent_launch(8) != 0
-    _cabi.check(lib.tgt_debug_set_dependent_launch(5))
+        _cabi.check(lib.tgt_debug_set_dependent_launch(7))     # the default: every link, for the tests that follow
+    assert lib.tgt_debug_set_dependent_launch(8) != 0          # refused, and changes nothing
     base = results[0][0]
     for links, runs in results.items():
         for res in runs:

@@ -22,13 +22,29 @@ def _own_tiles():
     _cabi.check(_cabi.load().tgt_debug_set_tile_edges(0))
 
 
-def _graph_with_rows_of(lengths, n, seed):
-    """Edges whose destinations (and, in a second copy turned round, sources) have exactly `lengths` edges each."""
+def _graph_with_rows_of(lengths, extra, seed):
+    """Edges in which row i is the destination of exactly lengths[i] edges and the source of as many; their other ends are
+    `extra` rows behind those."""
     rng = np.random.default_rng(seed)
     rows = np.concatenate([np.full(m, i) for i, m in enumerate(lengths)])
-    ends = rng.integers(0, n, rows.size)
-    ei = np.concatenate([np.stack([ends, rows]), np.stack([rows, ends])], axis=1)
+    ends = rng.integers(len(lengths), len(lengths) + extra, (2, rows.size))
+    ei = np.concatenate([np.stack([ends[0], rows]), np.stack([rows, ends[1]])], axis=1)
+    for side in ei:
+        assert np.array_equal(np.bincount(side, minlength=len(lengths))[:len(lengths)], lengths)
     return torch.from_numpy(ei[:, rng.permutation(ei.shape[1])])
+
+
+def _lengths(tile, slots):
+    """Edges per row: one less than, as many as and one more than fill 1 or 2 tiles, those on both sides of the line between
+    the finishing kernel's routes, and more than one round of its CTA's slots; each of these rows starts with a tile, the row
+    behind it fills its last one up.  Then rows that start anywhere in a tile."""
+    lengths, further = [], []
+    for m in (1, 2, GROUP_TILES, GROUP_TILES + 1, GROUP_TILES + 2, slots + 2):
+        for n in (m * tile - 1, m * tile, m * tile + 1):
+            lengths += [n, -n % tile]
+            further.append((n - 1) // tile)
+    assert set(further) >= {0, 1, GROUP_TILES, GROUP_TILES + 1, slots + 1, slots + 2}
+    return lengths + [3, 0, (GROUP_TILES - 1) * tile - 1, 1, 0, 0, 3 * tile + 1, 2]
 
 
 @pytest.mark.parametrize("heads,head_dim,dtype", [(8, 8, torch.float32), (1, 8, torch.float32), (2, 8, torch.float32),
@@ -37,12 +53,11 @@ def _graph_with_rows_of(lengths, n, seed):
 def test_rows_over_one_to_many_tiles_match_the_oracle(heads, head_dim, dtype, bias):
     from torchgt_b200 import SparseGraph, _cabi, sparse_graph_attention
     _cabi.check(_cabi.load().tgt_debug_set_tile_edges(4))
-    group = 4 * 128 // 32     # edges of a tile of the widest lane group; narrower ones have up to 512
-    tile = {(8, 8): 64 if dtype == torch.bfloat16 else 32, (1, 8): 256, (2, 8): 128, (8, 16): group, (3, 8): 256}[heads, head_dim]
-    lengths = [m * tile + d for m in (1, 2, GROUP_TILES - 1, GROUP_TILES, GROUP_TILES + 1, 3 * GROUP_TILES) for d in (-1, 0, 1)]
-    lengths = [3, 0] + lengths[:12 if tile > 100 else 18] + [1, 0, 0, 2]
+    # lanes of a group; a tile is 128 / lanes groups of 4 edges, the finishing CTA has 128 or 512 / lanes slots
+    lanes = {(8, 8): 8 if dtype == torch.bfloat16 else 16, (1, 8): 2, (2, 8): 4, (8, 16): 32, (3, 8): 2}[heads, head_dim]
+    lengths = _lengths(4 * 128 // lanes, (128 if lanes <= 4 else 512) // lanes)
     n = len(lengths) + 40
-    ei = _graph_with_rows_of(lengths, n, 5)
+    ei = _graph_with_rows_of(lengths, 40, 5)
     gen = torch.Generator().manual_seed(6)
     q, k, v, dout = (torch.randn(n, heads, head_dim, generator=gen).to(dtype) for _ in range(4))
     b = None if bias == "none" else torch.randn((ei.shape[1],) + ((heads,) if bias == "head" else ()), generator=gen) * 0.1
