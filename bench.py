@@ -50,8 +50,7 @@ ROTATING_SETS = 4
 
 def ncu_traffic(workload, dtype_name):
     """dram__bytes_read.sum + dram__bytes_write.sum per launch of each phase, as recorded next to the ncu
-    summary of that workload under profiles/ (taken before the dQ phase was one kernel); None when no capture of this
-    workload, or of a phase, is on file."""
+    summary of that workload under profiles/; None when no capture of this workload, or of a phase, is on file."""
     path = ROOT / "profiles" / f"sparse_attn_{workload}_{dtype_name}_traffic.json"
     try:
         return {k: float(v) for k, v in json.loads(path.read_text())["dram_bytes_per_launch"].items()}
@@ -76,7 +75,7 @@ def algorithmic_bytes(n_rows, n_edges, heads, head_dim, elem, bias_bytes):
     fwd = 2 * n_rows * r + n_edges * (2 * r + bias_bytes)
     dq = 4 * n_rows * r + n_edges * (2 * r + bias_bytes)
     dkv = 4 * n_rows * r + n_edges * (2 * r + bias_bytes)
-    return {"fwd_kernel": fwd, "bwd_dq_fused_kernel": dq, "bwd_dkv_kernel": dkv}
+    return {"fwd_kernel": fwd, "bwd_dq_fused_kernel": dq, "bwd_dkv_kernel": dkv, "backward": dq + dkv, "step": fwd + dq + dkv}
 
 
 class ClockSampler:
@@ -499,14 +498,14 @@ class OpBuffers:
             1 if self.bias is not None else 0, self.graph.by_dst.byref(), p(self.out), p(self.z), HEADS, HEAD_DIM,
             self.code, p(self.scratch_f), self.scratch_f.numel(), stream))
 
-    def bwd(self, stream, passes, with_dbias=True):
+    def bwd(self, stream, passes):
         from torchgt_b200 import _cabi
         lib = _cabi.load()
         p = lambda t: None if t is None else t.data_ptr()
         _cabi.check(lib.tgt_sparse_attn_bwd_strided(
             p(self.dout), self.row_bytes, p(self.q), self.row_bytes, p(self.k), p(self.v), self.kv_row_bytes,
             p(self.bias), 1 if self.bias is not None else 0, p(self.out), p(self.z), self.graph.by_dst.byref(),
-            self.graph.by_src.byref(), p(self.dq), p(self.dk), p(self.dv), p(self.dbias) if with_dbias else None, HEADS, HEAD_DIM,
+            self.graph.by_src.byref(), p(self.dq), p(self.dk), p(self.dv), p(self.dbias), HEADS, HEAD_DIM,
             self.code, p(self.scratch_b), self.scratch_b.numel(), stream, passes))
 
 
@@ -531,12 +530,11 @@ def kernels_per_step(dbias, dtype):
 
 def measure_device_resident(sets, steps, warmup):
     """CUDA-event timings of forward+backward through the C ABI on device-resident input sets: the whole
-    step (with dbias), the step with the bias as a plain input, and each phase on its own."""
+    step (with dbias) and its two phases, the step with the bias as a plain input and its three.  The backward with dbias
+    is one phase: its passes are other kernels than those that a call of one pass runs."""
     import copy
     n_sets = len(sets)
     step_graphs = [capture(lambda s, b=b: (b.fwd(s), b.bwd(s, 7 if b.dbias is not None else 6))) for b in sets]
-    phase_graphs = [[capture(lambda s, b=b: b.fwd(s)), capture(lambda s, b=b: b.bwd(s, 2, with_dbias=False)),
-                     capture(lambda s, b=b: b.bwd(s, 4))] for b in sets]
     torch.cuda.synchronize()
     start, stop = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
 
@@ -563,18 +561,30 @@ def measure_device_resident(sets, steps, warmup):
     ms_no_dbias = timed(plain_graphs)
     plain_graphs.clear()
     # ---- per-phase durations (each phase its own graph, events around every replay) ------------------
-    names = ["fwd_kernel", "bwd_dq_fused_kernel", "bwd_dkv_kernel"]
     phase_steps = min(steps, 200)
-    evs = [[torch.cuda.Event(enable_timing=True) for _ in range(4)] for _ in range(phase_steps)]
-    for i in range(phase_steps):
-        for j in range(3):
-            evs[i][j].record()
-            phase_graphs[i % n_sets][j].replay()
-        evs[i][3].record()
-    torch.cuda.synchronize()
-    phase_ms = {n: statistics.mean(evs[i][j].elapsed_time(evs[i][j + 1]) for i in range(phase_steps))
-                for j, n in enumerate(names)}
-    return {"ms_per_step": ms_per_step, "ms_no_dbias": ms_no_dbias, "phase_ms": phase_ms, "names": names}
+
+    def phases(of, calls):
+        graphs = [[capture(lambda s, b=b, call=call: call(b, s)) for call in calls.values()] for b in of]
+        evs = [[torch.cuda.Event(enable_timing=True) for _ in range(len(calls) + 1)] for _ in range(phase_steps)]
+        for i in range(phase_steps):
+            for j in range(len(calls)):
+                evs[i][j].record()
+                graphs[i % n_sets][j].replay()
+            evs[i][-1].record()
+        torch.cuda.synchronize()
+        return {n: statistics.mean(evs[i][j].elapsed_time(evs[i][j + 1]) for i in range(phase_steps))
+                for j, n in enumerate(calls)}
+
+    phase_ms = phases(sets, {"fwd_kernel": lambda b, s: b.fwd(s),
+                             "backward": lambda b, s: b.bwd(s, 7 if b.dbias is not None else 6)})
+    plain_ms = phases(plain_sets, {"fwd_kernel": lambda b, s: b.fwd(s), "bwd_dq_fused_kernel": lambda b, s: b.bwd(s, 2),
+                                   "bwd_dkv_kernel": lambda b, s: b.bwd(s, 4)})
+    return {"ms_per_step": ms_per_step, "ms_no_dbias": ms_no_dbias, "phase_ms": phase_ms, "plain_ms": plain_ms}
+
+
+def phase_report(phase_ms, bytes_, peak):
+    """Times and roofline fractions of phases by name."""
+    return {"phases_ms": phase_ms, "phases_frac": {n: bytes_[n] / (t * 1e-3) / 1e9 / peak for n, t in phase_ms.items()}}
 
 
 def extra_workload(name, dtype, steps, warmup, zipf=None):
@@ -599,8 +609,8 @@ def extra_workload(name, dtype, steps, warmup, zipf=None):
     elem = 4 if dtype == torch.float32 else 2
     peak, peak_kind = measured_hbm_peak()
     bytes_ = algorithmic_bytes(n_rows, n_edges, HEADS, HEAD_DIM, elem, 4)
-    dominant = max(m["names"], key=lambda n: m["phase_ms"][n])
-    step_bytes = sum(bytes_.values())
+    dominant = max(m["phase_ms"], key=m["phase_ms"].get)
+    step_bytes = bytes_["step"]
     del sets, graph
     torch.cuda.empty_cache()
     return {"rows": n_rows, "edges": n_edges, "io_dtype": "fp32" if elem == 4 else "bf16", "steps": steps,
@@ -608,9 +618,8 @@ def extra_workload(name, dtype, steps, warmup, zipf=None):
             "frac": step_bytes / (m["ms_per_step"] * 1e-3) / 1e9 / peak, "peak_kind": f"of {peak_kind}",
             "dominant_phase": dominant,
             "dominant_phase_frac": bytes_[dominant] / (m["phase_ms"][dominant] * 1e-3) / 1e9 / peak,
-            "phases_ms": m["phase_ms"],
-            "phases_frac": {n: bytes_[n] / (m["phase_ms"][n] * 1e-3) / 1e9 / peak for n in m["names"]},
-            "ms_per_step_without_dbias": m["ms_no_dbias"], "clocks": clocks}
+            **phase_report(m["phase_ms"], bytes_, peak), "ms_per_step_without_dbias": m["ms_no_dbias"],
+            "without_dbias": phase_report(m["plain_ms"], bytes_, peak), "clocks": clocks}
 
 
 def run_single_gpu(args, dtype):
@@ -644,7 +653,7 @@ def run_single_gpu(args, dtype):
         return
     sampler = ClockSampler(0)
     m = measure_device_resident(sets, args.steps, args.warmup)
-    ms_per_step, ms_no_dbias, phase_ms, names = m["ms_per_step"], m["ms_no_dbias"], m["phase_ms"], m["names"]
+    ms_per_step, ms_no_dbias, phase_ms = m["ms_per_step"], m["ms_no_dbias"], m["phase_ms"]
 
     # ---- end to end through the public API from pinned host memory -----------------------------------
     hq, hk, hv, hdout, hbias = (t.pin_memory() for t in make_inputs(n_rows, n_edges, dtype, 99, None))
@@ -711,9 +720,9 @@ def run_single_gpu(args, dtype):
     d2h = 4 * n_rows * HEADS * HEAD_DIM * elem + n_edges * 4
     peak, peak_kind = measured_hbm_peak()
     bytes_ = algorithmic_bytes(n_rows, n_edges, HEADS, HEAD_DIM, elem, 4)
-    dominant = max(names, key=lambda n: phase_ms[n])
+    dominant = max(phase_ms, key=phase_ms.get)
     achieved = bytes_[dominant] / (phase_ms[dominant] * 1e-3) / 1e9
-    step_bytes = sum(bytes_.values())
+    step_bytes = bytes_["step"]
     step_achieved = step_bytes / (ms_per_step * 1e-3) / 1e9
     cpu, _ = cpu_reference_rate(edge_index, n_rows, steps=5, warmup=2, time_limit_s=20.0)
     epoch = None
@@ -760,13 +769,13 @@ def run_single_gpu(args, dtype):
                      "frac": achieved / peak, "peak_kind": f"of {peak_kind}",
                      "traffic": (ncu_traffic(args.workload, args.dtype) or {}).get(dominant),
                      "algorithmic_bytes_per_launch": bytes_[dominant],
-                     "phases_ms": phase_ms,
-                     "phases_frac": {n: bytes_[n] / (phase_ms[n] * 1e-3) / 1e9 / peak for n in names},
+                     **phase_report(phase_ms, bytes_, peak),
                      "step": {"algorithmic_bytes": step_bytes, "achieved": step_achieved,
                               "frac": step_achieved / peak, "frac_of_nominal_8TBs": step_achieved / 8000.0},
                      "step_without_dbias": {
                          "ms_per_step": ms_no_dbias, "edges_per_s": n_edges / (ms_no_dbias * 1e-3),
                          "frac": step_bytes / (ms_no_dbias * 1e-3) / 1e9 / peak,
+                         **phase_report(m["plain_ms"], bytes_, peak),
                          "note": "bias read as an input, its gradient not computed (the byte count has no dbias "
                                  "term either); the headline step computes dbias as well"}},
         "cpu_baseline": cpu,
@@ -1082,7 +1091,7 @@ def run_multi_gpu(args, dtype, rank, world):
         elem = 4 if dtype == torch.float32 else 2
         peak, peak_kind = measured_hbm_peak()
         bytes_ = algorithmic_bytes(n_rows, n_edges, heads_local, HEAD_DIM, elem, 0)
-        step_bytes = sum(bytes_.values())
+        step_bytes = bytes_["step"]
         per_rank_io = 4 * (L + 1) * HEADS * HEAD_DIM * elem
         # kernels: the attention phases; per step two pushes, two pulls, four barriers, one global-row kernel
         launches = kernels_per_step(False, dtype) + (9 if px is not None else 12)
