@@ -56,9 +56,8 @@ def test_two_calls_in_a_row_match_the_allocating_entry_point():
     lib.tgt_debug_set_tile_edges(8)        # many tiles, so rows do cross tiles and the scratch is used
     try:
         # second call: other sizes and values, so leftovers of the first call would show
-        # The cases cover both ways rows that cross tiles are finished: inside the walk kernel (rows of more
-        # than 64 bytes: arrival counters in the built-in array) and by a second kernel (rows of at most 64
-        # bytes: 1 head x 8 and 2 heads x 8 in fp32), and both storage types.
+        # The cases cover both shapes of the kernel that finishes rows across tiles from the carries in the built-in array: CTAs
+        # of 512 threads, and of 128 for lane groups of up to four (1 head x 8, 2 heads x 8), and both storage types.
         cases = ((1, 3000, 8, 8, True, torch.float32), (2, 1777, 4, 16, False, torch.float32),
                  (3, 2500, 1, 8, True, torch.float32), (4, 2100, 2, 8, False, torch.float32),
                  (5, 2800, 8, 8, True, torch.bfloat16), (6, 1900, 2, 8, True, torch.bfloat16))

@@ -20,16 +20,11 @@
 //
 // Rows without edges are zero-filled.  The few between two rows of a range are filled by the group that walks over
 // them; aligned blocks of kGapRows rows that are empty as a whole are looked for by the first CTAs, 4,096 rows each, two
-// words of ptr[] per block.  Left to the walking group, the padding behind the graphs of a padded batch is one serial
-// chain of stores: 16 graphs padded to 20,000 rows (320,000 rows, half of them empty, gaps of up to 18,000, 8 heads of
-// 8) took 485 us forward, 192 us dQ and 475 us dK/dV per layer and take 59, 60 and 136.
-// What batches without empty rows pay for it decides who looks: CTAs of their own behind the tiles' hold up the launch
-// of the call's next kernel (64K step + 1.4 %), an equal share for every CTA costs each of them a round trip to memory
-// (one-head 512K step + 2.3 %), testing in front of the walk changes its registers (64K step + 4.6 %) and behind the
-// stitching its occupancy.  Loading the tested words with the tile's indices gains nothing (one-head 512K step 307.9 us
-// against 306.3), and as a function that is not inlined it costs the walk its registers (322 us; 64K step 172 against 162).
-// Between the walk and the stitching the search is free (without it 308.6 against 308.2); what is left, 303.9 -> 307.2 us
-// for the one-head 512K step and 160.5 -> 161.3 for the 64K step with bias gradient, is zero_gap's longer code in the walk.
+// words of ptr[] per block, between the walk and the stitching.  Left to the walking group, the padding behind the graphs of a
+// padded batch is one serial chain of stores: 16 graphs of 2,000 to 18,000 nodes padded to 20,000 rows (2.5 edges per node, 8
+// heads of 8) take 467 us forward, 217 dQ and 274 dK/dV that way and 84, 101 and 118 this way.  Batches without empty rows pay
+// nothing that shows: with the search taken out the 64K step takes 126.5 us against 126.5, one head at 512K rows 263.9 against
+// 264.4.
 #pragma once
 
 #include <type_traits>
@@ -101,7 +96,7 @@ struct SegWalk {
   const int32_t* seg;
   int n_rows;
   int n_edges;
-  int ge;          // edges per lane group per tile (multiple of kGeStep, <= GE_MAX)
+  int ge;          // edges per lane group per tile (a multiple of the walk's batch, <= GE_MAX; of kGeStep where forced)
   int n_tiles;
   int gap_ctas;    // CTAs that look for rows without edges (fill_gaps)
   float* gcarry;   // [n_tiles][2][gridDim.y * G * NACC] cross-tile partial sums
