@@ -662,11 +662,14 @@ at::Tensor layer_norm(const at::Tensor& x, const at::Tensor& w, const at::Tensor
 // without going back to Python between them: a layer's nine launches on 4,096 rows cost 100 us of host time one by one from
 // the modules.  The attention takes the projections as they are, so no views stand between the nodes.  `p`: weight and bias (or
 // none) of the first norm, the query, key, value and output projections, the second norm and the two feed-forward layers.
-at::Tensor encoder_layer(const at::Tensor& x, const std::shared_ptr<Graph>& graph, int heads, int head_dim,
+// Nothing, and nothing launched, where the projections are not heads * head_dim wide: the modules say what is wrong.
+std::optional<at::Tensor> encoder_layer(const at::Tensor& x, const std::shared_ptr<Graph>& graph, int heads, int head_dim,
                          const std::vector<std::optional<at::Tensor>>& p, double eps, double ffn_eps) {
   TORCH_CHECK(p.size() == 16, "encoder_layer takes eight weights and their biases");
   TORCH_CHECK(x.numel() == graph->n_rows * x.size(-1), "x and the graph have different numbers of rows");
   auto weight = [&p](int i) -> const at::Tensor& { return *p[2 * i]; };
+  for (int i = 1; i <= 3; ++i)
+    if (weight(i).dim() != 2 || weight(i).size(0) != int64_t(heads) * head_dim) return std::nullopt;
   const at::Tensor y = layer_norm(x, weight(0), *p[1], eps);
   const std::vector<at::Tensor> qkv = linear3(y, {weight(1), weight(2), weight(3)}, {p[3], p[5], p[7]});
   const at::Tensor attended = attention_over_rows(qkv[0], qkv[1], qkv[2], at::Tensor(), graph, heads, head_dim);

@@ -147,9 +147,6 @@ class EncoderLayer(nn.Module):
         tensors = [m._parameters.get(name) for m in layers for name in ("weight", "bias")]
         if any(t is None for t in tensors) or not plain_call(x, *tensors):
             return None
-        width = mha.num_heads * mha.att_size     # other projections: the modules say what is wrong
-        if not tensors[2].shape[0] == tensors[4].shape[0] == tensors[6].shape[0] == width:
-            return None
         graph = graph_for(edge_index, x.size(0) * x.size(1))
         graph.native.poll()
         return _cabi.native().encoder_layer(x, graph.native, mha.num_heads, mha.att_size, tensors, norm.eps, ffn_norm.eps)
