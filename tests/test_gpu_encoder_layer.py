@@ -98,3 +98,20 @@ def test_the_attention_itself_refuses_rows_that_are_not_the_graphs(wrong):
         for run in (lambda: native.attention(q, k, v, None, graph.native), lambda: native.attention_forward(q, k, v, None, graph.native)):
             with pytest.raises(TypeError if wrong == "dtype" else ValueError):
                 run()
+
+
+def test_the_attention_itself_refuses_a_bias_of_other_edges():
+    """A traced call checks its arguments when it is traced; it runs again on whatever it is given."""
+    from torchgt_b200 import _cabi, sparse_graph_attention
+    _, graph, _, _ = _layer(64, 8, 64, 300)
+    rows = [torch.randn(300, 8, 8, device="cuda") for _ in range(3)]
+    bias = torch.zeros(graph.n_edges, device="cuda")
+    traced = torch.jit.trace(lambda q, k, v, b: sparse_graph_attention(q, k, v, graph, b), (*rows, bias), check_trace=False)
+    assert torch.equal(traced(*rows, bias), sparse_graph_attention(*rows, graph, bias))
+    with pytest.raises(Exception, match="bias must be"):
+        traced(*rows, bias[:-1].contiguous())
+    for wrong in (bias[:-1], bias.double(), bias.view(-1, 1).expand(-1, 4)):
+        with pytest.raises(ValueError, match="bias must be"):
+            _cabi.native().attention(*rows, wrong, graph.native)
+    with pytest.raises(Exception, match="share the shape"):
+        traced(*(t[:299] for t in rows), bias)

@@ -282,9 +282,10 @@ int bias_heads(const at::Tensor& bias) {
 
 int dtype_of(const at::Tensor& q) { return q.scalar_type() == at::kFloat ? TGT_F32 : TGT_BF16; }
 
-// The kernels take bare pointers to n_rows rows of heads * head_dim values of one type, and the gradients are laid out like q, k
-// and v: whoever calls them, anything else stops here.
-void check_rows(const Graph& g, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, int heads, int head_dim) {
+// The kernels take bare pointers to n_rows rows of heads * head_dim values of one type and to one or `heads` bias values per edge,
+// and the gradients are laid out like q, k, v and the bias: whoever calls them, anything else stops here.
+void check_rows(const Graph& g, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& bias, int heads,
+                int head_dim) {
   if (q.sizes() != k.sizes() || q.sizes() != v.sizes() || q.numel() != g.n_rows * heads * head_dim) {
     std::ostringstream what;
     what << "q, k, v must share the shape [N, H, D], here " << g.n_rows << " rows of " << heads << " x " << head_dim << "; got "
@@ -294,6 +295,12 @@ void check_rows(const Graph& g, const at::Tensor& q, const at::Tensor& k, const 
   if ((q.scalar_type() != at::kFloat && q.scalar_type() != at::kBFloat16) || k.scalar_type() != q.scalar_type() ||
       v.scalar_type() != q.scalar_type())
     throw py::type_error("q, k, v must all be float32 or all bfloat16");
+  if (bias.defined() && (bias.scalar_type() != at::kFloat || bias.dim() < 1 || bias.dim() > 2 || bias.size(0) != g.n_edges ||
+                         (bias.dim() == 2 && bias.size(1) != heads))) {
+    std::ostringstream what;
+    what << "bias must be float32 [E] or [E, H] with E=" << g.n_edges << ", H=" << heads << "; got " << bias.sizes();
+    throw py::value_error(what.str());
+  }
 }
 
 at::Tensor scratch(Graph& g, int heads, int head_dim, int dtype, int phase, const at::Tensor& like) {
@@ -362,7 +369,7 @@ at::Tensor attention_over_rows(const at::Tensor& q_in, const at::Tensor& k_in, c
   for (const at::Tensor* t : {&q_in, &k_in, &v_in, &bias})
     TORCH_CHECK_NOT_IMPLEMENTED(!torch::autograd::isFwGradDefined(*t),
                                 "sparse_graph_attention does not support forward-mode AD");
-  check_rows(*graph, q_in, k_in, v_in, heads, head_dim);
+  check_rows(*graph, q_in, k_in, v_in, bias, heads, head_dim);
   const at::Tensor q = q_in.contiguous(), k = k_in.contiguous(), v = v_in.contiguous();
   const int dtype = dtype_of(q);
   const c10::cuda::CUDAGuard guard(q.device());
@@ -417,9 +424,10 @@ std::pair<at::Tensor, at::Tensor> forward_pass(const at::Tensor& q, const at::Te
                                                const std::optional<at::Tensor>& bias, const std::shared_ptr<Graph>& graph) {
   const c10::cuda::CUDAGuard guard(q.device());
   const int heads = int(q.size(1)), head_dim = int(q.size(2));
-  check_rows(*graph, q, k, v, heads, head_dim);
+  const at::Tensor bias_ = bias.value_or(at::Tensor());
+  check_rows(*graph, q, k, v, bias_, heads, head_dim);
   at::Tensor out = at::empty_like(q), z = at::empty({q.size(0), heads}, q.options().dtype(at::kFloat));
-  attention_forward(*graph, q, k, v, bias.value_or(at::Tensor()), out, z, heads, head_dim, dtype_of(q));
+  attention_forward(*graph, q, k, v, bias_, out, z, heads, head_dim, dtype_of(q));
   return {out, z};
 }
 
